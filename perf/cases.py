@@ -195,8 +195,14 @@ def run(s):
         out = {"loss": loss, "norm": norm}
         for b in model.engine.buckets:
             if b.numel:
-                out["grad." + b.name], out["weight." + b.name] = b.grad_flat, b.master
-                out["mean." + b.name], out["square." + b.name] = b.exp_avg, b.exp_avg_sq
+                # the embedding bucket goes out parameter by parameter: a table of mostly untouched rows next to vectors that sum
+                # over every token have no common scale to compare them on
+                parts = {b.name: slice(None)}
+                if b is model.engine.buckets[0]:
+                    parts = {"%s.%d" % (b.name, i): slice(o, o + p.numel()) for i, (p, o) in enumerate(zip(b.params, b.offsets))}
+                for name, at in parts.items():
+                    out["grad." + name], out["weight." + name] = b.grad_flat[at], b.master[at]
+                    out["mean." + name], out["square." + name] = b.exp_avg[at], b.exp_avg_sq[at]
         return out
     if s["kind"] == "forward":
         with torch.no_grad():
