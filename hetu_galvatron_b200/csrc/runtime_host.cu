@@ -7,6 +7,7 @@ extern "C" int gv_read_error_attn(unsigned int out[4]);
 extern "C" int gv_read_error_comm(unsigned int out[4]);
 extern "C" int gv_read_error_fgemm(unsigned int out[4]);
 extern "C" int gv_read_error_nvl(unsigned int out[4]);
+extern "C" int gv_read_error_norm(unsigned int out[4]);
 extern "C" int gv_read_error_bench(unsigned int out[4]);
 
 // Polls every translation unit that contains bounded waits. Returns 1 and fills `out`
@@ -21,6 +22,8 @@ extern "C" int gv_read_error(unsigned int out[4]) {
   r = gv_read_error_fgemm(out);
   if (r != 0) return r;
   r = gv_read_error_nvl(out);
+  if (r != 0) return r;
+  r = gv_read_error_norm(out);
   if (r != 0) return r;
   return gv_read_error_bench(out);
 }

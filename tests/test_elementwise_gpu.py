@@ -36,6 +36,38 @@ def test_rmsnorm(rows, cols):
     close(dw.cpu(), dwr)
 
 
+# edges of the row layouts: one vector, a lane short of and past a warp's share, each step of vectors per thread and of warps per
+# row, the widest row; single rows, odd rows, more rows than ring stages of every CTA
+NORM_EDGES = [(1, 8), (3, 248), (2, 264), (5, 1032), (131, 2048), (17, 2056), (9, 4104), (3, 8184), (4099, 768), (2500, 3584)]
+
+
+@pytest.mark.parametrize("layer", [False, True])
+@pytest.mark.parametrize("rows,cols", NORM_EDGES)
+def test_norms_at_layout_edges(rows, cols, layer):
+    """Both norms against fp64 sums of the same bf16 inputs. Outputs are rounded to bf16 once (2^-9 relative), dx adds a bf16
+    residual gradient to it; fp32 weight-gradient sums over `rows` terms stay within 1e-5 of their largest column sum."""
+    g = torch.Generator(device=DEV).manual_seed(rows + cols)
+    mk = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    x, dy, dres, w, b = mk(rows, cols), mk(rows, cols), mk(rows, cols), mk(cols), mk(cols)
+    if layer:
+        y, _, mean, rstd = Fn.layernorm_fwd(x, w, b, 1e-5)
+    else:
+        y, _, rstd = Fn.rmsnorm_fwd(x, w, 1e-5)
+    dw, db = torch.ones(cols, device=DEV), torch.ones(cols, device=DEV)
+    dx = Fn.layernorm_bwd(dy, x, w, mean, rstd, dres, dw, db) if layer else Fn.rmsnorm_bwd(dy, x, w, rstd, dres, dw)
+    xd, dyd, wd = x.double(), dy.double(), w.double()
+    mu = xd.mean(-1, keepdim=True) if layer else 0.0
+    r = ((xd - mu).pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt()
+    xh = (xd - mu) * r
+    gr = dyd * wd
+    yr = xh * wd + (b.double() if layer else 0.0)
+    dxr = r * (gr - (gr.mean(-1, keepdim=True) if layer else 0.0) - xh * (gr * xh).mean(-1, keepdim=True)) + dres.double()
+    for got, ref in ((y, yr), (dx, dxr)):
+        assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * ref.abs().max()).all()
+    for got, ref in [(dw, (dyd * xh).sum(0))] + ([(db, dyd.sum(0))] if layer else []):
+        assert (got.double() - 1 - ref).abs().max() <= 1e-5 * (dyd.abs() * (xh.abs() + 1)).sum(0).max()
+
+
 def test_norm_weight_gradients_are_bitwise_repeatable():
     """The weight (and bias) gradient is reduced in two stages in a fixed order, without atomics: same bits every run."""
     torch.manual_seed(1)
