@@ -5,10 +5,10 @@
 // column/row-parallel linears (megatron/core/tensor_parallel/layers.py:417 forward,
 // :462 input gradient, :534 weight gradient and the fused accumulate variant :498-509).
 //
-// One persistent CTA per SM, 6 warps:
+// One persistent CTA per SM, 10 warps:
 //   warp 0      : TMA producer (one elected lane)
 //   warp 1      : TMEM allocator + MMA issuer (one elected lane)
-//   warps 2..5  : epilogue; warp w owns TMEM lanes 32*(w%4)..+31
+//   warps 2..9  : epilogue; warp w owns TMEM lanes 32*(w%4)..+31 and half of the columns
 // Tile 128 x BN x 64 (BN = 256 or 128), 128-byte swizzled operands, both operand majors
 // supported through the shared-memory descriptors, so forward, dgrad and wgrad GEMMs all read
 // the tensors in the layout they already have (no transposes are materialised).
@@ -21,8 +21,14 @@ namespace gv {
 
 constexpr int BM = 128;
 constexpr int BK = 64;
-constexpr int GEMM_THREADS = 192;
+constexpr int GEMM_THREADS = 64 + 256;
 constexpr int GROUP_M = 8;
+constexpr int EPI_WARPS = 8;                     // epilogue: two warps per TMEM lane quarter
+constexpr int EPI_STAGE_BYTES = 32 * 32 * 4;     // a warp's staging buffer: one 32 x 32 chunk in fp32
+constexpr int EPI_BYTES = EPI_WARPS * EPI_STAGE_BYTES;
+// Epilogue kinds, a template parameter so that none carries the registers of the others: EPI_LINEAR (scale, bias, GELU,
+// residual, accumulate, rotary heads), EPI_SWIGLU (gated activation), EPI_XENT (cross-entropy statistics or gradient).
+constexpr int EPI_LINEAR = 0, EPI_SWIGLU = 1, EPI_XENT = 2;
 
 struct GemmDev {
   void* C;
@@ -61,7 +67,8 @@ struct GemmSmem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
+  static constexpr int EPI_OFFSET = STAGES * STAGE_BYTES;
+  static constexpr int BAR_OFFSET = EPI_OFFSET + EPI_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;  // barriers + alignment slack
 };
 
@@ -81,108 +88,174 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   return 0.5f * x * (1.0f + tanhf(u));
 }
 
-// Epilogue of one 32-column chunk of one output row: alpha, bias, GELU, residual, accumulate, store (bf16 or fp32).
-__device__ __forceinline__ void epilogue_chunk(const GemmDev& p, const uint32_t (&r)[32], int row, int col0) {
-        float v[32];
+// ------------------------------ epilogue ------------------------------
+// Eight warps: TMEM lets a warp read only the 32 lanes (rows) of its quarter, so the two warps of a quarter share its rows
+// and split the tile's columns. A warp works on 32 x 32 chunks. The accumulators arrive one row per lane; everything that
+// needs whole rows (rotary pairs, gated activation, cross entropy) is done in that form, then the chunk goes through 4 KB of
+// shared memory of this warp's own and is stored with eight lanes per row, four rows per instruction. Bound by latency, not
+// by bandwidth: what the store needs from memory (residual, old value of C) is loaded one chunk ahead.
+// With four warps and one row per lane (32 rows x 16 bytes per store) the epilogue, not the tensor cores, set the time of
+// most products with K <= 2048. M x N x K, before -> now: gated 8192 x 5632 x 1024 276 -> 109 us, rotary 8192 x 3072 x 1024
+// 180 -> 131, cross-entropy gradient 8192 x 30592 x 1280 607 -> 480, fp32 accumulation 5632 x 1024 x 8192 128 -> 106,
+// 6144 x 1536 x 576 56 -> 37, bias 36864 x 768 x 192 60 -> 41; with K >= 4096 within 5 %.
+// What a chunk's store reads from memory, in the store's own layout: lane l holds columns 4 (l % 8) .. + 3 of rows
+// l / 8 + 4 i of the chunk.
+struct EpiOld { uint4 v[8]; };
+
+__device__ __forceinline__ float4 bf16x4_to_f4(uint32_t lo, uint32_t hi) {
+  const float2 a = unpack_bf16x2(lo), b = unpack_bf16x2(hi);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+__device__ __forceinline__ bool epi_has_old(const GemmDev& p) { return p.residual != nullptr || p.accumulate; }
+
+// The residual, or without one the old C, of a chunk. Column groups that N cuts are read by epi_store itself.
+__device__ __forceinline__ void epi_load_old(const GemmDev& p, int row0, int col0, int lane, EpiOld& old) {
+  const int col = col0 + (lane & 7) * 4;
+  if (col + 4 > p.N) return;
+  const int r0 = row0 + (lane >> 3);
+  const bool wide = p.residual == nullptr && p.c_f32;
+  const char* src;
+  size_t step;                                             // bytes from one of this lane's rows to the next
+  if (p.residual != nullptr) {
+    src = reinterpret_cast<const char*>(p.residual + static_cast<size_t>(r0) * p.ldr + col);
+    step = static_cast<size_t>(p.ldr) * 8;
+  } else {
+    src = reinterpret_cast<const char*>(p.C) + (static_cast<size_t>(r0) * p.ldc + col) * (wide ? 4 : 2);
+    step = static_cast<size_t>(p.ldc) * (wide ? 16 : 8);
+  }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
-        const bool full = col0 + 32 <= p.N;
-        if (p.bias != nullptr) {
-          if (full) {
-            const uint4* bp = reinterpret_cast<const uint4*>(p.bias + col0);
+  for (int i = 0; i < 8; ++i, src += step) {
+    if (r0 + 4 * i >= p.M) continue;
+    if (wide) {
+      old.v[i] = *reinterpret_cast<const uint4*>(src);
+    } else {
+      const uint2 u = *reinterpret_cast<const uint2*>(src);
+      old.v[i].x = u.x; old.v[i].y = u.y;
+    }
+  }
+}
+
+// One row per lane -> the warp's staging buffer (16-byte pieces XOR-swizzled by the row: no bank conflicts either way).
+__device__ __forceinline__ void epi_stage(const uint32_t (&r)[32], float4* stage, int lane) {
+  __syncwarp();                                // the previous chunk has been read by all lanes
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 b = __ldg(bp + j);
-              float2 f0 = unpack_bf16x2(b.x), f1 = unpack_bf16x2(b.y), f2 = unpack_bf16x2(b.z), f3 = unpack_bf16x2(b.w);
-              v[j * 8 + 0] += f0.x; v[j * 8 + 1] += f0.y; v[j * 8 + 2] += f1.x; v[j * 8 + 3] += f1.y;
-              v[j * 8 + 4] += f2.x; v[j * 8 + 5] += f2.y; v[j * 8 + 6] += f3.x; v[j * 8 + 7] += f3.y;
-            }
-          } else {
-            for (int i = 0; i < 32; ++i)
-              if (col0 + i < p.N) v[i] += __bfloat162float(p.bias[col0 + i]);
-          }
-        }
-        if (p.xent_mode == 2) {
-          // gradient of the cross entropy w.r.t. the logits, straight from the recomputed fp32 logits
-          const float l = p.lse[row], g = p.gscale[row];
-          const long long lab = p.labels[row];
-          const long long tcol = (lab == p.ignore_index) ? -1 : lab - p.vocab_start - col0;
+  for (int j = 0; j < 8; ++j)
+    stage[lane * 8 + (j ^ (lane & 7))] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                     __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+  __syncwarp();
+}
+
+// This lane's part of the staged chunk: four columns of eight rows.
+__device__ __forceinline__ void epi_fetch(const float4* stage, int lane, float4 (&v)[8]) {
+  const int piece = lane & 7, l0 = lane >> 3;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = (__expf(v[i] - l) - (tcol == i ? 1.f : 0.f)) * g;
-        }
-        if (p.act == 1) {
+  for (int i = 0; i < 8; ++i) v[i] = stage[(l0 + 4 * i) * 8 + (piece ^ ((l0 + 4 * i) & 7))];
+}
+
+// Stores the staged chunk to C: alpha, bias, GELU, residual, accumulate. PLAIN: alpha alone, bf16.
+template <bool PLAIN>
+__device__ __forceinline__ void epi_store(const GemmDev& p, const float4* stage, int row0, int col0, int lane, const EpiOld& old) {
+  const int col = col0 + (lane & 7) * 4;
+  if (col >= p.N) return;
+  const int r0 = row0 + (lane >> 3);
+  if (PLAIN || col + 4 <= p.N) {
+    float4 v[8];
+    epi_fetch(stage, lane, v);
+    if constexpr (PLAIN) {
+      __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(r0) * p.ldc + col;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
-        }
+      for (int i = 0; i < 8; ++i, cp += 4 * static_cast<size_t>(p.ldc))
+        if (r0 + 4 * i < p.M)
+          *reinterpret_cast<uint2*>(cp) = make_uint2(pack_bf16x2(v[i].x * p.alpha, v[i].y * p.alpha), pack_bf16x2(v[i].z * p.alpha, v[i].w * p.alpha));
+      return;
+    }
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.bias != nullptr) {
+      const uint2 u = __ldg(reinterpret_cast<const uint2*>(p.bias + col));
+      b = bf16x4_to_f4(u.x, u.y);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[i].x = v[i].x * p.alpha + b.x; v[i].y = v[i].y * p.alpha + b.y;
+      v[i].z = v[i].z * p.alpha + b.z; v[i].w = v[i].w * p.alpha + b.w;
+    }
+    if (p.act == 1) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[i].x = gelu_tanh(v[i].x); v[i].y = gelu_tanh(v[i].y); v[i].z = gelu_tanh(v[i].z); v[i].w = gelu_tanh(v[i].w);
+      }
+    }
+    if (p.residual != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 o = bf16x4_to_f4(old.v[i].x, old.v[i].y);
+        v[i].x += o.x; v[i].y += o.y; v[i].z += o.z; v[i].w += o.w;
+      }
+    }
+    char* cp = reinterpret_cast<char*>(p.C) + (static_cast<size_t>(r0) * p.ldc + col) * (p.c_f32 ? 4 : 2);
+    const size_t step = static_cast<size_t>(p.ldc) * (p.c_f32 ? 16 : 8);
+    if (p.accumulate) {
+      char* op = cp;
+#pragma unroll
+      for (int i = 0; i < 8; ++i, op += step) {
+        if (r0 + 4 * i >= p.M) continue;
+        uint4 u = old.v[i];
         if (p.residual != nullptr) {
-          const __nv_bfloat16* rp = p.residual + static_cast<size_t>(row) * p.ldr + col0;
-          if (full) {
-            const uint4* rp4 = reinterpret_cast<const uint4*>(rp);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 b = rp4[j];
-              float2 f0 = unpack_bf16x2(b.x), f1 = unpack_bf16x2(b.y), f2 = unpack_bf16x2(b.z), f3 = unpack_bf16x2(b.w);
-              v[j * 8 + 0] += f0.x; v[j * 8 + 1] += f0.y; v[j * 8 + 2] += f1.x; v[j * 8 + 3] += f1.y;
-              v[j * 8 + 4] += f2.x; v[j * 8 + 5] += f2.y; v[j * 8 + 6] += f3.x; v[j * 8 + 7] += f3.y;
-            }
-          } else {
-            for (int i = 0; i < 32; ++i)
-              if (col0 + i < p.N) v[i] += __bfloat162float(rp[i]);
-          }
+          if (p.c_f32) u = *reinterpret_cast<const uint4*>(op);
+          else { const uint2 w = *reinterpret_cast<const uint2*>(op); u.x = w.x; u.y = w.y; }
         }
+        const float4 o = p.c_f32 ? make_float4(__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w))
+                                 : bf16x4_to_f4(u.x, u.y);
+        v[i].x += o.x; v[i].y += o.y; v[i].z += o.z; v[i].w += o.w;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i, cp += step) {
+      if (r0 + 4 * i >= p.M) continue;
+      if (p.c_f32) *reinterpret_cast<float4*>(cp) = v[i];
+      else *reinterpret_cast<uint2*>(cp) = make_uint2(pack_bf16x2(v[i].x, v[i].y), pack_bf16x2(v[i].z, v[i].w));
+    }
+  } else {
+    // the last columns of an N that is not a multiple of four
+    const int piece = lane & 7, l0 = lane >> 3;
+    for (int i = 0; i < 8; ++i) {
+      const int lr = l0 + 4 * i, row = row0 + lr;
+      if (row >= p.M) break;
+      const float* sv = reinterpret_cast<const float*>(stage + lr * 8 + (piece ^ (lr & 7)));
+      for (int e = 0; col + e < p.N; ++e) {
+        float v = sv[e] * p.alpha;
+        if (p.bias != nullptr) v += __bfloat162float(p.bias[col + e]);
+        if (p.act == 1) v = gelu_tanh(v);
+        if (p.residual != nullptr) v += __bfloat162float(p.residual[static_cast<size_t>(row) * p.ldr + col + e]);
+        const size_t at = static_cast<size_t>(row) * p.ldc + col + e;
         if (p.c_f32) {
-          float* cp = reinterpret_cast<float*>(p.C) + static_cast<size_t>(row) * p.ldc + col0;
-          if (full) {
-            float4* cp4 = reinterpret_cast<float4*>(cp);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              float4 o = make_float4(v[j * 4], v[j * 4 + 1], v[j * 4 + 2], v[j * 4 + 3]);
-              if (p.accumulate) {
-                float4 old = cp4[j];
-                o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-              }
-              cp4[j] = o;
-            }
-          } else {
-            for (int i = 0; i < 32; ++i)
-              if (col0 + i < p.N) cp[i] = p.accumulate ? cp[i] + v[i] : v[i];
-          }
+          float* cp = reinterpret_cast<float*>(p.C) + at;
+          *cp = p.accumulate ? *cp + v : v;
         } else {
-          __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + col0;
-          if (full) {
-            uint4* cp4 = reinterpret_cast<uint4*>(cp);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (p.accumulate) {
-                uint4 b = cp4[j];
-                float2 f0 = unpack_bf16x2(b.x), f1 = unpack_bf16x2(b.y), f2 = unpack_bf16x2(b.z), f3 = unpack_bf16x2(b.w);
-                v[j * 8 + 0] += f0.x; v[j * 8 + 1] += f0.y; v[j * 8 + 2] += f1.x; v[j * 8 + 3] += f1.y;
-                v[j * 8 + 4] += f2.x; v[j * 8 + 5] += f2.y; v[j * 8 + 6] += f3.x; v[j * 8 + 7] += f3.y;
-              }
-              uint4 o;
-              o.x = pack_bf16x2(v[j * 8 + 0], v[j * 8 + 1]);
-              o.y = pack_bf16x2(v[j * 8 + 2], v[j * 8 + 3]);
-              o.z = pack_bf16x2(v[j * 8 + 4], v[j * 8 + 5]);
-              o.w = pack_bf16x2(v[j * 8 + 6], v[j * 8 + 7]);
-              cp4[j] = o;
-            }
-          } else {
-            for (int i = 0; i < 32; ++i)
-              if (col0 + i < p.N) {
-                float o = v[i];
-                if (p.accumulate) o += __bfloat162float(cp[i]);
-                cp[i] = __float2bfloat16(o);
-              }
-          }
+          __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(p.C) + at;
+          *cp = __float2bfloat16(p.accumulate ? __bfloat162float(*cp) + v : v);
         }
+      }
+    }
+  }
+}
+
+// Stores the staged chunk as bf16, no scaling, to the activation output.
+__device__ __forceinline__ void epi_store_act(const GemmDev& p, const float4* stage, int row0, int unit0, int lane) {
+  const int r0 = row0 + (lane >> 3);
+  float4 v[8];
+  epi_fetch(stage, lane, v);
+  __nv_bfloat16* ap = p.act_out + static_cast<size_t>(r0) * p.ld_act + unit0 + (lane & 7) * 4;
+#pragma unroll
+  for (int i = 0; i < 8; ++i, ap += 4 * static_cast<size_t>(p.ld_act))
+    if (r0 + 4 * i < p.M) *reinterpret_cast<uint2*>(ap) = make_uint2(pack_bf16x2(v[i].x, v[i].y), pack_bf16x2(v[i].z, v[i].w));
 }
 
 // Rotary embedding (non-interleaved halves) on two 32-column chunks of one output row that sit half a head apart:
 // r1 holds columns [c, c + 32) of the head's first half, r2 the same columns of its second half
 // (reference: megatron/core/models/common/embeddings/rotary_pos_embedding.py:204-227 as a separate pass over q and k).
-__device__ __forceinline__ void rope_rotate_chunks(const GemmDev& p, uint32_t (&r1)[32], uint32_t (&r2)[32], int row, int freq0) {
-  const float pos = p.rope_pos ? static_cast<float>(p.rope_pos[row])
-                               : static_cast<float>((row / p.rope_pos_div) % p.rope_pos_mod + p.rope_pos_offset);
+__device__ __forceinline__ void rope_rotate_chunks(const GemmDev& p, uint32_t (&r1)[32], uint32_t (&r2)[32], float pos, int freq0) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     float sn, cs;
@@ -193,36 +266,12 @@ __device__ __forceinline__ void rope_rotate_chunks(const GemmDev& p, uint32_t (&
   }
 }
 
-// SwiGLU on two accumulator chunks of one row: rg = gate pre-activations, ru = up values of the same 32 hidden units.
-// Stores both (bf16) into C = [gate | up] and silu(gate) * up into the activation output
-// (reference: chunk + silu * mul as separate passes, galvatron/core/runtime/tensor_parallel/transformer.py:122-124).
-__device__ __forceinline__ void swiglu_chunks(const GemmDev& p, const uint32_t (&rg)[32], const uint32_t (&ru)[32], int row,
-                                              int unit0) {
-  epilogue_chunk(p, rg, row, unit0);
-  epilogue_chunk(p, ru, row, p.swiglu_f + unit0);
-  __nv_bfloat16* ap = p.act_out + static_cast<size_t>(row) * p.ld_act + unit0;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    float o[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      // on the bf16-rounded values, like the stand-alone kernel that reads the stored projection
-      const float g = __bfloat162float(__float2bfloat16(__uint_as_float(rg[j * 8 + e]) * p.alpha));
-      const float u = __bfloat162float(__float2bfloat16(__uint_as_float(ru[j * 8 + e]) * p.alpha));
-      o[e] = g / (1.f + __expf(-g)) * u;
-    }
-    uint4 w;
-    w.x = pack_bf16x2(o[0], o[1]); w.y = pack_bf16x2(o[2], o[3]); w.z = pack_bf16x2(o[4], o[5]); w.w = pack_bf16x2(o[6], o[7]);
-    reinterpret_cast<uint4*>(ap)[j] = w;
-  }
-}
-
 // Cross-entropy statistics of one 32-column chunk of one row of logits (fp32, straight from the accumulator): the
-// running (max, sum exp(x - max)) of the row over the current tile, and the target logit when the label's column is
-// in this chunk. Replaces the passes over materialised logits of the reference's vocab-parallel cross entropy
-// (megatron/core/tensor_parallel/cross_entropy.py:16-152).
-__device__ __forceinline__ void xent_stats_chunk(const GemmDev& p, const uint32_t (&r)[32], int row, int col0, float& xm,
-                                                 float& xl) {
+// running (max, sum exp(x - max)) of the row over this warp's columns, and the target logit when the label's column is
+// in this chunk (lcol = label - vocab_start, or negative when it is not counted). Replaces the passes over materialised
+// logits of the reference's vocab-parallel cross entropy (megatron/core/tensor_parallel/cross_entropy.py:16-152).
+__device__ __forceinline__ void xent_stats_chunk(const GemmDev& p, const uint32_t (&r)[32], int row, int col0, long long lcol,
+                                                 float& xm, float& xl) {
   float v[32];
   const int valid = min(32, p.N - col0);
   float mx = -INFINITY;
@@ -237,19 +286,155 @@ __device__ __forceinline__ void xent_stats_chunk(const GemmDev& p, const uint32_
   for (int i = 0; i < 32; ++i) sum += __expf(v[i] - m_new);
   xl = xl * __expf(xm - m_new) + sum;
   xm = m_new;
-  const long long lab = p.labels[row];
-  if (lab != p.ignore_index) {
-    const long long t = lab - p.vocab_start - col0;
-    if (t >= 0 && t < valid) {
-      float tv = 0.f;
+  const long long t = lcol - col0;
+  if (lcol >= 0 && t >= 0 && t < valid) {
+    float tv = 0.f;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) tv = (t == i) ? v[i] : tv;
-      p.target[row] = tv;
-    }
+    for (int i = 0; i < 32; ++i) tv = (t == i) ? v[i] : tv;
+    p.target[row] = tv;
   }
 }
 
-template <int BN, bool A_MN, bool B_MN>
+// One thread polls for the epilogue, the other warps sleep in a barrier. A wait that gave up is everybody's result, so all
+// warps leave together.
+__device__ __forceinline__ bool epilogue_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned int site) {
+  bool done = true;
+  if (threadIdx.x == 64) done = mbar_wait(bar, parity, abort_flag, site);
+  done = named_bar_all<1, 32 * EPI_WARPS>(done);
+  tc_fence_after();
+  return done;
+}
+
+// The epilogue of one tile for one warp: rows row0 .. row0 + 31 of the output, this warp's part of its BN columns.
+// `t_addr` addresses the tile's accumulator columns in the warp's own TMEM lanes; `wait()` returns once they are complete
+// (false: given up). `xslot` are the two warps' 2 x 32 float2 slots for joining row statistics, `parity` alternates per tile.
+template <int BN, int EPI, class Wait>
+__device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr, int row0, int tn, int half, int quarter, int lane,
+                                              int parity, float4* stage, Wait wait) {
+  const int n0 = tn * BN, row = row0 + lane;
+  const bool row_ok = row < p.M;
+  EpiOld old;
+  uint32_t r[32];
+  if constexpr (EPI == EPI_SWIGLU) {
+    // columns [0, 128) of the tile are gate, [128, 256) up, of hidden units tn * 128 ...: this warp takes 64 units.
+    // (reference: chunk + silu * mul as separate passes, galvatron/core/runtime/tensor_parallel/transformer.py:122-124)
+    if (!wait()) return false;
+#pragma unroll 1
+    for (int c = 2 * half; c < 2 * half + 2; ++c) {
+      uint32_t u[32];
+      __syncwarp();
+      tmem_ld_32x32b_x32(t_addr + c * 32, r);
+      tmem_ld_32x32b_x32(t_addr + (c + 4) * 32, u);
+      tmem_ld_wait();
+      const int unit0 = tn * 128 + c * 32;
+      epi_stage(r, stage, lane);
+      epi_store<true>(p, stage, row0, unit0, lane, old);
+      epi_stage(u, stage, lane);
+      epi_store<true>(p, stage, row0, p.swiglu_f + unit0, lane, old);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        // on the bf16-rounded values, like the stand-alone kernel that reads the stored projection
+        const float g = __bfloat162float(__float2bfloat16(__uint_as_float(r[i]) * p.alpha));
+        const float up = __bfloat162float(__float2bfloat16(__uint_as_float(u[i]) * p.alpha));
+        r[i] = __float_as_uint(g / (1.f + __expf(-g)) * up);
+      }
+      epi_stage(r, stage, lane);
+      epi_store_act(p, stage, row0, unit0, lane);
+    }
+    return true;
+  } else if constexpr (EPI == EPI_XENT) {
+    constexpr int CHUNKS = BN / 64;                       // of this warp
+    const int c0 = half * CHUNKS;
+    long long lcol = -1;
+    float l = 0.f, g = 0.f;
+    if (row_ok) {
+      const long long lab = p.labels[row];
+      if (lab != p.ignore_index) lcol = lab - p.vocab_start;
+      if (p.xent_mode == 2) { l = p.lse[row]; g = p.gscale[row]; }
+    }
+    float xm = -INFINITY, xl = 0.f;
+    if (!wait()) return false;
+#pragma unroll 1
+    for (int c = c0; c < c0 + CHUNKS; ++c) {
+      const int col0 = n0 + c * 32;
+      if (col0 >= p.N) break;
+      __syncwarp();
+      tmem_ld_32x32b_x32(t_addr + c * 32, r);
+      tmem_ld_wait();
+      if (p.xent_mode == 1) {
+        if (row_ok) xent_stats_chunk(p, r, row, col0, lcol, xm, xl);
+      } else {
+        // gradient of the cross entropy w.r.t. the logits, straight from the recomputed fp32 logits
+        const int t = (lcol >= col0 && lcol < col0 + 32) ? static_cast<int>(lcol - col0) : -1;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          r[i] = __float_as_uint((__expf(__uint_as_float(r[i]) * p.alpha - l) - (t == i ? 1.f : 0.f)) * g);
+        epi_stage(r, stage, lane);
+        epi_store<false>(p, stage, row0, col0, lane, old);
+      }
+    }
+    if (p.xent_mode == 1) {
+      // the quarter's second warp hands its half of the statistics to the first; two slots, one barrier per tile: a slot
+      // is written again only after the next tile's barrier, which the reader reaches after reading
+      float2* slot = reinterpret_cast<float2*>(stage - (half ? 4 * (EPI_STAGE_BYTES / 16) : 0)) + parity * 32 + lane;
+      if (half == 1) *slot = make_float2(xm, xl);
+      named_bar_sync_id(2 + quarter, 64);
+      if (half == 0 && row_ok) {
+        const float2 o = *slot;
+        const float m = fmaxf(xm, o.x);
+        float* st = p.stats + (static_cast<size_t>(row) * p.stat_tiles + tn) * 2;
+        st[0] = m;
+        st[1] = xl * __expf(xm - m) + (o.x == -INFINITY ? 0.f : o.y * __expf(o.x - m));
+      }
+    }
+    return true;
+  } else {
+  if (p.rope_cols > 0) {
+    // q / k heads: a chunk and its partner half a head further right are rotated together
+    const float pos = p.rope_pos ? (row_ok ? static_cast<float>(p.rope_pos[row]) : 0.f)
+                                 : static_cast<float>((row / p.rope_pos_div) % p.rope_pos_mod + p.rope_pos_offset);
+    const int hc = p.rope_dh >> 6;                        // chunks per half head
+    if (!wait()) return false;
+#pragma unroll 1
+    for (int pi = half * (BN / 128); pi < (half + 1) * (BN / 128); ++pi) {
+      const int in_head = pi % hc, c = (pi / hc) * 2 * hc + in_head;
+      uint32_t u[32];
+      __syncwarp();
+      tmem_ld_32x32b_x32(t_addr + c * 32, r);
+      tmem_ld_32x32b_x32(t_addr + (c + hc) * 32, u);
+      tmem_ld_wait();
+      const int col0 = n0 + c * 32;
+      if (col0 < p.rope_cols) rope_rotate_chunks(p, r, u, pos, in_head * 32);
+      epi_stage(r, stage, lane);
+      epi_store<false>(p, stage, row0, col0, lane, old);
+      epi_stage(u, stage, lane);
+      epi_store<false>(p, stage, row0, col0 + hc * 32, lane, old);
+    }
+    return true;
+  }
+  constexpr int CHUNKS = BN / 64;                         // of this warp
+  const int c0 = half * CHUNKS;
+  const bool has_old = epi_has_old(p);
+  if (has_old) epi_load_old(p, row0, n0 + c0 * 32, lane, old);
+  if (!wait()) return false;
+#pragma unroll 1
+  for (int c = c0; c < c0 + CHUNKS; ++c) {
+    const int col0 = n0 + c * 32;
+    if (col0 >= p.N) break;
+    __syncwarp();
+    tmem_ld_32x32b_x32(t_addr + c * 32, r);
+    EpiOld next;
+    if (has_old && c + 1 < c0 + CHUNKS) epi_load_old(p, row0, col0 + 32, lane, next);
+    tmem_ld_wait();
+    epi_stage(r, stage, lane);
+    epi_store<false>(p, stage, row0, col0, lane, old);
+    old = next;
+  }
+  return true;
+  }
+}
+
+template <int BN, bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmDev p) {
   using S = GemmSmem<BN>;
@@ -266,7 +451,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int num_m = (p.M + BM - 1) / BM;
-  const int num_n = p.swiglu_f > 0 ? p.swiglu_f / 128 : (p.N + BN - 1) / BN;   // gated: a tile = 128 hidden units
+  const int num_n = EPI == EPI_SWIGLU ? p.swiglu_f / 128 : (p.N + BN - 1) / BN;   // gated: a tile = 128 hidden units
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
   constexpr uint32_t TMEM_COLS = 2 * BN;  // two accumulator buffers (512 or 256 columns)
@@ -278,7 +463,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 128);
+      mbar_init(&acc_empty[a], 32 * EPI_WARPS);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -316,7 +501,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             for (int q = 0; q < BM / 64; ++q) tma_load_2d(sA + q * (BK * 128), &tmA, &full_bar[stage], m0 + q * 64, kb * BK);
           }
           if constexpr (!B_MN) {
-            if (p.swiglu_f > 0) {
+            if constexpr (EPI == EPI_SWIGLU) {
               // 128 gate rows and the 128 up rows of the same hidden units (the map's box is 128 rows in this mode)
               tma_load_2d(sB, &tmB, &full_bar[stage], kb * BK, tn * 128);
               tma_load_2d(sB + 128 * 128, &tmB, &full_bar[stage], kb * BK, p.swiglu_f + tn * 128);
@@ -370,60 +555,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else {
     // ------------------------------ epilogue ----------------------------------
     const int quarter = warp & 3;  // TMEM lane group this warp may access
+    const int half = (warp - 2) >> 2;
+    float4* stage_buf = reinterpret_cast<float4*>(smem + S::EPI_OFFSET + (warp - 2) * EPI_STAGE_BYTES);
     int acc = 0;
     uint32_t acc_phase = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
       int tm, tn;
       tile_coords(tile, num_m, num_n, tm, tn);
-      const int row = tm * BM + quarter * 32 + lane;
-      const int n0 = tn * BN;
-      if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag, 4)) { ok = false; break; }
-      tc_fence_after();
       const uint32_t t_addr = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
-      const bool row_ok = row < p.M;
-      float xm = -INFINITY, xl = 0.f;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        __syncwarp();
-        tmem_ld_32x32b_x32(t_addr + c * 32, r);
-        tmem_ld_wait();
-        const int col0 = n0 + c * 32;
-        if (p.swiglu_f > 0) {
-          // columns [0, 128) of the tile are gate, [128, 256) up, of hidden units tn * 128 ...
-          if (c >= 4) continue;
-          uint32_t r2[32];
-          tmem_ld_32x32b_x32(t_addr + (c + 4) * 32, r2);
-          tmem_ld_wait();
-          if (row_ok) swiglu_chunks(p, r, r2, row, tn * 128 + c * 32);
-          continue;
-        }
-        if (p.rope_cols > 0 && col0 < p.rope_cols) {
-          // q / k heads: the chunk and its partner half a head further right are rotated together
-          const int hc = p.rope_dh >> 6;                      // chunks per half head
-          const int in_head = (col0 % p.rope_dh) >> 5;
-          if (in_head >= hc) continue;                        // second halves were stored with their partners
-          uint32_t r2[32];
-          tmem_ld_32x32b_x32(t_addr + (c + hc) * 32, r2);
-          tmem_ld_wait();
-          if (row_ok) {
-            rope_rotate_chunks(p, r, r2, row, in_head * 32);
-            epilogue_chunk(p, r, row, col0);
-            epilogue_chunk(p, r2, row, col0 + hc * 32);
-          }
-          continue;
-        }
-        if (row_ok && col0 < p.N) {
-          if (p.xent_mode == 1) xent_stats_chunk(p, r, row, col0, xm, xl);
-          else epilogue_chunk(p, r, row, col0);
-        }
-      }
-      if (p.xent_mode == 1 && row_ok) {
-        float* st = p.stats + (static_cast<size_t>(row) * p.stat_tiles + tn) * 2;
-        st[0] = xm;
-        st[1] = xl;
-      }
+      const bool ok = epilogue_tile<BN, EPI>(p, t_addr, tm * BM + quarter * 32, tn, half, quarter, lane, acc, stage_buf, [&] {
+        return epilogue_wait(&acc_full[acc], acc_phase, abort_flag, 4);
+      });
+      if (!ok) break;
       __syncwarp();
       tc_fence_before();
       mbar_arrive(&acc_empty[acc]);
@@ -452,7 +595,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 constexpr int P_STAGES = 6;
 constexpr int P_HALF_BYTES = BM * BK * 2;                  // 16 KB: A half or B half of one k-block
 constexpr int P_STAGE_BYTES = 2 * P_HALF_BYTES;
-constexpr int P_BAR_OFFSET = P_STAGES * P_STAGE_BYTES;
+constexpr int P_EPI_OFFSET = P_STAGES * P_STAGE_BYTES;
+constexpr int P_BAR_OFFSET = P_EPI_OFFSET + EPI_BYTES;
 constexpr int P_SMEM_TOTAL = P_BAR_OFFSET + 256 + 1024;
 
 // TMA tile load of this CTA's shared memory whose completion is counted on CTA 0's barrier (pair form of the load)
@@ -473,7 +617,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
       : "memory");
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmDev p) {
   extern __shared__ uint8_t smem_raw[];
@@ -489,7 +633,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const uint32_t cta = cluster_ctarank();               // 0: issues the MMAs; 1: peer
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   constexpr int TM = 2 * BM, TN = 256;
-  const int num_m = (p.M + TM - 1) / TM, num_n = p.swiglu_f > 0 ? p.swiglu_f / 128 : (p.N + TN - 1) / TN;
+  const int num_m = (p.M + TM - 1) / TM, num_n = EPI == EPI_SWIGLU ? p.swiglu_f / 128 : (p.N + TN - 1) / TN;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
   constexpr uint32_t TMEM_COLS = 2 * TN;
@@ -501,7 +645,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 256);    // the epilogue threads of both CTAs
+      mbar_init(&acc_empty[a], 2 * 32 * EPI_WARPS);    // the epilogue threads of both CTAs
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -529,7 +673,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         tile_coords(tile, num_m, num_n, tm, tn);
         const int m0 = tm * TM + static_cast<int>(cta) * BM;      // this CTA's rows of A and of the output
         // this CTA's 128 rows of B (columns of the output); gated mode: CTA 0 stages the gate rows, CTA 1 the up rows
-        const int nb0 = p.swiglu_f > 0 ? tn * 128 + static_cast<int>(cta) * p.swiglu_f : tn * TN + static_cast<int>(cta) * BM;
+        const int nb0 = EPI == EPI_SWIGLU ? tn * 128 + static_cast<int>(cta) * p.swiglu_f : tn * TN + static_cast<int>(cta) * BM;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, 5)) { ok = false; break; }
           uint8_t* sA = smem + stage * P_STAGE_BYTES;
@@ -588,60 +732,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   } else {
     // ------------------------------ epilogue (both CTAs, own 128 rows) ----------------------------------
     const int quarter = warp & 3;
+    const int half = (warp - 2) >> 2;
+    float4* stage_buf = reinterpret_cast<float4*>(smem + P_EPI_OFFSET + (warp - 2) * EPI_STAGE_BYTES);
     int acc = 0;
     uint32_t acc_phase = 0;
-    bool ok = true;
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       int tm, tn;
       tile_coords(tile, num_m, num_n, tm, tn);
-      const int row = tm * TM + static_cast<int>(cta) * BM + quarter * 32 + lane;
-      const int n0 = tn * TN;
-      if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag, 8)) { ok = false; break; }
-      tc_fence_after();
       const uint32_t t_addr = tmem_base + acc * TN + (static_cast<uint32_t>(quarter * 32) << 16);
-      const bool row_ok = row < p.M;
-      float xm = -INFINITY, xl = 0.f;
-#pragma unroll 1
-      for (int c = 0; c < TN / 32; ++c) {
-        uint32_t r[32];
-        __syncwarp();
-        tmem_ld_32x32b_x32(t_addr + c * 32, r);
-        tmem_ld_wait();
-        const int col0 = n0 + c * 32;
-        if (p.swiglu_f > 0) {
-          // columns [0, 128) of the tile are gate, [128, 256) up, of hidden units tn * 128 ...
-          if (c >= 4) continue;
-          uint32_t r2[32];
-          tmem_ld_32x32b_x32(t_addr + (c + 4) * 32, r2);
-          tmem_ld_wait();
-          if (row_ok) swiglu_chunks(p, r, r2, row, tn * 128 + c * 32);
-          continue;
-        }
-        if (p.rope_cols > 0 && col0 < p.rope_cols) {
-          // q / k heads: the chunk and its partner half a head further right are rotated together
-          const int hc = p.rope_dh >> 6;                      // chunks per half head
-          const int in_head = (col0 % p.rope_dh) >> 5;
-          if (in_head >= hc) continue;                        // second halves were stored with their partners
-          uint32_t r2[32];
-          tmem_ld_32x32b_x32(t_addr + (c + hc) * 32, r2);
-          tmem_ld_wait();
-          if (row_ok) {
-            rope_rotate_chunks(p, r, r2, row, in_head * 32);
-            epilogue_chunk(p, r, row, col0);
-            epilogue_chunk(p, r2, row, col0 + hc * 32);
-          }
-          continue;
-        }
-        if (row_ok && col0 < p.N) {
-          if (p.xent_mode == 1) xent_stats_chunk(p, r, row, col0, xm, xl);
-          else epilogue_chunk(p, r, row, col0);
-        }
-      }
-      if (p.xent_mode == 1 && row_ok) {
-        float* st = p.stats + (static_cast<size_t>(row) * p.stat_tiles + tn) * 2;
-        st[0] = xm;
-        st[1] = xl;
-      }
+      const int row0 = tm * TM + static_cast<int>(cta) * BM + quarter * 32;
+      const bool ok = epilogue_tile<TN, EPI>(p, t_addr, row0, tn, half, quarter, lane, acc, stage_buf, [&] {
+        return epilogue_wait(&acc_full[acc], acc_phase, abort_flag, 8);
+      });
+      if (!ok) break;
       __syncwarp();
       tc_fence_before();
       mbar_arrive_cluster(&acc_empty[acc], 0);   // both CTAs report to the issuing CTA
@@ -747,7 +850,7 @@ static void fill_rope(GemmDev& p, const gv_gemm_args* a) {
   p.rope_pos_offset = a->rope_pos_offset;
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, int EPI = EPI_LINEAR>
 static int launch_gemm(const gv_gemm_args* a, cudaStream_t stream, const gv_xent_args* x = nullptr) {
   CUtensorMap tmA, tmB;
   int rc;
@@ -772,7 +875,7 @@ static int launch_gemm(const gv_gemm_args* a, cudaStream_t stream, const gv_xent
   fill_xent(p, x, BN);
   fill_rope(p, a);
   fill_swiglu(p, a);
-  auto kern = gemm_bf16_kernel<BN, A_MN, B_MN>;
+  auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, EPI>;
   constexpr int smem = GemmSmem<BN>::TOTAL;
   static PerDeviceOnce smem_once;
   {
@@ -785,7 +888,7 @@ static int launch_gemm(const gv_gemm_args* a, cudaStream_t stream, const gv_xent
   return static_cast<int>(cudaGetLastError());
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int EPI = EPI_LINEAR>
 static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv_xent_args* x = nullptr) {
   CUtensorMap tmA, tmB;
   int rc;
@@ -810,7 +913,7 @@ static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv
   fill_xent(p, x, 256);
   fill_rope(p, a);
   fill_swiglu(p, a);
-  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN>;
+  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, EPI>;
   static PerDeviceOnce smem_once;
   {
     cudaError_t e = ensure_max_dynamic_smem(smem_once, kern, P_SMEM_TOTAL);
@@ -878,8 +981,8 @@ extern "C" int gv_gemm_bf16(const gv_gemm_args* a, gv_stream_t s) {
         (a->N % 256) || (a->swiglu_ld % 8) || (reinterpret_cast<uintptr_t>(a->swiglu_out) & 15))
       return 2007;
     const long pair_tiles = static_cast<long>((a->M + 255) / 256) * (a->N / 256);
-    if (pair_mode() != 0 && (pair_mode() == 2 || pair_tiles >= num_sms() / 2)) return launch_gemm_pair<false, false>(a, stream);
-    return launch_gemm<256, false, false>(a, stream);
+    if (pair_mode() != 0 && (pair_mode() == 2 || pair_tiles >= num_sms() / 2)) return launch_gemm_pair<false, false, EPI_SWIGLU>(a, stream);
+    return launch_gemm<256, false, false, EPI_SWIGLU>(a, stream);
   }
   // Narrow tiles when wide ones would leave most SMs idle.
   const long tiles256 = static_cast<long>((a->M + BM - 1) / BM) * ((a->N + 255) / 256);
@@ -927,6 +1030,6 @@ extern "C" int gv_gemm_xent(const gv_gemm_args* a, const gv_xent_args* x, gv_str
   if ((a->K % 8) || (a->lda % 8) || (a->ldb % 8) || (x->mode == 2 && (a->ldc % 8))) return 2001;
   if ((reinterpret_cast<uintptr_t>(a->A) | reinterpret_cast<uintptr_t>(a->B) | reinterpret_cast<uintptr_t>(a->C)) & 15) return 2002;
   const long pair_tiles = static_cast<long>((a->M + 255) / 256) * ((a->N + 255) / 256);
-  if (pair_mode() != 0 && (pair_mode() == 2 || pair_tiles >= num_sms() / 2)) return launch_gemm_pair<false, false>(a, stream, x);
-  return launch_gemm<256, false, false>(a, stream, x);
+  if (pair_mode() != 0 && (pair_mode() == 2 || pair_tiles >= num_sms() / 2)) return launch_gemm_pair<false, false, EPI_XENT>(a, stream, x);
+  return launch_gemm<256, false, false, EPI_XENT>(a, stream, x);
 }

@@ -206,6 +206,10 @@ template <int ID, int COUNT>
 __device__ __forceinline__ void named_bar_sync() {
   asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(COUNT) : "memory");
 }
+// The same with the barrier chosen at run time.
+__device__ __forceinline__ void named_bar_sync_id(int id, int count) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
 // Same barrier, also AND-reducing a predicate over its threads: when one thread's bounded wait gave up, all of them
 // learn it at the same point and nobody is left alone at a later barrier.
 template <int ID, int COUNT>

@@ -68,6 +68,28 @@ def test_gemm_epilogues():
     _check(accb, accb0.float() + ref, K)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 6, 8), (33, 36, 72), (129, 130, 64), (300, 257, 200), (2500, 2046, 136)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_epilogue_edges(M, N, K, f32):
+    """Every store option at once, at row and column counts that cut tiles, 32 x 32 chunks and groups of four columns; the
+    last size runs on CTA pairs. Columns of the output buffer beyond N stay untouched."""
+    g = torch.Generator(device="cuda").manual_seed(M * N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", dtype=torch.bfloat16, generator=g)
+    ld = (N + 7) // 8 * 8 + 8
+    a, b, bias, res = rnd(M, K), rnd(N, K), rnd(ld)[:N], rnd(M, ld)[:, :N]
+    buf = rnd(M, ld).to(torch.float32 if f32 else torch.bfloat16)
+    old = buf.clone()
+    gemm(a, b, out=buf[:, :N], bias=bias, gelu=True, residual=res, accumulate=True, alpha=0.25)
+    x = 0.25 * (a.double() @ b.double().t()) + bias.double()
+    ref = torch.nn.functional.gelu(x, approximate="tanh") + res.double() + old[:, :N].double()
+    # fp32 sums of K products and a handful of fp32 roundings (the GELU's slope is below 1.13), then one rounding to bf16
+    size = 0.25 * (a.double().abs() @ b.double().abs().t()) + x.abs() + res.double().abs() + old[:, :N].double().abs() + 1
+    bound = (K + 16) * 2.0 ** -23 * size + (0 if f32 else 2.0 ** -8 * ref.abs())
+    assert ((buf[:, :N].double() - ref).abs() <= bound).all()
+    assert torch.equal(buf[:, N:], old[:, N:])
+    assert _lib.read_error() is None
+
+
 def test_gemm_linear_grads_match_torch():
     torch.manual_seed(2)
     M, N, K = 1024, 768, 512
