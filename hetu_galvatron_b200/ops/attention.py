@@ -13,17 +13,19 @@ def supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
     if dh % 8 != 0 or dh > 128:
         return False
     for t in (q, k, v):
-        if t.dtype != torch.bfloat16 or t.stride(-1) != 1 or t.data_ptr() % 16 != 0:
+        if t.dtype != torch.bfloat16 or t.data_ptr() % 16 != 0:
             return False
-        if any(s % 8 for s in t.stride()[:-1]):
+        sb, ss, sh, inner = t.stride()
+        if inner != 1 or (sb | ss | sh) % 8:
             return False
     return q.shape[2] % k.shape[2] == 0
 
 
 def _strides(t):
-    return t.stride(0), t.stride(1), t.stride(2)
+    return t.stride()[:3]
 
 
+_NO_GRAD_STRIDES = (0,) * 12          # do, dq, dk, dv of a forward call
 _READY = False
 
 
@@ -106,17 +108,13 @@ def fwd(q, k, v, causal: bool, scale: float, out=None, kv_lens=None, dropout=Non
     sk, hk = k.shape[1], k.shape[2]
     o = out if out is not None else torch.empty((b, sq, hq, dh), dtype=q.dtype, device=q.device)
     lse = torch.empty((b, hq, sq), dtype=torch.float32, device=q.device)
-    a = _lib.AttnArgs(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), o=o.data_ptr(), lse=lse.data_ptr(),
-                      b=b, sq=sq, sk=sk, hq=hq, hk=hk, dh=dh, causal=int(causal), scale=float(scale))
     lens = _lens(kv_lens, b, q.device)
-    a.kv_lens = _lib.p(lens) or None
+    a = _lib.AttnArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), 0, 0, 0, 0, 0, 0,
+                      b, sq, sk, hq, hk, dh, *_strides(q), *_strides(k), *_strides(v), *_strides(o), *_NO_GRAD_STRIDES,
+                      int(causal), float(scale), 0 if lens is None else lens.data_ptr())
     _set_dropout(a, dropout)
     if additive is not None:
         additive.apply(a, hq)
-    (a.q_stride_b, a.q_stride_s, a.q_stride_h) = _strides(q)
-    (a.k_stride_b, a.k_stride_s, a.k_stride_h) = _strides(k)
-    (a.v_stride_b, a.v_stride_s, a.v_stride_h) = _strides(v)
-    (a.o_stride_b, a.o_stride_s, a.o_stride_h) = _strides(o)
     _lib.check(lib.gv_attn_fwd(a, _lib.stream_ptr()), "gv_attn_fwd")
     return o, lse
 
@@ -137,16 +135,11 @@ def bwd(dout, q, k, v, o, lse, causal: bool, scale: float, dq=None, dk=None, dv=
         dv = torch.empty((b, sk, hk, dh), dtype=q.dtype, device=q.device)
     dq_accum = torch.empty((b, sq, hq, dh), dtype=torch.float32, device=q.device)
     delta = torch.empty((b, hq, sq), dtype=torch.float32, device=q.device)
-    a = _lib.AttnArgs(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), o=o.data_ptr(), lse=lse.data_ptr(),
-                      dout=dout.data_ptr(), dq=dq.data_ptr(), dk=dk.data_ptr(), dv=dv.data_ptr(),
-                      dq_accum=dq_accum.data_ptr(), delta=delta.data_ptr(),
-                      b=b, sq=sq, sk=sk, hq=hq, hk=hk, dh=dh, causal=int(causal), scale=float(scale))
     lens = _lens(kv_lens, b, q.device)
-    a.kv_lens = _lib.p(lens) or None
-    (a.q_stride_b, a.q_stride_s, a.q_stride_h) = _strides(q)
-    (a.k_stride_b, a.k_stride_s, a.k_stride_h) = _strides(k)
-    (a.v_stride_b, a.v_stride_s, a.v_stride_h) = _strides(v)
-    (a.o_stride_b, a.o_stride_s, a.o_stride_h) = _strides(o)
+    a = _lib.AttnArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), dout.data_ptr(), dq.data_ptr(),
+                      dk.data_ptr(), dv.data_ptr(), dq_accum.data_ptr(), delta.data_ptr(), b, sq, sk, hq, hk, dh,
+                      *_strides(q), *_strides(k), *_strides(v), *_strides(o), *_strides(dout), *_strides(dq), *_strides(dk),
+                      *_strides(dv), int(causal), float(scale), 0 if lens is None else lens.data_ptr())
     _set_dropout(a, dropout)
     if additive is not None:
         additive.apply(a, hq)
@@ -158,9 +151,5 @@ def bwd(dout, q, k, v, o, lse, causal: bool, scale: float, dq=None, dk=None, dv=
         inv_freq, pos, off = dq_rope
         pos = None if pos is None else pos.to(device=q.device, dtype=torch.int32).contiguous()
         a.dq_rope_inv_freq, a.dq_rope_pos, a.dq_rope_pos_offset = inv_freq.data_ptr(), (_lib.p(pos) or None), int(off)
-    (a.do_stride_b, a.do_stride_s, a.do_stride_h) = _strides(dout)
-    (a.dq_stride_b, a.dq_stride_s, a.dq_stride_h) = _strides(dq)
-    (a.dk_stride_b, a.dk_stride_s, a.dk_stride_h) = _strides(dk)
-    (a.dv_stride_b, a.dv_stride_s, a.dv_stride_h) = _strides(dv)
     _lib.check(lib.gv_attn_bwd(a, _lib.stream_ptr()), "gv_attn_bwd")
     return dq, dk, dv

@@ -334,6 +334,22 @@ def rmsnorm_branch(x, w, eps: float = 1e-5):
     return RMSNormBranchFn.apply(x, w, eps)
 
 
+def _layernorm_grads(dy, x, w, b, mean, rstd, dres):
+    """dx and what autograd gets for weight and bias: the kernel adds both into their fp32 gradient buffers when there are
+    such, else into a scratch pair that is handed on."""
+    mw, mb = getattr(w, "main_grad", None), getattr(b, "main_grad", None)
+    if mw is not None and mb is not None and mw.dtype == mb.dtype == torch.float32:
+        dx = Fn.layernorm_bwd(dy, x, w, mean, rstd, dres, mw.view(-1), mb.view(-1))
+        for p in (w, b):
+            hook = getattr(p, "grad_ready_hook", None)
+            if hook is not None:
+                hook(p)
+        return dx, None, None
+    dwb = torch.zeros(2, w.numel(), dtype=torch.float32, device=w.device)
+    dx = Fn.layernorm_bwd(dy, x, w, mean, rstd, dres, dwb[0], dwb[1])
+    return dx, _vec_grad(w, lambda buf: buf.add_(dwb[0])), _vec_grad(b, lambda buf: buf.add_(dwb[1]))
+
+
 class LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b, eps):
@@ -344,11 +360,7 @@ class LayerNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, b, mean, rstd = ctx.saved_tensors
-        dwb = torch.zeros(2, w.numel(), dtype=torch.float32, device=w.device)
-        dx = Fn.layernorm_bwd(dy, x, w, mean, rstd, None, dwb[0], dwb[1])
-        dw = _vec_grad(w, lambda buf: buf.add_(dwb[0]))
-        db = _vec_grad(b, lambda buf: buf.add_(dwb[1]))
-        return dx, dw, db, None
+        return (*_layernorm_grads(dy, x, w, b, mean, rstd, None), None)
 
 
 def layernorm(x, w, b, eps: float = 1e-5):
@@ -369,11 +381,7 @@ class LayerNormBranchFn(torch.autograd.Function):
         x, w, b, mean, rstd = ctx.saved_tensors
         if dy is None:
             return dres, None, None, None
-        dwb = torch.zeros(2, w.numel(), dtype=torch.float32, device=w.device)
-        dx = Fn.layernorm_bwd(dy, x, w, mean, rstd, dres, dwb[0], dwb[1])
-        dw = _vec_grad(w, lambda buf: buf.add_(dwb[0]))
-        db = _vec_grad(b, lambda buf: buf.add_(dwb[1]))
-        return dx, dw, db, None
+        return (*_layernorm_grads(dy, x, w, b, mean, rstd, dres), None)
 
 
 def layernorm_branch(x, w, b, eps: float = 1e-5):
@@ -397,13 +405,15 @@ class AttnCfg:
 
 
 def _qkv_views(qkv: torch.Tensor, cfg: AttnCfg):
-    tokens = qkv.shape[0]
-    s = tokens // cfg.batch
-    hq, hk, dh = cfg.hq, cfg.hk, cfg.dh
-    q = qkv[:, : hq * dh].view(s, cfg.batch, hq, dh).transpose(0, 1)
-    k = qkv[:, hq * dh:(hq + hk) * dh].view(s, cfg.batch, hk, dh).transpose(0, 1)
-    v = qkv[:, (hq + hk) * dh:].view(s, cfg.batch, hk, dh).transpose(0, 1)
-    return q, k, v
+    """q, k, v [batch, s, heads, dh] as views of the contiguous packed projection."""
+    tokens, ld = qkv.shape
+    b, hq, hk, dh = cfg.batch, cfg.hq, cfg.hk, cfg.dh
+    s, at, strides = tokens // b, qkv.storage_offset(), (ld, b * ld, dh, 1)
+    if s * b != tokens or (hq + 2 * hk) * dh != ld:
+        raise ValueError("packed projection %s does not hold %d + 2 x %d heads of %d for whole sequences of %d elements"
+                         % (tuple(qkv.shape), hq, hk, dh, b))
+    return (qkv.as_strided((b, s, hq, dh), strides, at), qkv.as_strided((b, s, hk, dh), strides, at + hq * dh),
+            qkv.as_strided((b, s, hk, dh), strides, at + (hq + hk) * dh))
 
 
 def _rope_packed_(qkv: torch.Tensor, cfg: AttnCfg, inv_freq, positions, inverse: bool):

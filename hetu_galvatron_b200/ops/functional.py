@@ -7,7 +7,6 @@ oracle of the GPU tests). Function names mirror csrc/include/gv_kernels.h.
 from __future__ import annotations
 
 import math
-from ctypes import c_void_p
 
 import torch
 import torch.nn.functional as F
@@ -21,21 +20,18 @@ def _native(t: torch.Tensor) -> bool:
     return t.is_cuda and t.dtype == torch.bfloat16
 
 
+# Addresses and the stream go over as ints: every entry point called here has its argument types in ``_lib.PROTOTYPES``.
 def _vp(t):
-    return c_void_p(0 if t is None else t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
-def _s():
-    return c_void_p(_lib.stream_ptr())
+_s = _lib.stream_ptr
 
 
 # ----------------------------------------------------------------------------- normalisation
 def _norm_scratch(rows: int, cols: int, layer: int, device) -> torch.Tensor:
     """Partial weight-gradient rows of the two-stage (atomic-free, bitwise repeatable) norm backward: one per CTA."""
-    fn = _lib.lib().gv_norm_bwd_scratch_elems
-    raw = getattr(fn, "raw", fn)
-    raw.restype = _lib.c_longlong
-    n = int(raw(int(rows), int(cols), int(layer)))
+    n = _lib.lib().gv_norm_bwd_scratch_elems(rows, cols, layer)
     return torch.empty(max(n, 1), dtype=torch.float32, device=device)
 
 
@@ -50,7 +46,7 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float, residual: torch.Te
         if residual is not None:
             residual = residual.contiguous()
         rc = _lib.lib().gv_rmsnorm_fwd(_vp(x), _vp(residual), _vp(w), _vp(y), _vp(h if residual is not None else None),
-                                       _vp(rstd), rows, cols, _lib.c_float(eps), _s())
+                                       _vp(rstd), rows, cols, eps, _s())
         _lib.check(rc, "gv_rmsnorm_fwd")
         return y, h, rstd
     h = x if residual is None else (x + residual)
@@ -70,7 +66,7 @@ def rmsnorm_bwd(dy, h, w, rstd, dres=None, dw_accum: torch.Tensor | None = None)
             dres = dres.contiguous()
         scratch = _norm_scratch(rows, cols, 0, h.device)
         rc = _lib.lib().gv_rmsnorm_bwd(_vp(dy), _vp(h), _vp(w), _vp(rstd), _vp(dres), _vp(dx), _vp(dw_accum), _vp(scratch),
-                                       _lib.c_longlong(scratch.numel()), rows, cols, _s())
+                                       scratch.numel(), rows, cols, _s())
         _lib.check(rc, "gv_rmsnorm_bwd")
         return dx
     hf = h.float().reshape(rows, cols)
@@ -99,7 +95,7 @@ def layernorm_fwd(x, w, b, eps, residual=None):
             residual = residual.contiguous()
         rc = _lib.lib().gv_layernorm_fwd(_vp(x), _vp(residual), _vp(w), _vp(b), _vp(y),
                                          _vp(h if residual is not None else None), _vp(mean), _vp(rstd), rows, cols,
-                                         _lib.c_float(eps), _s())
+                                         eps, _s())
         _lib.check(rc, "gv_layernorm_fwd")
         return y, h, mean, rstd
     h = x if residual is None else (x + residual)
@@ -121,7 +117,7 @@ def layernorm_bwd(dy, h, w, mean, rstd, dres=None, dw_accum=None, db_accum=None)
             dres = dres.contiguous()
         scratch = _norm_scratch(rows, cols, 1, h.device)
         rc = _lib.lib().gv_layernorm_bwd(_vp(dy), _vp(h), _vp(w), _vp(mean), _vp(rstd), _vp(dres), _vp(dx),
-                                         _vp(dw_accum), _vp(db_accum), _vp(scratch), _lib.c_longlong(scratch.numel()),
+                                         _vp(dw_accum), _vp(db_accum), _vp(scratch), scratch.numel(),
                                          rows, cols, _s())
         _lib.check(rc, "gv_layernorm_bwd")
         return dx
@@ -158,8 +154,8 @@ def rope_(x: torch.Tensor, inv_freq: torch.Tensor, pos_div: int = 1, pos_mod: in
         pos32 = None
         if positions is not None:
             pos32 = positions.to(torch.int32).contiguous()
-        rc = _lib.lib().gv_rope(_vp(x), _vp(pos32), _vp(inv_freq), _lib.c_longlong(tokens), heads, dh,
-                                _lib.c_longlong(x.stride(0)), int(pos_div), int(pos_mod), int(pos_offset), int(inverse),
+        rc = _lib.lib().gv_rope(_vp(x), _vp(pos32), _vp(inv_freq), tokens, heads, dh,
+                                x.stride(0), int(pos_div), int(pos_mod), int(pos_offset), int(inverse),
                                 _s())
         _lib.check(rc, "gv_rope")
         return x
@@ -185,7 +181,7 @@ def swiglu_fwd(gu: torch.Tensor) -> torch.Tensor:
     rows = gu.numel() // gu.shape[-1]
     if _native(gu) and f % 8 == 0 and gu.is_contiguous():
         out = torch.empty(*gu.shape[:-1], f, dtype=gu.dtype, device=gu.device)
-        _lib.check(_lib.lib().gv_swiglu_fwd(_vp(gu), _vp(out), _lib.c_longlong(rows), f, _s()), "gv_swiglu_fwd")
+        _lib.check(_lib.lib().gv_swiglu_fwd(_vp(gu), _vp(out), rows, f, _s()), "gv_swiglu_fwd")
         return out
     g, u = gu.float().chunk(2, dim=-1)
     return (F.silu(g) * u).to(gu.dtype)
@@ -197,7 +193,7 @@ def swiglu_bwd(dout: torch.Tensor, gu: torch.Tensor) -> torch.Tensor:
     if _native(gu) and f % 8 == 0 and gu.is_contiguous():
         dout = dout.contiguous()
         dgu = torch.empty_like(gu)
-        _lib.check(_lib.lib().gv_swiglu_bwd(_vp(dout), _vp(gu), _vp(dgu), _lib.c_longlong(rows), f, _s()),
+        _lib.check(_lib.lib().gv_swiglu_bwd(_vp(dout), _vp(gu), _vp(dgu), rows, f, _s()),
                    "gv_swiglu_bwd")
         return dgu
     g, u = gu.float().chunk(2, dim=-1)
@@ -210,7 +206,7 @@ def swiglu_bwd(dout: torch.Tensor, gu: torch.Tensor) -> torch.Tensor:
 def gelu_fwd(x: torch.Tensor) -> torch.Tensor:
     if _native(x) and x.numel() % 8 == 0 and x.is_contiguous():
         y = torch.empty_like(x)
-        _lib.check(_lib.lib().gv_gelu_fwd(_vp(x), _vp(y), _lib.c_longlong(x.numel()), _s()), "gv_gelu_fwd")
+        _lib.check(_lib.lib().gv_gelu_fwd(_vp(x), _vp(y), x.numel(), _s()), "gv_gelu_fwd")
         return y
     return F.gelu(x.float(), approximate="tanh").to(x.dtype)
 
@@ -219,7 +215,7 @@ def gelu_bwd(dy: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
     if _native(x) and x.numel() % 8 == 0 and x.is_contiguous():
         dy = dy.contiguous()
         dx = torch.empty_like(x)
-        _lib.check(_lib.lib().gv_gelu_bwd(_vp(dy), _vp(x), _vp(dx), _lib.c_longlong(x.numel()), _s()), "gv_gelu_bwd")
+        _lib.check(_lib.lib().gv_gelu_bwd(_vp(dy), _vp(x), _vp(dx), x.numel(), _s()), "gv_gelu_bwd")
         return dx
     xf = x.float()
     k0, k1 = 0.7978845608028654, 0.044715
@@ -233,7 +229,7 @@ def colsum_accum(dy: torch.Tensor, out: torch.Tensor) -> None:
     cols = dy.shape[-1]
     rows = dy.numel() // cols
     if _native(dy) and cols % 8 == 0 and out.dtype == torch.float32 and dy.is_contiguous():
-        _lib.check(_lib.lib().gv_colsum_accum(_vp(dy), _vp(out), _lib.c_longlong(rows), cols, _s()), "gv_colsum_accum")
+        _lib.check(_lib.lib().gv_colsum_accum(_vp(dy), _vp(out), rows, cols, _s()), "gv_colsum_accum")
         return
     out.add_(dy.float().reshape(rows, cols).sum(0).to(out.dtype))
 
@@ -249,8 +245,8 @@ def embedding_fwd(ids: torch.Tensor, table: torch.Tensor, vocab_start: int = 0,
         out = torch.empty(flat.numel(), hidden, dtype=table.dtype, device=table.device)
         p32 = pos_ids.reshape(-1).to(torch.int32).contiguous() if pos_table is not None else None
         rc = _lib.lib().gv_embedding_fwd(_vp(flat), _vp(table), _vp(p32), _vp(pos_table), _vp(out),
-                                         _lib.c_longlong(flat.numel()), hidden, _lib.c_longlong(vocab_start),
-                                         _lib.c_longlong(table.shape[0]), _s())
+                                         flat.numel(), hidden, vocab_start,
+                                         table.shape[0], _s())
         _lib.check(rc, "gv_embedding_fwd")
         return out.reshape(*ids.shape, hidden)
     local = flat - vocab_start
@@ -267,8 +263,8 @@ def embedding_bwd(ids: torch.Tensor, dout: torch.Tensor, dtable_accum: torch.Ten
     if _native(dout) and hidden % 8 == 0 and dtable_accum.dtype == torch.float32:
         flat = flat.to(torch.int64).contiguous()
         dout = dout.contiguous()
-        rc = _lib.lib().gv_embedding_bwd(_vp(flat), _vp(dout), _vp(dtable_accum), _lib.c_longlong(flat.numel()), hidden,
-                                         _lib.c_longlong(vocab_start), _lib.c_longlong(dtable_accum.shape[0]), _s())
+        rc = _lib.lib().gv_embedding_bwd(_vp(flat), _vp(dout), _vp(dtable_accum), flat.numel(), hidden,
+                                         vocab_start, dtable_accum.shape[0], _s())
         _lib.check(rc, "gv_embedding_bwd")
         return
     local = flat - vocab_start
@@ -286,8 +282,8 @@ def xent_stats(logits: torch.Tensor, labels: torch.Tensor, vocab_start: int = 0)
         mx = torch.empty(rows, dtype=torch.float32, device=logits.device)
         se = torch.empty_like(mx)
         tg = torch.empty_like(mx)
-        rc = _lib.lib().gv_xent_stats(_vp(logits), _vp(labels), _vp(mx), _vp(se), _vp(tg), _lib.c_longlong(rows), v,
-                                      _lib.c_longlong(logits.stride(0)), _lib.c_longlong(vocab_start), _s())
+        rc = _lib.lib().gv_xent_stats(_vp(logits), _vp(labels), _vp(mx), _vp(se), _vp(tg), rows, v,
+                                      logits.stride(0), vocab_start, _s())
         _lib.check(rc, "gv_xent_stats")
         return mx, se, tg
     lf = logits.float()
@@ -310,9 +306,9 @@ def xent_loss_grad_(logits: torch.Tensor, labels: torch.Tensor, mx, se, tg, grad
         labels = labels.to(torch.int64).contiguous()
         loss = torch.empty(rows, dtype=torch.float32, device=logits.device)
         rc = _lib.lib().gv_xent_loss_grad(_vp(logits), _vp(labels), _vp(mx), _vp(se), _vp(tg), _vp(loss),
-                                          _lib.c_float(grad_scale), _vp(scale_tensor), _lib.c_longlong(rows), v,
-                                          _lib.c_longlong(logits.stride(0)), _lib.c_longlong(vocab_start),
-                                          _lib.c_longlong(ignore_index), _s())
+                                          grad_scale, _vp(scale_tensor), rows, v,
+                                          logits.stride(0), vocab_start,
+                                          ignore_index, _s())
         _lib.check(rc, "gv_xent_loss_grad")
         return loss
     lf = logits.float()
@@ -340,9 +336,9 @@ def adamw_step_(master, m, v, grad, param, *, lr, beta1, beta2, eps, weight_deca
     if master.is_cuda and master.dtype == torch.float32 and grad.dtype in (torch.float32, torch.bfloat16) and \
             (param is None or param.dtype == torch.bfloat16):
         rc = _lib.lib().gv_adamw(_vp(master), _vp(m), _vp(v), _vp(grad), int(grad.dtype == torch.bfloat16), _vp(param),
-                                 _lib.c_longlong(n), _lib.c_float(lr), _lib.c_float(beta1), _lib.c_float(beta2),
-                                 _lib.c_float(eps), _lib.c_float(weight_decay), _lib.c_float(bc1), _lib.c_float(bc2),
-                                 _lib.c_float(grad_scale), _vp(clip_coef), _s())
+                                 n, lr, beta1, beta2,
+                                 eps, weight_decay, bc1, bc2,
+                                 grad_scale, _vp(clip_coef), _s())
         _lib.check(rc, "gv_adamw")
         return
     g = grad.to(master.dtype) * grad_scale
@@ -359,7 +355,7 @@ def adamw_step_(master, m, v, grad, param, *, lr, beta1, beta2, eps, weight_deca
 def sumsq_accum(x: torch.Tensor, out: torch.Tensor) -> None:
     """out[0] += sum(x^2) (fp32)."""
     if x.is_cuda and x.dtype in (torch.float32, torch.bfloat16) and x.is_contiguous() and out.dtype == torch.float32:
-        rc = _lib.lib().gv_sumsq_accum(_vp(x), int(x.dtype == torch.bfloat16), _lib.c_longlong(x.numel()), _vp(out), _s())
+        rc = _lib.lib().gv_sumsq_accum(_vp(x), int(x.dtype == torch.bfloat16), x.numel(), _vp(out), _s())
         _lib.check(rc, "gv_sumsq_accum")
         return
     out.add_(x.float().pow(2).sum().to(out.dtype))
@@ -375,8 +371,8 @@ def lse_merge_(acc: torch.Tensor, lse_acc: torch.Tensor, o_blk: torch.Tensor, ls
             and o_blk.dtype == torch.bfloat16 and o_blk.stride(-1) == 1 and lse_blk.dtype == torch.float32):
         lse_blk = lse_blk.contiguous()
         rc = _lib.lib().gv_lse_merge(_vp(acc), _vp(lse_acc), _vp(o_blk), _vp(lse_blk), b, s, sb, s_off, h, dh,
-                                     _lib.c_longlong(o_blk.stride(0)), _lib.c_longlong(o_blk.stride(1)),
-                                     _lib.c_longlong(o_blk.stride(2)), _s())
+                                     o_blk.stride(0), o_blk.stride(1),
+                                     o_blk.stride(2), _s())
         _lib.check(rc, "gv_lse_merge")
         return
     la = lse_acc[:, :, s_off:s_off + sb]

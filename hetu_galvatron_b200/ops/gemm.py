@@ -13,16 +13,17 @@ from . import _lib
 
 
 def _use_native(*ts) -> bool:
-    t0 = ts[0]
-    if not t0.is_cuda:
-        return False
-    return all(t is None or (t.is_cuda and t.dtype == torch.bfloat16) for t in ts)
+    for t in ts:
+        if t is not None and not (t.is_cuda and t.dtype == torch.bfloat16):
+            return False
+    return True
 
 
 def _row_major_2d(t: torch.Tensor) -> torch.Tensor:
     if t.dim() != 2:
         t = t.reshape(-1, t.shape[-1])
-    if t.stride(1) != 1 or t.stride(0) % 8 != 0 or t.data_ptr() % 16 != 0:
+    ld, inner = t.stride()
+    if inner != 1 or ld % 8 != 0 or t.data_ptr() % 16 != 0:
         t = t.contiguous()
     return t
 
@@ -76,11 +77,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if residual is not None:
             residual = _row_major_2d(residual)
         args = _lib.GemmArgs(
-            A=a.data_ptr(), B=b.data_ptr(), C=out.data_ptr(), bias=_lib.p(bias), residual=_lib.p(residual),
-            M=M, N=N, K=K, lda=a.stride(0), ldb=b.stride(0), ldc=out.stride(0),
-            ldr=residual.stride(0) if residual is not None else 0,
-            a_mn_major=int(a_mn), b_mn_major=int(b_mn), c_f32=int(out.dtype == torch.float32),
-            accumulate=int(accumulate), act=int(gelu), alpha=float(alpha))
+            a.data_ptr(), b.data_ptr(), out.data_ptr(), 0 if bias is None else bias.data_ptr(),
+            0 if residual is None else residual.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+            0 if residual is None else residual.stride(0), int(a_mn), int(b_mn), int(out.dtype == torch.float32),
+            int(accumulate), int(gelu), float(alpha))
         if swiglu_out is not None:
             args.swiglu_out, args.swiglu_ld = swiglu_out.data_ptr(), swiglu_out.stride(0)
         if rope is not None:

@@ -215,12 +215,16 @@ class ParamBucket:
     def _remember_shapes(self) -> None:
         for p in self.params:
             p._gv_shape, p._gv_numel = tuple(p.shape), p.numel()
+        self._grad_views = None
 
     def _ensure_grad(self) -> None:
         if self.grad_flat is None:
             self.grad_flat = torch.zeros(self.numel, dtype=self.grad_dtype, device=self.device)
-        for p, o in zip(self.params, self.offsets):
-            p.main_grad = self.grad_flat[o:o + p._gv_numel].view(p._gv_shape)
+        if self._grad_views is None or self._grad_views[0] is not self.grad_flat:
+            self._grad_views = (self.grad_flat, [self.grad_flat[o:o + p._gv_numel].view(p._gv_shape)
+                                                 for p, o in zip(self.params, self.offsets)])
+        for p, view in zip(self.params, self._grad_views[1]):
+            p.main_grad = view
 
     # ------------------------------------------------------------------ ZeRO-3 gather / release
     def wait_params(self) -> None:
@@ -426,6 +430,9 @@ class ParamBucket:
     def grad_sumsq(self, out: torch.Tensor, tp_size: int) -> None:
         """Adds this bucket's share of the squared global gradient norm (already divided by d^2) into out[0]."""
         if self.numel == 0 or self.grad_shard is None:
+            return
+        if self.d == 1 and not self.skip_params and not (self.dup_params and tp_size > 1):
+            Fn.sumsq_accum(self.grad_shard, out)        # the whole bucket counts, with weight one
             return
         tmp = torch.zeros(1, dtype=torch.float32, device=self.device)
         Fn.sumsq_accum(self.grad_shard, tmp)
