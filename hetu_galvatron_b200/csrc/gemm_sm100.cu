@@ -12,7 +12,9 @@
 // Tile 128 x BN x 64 (BN = 256 or 128), 128-byte swizzled operands, both operand majors
 // supported through the shared-memory descriptors, so forward, dgrad and wgrad GEMMs all read
 // the tensors in the layout they already have (no transposes are materialised).
+#include <atomic>
 #include <cstdlib>
+#include <type_traits>
 #include "include/gv_kernels.h"
 #include "include/gv_host.h"
 #include "include/gv_ptx.cuh"
@@ -153,23 +155,14 @@ __device__ __forceinline__ void epi_fetch(const float4* stage, int lane, float4 
   for (int i = 0; i < 8; ++i) v[i] = stage[(l0 + 4 * i) * 8 + (piece ^ ((l0 + 4 * i) & 7))];
 }
 
-// Stores the staged chunk to C: alpha, bias, GELU, residual, accumulate. PLAIN: alpha alone, bf16.
-template <bool PLAIN>
+// Stores the staged chunk to C: alpha, bias, GELU, residual, accumulate.
 __device__ __forceinline__ void epi_store(const GemmDev& p, const float4* stage, int row0, int col0, int lane, const EpiOld& old) {
   const int col = col0 + (lane & 7) * 4;
   if (col >= p.N) return;
   const int r0 = row0 + (lane >> 3);
-  if (PLAIN || col + 4 <= p.N) {
+  if (col + 4 <= p.N) {
     float4 v[8];
     epi_fetch(stage, lane, v);
-    if constexpr (PLAIN) {
-      __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(r0) * p.ldc + col;
-#pragma unroll
-      for (int i = 0; i < 8; ++i, cp += 4 * static_cast<size_t>(p.ldc))
-        if (r0 + 4 * i < p.M)
-          *reinterpret_cast<uint2*>(cp) = make_uint2(pack_bf16x2(v[i].x * p.alpha, v[i].y * p.alpha), pack_bf16x2(v[i].z * p.alpha, v[i].w * p.alpha));
-      return;
-    }
     float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
     if (p.bias != nullptr) {
       const uint2 u = __ldg(reinterpret_cast<const uint2*>(p.bias + col));
@@ -241,28 +234,128 @@ __device__ __forceinline__ void epi_store(const GemmDev& p, const float4* stage,
   }
 }
 
-// Stores the staged chunk as bf16, no scaling, to the activation output.
-__device__ __forceinline__ void epi_store_act(const GemmDev& p, const float4* stage, int row0, int unit0, int lane) {
-  const int r0 = row0 + (lane >> 3);
-  float4 v[8];
-  epi_fetch(stage, lane, v);
-  __nv_bfloat16* ap = p.act_out + static_cast<size_t>(r0) * p.ld_act + unit0 + (lane & 7) * 4;
+// One row per lane, 64 columns as bf16 pairs -> memory: 4 KB of staging again, sixteen bytes per lane and eight lanes per row,
+// so every store covers four whole lines. Outputs that only need scale, bias and activation take this way (the fp32 one above
+// moves twice the staging bytes and half a line per row: 8192 x 4096 x 1024 took 63 us with it).
+__device__ __forceinline__ void epi_put64(const uint32_t (&w)[32], float4* stage, int lane, __nv_bfloat16* C, int ld, int M, int N,
+                                          int row0, int col0) {
+  uint4* st = reinterpret_cast<uint4*>(stage);
+  __syncwarp();
 #pragma unroll
-  for (int i = 0; i < 8; ++i, ap += 4 * static_cast<size_t>(p.ld_act))
-    if (r0 + 4 * i < p.M) *reinterpret_cast<uint2*>(ap) = make_uint2(pack_bf16x2(v[i].x, v[i].y), pack_bf16x2(v[i].z, v[i].w));
+  for (int j = 0; j < 8; ++j) st[lane * 8 + (j ^ (lane & 7))] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+  __syncwarp();
+  const int piece = lane & 7, l0 = lane >> 3, r0 = row0 + l0, col = col0 + piece * 8;
+  if (col >= N) return;
+  uint4 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = st[(l0 + 4 * i) * 8 + (piece ^ ((l0 + 4 * i) & 7))];
+  __nv_bfloat16* cp = C + static_cast<size_t>(r0) * ld + col;
+  if (col + 8 <= N) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i, cp += 4 * static_cast<size_t>(ld))
+      if (r0 + 4 * i < M) *reinterpret_cast<uint4*>(cp) = v[i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i, cp += 4 * static_cast<size_t>(ld)) {
+      if (r0 + 4 * i >= M) continue;
+      const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (col + e < N) cp[e] = __ushort_as_bfloat16(static_cast<unsigned short>(u[e >> 1] >> (16 * (e & 1))));
+    }
+  }
+}
+
+// alpha, bias and GELU on one row's 32 columns, rounded to bf16 pairs. The bias is the same for all lanes: broadcast loads.
+__device__ __forceinline__ void epi_pack32(const GemmDev& p, const uint32_t (&r)[32], int col0, uint32_t* w) {
+  float v[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+  if (p.bias != nullptr) {
+    if (col0 + 32 <= p.N) {
+      const uint2* bp = reinterpret_cast<const uint2*>(p.bias + col0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint2 u = __ldg(bp + j);
+        const float4 b = bf16x4_to_f4(u.x, u.y);
+        v[4 * j] += b.x; v[4 * j + 1] += b.y; v[4 * j + 2] += b.z; v[4 * j + 3] += b.w;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (col0 + i < p.N) v[i] += __bfloat162float(p.bias[col0 + i]);
+    }
+  }
+  if (p.act == 1) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+}
+
+// sin and cos without branches, for |x| <= SINCOS_MAX: reduction by multiples of pi / 2 kept in two floats (Cody and Waite),
+// then the polynomials of the Cephes library's sinf / cosf (Moshier) on [-pi / 4, pi / 4]. Largest error against 64 bits up to
+// SINCOS_MAX: 6.4e-8 (CUDA's own: 8.8e-8). sincosf's slow path for huge arguments is a branch per element, and with two warps per
+// scheduler the epilogue waited for those branches: 8192 x 3072 x 1024 with 64-wide heads 81 -> 61 us.
+constexpr float SINCOS_MAX = 65536.f;
+__device__ __forceinline__ void sincos_reduced(float x, float& sn, float& cs) {
+  const float k = rintf(x * 0.636619772f);
+  const int q = static_cast<int>(k);
+  const float r = fmaf(-k, -4.37113900019e-8f, fmaf(-k, 1.57079637051f, x));
+  const float t = r * r;
+  const float s = fmaf(fmaf(fmaf(-1.9515295891e-4f, t, 8.3321608736e-3f), t, -1.6666654611e-1f) * t, r, r);
+  const float w = 0.5f * t, u = 1.f - w;                   // 1 - w in two parts: u and what its rounding lost
+  const float c = u + fmaf(fmaf(fmaf(2.443315711809948e-5f, t, -1.388731625493765e-3f), t, 4.166664568298827e-2f) * t, t, (1.f - u) - w);
+  const float a = (q & 1) ? c : s, b = (q & 1) ? s : c;
+  sn = __uint_as_float(__float_as_uint(a) ^ (static_cast<uint32_t>(q & 2) << 30));
+  cs = __uint_as_float(__float_as_uint(b) ^ (static_cast<uint32_t>((q + 1) & 2) << 30));
+}
+
+// x / (1 + exp(-x)) without the branch per element of an IEEE division: a reciprocal with one Newton step, which is left out
+// where the denominator has overflowed (there x * 0 is the answer). 8192 x 5632 x 1024 gated: 129 -> 98 us.
+__device__ __forceinline__ float silu(float x) {
+  const float d = 1.f + __expf(-x);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  const float z = fmaf(y, fmaf(-d, y, 1.f), y);
+  return x * (d < 1e38f ? z : y);
 }
 
 // Rotary embedding (non-interleaved halves) on two 32-column chunks of one output row that sit half a head apart:
 // r1 holds columns [c, c + 32) of the head's first half, r2 the same columns of its second half
 // (reference: megatron/core/models/common/embeddings/rotary_pos_embedding.py:204-227 as a separate pass over q and k).
 __device__ __forceinline__ void rope_rotate_chunks(const GemmDev& p, uint32_t (&r1)[32], uint32_t (&r2)[32], float pos, int freq0) {
+  float largest = 0.f;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    float sn, cs;
-    sincosf(pos * __ldg(p.rope_inv_freq + freq0 + i), &sn, &cs);
-    const float a = __uint_as_float(r1[i]), b = __uint_as_float(r2[i]);
-    r1[i] = __float_as_uint(a * cs - b * sn);
-    r2[i] = __float_as_uint(b * cs + a * sn);
+  for (int i = 0; i < 32; ++i) largest = fmaxf(largest, fabsf(pos * __ldg(p.rope_inv_freq + freq0 + i)));
+  if (largest <= SINCOS_MAX) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      float sn, cs;
+      sincos_reduced(pos * __ldg(p.rope_inv_freq + freq0 + i), sn, cs);
+      const float a = __uint_as_float(r1[i]), b = __uint_as_float(r2[i]);
+      r1[i] = __float_as_uint(a * cs - b * sn);
+      r2[i] = __float_as_uint(b * cs + a * sn);
+    }
+  } else {
+#pragma unroll 1
+    for (int i0 = 0; i0 < 32; i0 += 8) {
+      // (rolled, so the registers of the chunk are walked by rotating them eight at a time)
+      uint32_t h1[8], h2[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        float sn, cs;
+        sincosf(pos * __ldg(p.rope_inv_freq + freq0 + i0 + e), &sn, &cs);
+        const float a = __uint_as_float(r1[e]), b = __uint_as_float(r2[e]);
+        h1[e] = __float_as_uint(a * cs - b * sn);
+        h2[e] = __float_as_uint(b * cs + a * sn);
+      }
+#pragma unroll
+      for (int e = 0; e < 24; ++e) { r1[e] = r1[e + 8]; r2[e] = r2[e + 8]; }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { r1[24 + e] = h1[e]; r2[24 + e] = h2[e]; }
+    }
   }
 }
 
@@ -305,12 +398,21 @@ __device__ __forceinline__ bool epilogue_wait(uint64_t* bar, uint32_t parity, vo
   return done;
 }
 
+// How the CTAs that share a tile's reduction join their partial sums; this one does not split it.
+struct NoExchange {
+  static constexpr bool SPLIT = false;
+  __device__ __forceinline__ int first(int) const { return 0; }
+  __device__ __forceinline__ int step() const { return 1; }
+  __device__ __forceinline__ bool hand_over(uint32_t, int, int, int, int, int, int) { return true; }
+  __device__ __forceinline__ void add_peers(uint32_t (&)[32], int, int, int, int) const {}
+};
+
 // The epilogue of one tile for one warp: rows row0 .. row0 + 31 of the output, this warp's part of its BN columns.
 // `t_addr` addresses the tile's accumulator columns in the warp's own TMEM lanes; `wait()` returns once they are complete
 // (false: given up). `xslot` are the two warps' 2 x 32 float2 slots for joining row statistics, `parity` alternates per tile.
-template <int BN, int EPI, class Wait>
+template <int BN, int EPI, class Wait, class Exchange>
 __device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr, int row0, int tn, int half, int quarter, int lane,
-                                              int parity, float4* stage, Wait wait) {
+                                              int parity, float4* stage, Wait wait, Exchange&& ex) {
   const int n0 = tn * BN, row = row0 + lane;
   const bool row_ok = row < p.M;
   EpiOld old;
@@ -319,28 +421,36 @@ __device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr,
     // columns [0, 128) of the tile are gate, [128, 256) up, of hidden units tn * 128 ...: this warp takes 64 units.
     // (reference: chunk + silu * mul as separate passes, galvatron/core/runtime/tensor_parallel/transformer.py:122-124)
     if (!wait()) return false;
-#pragma unroll 1
-    for (int c = 2 * half; c < 2 * half + 2; ++c) {
-      uint32_t u[32];
-      __syncwarp();
-      tmem_ld_32x32b_x32(t_addr + c * 32, r);
-      tmem_ld_32x32b_x32(t_addr + (c + 4) * 32, u);
-      tmem_ld_wait();
-      const int unit0 = tn * 128 + c * 32;
-      epi_stage(r, stage, lane);
-      epi_store<true>(p, stage, row0, unit0, lane, old);
-      epi_stage(u, stage, lane);
-      epi_store<true>(p, stage, row0, p.swiglu_f + unit0, lane, old);
+    uint32_t g[32], u[32];                          // bf16 pairs of the 64 gate and the 64 up columns
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        // on the bf16-rounded values, like the stand-alone kernel that reads the stored projection
-        const float g = __bfloat162float(__float2bfloat16(__uint_as_float(r[i]) * p.alpha));
-        const float up = __bfloat162float(__float2bfloat16(__uint_as_float(u[i]) * p.alpha));
-        r[i] = __float_as_uint(g / (1.f + __expf(-g)) * up);
-      }
-      epi_stage(r, stage, lane);
-      epi_store_act(p, stage, row0, unit0, lane);
+    for (int h = 0; h < 2; ++h) {
+      __syncwarp();
+      tmem_ld_32x32b_x32(t_addr + (2 * half + h) * 32, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        g[16 * h + i] = pack_bf16x2(__uint_as_float(r[2 * i]) * p.alpha, __uint_as_float(r[2 * i + 1]) * p.alpha);
     }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      __syncwarp();
+      tmem_ld_32x32b_x32(t_addr + (4 + 2 * half + h) * 32, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        u[16 * h + i] = pack_bf16x2(__uint_as_float(r[2 * i]) * p.alpha, __uint_as_float(r[2 * i + 1]) * p.alpha);
+    }
+    const int unit0 = tn * 128 + half * 64;
+    __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C);
+    epi_put64(g, stage, lane, C, p.ldc, p.M, p.N, row0, unit0);
+    epi_put64(u, stage, lane, C, p.ldc, p.M, p.N, row0, p.swiglu_f + unit0);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      // on the bf16-rounded values, like the stand-alone kernel that reads the stored projection
+      const float2 gf = unpack_bf16x2(g[i]), uf = unpack_bf16x2(u[i]);
+      g[i] = pack_bf16x2(silu(gf.x) * uf.x, silu(gf.y) * uf.y);
+    }
+    epi_put64(g, stage, lane, p.act_out, p.ld_act, p.M, p.swiglu_f, row0, unit0);
     return true;
   } else if constexpr (EPI == EPI_XENT) {
     constexpr int CHUNKS = BN / 64;                       // of this warp
@@ -355,23 +465,28 @@ __device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr,
     float xm = -INFINITY, xl = 0.f;
     if (!wait()) return false;
 #pragma unroll 1
-    for (int c = c0; c < c0 + CHUNKS; ++c) {
-      const int col0 = n0 + c * 32;
-      if (col0 >= p.N) break;
-      __syncwarp();
-      tmem_ld_32x32b_x32(t_addr + c * 32, r);
-      tmem_ld_wait();
-      if (p.xent_mode == 1) {
-        if (row_ok) xent_stats_chunk(p, r, row, col0, lcol, xm, xl);
-      } else {
-        // gradient of the cross entropy w.r.t. the logits, straight from the recomputed fp32 logits
-        const int t = (lcol >= col0 && lcol < col0 + 32) ? static_cast<int>(lcol - col0) : -1;
+    for (int c = c0; c < c0 + CHUNKS; c += 2) {
+      if (n0 + c * 32 >= p.N) break;
+      uint32_t w[32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          r[i] = __float_as_uint((__expf(__uint_as_float(r[i]) * p.alpha - l) - (t == i ? 1.f : 0.f)) * g);
-        epi_stage(r, stage, lane);
-        epi_store<false>(p, stage, row0, col0, lane, old);
+      for (int h = 0; h < 2; ++h) {
+        const int col0 = n0 + (c + h) * 32;
+        __syncwarp();
+        tmem_ld_32x32b_x32(t_addr + (c + h) * 32, r);
+        tmem_ld_wait();
+        if (p.xent_mode == 1) {
+          if (row_ok && col0 < p.N) xent_stats_chunk(p, r, row, col0, lcol, xm, xl);
+        } else {
+          // gradient of the cross entropy w.r.t. the logits, straight from the recomputed fp32 logits
+          const int t = (lcol >= col0 && lcol < col0 + 32) ? static_cast<int>(lcol - col0) : -1;
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            w[16 * h + i] = pack_bf16x2((__expf(__uint_as_float(r[2 * i]) * p.alpha - l) - (t == 2 * i ? 1.f : 0.f)) * g,
+                                        (__expf(__uint_as_float(r[2 * i + 1]) * p.alpha - l) - (t == 2 * i + 1 ? 1.f : 0.f)) * g);
+        }
       }
+      if (p.xent_mode == 2)
+        epi_put64(w, stage, lane, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.M, p.N, row0, n0 + c * 32);
     }
     if (p.xent_mode == 1) {
       // the quarter's second warp hands its half of the statistics to the first; two slots, one barrier per tile: a slot
@@ -389,7 +504,8 @@ __device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr,
     }
     return true;
   } else {
-  if (p.rope_cols > 0) {
+  constexpr bool SPLIT = std::remove_reference<Exchange>::type::SPLIT;
+  if (!SPLIT && p.rope_cols > 0) {          // a split product has no rotary columns
     // q / k heads: a chunk and its partner half a head further right are rotated together
     const float pos = p.rope_pos ? (row_ok ? static_cast<float>(p.rope_pos[row]) : 0.f)
                                  : static_cast<float>((row / p.rope_pos_div) % p.rope_pos_mod + p.rope_pos_offset);
@@ -406,29 +522,51 @@ __device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr,
       const int col0 = n0 + c * 32;
       if (col0 < p.rope_cols) rope_rotate_chunks(p, r, u, pos, in_head * 32);
       epi_stage(r, stage, lane);
-      epi_store<false>(p, stage, row0, col0, lane, old);
+      epi_store(p, stage, row0, col0, lane, old);
       epi_stage(u, stage, lane);
-      epi_store<false>(p, stage, row0, col0 + hc * 32, lane, old);
+      epi_store(p, stage, row0, col0 + hc * 32, lane, old);
     }
     return true;
   }
   constexpr int CHUNKS = BN / 64;                         // of this warp
   const int c0 = half * CHUNKS;
   const bool has_old = epi_has_old(p);
-  if (has_old) epi_load_old(p, row0, n0 + c0 * 32, lane, old);
-  if (!wait()) return false;
+  if (!SPLIT && !has_old && !p.c_f32) {
+    if (!wait()) return false;
 #pragma unroll 1
-  for (int c = c0; c < c0 + CHUNKS; ++c) {
+    for (int c = c0; c < c0 + CHUNKS; c += 2) {
+      if (n0 + c * 32 >= p.N) break;
+      uint32_t w[32];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        __syncwarp();
+        tmem_ld_32x32b_x32(t_addr + (c + h) * 32, r);
+        tmem_ld_wait();
+        epi_pack32(p, r, n0 + (c + h) * 32, w + 16 * h);
+      }
+      epi_put64(w, stage, lane, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.M, p.N, row0, n0 + c * 32);
+    }
+    return true;
+  }
+  // chunks that this CTA finishes: all of them, or with a split reduction every ex.step-th
+  const int first = c0 + ex.first(c0), step = ex.step();
+  if (has_old) epi_load_old(p, row0, n0 + first * 32, lane, old);
+  if (!wait()) return false;
+  if (!ex.hand_over(t_addr, c0, CHUNKS, quarter, half, lane, parity)) return false;
+#pragma unroll 1
+  for (int c = first; c < c0 + CHUNKS; c += step) {
     const int col0 = n0 + c * 32;
     if (col0 >= p.N) break;
     __syncwarp();
     tmem_ld_32x32b_x32(t_addr + c * 32, r);
     EpiOld next;
-    if (has_old && c + 1 < c0 + CHUNKS) epi_load_old(p, row0, col0 + 32, lane, next);
+    if (!SPLIT && has_old && c + step < c0 + CHUNKS) epi_load_old(p, row0, n0 + (c + step) * 32, lane, next);
     tmem_ld_wait();
+    ex.add_peers(r, c, quarter, lane, parity);
+    if (SPLIT && has_old && c != first) epi_load_old(p, row0, col0, lane, old);
     epi_stage(r, stage, lane);
-    epi_store<false>(p, stage, row0, col0, lane, old);
-    old = next;
+    epi_store(p, stage, row0, col0, lane, old);
+    if (!SPLIT) old = next;
   }
   return true;
   }
@@ -565,7 +703,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t t_addr = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
       const bool ok = epilogue_tile<BN, EPI>(p, t_addr, tm * BM + quarter * 32, tn, half, quarter, lane, acc, stage_buf, [&] {
         return epilogue_wait(&acc_full[acc], acc_phase, abort_flag, 4);
-      });
+      }, NoExchange());
       if (!ok) break;
       __syncwarp();
       tc_fence_before();
@@ -599,10 +737,10 @@ constexpr int P_EPI_OFFSET = P_STAGES * P_STAGE_BYTES;
 constexpr int P_BAR_OFFSET = P_EPI_OFFSET + EPI_BYTES;
 constexpr int P_SMEM_TOTAL = P_BAR_OFFSET + 256 + 1024;
 
-// TMA tile load of this CTA's shared memory whose completion is counted on CTA 0's barrier (pair form of the load)
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* desc, uint64_t* bar, int32_t c0, int32_t c1) {
+// TMA tile load of this CTA's shared memory whose completion is counted on the barrier of the pair's even CTA (`leader`)
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* desc, uint64_t* bar, uint32_t leader, int32_t c0, int32_t c1) {
   uint32_t leader_bar;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(leader_bar) : "r"(smem_u32(bar)), "r"(0));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(leader_bar) : "r"(smem_u32(bar)), "r"(leader));
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       :
@@ -610,16 +748,79 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       : "memory");
 }
 // commit of the pair's MMAs: arrives on the same barrier in both CTAs
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t leader) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-      "h"(static_cast<uint16_t>(3))
+      "h"(static_cast<uint16_t>(3u << leader))
       : "memory");
 }
 
-template <bool A_MN, bool B_MN, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmDev p) {
+// Split reduction: the S pairs of a cluster of 2 S CTAs each multiply a part of K for the same 256 x 256 tile and then
+// join their sums. Chunk c of the tile (32 columns) is finished by the pair c % S; the other pairs leave theirs in `ws`
+// (global memory that stays in L2), arrive on the finisher's barrier, and the finisher adds them to its own in
+// pair order, so the result is repeatable. Two slots alternate: whoever writes a slot again has seen every pair arrive for the tile in
+// between, which each does after reading.
+constexpr int SPLIT_CHUNK = 256;                             // float4 of one 32 x 32 chunk, as [piece of 4 columns][row]
+constexpr int SPLIT_PART = 4 * 8 * SPLIT_CHUNK;              // of one CTA's 128 x 256 partial tile
+struct SplitExchange {
+  static constexpr bool SPLIT = true;
+  float4* ws;                // of this cluster and half: [slot][pair][quarter][chunk]
+  uint64_t* joined;          // [2] one per slot: 8 warps x (S - 1) pairs arrive
+  volatile uint32_t* abort_flag;
+  int S, rank;               // pairs of the cluster, and which one this is
+  uint32_t cta, phase[2];
+
+  __device__ __forceinline__ int first(int c0) const { return (rank - c0 % S + S) % S; }
+  __device__ __forceinline__ int step() const { return S; }
+  __device__ __forceinline__ float4* part(int pair, int c, int quarter, int slot) const {
+    return ws + static_cast<size_t>(slot * S + pair) * SPLIT_PART + (quarter * 8 + c) * SPLIT_CHUNK;
+  }
+  __device__ __forceinline__ bool hand_over(uint32_t t_addr, int c0, int chunks, int quarter, int half, int lane, int slot) {
+#pragma unroll 1
+    for (int c = c0; c < c0 + chunks; ++c) {
+      if (c % S == rank) continue;
+      uint32_t r[32];
+      __syncwarp();
+      tmem_ld_32x32b_x32(t_addr + c * 32, r);
+      tmem_ld_wait();
+      float4* dst = part(rank, c, quarter, slot) + lane;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        __stcg(dst + j * 32, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
+                                         __uint_as_float(r[4 * j + 3])));
+    }
+    __syncwarp();
+    if (lane < S && lane != rank) mbar_arrive_cluster(&joined[slot], 2 * lane + cta);
+    bool done = true;
+    if (threadIdx.x == 64) done = mbar_wait_cluster(&joined[slot], phase[slot], abort_flag, 9);
+    phase[slot] ^= 1;
+    return named_bar_all<1, 32 * EPI_WARPS>(done);
+  }
+  __device__ __forceinline__ void add_peers(uint32_t (&r)[32], int c, int quarter, int lane, int slot) const {
+#pragma unroll 1
+    for (int q = 0; q < S; ++q) {
+      if (q == rank) continue;
+      const float4* src = part(q, c, quarter, slot) + lane;
+      float4 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __ldcg(src + j * 32);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + v[j].x);
+        r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + v[j].y);
+        r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + v[j].z);
+        r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + v[j].w);
+      }
+    }
+  }
+};
+
+template <bool SPLIT> struct ExchangeOf { using type = NoExchange; };
+template <> struct ExchangeOf<true> { using type = SplitExchange; };
+
+// SPLIT: S pairs of the cluster share each tile; otherwise the cluster is one pair and S and ws are unused.
+template <bool A_MN, bool B_MN, int EPI, bool SPLIT>
+__device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmDev& p, int S, float4* ws) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + P_BAR_OFFSET);   // used in CTA 0 only
@@ -628,14 +829,20 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   uint64_t* acc_empty = acc_full + 2;                                       // [2], used in CTA 0 only (256 arrivals)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  uint64_t* joined = acc_empty + 4;                                         // [2], SPLIT only
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t cta = cluster_ctarank();               // 0: issues the MMAs; 1: peer
-  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const uint32_t cta_rank = cluster_ctarank(), cta = cta_rank & 1;          // 0: issues the pair's MMAs; 1: peer
+  const uint32_t leader = SPLIT ? cta_rank & ~1u : 0u;                       // rank of the pair's issuing CTA
+  // `pair`, `num_pairs`: the group of CTAs that works on one tile, and how many there are
+  const int pair = SPLIT ? blockIdx.x / (2 * S) : blockIdx.x >> 1, num_pairs = SPLIT ? gridDim.x / (2 * S) : gridDim.x >> 1;
   constexpr int TM = 2 * BM, TN = 256;
   const int num_m = (p.M + TM - 1) / TM, num_n = EPI == EPI_SWIGLU ? p.swiglu_f / 128 : (p.N + TN - 1) / TN;
   const int num_tiles = num_m * num_n;
-  const int num_kb = (p.K + BK - 1) / BK;
+  const int all_kb = (p.K + BK - 1) / BK;
+  const int split = static_cast<int>(cta_rank >> 1);
+  const int kb0 = SPLIT ? static_cast<int>(static_cast<long long>(all_kb) * split / S) : 0;
+  const int kb1 = SPLIT ? static_cast<int>(static_cast<long long>(all_kb) * (split + 1) / S) : all_kb;
   constexpr uint32_t TMEM_COLS = 2 * TN;
 
   if (threadIdx.x == 0) {
@@ -646,6 +853,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], 2 * 32 * EPI_WARPS);    // the epilogue threads of both CTAs
+    }
+    if constexpr (SPLIT) {
+      for (int a = 0; a < 2; ++a) mbar_init(&joined[a], EPI_WARPS * (S - 1));
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -674,7 +884,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const int m0 = tm * TM + static_cast<int>(cta) * BM;      // this CTA's rows of A and of the output
         // this CTA's 128 rows of B (columns of the output); gated mode: CTA 0 stages the gate rows, CTA 1 the up rows
         const int nb0 = EPI == EPI_SWIGLU ? tn * 128 + static_cast<int>(cta) * p.swiglu_f : tn * TN + static_cast<int>(cta) * BM;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, 5)) { ok = false; break; }
           uint8_t* sA = smem + stage * P_STAGE_BYTES;
           uint8_t* sB = sA + P_HALF_BYTES;
@@ -683,16 +893,16 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           // stage from the peer would put a cluster round trip into its producer loop.
           if (cta == 0) mbar_expect_tx(&full_bar[stage], 2 * P_STAGE_BYTES);
           if constexpr (!A_MN) {
-            tma_load_2d_pair(sA, &tmA, &full_bar[stage], kb * BK, m0);
+            tma_load_2d_pair(sA, &tmA, &full_bar[stage], leader, kb * BK, m0);
           } else {
 #pragma unroll
-            for (int q = 0; q < BM / 64; ++q) tma_load_2d_pair(sA + q * (BK * 128), &tmA, &full_bar[stage], m0 + q * 64, kb * BK);
+            for (int q = 0; q < BM / 64; ++q) tma_load_2d_pair(sA + q * (BK * 128), &tmA, &full_bar[stage], leader, m0 + q * 64, kb * BK);
           }
           if constexpr (!B_MN) {
-            tma_load_2d_pair(sB, &tmB, &full_bar[stage], kb * BK, nb0);
+            tma_load_2d_pair(sB, &tmB, &full_bar[stage], leader, kb * BK, nb0);
           } else {
 #pragma unroll
-            for (int q = 0; q < BM / 64; ++q) tma_load_2d_pair(sB + q * (BK * 128), &tmB, &full_bar[stage], nb0 + q * 64, kb * BK);
+            for (int q = 0; q < BM / 64; ++q) tma_load_2d_pair(sB + q * (BK * 128), &tmB, &full_bar[stage], leader, nb0 + q * 64, kb * BK);
           }
           if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
         }
@@ -714,18 +924,18 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, 6)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag, 7)) { ok = false; break; }
           tc_fence_after();
           const uint64_t so = static_cast<uint64_t>(stage) * (P_STAGE_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            umma_f16_ss<2>(d_tmem, a_desc0 + so + k * A_STEP, b_desc0 + so + k * B_STEP, idesc, (kb | k) != 0 ? 1u : 0u);
-          umma_commit_pair(&empty_bar[stage]);   // frees this stage in both CTAs once these MMAs retire
+            umma_f16_ss<2>(d_tmem, a_desc0 + so + k * A_STEP, b_desc0 + so + k * B_STEP, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+          umma_commit_pair(&empty_bar[stage], leader);   // frees this stage in both CTAs once these MMAs retire
           if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit_pair(&acc_full[acc]);
+        umma_commit_pair(&acc_full[acc], leader);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
@@ -736,6 +946,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     float4* stage_buf = reinterpret_cast<float4*>(smem + P_EPI_OFFSET + (warp - 2) * EPI_STAGE_BYTES);
     int acc = 0;
     uint32_t acc_phase = 0;
+    typename ExchangeOf<SPLIT>::type ex;
+    if constexpr (SPLIT)
+      ex = {ws + (static_cast<size_t>(pair) * 2 + cta) * 2 * S * SPLIT_PART, joined, abort_flag, S, split, cta, {0u, 0u}};
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       int tm, tn;
       tile_coords(tile, num_m, num_n, tm, tn);
@@ -743,11 +956,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const int row0 = tm * TM + static_cast<int>(cta) * BM + quarter * 32;
       const bool ok = epilogue_tile<TN, EPI>(p, t_addr, row0, tn, half, quarter, lane, acc, stage_buf, [&] {
         return epilogue_wait(&acc_full[acc], acc_phase, abort_flag, 8);
-      });
+      }, ex);
       if (!ok) break;
       __syncwarp();
       tc_fence_before();
-      mbar_arrive_cluster(&acc_empty[acc], 0);   // both CTAs report to the issuing CTA
+      mbar_arrive_cluster(&acc_empty[acc], leader);   // both CTAs report to the issuing CTA
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   }
@@ -759,6 +972,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     tc_fence_after();
     tmem_dealloc<2>(tmem_base, TMEM_COLS);
   }
+}
+
+template <bool A_MN, bool B_MN, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmDev p) {
+  pair_body<A_MN, B_MN, EPI, false>(tmA, tmB, p, 1, nullptr);
+}
+
+// Launched with clusters of 2 S CTAs.
+template <bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_bf16_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmDev p, int S, float4* ws) {
+  pair_body<A_MN, B_MN, EPI_LINEAR, true>(tmA, tmB, p, S, ws);
 }
 
 // ----------------------------------------------------------------------------------
@@ -888,9 +1114,9 @@ static int launch_gemm(const gv_gemm_args* a, cudaStream_t stream, const gv_xent
   return static_cast<int>(cudaGetLastError());
 }
 
-template <bool A_MN, bool B_MN, int EPI = EPI_LINEAR>
-static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv_xent_args* x = nullptr) {
-  CUtensorMap tmA, tmB;
+// Tensor maps and device parameters of a launch on CTA pairs: each CTA loads 128 of the 256 rows of either operand.
+template <bool A_MN, bool B_MN>
+static int fill_pair(const gv_gemm_args* a, const gv_xent_args* x, CUtensorMap& tmA, CUtensorMap& tmB, GemmDev& p) {
   int rc;
   if (!A_MN)
     rc = make_tmap_bf16_2d(&tmA, a->A, a->M, a->K, a->lda, 64, BM);
@@ -898,11 +1124,10 @@ static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv
     rc = make_tmap_bf16_2d(&tmA, a->A, a->K, a->M, a->lda, 64, BK);
   if (rc) return rc;
   if (!B_MN)
-    rc = make_tmap_bf16_2d(&tmB, a->B, a->N, a->K, a->ldb, 64, BM);   // each CTA of the pair loads 128 of the 256 B rows
+    rc = make_tmap_bf16_2d(&tmB, a->B, a->N, a->K, a->ldb, 64, BM);
   else
     rc = make_tmap_bf16_2d(&tmB, a->B, a->K, a->N, a->ldb, 64, BK);
   if (rc) return rc;
-  GemmDev p;
   p.C = a->C;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(a->bias);
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a->residual);
@@ -913,6 +1138,36 @@ static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv
   fill_xent(p, x, 256);
   fill_rope(p, a);
   fill_swiglu(p, a);
+  return 0;
+}
+
+// How many clusters of `ctas` CTAs with one CTA per SM the device holds at once. A persistent grid must not exceed it (a part
+// with an odd number of SMs enabled in some TPCs holds fewer than num_sms / ctas): what is left over would run as a second wave.
+template <class Kernel>
+static int resident_clusters(Kernel kern, int ctas) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(num_sms() / ctas * ctas));
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = P_SMEM_TOTAL;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(ctas); attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    n = num_sms() / ctas;
+  }
+  return n;
+}
+
+template <bool A_MN, bool B_MN, int EPI = EPI_LINEAR>
+static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv_xent_args* x = nullptr) {
+  CUtensorMap tmA, tmB;
+  GemmDev p;
+  const int rc = fill_pair<A_MN, B_MN>(a, x, tmA, tmB, p);
+  if (rc) return rc;
   auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, EPI>;
   static PerDeviceOnce smem_once;
   {
@@ -920,30 +1175,56 @@ static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   const int tiles = ((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + 255) / 256);
-  // A persistent grid must not exceed the number of CTA pairs the device can hold at once (a part with an odd number
-  // of SMs enabled in some TPCs holds fewer than num_sms / 2): the pairs left over would run as a second wave.
   static int max_pairs = 0;
-  if (max_pairs == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(num_sms() / 2 * 2));
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = P_SMEM_TOTAL;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      n = num_sms() / 2;
-    }
-    max_pairs = n;
-  }
-  int pairs = max_pairs;
-  if (tiles < pairs) pairs = tiles;
+  if (max_pairs == 0) max_pairs = resident_clusters(kern, 2);
+  const int pairs = tiles < max_pairs ? tiles : max_pairs;
   kern<<<2 * pairs, GEMM_THREADS, P_SMEM_TOTAL, stream>>>(tmA, tmB, p);
   return static_cast<int>(cudaGetLastError());
+}
+
+constexpr int MAX_SPLIT = 4;      // pairs per cluster: eight CTAs is the portable cluster size
+
+// Clusters of 2 S CTAs of the split kernel that fit at once (the four layouts need the same resources), for S = 2 .. 4.
+static int split_clusters(int S) {
+  static std::atomic<int> n[MAX_SPLIT + 1];
+  int v = n[S].load(std::memory_order_relaxed);
+  if (v == 0) {
+    auto kern = gemm_bf16_split_kernel<false, false>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_TOTAL) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    v = resident_clusters(kern, 2 * S);
+    n[S].store(v, std::memory_order_relaxed);
+  }
+  return v;
+}
+
+template <bool A_MN, bool B_MN>
+static int launch_gemm_split(const gv_gemm_args* a, cudaStream_t stream, int S) {
+  CUtensorMap tmA, tmB;
+  GemmDev p;
+  const int rc = fill_pair<A_MN, B_MN>(a, nullptr, tmA, tmB, p);
+  if (rc) return rc;
+  auto kern = gemm_bf16_split_kernel<A_MN, B_MN>;
+  static PerDeviceOnce smem_once;
+  {
+    cudaError_t e = ensure_max_dynamic_smem(smem_once, kern, P_SMEM_TOTAL);
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  const int tiles = ((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + 255) / 256);
+  const int clusters = tiles < split_clusters(S) ? tiles : split_clusters(S);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(2 * S * clusters));
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = P_SMEM_TOTAL;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(2 * S); attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, S, reinterpret_cast<float4*>(a->workspace)));
 }
 
 // GV_GEMM_PAIR: 0 never, 1 (default) when there is a 256 x 256 tile for every SM pair, 2 always (used by the
@@ -956,6 +1237,51 @@ static int pair_mode() {
     if (mode < 0 || mode > 2) mode = 1;
   }
   return mode;
+}
+
+// Narrow tiles when wide ones would leave most SMs idle.
+static bool narrow_tiles(const gv_gemm_args* a) {
+  return a->N <= 128 || static_cast<long>((a->M + BM - 1) / BM) * ((a->N + 255) / 256) < num_sms();
+}
+
+// Pairs per tile of the split kernel for this product, 1 = no split. The estimate counts waves of tiles: microseconds per
+// 64-deep k-block are 0.36 for a pair's 256 x 256 tile and 0.2 for a CTA's 128 x 128 tile (both measured at 8192 deep and
+// more), plus what joining the sums costs. Splitting pays where the last wave is nearly empty (75 tiles on 74 pairs: 2
+// waves, or 5 quarter waves) or where there is less than one wave of tiles; it must promise 7 %, since the estimate is no
+// better. GV_GEMM_SPLIT = 2 .. 4 forces that split (numerics tests), 1 turns it off.
+static int split_plan(const gv_gemm_args* a) {
+  static const int forced = [] {
+    const char* e = getenv("GV_GEMM_SPLIT");
+    return e && e[0] >= '1' && e[0] <= '4' ? e[0] - '0' : 0;
+  }();
+  if (forced == 1 || a->rope_cols > 0 || a->swiglu_out || a->M <= 0 || a->N <= 0 || a->K <= 0) return 1;
+  const int kb = (a->K + BK - 1) / BK;
+  if (forced) return kb >= forced ? forced : 1;
+  if (pair_mode() != 1 || kb < 16) return 1;
+  const long tiles = static_cast<long>((a->M + 255) / 256) * ((a->N + 255) / 256);
+  const long sms = num_sms();
+  const bool on_pairs = !narrow_tiles(a) && tiles >= sms / 2;
+  const long small = static_cast<long>((a->M + BM - 1) / BM) * ((a->N + BM - 1) / BM);
+  double best = on_pairs ? static_cast<double>((tiles + sms / 2 - 1) / (sms / 2)) * kb * 0.36
+                         : static_cast<double>((small + sms - 1) / sms) * kb * 0.2;
+  if (!on_pairs && !narrow_tiles(a)) return 1;       // 128 x 256 tiles on single CTAs: one and a half waves, left alone
+  best *= 0.93;
+  int S = 1;
+  for (int s = 2; s <= MAX_SPLIT; ++s) {
+    if (kb / s < 8) break;
+    const int c = split_clusters(s);
+    if (c <= 0) continue;
+    const double t = static_cast<double>((tiles + c - 1) / c) * ((kb + s - 1) / s) * 0.36 + 3.0 + s;
+    if (t < best) { best = t; S = s; }
+  }
+  return S;
+}
+
+// Two slots per cluster and half, S partial tiles of one CTA each.
+static long long split_bytes(const gv_gemm_args* a, int S) {
+  const long tiles = static_cast<long>((a->M + 255) / 256) * ((a->N + 255) / 256);
+  const long clusters = tiles < split_clusters(S) ? tiles : split_clusters(S);
+  return static_cast<long long>(clusters) * 2 * 2 * S * SPLIT_PART * 16;
 }
 
 }  // namespace gv
@@ -984,10 +1310,20 @@ extern "C" int gv_gemm_bf16(const gv_gemm_args* a, gv_stream_t s) {
     if (pair_mode() != 0 && (pair_mode() == 2 || pair_tiles >= num_sms() / 2)) return launch_gemm_pair<false, false, EPI_SWIGLU>(a, stream);
     return launch_gemm<256, false, false, EPI_SWIGLU>(a, stream);
   }
-  // Narrow tiles when wide ones would leave most SMs idle.
-  const long tiles256 = static_cast<long>((a->M + BM - 1) / BM) * ((a->N + 255) / 256);
-  const bool narrow = (a->N <= 128) || (tiles256 < num_sms());
   const int key = (a->a_mn_major ? 2 : 0) | (a->b_mn_major ? 1 : 0);
+  if (a->workspace != nullptr) {
+    const int S = split_plan(a);
+    if (S > 1) {
+      if (a->workspace_bytes < split_bytes(a, S) || (reinterpret_cast<uintptr_t>(a->workspace) & 15)) return 2008;
+      switch (key) {
+        case 0: return launch_gemm_split<false, false>(a, stream, S);
+        case 1: return launch_gemm_split<false, true>(a, stream, S);
+        case 2: return launch_gemm_split<true, false>(a, stream, S);
+        default: return launch_gemm_split<true, true>(a, stream, S);
+      }
+    }
+  }
+  const bool narrow = narrow_tiles(a);
   // K-major operands and enough 256 x 256 tiles for every SM pair: the two-CTA kernel
   if (pair_mode() != 0) {
     const long pair_tiles = static_cast<long>((a->M + 255) / 256) * ((a->N + 255) / 256);
@@ -1015,6 +1351,11 @@ extern "C" int gv_gemm_bf16(const gv_gemm_args* a, gv_stream_t s) {
       default: return launch_gemm<128, true, true>(a, stream);
     }
   }
+}
+
+extern "C" long long gv_gemm_workspace_bytes(const gv_gemm_args* a) {
+  const int S = gv::split_plan(a);
+  return S > 1 ? gv::split_bytes(a, S) : 0;
 }
 
 // Language-model head with the cross entropy in the GEMM epilogue. Always runs the 256-column-wide tiles, so the

@@ -52,8 +52,15 @@ typedef struct {
   // silu(gate) * up. Needs K-major A and B, bf16 C, no bias / residual / activation / accumulate.
   void* swiglu_out;
   int swiglu_ld;
+  // Scratch for a split reduction (NULL: the reduction is not split): gv_gemm_workspace_bytes of the same arguments,
+  // 16-byte aligned, uninitialised, in use until the launch has finished.
+  void* workspace;
+  long long workspace_bytes;
 } gv_gemm_args;
 int gv_gemm_bf16(const gv_gemm_args* args, gv_stream_t stream);
+// Bytes of scratch with which gv_gemm_bf16 would split this product's reduction over several CTA pairs per tile; 0 when it
+// would not. Depends on sizes and options only, not on addresses.
+long long gv_gemm_workspace_bytes(const gv_gemm_args* args);
 
 // Language-model head GEMM (logits = A * B^T, both K-major) with the cross entropy in its epilogue; the logits
 // themselves are never stored.

@@ -146,6 +146,38 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// The same for a barrier that other CTAs of the cluster arrive on after writing global memory: what they wrote before
+// their arrival is visible afterwards.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
+                                          unsigned int site) {
+  uint32_t addr = smem_u32(bar);
+  uint32_t ok = 0;
+  uint64_t t0 = 0;
+  for (uint32_t spin = 0;; ++spin) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((spin & 0xff) == 0xff) {
+      if (*abort_flag) return false;
+      uint64_t now = global_timer_ns();
+      if (t0 == 0) {
+        t0 = now;
+      } else if (now - t0 > GV_WAIT_NS) {
+        *abort_flag = 1;
+        record_error((site << 16) | 1u, parity, spin);
+        return false;
+      }
+    }
+  }
+}
+
 // ----------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies). Loads complete on an mbarrier; stores use bulk groups.
 // ----------------------------------------------------------------------------

@@ -17,7 +17,7 @@ _LIB = None
 
 # Kernel launches per library call (for launch accounting in benchmarks).
 KERNELS_PER_CALL = {"gv_attn_bwd": 3, "gv_read_error": 0, "gv_norm_bwd_scratch_elems": 0, "gv_rmsnorm_bwd": 2,
-                    "gv_layernorm_bwd": 2, "gv_device_sm_count": 0}
+                    "gv_layernorm_bwd": 2, "gv_device_sm_count": 0, "gv_gemm_workspace_bytes": 0}
 LAUNCH_COUNT = 0
 
 
@@ -57,6 +57,7 @@ class GemmArgs(Structure):
         ("rope_cols", c_int), ("rope_dh", c_int), ("rope_inv_freq", c_void_p), ("rope_pos", c_void_p),
         ("rope_pos_div", c_int), ("rope_pos_mod", c_int), ("rope_pos_offset", c_int),
         ("swiglu_out", c_void_p), ("swiglu_ld", c_int),
+        ("workspace", c_void_p), ("workspace_bytes", c_longlong),
     ]
 
 
@@ -130,6 +131,8 @@ def lib():
         cdll.gv_gemm_bf16.restype = c_int
         cdll.gv_gemm_xent.argtypes = [POINTER(GemmArgs), POINTER(XentArgs), c_void_p]
         cdll.gv_gemm_xent.restype = c_int
+        cdll.gv_gemm_workspace_bytes.argtypes = [POINTER(GemmArgs)]
+        cdll.gv_gemm_workspace_bytes.restype = c_longlong
         for name, types in PROTOTYPES.items():
             getattr(cdll, name).argtypes = types
             getattr(cdll, name).restype = c_longlong if name == "gv_norm_bwd_scratch_elems" else c_int

@@ -7,6 +7,8 @@ transpose (reference: megatron/core/tensor_parallel/layers.py:417,462,534).
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import _lib
@@ -41,6 +43,12 @@ class RopeEpilogue:
     @staticmethod
     def supported(x: torch.Tensor, dh: int, bias) -> bool:
         return x.is_cuda and x.dtype == torch.bfloat16 and dh in (64, 128) and bias is None
+
+
+@functools.lru_cache(maxsize=1024)
+def _workspace_bytes(M: int, N: int, K: int) -> int:
+    """Scratch of a split reduction for a product of these sizes (at most 38 MB); 0: not split."""
+    return _lib.lib().gv_gemm_workspace_bytes(_lib.GemmArgs(M=M, N=N, K=K))
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,
@@ -88,6 +96,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             args.rope_inv_freq = rope.inv_freq.data_ptr()
             args.rope_pos = _lib.p(rope.positions) or None
             args.rope_pos_div, args.rope_pos_mod, args.rope_pos_offset = rope.pos_div, 0, rope.pos_offset
+        elif swiglu_out is None:
+            need = _workspace_bytes(M, N, K)
+            if need:
+                try:
+                    scratch = torch.empty(need, dtype=torch.uint8, device=a.device)
+                    args.workspace, args.workspace_bytes = scratch.data_ptr(), need
+                except torch.cuda.OutOfMemoryError:
+                    pass                    # no room for the partial sums: the product runs unsplit
         _lib.check(_lib.lib().gv_gemm_bf16(args, _lib.stream_ptr()), "gv_gemm_bf16")
         return out
     if rope is not None or swiglu_out is not None:

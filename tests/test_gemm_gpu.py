@@ -164,6 +164,31 @@ def test_pair_kernel_matches_fp32_reference():
         assert v < 1e-2, (k, v, res)
 
 
+@pytest.mark.parametrize("split", [2, 3, 4])
+def test_split_reduction_matches_fp32_reference(split):
+    """The reduction of every product shared by ``split`` CTA pairs per tile: the same shapes, layouts and epilogues (tails
+    of M, N and K, one tile, several tiles per cluster, fewer k-blocks than pairs), and bit-equal repeats."""
+    import json
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    extra = """
+from hetu_galvatron_b200.ops.gemm import _workspace_bytes
+assert _workspace_bytes(4096, 2048, 512) > 0 and _workspace_bytes(256, 256, 64) == 0
+a, w = torch.randn(300, 4160, device="cuda", dtype=torch.bfloat16), torch.randn(776, 4160, device="cuda", dtype=torch.bfloat16)
+first = gemm(a, w, out_dtype=torch.float32)
+assert all(torch.equal(gemm(a, w, out_dtype=torch.float32), first) for _ in range(3))
+"""
+    env = dict(os.environ, GV_GEMM_SPLIT=str(split))
+    r = subprocess.run([sys.executable, "-c", PAIR_SCRIPT % root + extra], capture_output=True, text=True, timeout=300, env=env)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
+    res = json.loads([l for l in r.stdout.splitlines() if l.startswith("PAIR ")][0][5:])
+    assert res.pop("error") is None
+    for k, v in res.items():
+        assert v < 1e-2, (k, v, res)
+
+
 @pytest.mark.parametrize("M,V,K,vocab_start", [(256, 1000, 256, 0), (300, 4096, 512, 4096), (8192, 32000, 1024, 0), (128, 264, 64, 0)])
 def test_lm_head_cross_entropy_epilogues(M, V, K, vocab_start):
     """Head GEMM whose epilogue computes the cross-entropy statistics (no logits stored), and its backward twin whose
@@ -245,3 +270,40 @@ def test_up_projection_with_gated_activation_epilogue(M, f, K):
     assert (act.float() - ref32).abs().max().item() < 3e-2 * ref32.abs().max().item()
     torch.cuda.synchronize()
     assert _lib.read_error() is None
+
+
+@pytest.mark.parametrize("largest", [100, 65536, 3000000])
+@pytest.mark.parametrize("M,dh", [(40, 64), (300, 128), (9500, 64)])
+def test_rotary_epilogue_positions(M, dh, largest):
+    """Explicit positions on either side of the limit of the branch-free sines, against the rotation in 64 bits of the same
+    fp32 angles; odd row counts, single CTAs and pairs."""
+    from hetu_galvatron_b200.ops.gemm import RopeEpilogue
+    g = torch.Generator(device="cuda").manual_seed(M + dh)
+    x = torch.randn(M, 64, device="cuda", dtype=torch.bfloat16, generator=g)
+    w = torch.randn(4 * dh, 64, device="cuda", dtype=torch.bfloat16, generator=g)
+    pos = torch.randint(0, largest + 1, (M,), device="cuda", dtype=torch.int32, generator=g)
+    freq = 1.0 / (10000.0 ** (torch.arange(0, dh, 2, device="cuda").float() / dh))
+    y = gemm(x, w, rope=RopeEpilogue(3 * dh, dh, freq, pos)).double().view(M, 4, dh)
+    h = (x.double() @ w.double().t()).view(M, 4, dh)
+    ang = (pos.float()[:, None] * freq[None]).double()[:, None]
+    a, b = h[:, :3, :dh // 2], h[:, :3, dh // 2:]
+    ref = torch.cat([a * ang.cos() - b * ang.sin(), b * ang.cos() + a * ang.sin()], -1)
+    # bf16 rounding of the result, fp32 sums of 64 products, sines to 1e-7
+    bound = 2.0 ** -8 * ref.abs() + 1e-5 * (a.abs() + b.abs() + 1).repeat(1, 1, 2)
+    assert ((y[:, :3] - ref).abs() <= bound).all()
+    assert ((y[:, 3] - h[:, 3]).abs() <= 2.0 ** -8 * h[:, 3].abs() + 1e-5).all()
+    assert _lib.read_error() is None
+
+
+def test_gated_activation_extremes():
+    """Gates far outside the range of exp: silu goes to 0 on the left and to the gate itself on the right."""
+    f, K = 128, 8
+    x = torch.zeros(130, K, device="cuda", dtype=torch.bfloat16)
+    x[:, 0] = torch.linspace(-200, 200, 130, device="cuda")
+    w = torch.zeros(2 * f, K, device="cuda", dtype=torch.bfloat16)
+    w[:, 0] = 1.0
+    act = torch.empty(130, f, device="cuda", dtype=torch.bfloat16)
+    gemm(x, w, swiglu_out=act)
+    v = x[:, :1].double()
+    ref = v * torch.sigmoid(v) * v
+    assert ((act.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-30).all()
