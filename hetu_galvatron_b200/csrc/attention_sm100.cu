@@ -12,8 +12,8 @@
 //
 // Backward: one CTA = 128 KV rows of one (batch, kv head); it loops over the query heads of its group and
 // over 64-row query blocks, holding dK and dV in TMEM. Per block: S^T = K Q^T, dP^T = V dO^T (TMEM),
-// P^T and dS^T are written to shared memory by two epilogue warpgroups, dV += P^T dO, dK += dS^T Q,
-// dQ^T = K^T dS^T is read back from TMEM and added into an fp32 dQ buffer with coalesced reductions.
+// two epilogue warpgroups write P^T back to TMEM and dS^T to shared memory, dV += P^T dO, dK += dS^T Q,
+// dQ^T = K^T dS^T is read back from TMEM and added into an fp32 dQ buffer with bulk reductions.
 // Every operand is consumed in the layout it has in shared memory (K-major or MN-major descriptors).
 #include "include/gv_kernels.h"
 #include "include/gv_host.h"
@@ -84,6 +84,23 @@ __device__ __forceinline__ bool drop_keep(uint32_t bh_key, int q, int k, uint32_
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
 
+// Which (tile of `tiles`, head-and-batch of `heads`) a block works on. Causal tiles differ in length: the hardware starts blocks
+// in order of their index, so tiles of several heads are interleaved, longest first, in groups of `group` heads. One head
+// after the other (group 1) left SMs idle at the end, since a long tile of the last head started late: 16 heads of 2048 tokens
+// ran 182 units of work on the busiest SM for a mean of 159, eight heads interleaved 164. About 256 (backward) or 512
+// (forward, two blocks per SM) tiles per group keep a group's operands within L2.
+__device__ __forceinline__ void tile_of_block(int block, int tiles, int heads, int group, int& tile, int& head) {
+  const int g0 = block / (group * tiles) * group;
+  const int n = min(group, heads - g0), r = block - g0 * tiles;
+  tile = r / n;
+  head = g0 + r % n;
+}
+static int tile_group(bool causal, int tiles, int heads, int per_group) {
+  if (!causal) return 1;                        // equal lengths: neighbours share K and V (or Q and dO) in L2
+  const int g = (per_group + tiles - 1) / tiles;
+  return g < heads ? g : heads;
+}
+
 // =====================================================================================
 // Forward
 // =====================================================================================
@@ -116,6 +133,7 @@ struct FwdParams {
   int b, sq, sk, hq, hk, dh;
   long long o_sb, o_ss, o_sh;
   int causal;
+  int tile_group;              // see tile_of_block
   float scale_log2;
   // BIAS instantiation only (each may be null): bias bf16 [hq, sq, bias_ld], additive mask fp32 [mask_n, sq, bias_ld],
   // group ids int32 [mask_n, bias_ld]
@@ -157,8 +175,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_q_tiles = (p.sq + FWD_BM - 1) / FWD_BM;
-  const int q_tile = num_q_tiles - 1 - blockIdx.x;  // heavy (late) causal tiles first
-  const int head = blockIdx.y, batch = blockIdx.z;
+  int q_tile, head_batch;
+  tile_of_block(blockIdx.x, num_q_tiles, p.hq * p.b, p.tile_group, q_tile, head_batch);
+  q_tile = num_q_tiles - 1 - q_tile;                // long (late) causal tiles first
+  const int head = head_batch % p.hq, batch = head_batch / p.hq;
   const int kv_head = head / (p.hq / p.hk);
   const int q0 = q_tile * FWD_BM;
   const int shift = p.sk - p.sq;  // causal: query i sees keys <= i + shift
@@ -455,15 +475,21 @@ constexpr int BWD_THREADS = 64 + 256;
 constexpr int BWD_QSTAGES = 3;
 
 // Two (kv tile, q block) iterations are in flight per CTA: epilogue group 0 (warps 2-5) owns the even iterations,
-// group 1 (warps 6-9) the odd ones, each with its own S / dP accumulators in TMEM and its own P^T / dS^T tile in
-// shared memory, so the tensor cores work for one group while the other does its exponentials.
-// TMEM (512 columns): group g: S^T at g*128 (reused for dQ^T once P^T has been extracted), dP^T at g*128 + 64;
+// group 1 (warps 6-9) the odd ones, each with its own accumulators in TMEM, so the tensor cores work for one group while
+// the other does its exponentials. Within a group the steps of neighbouring iterations overlap too: P is computed as soon as
+// S is there and goes back to TMEM, where it is the A operand of dV += P^T dO (no shared memory, no fence); S of the next
+// iteration follows that product, so the group finds it ready when it has written dS; and the dQ block of an iteration is
+// read back between P and dS of the next one, when its products have long finished.
+// TMEM (512 columns): group g: S^T at g*128, overwritten by P^T (bf16, 32 columns); dP^T at g*128 + 64, overwritten by dQ^T;
 // dV at 256, dK at 384.
 struct BwdSmem {
   static constexpr int K_BYTES = BWD_BKV * BWD_DH * 2;   // 32 KB, 2 panels of [128 x 128 B]
   static constexpr int Q_BYTES = BWD_BQ * BWD_DH * 2;    // 16 KB, 2 panels of [64 x 128 B]
-  static constexpr int PT_BYTES = BWD_BKV * BWD_BQ * 2;  // 16 KB, 1 panel of [128 x 128 B]
-  static constexpr int R_BYTES = 2 * PT_BYTES;           // per group: P^T | dS^T, later the dQ block [64][dh] fp32
+  static constexpr int DS_BYTES = BWD_BKV * BWD_BQ * 2;  // 16 KB, 1 panel of [128 x 128 B]
+  // per group: 16 KB for the dQ block [64][dh] fp32 on its way out, then dS^T; a head size above 64 makes the block 32 KB,
+  // and its second half of the rows goes where the (consumed) dS^T was
+  static constexpr int OFF_DS_IN_R = 32 * BWD_DH * 4;
+  static constexpr int R_BYTES = OFF_DS_IN_R + DS_BYTES;
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = K_BYTES;
   static constexpr int OFF_Q = 2 * K_BYTES;                       // [BWD_QSTAGES]
@@ -491,6 +517,7 @@ struct BwdParams {
   long long dk_sb, dk_ss, dk_sh;
   long long dv_sb, dv_ss, dv_sh;
   int causal;
+  int tile_group;              // see tile_of_block
   float scale;
   float scale_log2;
   // BIAS instantiation only (each may be null): transposed bias bf16 [hq, sk, bias_ld], additive mask fp32
@@ -520,13 +547,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* stat_full = bars + 7;   // [3]
   // per group g (7 barriers each, starting at 10 + 7 g)
   auto gbar = [&](int g, int which) { return bars + 10 + 7 * g + which; };
-  enum { B_S_FULL = 0, B_DP_FULL, B_PT_FULL, B_DS_FULL, B_DQ_FULL, B_S_FREE, B_DP_FREE };
+  enum { B_S_FULL = 0, B_DP_FULL, B_PT_FULL, B_DS_FULL, B_DQ_FULL, B_PV_DONE, B_DP_FREE };
   uint64_t* all_done = bars + 24;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kv_tile = blockIdx.x, kv_head = blockIdx.y, batch = blockIdx.z;
+  int kv_tile, head_batch;
+  tile_of_block(blockIdx.x, (p.sk + BWD_BKV - 1) / BWD_BKV, p.hk * p.b, p.tile_group, kv_tile, head_batch);
+  const int kv_head = head_batch % p.hk, batch = head_batch / p.hk;
   const int kv0 = kv_tile * BWD_BKV;
   const int rep = p.hq / p.hk;
   const int shift = p.sk - p.sq;
@@ -556,7 +585,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(gbar(g, B_PT_FULL), 128);
       mbar_init(gbar(g, B_DS_FULL), 128);
       mbar_init(gbar(g, B_DQ_FULL), 1);
-      mbar_init(gbar(g, B_S_FREE), 128);
+      mbar_init(gbar(g, B_PV_DONE), 1);
       mbar_init(gbar(g, B_DP_FREE), 128);
     }
     mbar_init(all_done, 1);
@@ -620,7 +649,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       constexpr uint32_t idesc_dq = make_idesc_bf16(BWD_DH, BWD_BQ, 1, 1);    // dQ^T: A=K (MN-major), B=dS^T (MN-major)
       // Base descriptors, built once (an operand advances by adding (bytes >> 4)): K and V as K-major A operands, K
       // again as the MN-major A operand of dQ^T; Q / dO per ring stage as K-major B (S^T, dP^T) and MN-major B (dK, dV);
-      // P^T / dS^T per group as K-major A (dV, dK) and dS^T as MN-major B (dQ^T).
+      // dS^T per group as K-major A (dK) and as MN-major B (dQ^T). P^T, the A operand of dV, is read from TMEM.
       const uint64_t k_kmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_K), 0, 1024);
       const uint64_t v_kmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_V), 0, 1024);
       const uint64_t k_mnmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_K), BWD_BKV * 128, 1024);
@@ -628,49 +657,58 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint64_t do_kmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_DO), 0, 1024);
       const uint64_t q_mnmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_Q), BWD_BQ * 128, 1024);
       const uint64_t do_mnmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_DO), BWD_BQ * 128, 1024);
-      const uint64_t pt_kmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_R), 0, 1024);
-      const uint64_t dst_kmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_R + S::PT_BYTES), 0, 1024);
-      const uint64_t dst_mnmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_R + S::PT_BYTES), BWD_BKV * 128, 1024);
+      const uint64_t dst_kmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_R + S::OFF_DS_IN_R), 0, 1024);
+      const uint64_t dst_mnmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_R + S::OFF_DS_IN_R), BWD_BKV * 128, 1024);
       constexpr uint64_t Q_STEP = S::Q_BYTES >> 4, R_STEP = S::R_BYTES >> 4;
       bool dv_started = false, dk_started = false;
-      // A(it): S^T = K Q^T and dP^T = V dO^T of iteration `it` into its group's accumulators
-      auto issue_a = [&](int it) {
+      // S^T = K Q^T and dP^T = V dO^T of iteration `it` into its group's accumulators
+      auto issue_s = [&](int it) {
         const int g = it & 1, st = it % BWD_QSTAGES;
-        const uint64_t qd = q_kmaj0 + st * Q_STEP, dod = do_kmaj0 + st * Q_STEP;
-        const uint32_t d_s = tmem_base + g * 128;
+        const uint64_t qd = q_kmaj0 + st * Q_STEP;
 #pragma unroll
         for (int kk = 0; kk < BWD_DH / 16; ++kk) {
           if (kk >= ksteps) break;
           const uint64_t da = k_kmaj + static_cast<uint64_t>(((kk >> 2) * (BWD_BKV * 128) + (kk & 3) * 32) >> 4);
           const uint64_t db = qd + static_cast<uint64_t>(((kk >> 2) * (BWD_BQ * 128) + (kk & 3) * 32) >> 4);
-          umma_f16_ss<1>(d_s, da, db, idesc_st, kk != 0 ? 1u : 0u);
+          umma_f16_ss<1>(tmem_base + g * 128, da, db, idesc_st, kk != 0 ? 1u : 0u);
         }
         umma_commit<1>(gbar(g, B_S_FULL));
+      };
+      auto issue_dp = [&](int it) {
+        const int g = it & 1, st = it % BWD_QSTAGES;
+        const uint64_t dod = do_kmaj0 + st * Q_STEP;
 #pragma unroll
         for (int kk = 0; kk < BWD_DH / 16; ++kk) {
           if (kk >= ksteps) break;
           const uint64_t da = v_kmaj + static_cast<uint64_t>(((kk >> 2) * (BWD_BKV * 128) + (kk & 3) * 32) >> 4);
           const uint64_t db = dod + static_cast<uint64_t>(((kk >> 2) * (BWD_BQ * 128) + (kk & 3) * 32) >> 4);
-          umma_f16_ss<1>(d_s + 64, da, db, idesc_st, kk != 0 ? 1u : 0u);
+          umma_f16_ss<1>(tmem_base + g * 128 + 64, da, db, idesc_st, kk != 0 ? 1u : 0u);
         }
         umma_commit<1>(gbar(g, B_DP_FULL));
       };
-      // B(it): dV += P^T dO (reduction over the 64 query rows)
-      auto issue_b = [&](int it) {
+      // dV += P^T dO (reduction over the 64 query rows: 8 columns of P^T hold 16 of them)
+      auto issue_dv = [&](int it) {
         const int g = it & 1, st = it % BWD_QSTAGES;
-        const uint64_t ptd = pt_kmaj0 + g * R_STEP, dod = do_mnmaj0 + st * Q_STEP;
+        const uint64_t dod = do_mnmaj0 + st * Q_STEP;
 #pragma unroll
-        for (int kk = 0; kk < BWD_BQ / 16; ++kk) {
-          const uint64_t da = ptd + static_cast<uint64_t>((kk * 32) >> 4);
-          const uint64_t db = dod + static_cast<uint64_t>((kk * 2048) >> 4);
-          umma_f16_ss<1>(tmem_base + TM_DV, da, db, idesc_dv, (dv_started || kk != 0) ? 1u : 0u);
-        }
+        for (int kk = 0; kk < BWD_BQ / 16; ++kk)
+          umma_f16_ts(tmem_base + TM_DV, tmem_base + g * 128 + kk * 8, dod + static_cast<uint64_t>((kk * 2048) >> 4), idesc_dv,
+                      (dv_started || kk != 0) ? 1u : 0u);
         dv_started = true;
+        umma_commit<1>(gbar(g, B_PV_DONE));
       };
-      // C(it): dK += dS^T Q ; dQ^T = K^T dS^T into the group's S columns (P^T has been extracted by then)
+      // dK += dS^T Q ; dQ^T = K^T dS^T into the group's dP columns (the group has read dP by then)
       auto issue_c = [&](int it) {
         const int g = it & 1, st = it % BWD_QSTAGES;
         const uint64_t dsd = dst_kmaj0 + g * R_STEP, dsd_mn = dst_mnmaj0 + g * R_STEP, qd = q_mnmaj0 + st * Q_STEP;
+#pragma unroll
+        for (int kk = 0; kk < BWD_BKV / 16; ++kk) {
+          // A = K as [M = dh, K = kv]: MN-major, dh panels 128 rows * 128 B apart, 16 kv rows per step;
+          // B = dS^T as [N = q, K = kv]: MN-major, a single 64-wide panel
+          const uint64_t da = k_mnmaj + static_cast<uint64_t>((kk * 2048) >> 4);
+          const uint64_t db = dsd_mn + static_cast<uint64_t>((kk * 2048) >> 4);
+          umma_f16_ss<1>(tmem_base + g * 128 + 64, da, db, idesc_dq, kk != 0 ? 1u : 0u);
+        }
 #pragma unroll
         for (int kk = 0; kk < BWD_BQ / 16; ++kk) {
           const uint64_t da = dsd + static_cast<uint64_t>((kk * 32) >> 4);
@@ -678,21 +716,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           umma_f16_ss<1>(tmem_base + TM_DK, da, db, idesc_dv, (dk_started || kk != 0) ? 1u : 0u);
         }
         dk_started = true;
-#pragma unroll
-        for (int kk = 0; kk < BWD_BKV / 16; ++kk) {
-          // A = K as [M = dh, K = kv]: MN-major, dh panels 128 rows * 128 B apart, 16 kv rows per step;
-          // B = dS^T as [N = q, K = kv]: MN-major, a single 64-wide panel
-          const uint64_t da = k_mnmaj + static_cast<uint64_t>((kk * 2048) >> 4);
-          const uint64_t db = dsd_mn + static_cast<uint64_t>((kk * 2048) >> 4);
-          umma_f16_ss<1>(tmem_base + g * 128, da, db, idesc_dq, kk != 0 ? 1u : 0u);
-        }
+        // one commit for both: the group overwrites dS^T once it has seen the dQ block
         umma_commit<1>(gbar(g, B_DQ_FULL));
         umma_commit<1>(&qdo_empty[st]);
       };
       bool ok = n_iter == 0 || mbar_wait(kv_full, 0, abort_flag, 0x22);
-      // next iteration to issue per kind: A in global order (a ring stage must not be probed two uses ahead),
-      // B and C in order within each group
-      int next_a = 0, next_b[2] = {0, 1}, next_c[2] = {0, 1};
+      // next iteration to issue per kind: S and dP in global order (a ring stage must not be probed two uses ahead),
+      // the others in order within each group
+      int next_s = 0, next_dp = 0, next_dv[2] = {0, 1}, next_c[2] = {0, 1};
       uint32_t idle = 0;
       uint64_t t0 = 0;
       while (ok && (next_c[0] < n_iter || next_c[1] < n_iter)) {
@@ -700,29 +731,39 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
           int it = next_c[g];
-          if (it < n_iter && next_b[g] > it && mbar_test(gbar(g, B_DS_FULL), (it >> 1) & 1)) {
+          if (it < n_iter && next_dp > it && next_dv[g] > it && mbar_test(gbar(g, B_DS_FULL), (it >> 1) & 1)) {
             tc_fence_after();
             issue_c(it);
             next_c[g] += 2;
             progress = true;
           }
-          it = next_b[g];
-          if (it < n_iter && next_a > it && mbar_test(gbar(g, B_PT_FULL), (it >> 1) & 1)) {
+          it = next_dv[g];
+          if (it < n_iter && next_s > it && mbar_test(gbar(g, B_PT_FULL), (it >> 1) & 1)) {
             tc_fence_after();
-            issue_b(it);
-            next_b[g] += 2;
+            issue_dv(it);
+            next_dv[g] += 2;
             progress = true;
           }
         }
-        if (next_a < n_iter) {
-          const int it = next_a, g = it & 1, j = it >> 1, st = it % BWD_QSTAGES;
+        if (next_dp < next_s) {
+          const int it = next_dp, g = it & 1, j = it >> 1;
+          // the group's dQ block of its previous iteration has left these columns
+          if (j == 0 || (next_c[g] >= it && mbar_test(gbar(g, B_DP_FREE), (j - 1) & 1))) {
+            tc_fence_after();
+            issue_dp(it);
+            ++next_dp;
+            progress = true;
+          }
+        }
+        if (next_s < n_iter) {
+          const int it = next_s, g = it & 1, j = it >> 1, st = it % BWD_QSTAGES;
           bool ready = mbar_test(&qdo_full[st], (it / BWD_QSTAGES) & 1);
-          if (ready && j > 0)
-            ready = mbar_test(gbar(g, B_S_FREE), (j - 1) & 1) && mbar_test(gbar(g, B_DP_FREE), (j - 1) & 1);
+          // dV of the group's previous iteration has read P^T out of these columns
+          if (ready && j > 0) ready = next_dv[g] >= it && mbar_test(gbar(g, B_PV_DONE), (j - 1) & 1);
           if (ready) {
             tc_fence_after();
-            issue_a(it);
-            ++next_a;
+            issue_s(it);
+            ++next_s;
             progress = true;
           }
         }
@@ -736,7 +777,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             t0 = now;
           } else if (now - t0 > GV_WAIT_NS) {
             *abort_flag = 1;
-            record_error((0x30u << 16) | 1u, static_cast<unsigned>(next_a), static_cast<unsigned>(next_c[0]));
+            record_error((0x30u << 16) | 1u, static_cast<unsigned>(next_s), static_cast<unsigned>(next_c[0]));
             ok = false;
             break;
           }
@@ -753,124 +794,201 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t tm_s = tmem_base + lane_off + g * 128, tm_dp = tm_s + 64;
     uint8_t* region = smem + S::OFF_R + g * S::R_BYTES;
-    uint8_t* pt_row = region + rloc * 128;
-    uint8_t* dst_row = region + S::PT_BYTES + rloc * 128;
+    uint8_t* dst_row = region + S::OFF_DS_IN_R + rloc * 128;
+    const int half_rows = p.dh <= 64 ? 32 * p.dh : S::OFF_DS_IN_R / 4;   // floats between the two halves of a dQ block
     float* dq_stage = reinterpret_cast<float*>(region);
     const bool issuer = (threadIdx.x == 64 + g * 128);   // first thread of the group issues its dQ bulk reductions
+    auto vote = [&](bool good) { return g == 0 ? named_bar_all<2, 128>(good) : named_bar_all<3, 128>(good); };
     bool ok = true;
-    for (int it = g; it < n_iter; it += 2) {
+    // One round: P of iteration `it`, the dQ block of the group's previous iteration, dS of `it`; the last round only has
+    // the dQ block. A wait that gave up is carried to the next vote, which all 128 threads reach: the loop is only left
+    // right after one, and the .sync.aligned TMEM accesses stay warp-uniform.
+    for (int it = g; it < n_iter + 2; it += 2) {
+      const bool cur = it < n_iter, prev = it >= 2 + g;
+      if (!cur && !prev) break;
       const int j = it >> 1, st = it % BWD_QSTAGES;
       const int head = kv_head * rep + it / n_q;
       const int qb = q_start + it % n_q;
       const int qbase = qb * BWD_BQ;
       const uint32_t bh_key = DROP ? drop_key(p.drop_seed, batch, head + p.drop_head_offset) : 0u;
-      // `good` stays warp-uniform (voted) so the .sync.aligned TMEM loads never diverge; every barrier of the group is
-      // a vote that all 128 threads reach, and the loop is only left right after a vote.
-      bool good = mbar_wait(gbar(g, B_S_FULL), j & 1, abort_flag, 0x2b);
-      good = good && mbar_wait(&stat_full[st], (it / BWD_QSTAGES) & 1, abort_flag, 0x2a);
-      good = good && mbar_wait(gbar(g, B_DP_FULL), j & 1, abort_flag, 0x2d);
-      // the group's region still holds the dQ block of its previous iteration until that bulk reduction has read it
-      if (issuer) tma_store_wait_read<0>();
-      const bool v1 = g == 0 ? named_bar_all<2, 128>(good) : named_bar_all<3, 128>(good);
-      if (!v1) { ok = false; break; }
-      tc_fence_after();
       const bool boundary = (kv0 + BWD_BKV > sk_eff) || (p.causal && (kv0 + BWD_BKV - 1 > qbase + shift));
-      // P^T = exp2(S^T * scale - lse), dS^T = P^T * (dP^T - delta) * scale; S and dP of a 32-column half are loaded
-      // together so one TMEM round trip covers both
+      const int kr = min(kvrow, p.sk - 1);
+      bool good = true;
+      float pr[64];                    // probabilities of this thread's key at the 64 query columns, before dropout
+      uint32_t keep[2] = {0u, 0u};     // DROP: which of them survive
+      if (cur) {
+        good = mbar_wait(gbar(g, B_S_FULL), j & 1, abort_flag, 0x2b);
+        good = good && mbar_wait(&stat_full[st], (it / BWD_QSTAGES) & 1, abort_flag, 0x2a);
+        good = __all_sync(0xffffffffu, good);
+      }
+      if (cur && good) {
+        tc_fence_after();
+        const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t rs[32], rd[32];
-        tmem_ld_32x32b_x32(tm_s + h * 32, rs);
-        tmem_ld_32x32b_x32(tm_dp + h * 32, rd);
-        tmem_ld_wait();
-        // per-row statistics of these 32 query columns: the same for every thread -> broadcast 16-byte loads
-        const float4* lse4 = reinterpret_cast<const float4*>(s_lse + st * 64 + h * 32);
-        const float4* del4 = reinterpret_cast<const float4*>(s_delta + st * 64 + h * 32);
-        const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), ps2 = f2_pack(p.scale, p.scale);
-        // BIAS: this thread's key in the bias / mask / gradient matrices and in the group ids, at the 32 query columns of this half
-        const int kr = min(kvrow, p.sk - 1);
-        const bf16* bt_row = nullptr;
-        uint4 bt4[4];
-        const int* qid_row = nullptr;
-        const float* mask_col = nullptr;     // entry (first query column of this half, this thread's key) of the additive mask
-        float* dbias_col = nullptr;          // ... and of the bias gradient; column c of the half is c * bias_ld further
-        const int qlim = p.sq - (qbase + h * 32);      // columns of this half that are real queries
-        int kid = 0;
-        if constexpr (BIAS) {
-          if (kvrow < p.sk) {
-            const long long col0 = static_cast<long long>(qbase + h * 32) * p.bias_ld + kvrow;
-            if (p.mask) mask_col = p.mask + static_cast<long long>(batch % p.mask_n) * p.sq * p.bias_ld + col0;
-            if (p.dbias) dbias_col = p.dbias + static_cast<long long>(head) * p.sq * p.bias_ld + col0;
-          }
-          // this thread's key row of the transposed bias at the 32 query columns of this half: four 16-byte loads up front
-          if (p.bias_t) {
-            bt_row = p.bias_t + (static_cast<long long>(head) * p.sk + kr) * p.bias_ld + qbase + h * 32;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) bt4[i] = __ldg(reinterpret_cast<const uint4*>(bt_row) + i);
-          }
-          if (p.ids) {
-            const int* idw = p.ids + static_cast<long long>(batch % p.mask_n) * p.bias_ld;
-            kid = __ldg(idw + kr);
-            qid_row = idw + qbase + h * 32;
-          }
-        }
-#pragma unroll
-        for (int c4 = 0; c4 < 8; ++c4) {
-          const float4 ls = lse4[c4], dl = del4[c4];
-          const uint64_t nl2[2] = {f2_pack(-ls.x, -ls.y), f2_pack(-ls.z, -ls.w)};
-          const uint64_t nd2[2] = {f2_pack(-dl.x, -dl.y), f2_pack(-dl.z, -dl.w)};
-          float badd[4] = {0.f, 0.f, 0.f, 0.f};
-          int qid[4] = {0, 0, 0, 0};
+        for (int h = 0; h < 2; ++h) {
+          uint32_t rs[32], pk[16];
+          tmem_ld_32x32b_x32(tm_s + h * 32, rs);
+          // per-row statistics of these 32 query columns: the same for every thread -> broadcast 16-byte loads
+          const float4* lse4 = reinterpret_cast<const float4*>(s_lse + st * 64 + h * 32);
+          // BIAS: this thread's key in the bias / mask matrices and in the group ids, at the 32 query columns of this half
+          const bf16* bt_row = nullptr;
+          uint4 bt4[4];
+          const int* qid_row = nullptr;
+          const float* mask_col = nullptr;     // entry (first query column of this half, this thread's key) of the additive mask
+          const int qlim = p.sq - (qbase + h * 32);      // columns of this half that are real queries
+          int kid = 0;
           if constexpr (BIAS) {
-            if (bt_row) {
-              const uint4 u = bt4[c4 >> 1];
-              const float2 f0 = unpack_bf16x2((c4 & 1) ? u.z : u.x), f1 = unpack_bf16x2((c4 & 1) ? u.w : u.y);
-              badd[0] = f0.x; badd[1] = f0.y; badd[2] = f1.x; badd[3] = f1.y;
+            if (kvrow < p.sk && p.mask)
+              mask_col = p.mask + static_cast<long long>(batch % p.mask_n) * p.sq * p.bias_ld +
+                         static_cast<long long>(qbase + h * 32) * p.bias_ld + kvrow;
+            // this thread's key row of the transposed bias at the 32 query columns of this half: four 16-byte loads up front
+            if (p.bias_t) {
+              bt_row = p.bias_t + (static_cast<long long>(head) * p.sk + kr) * p.bias_ld + qbase + h * 32;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) bt4[i] = __ldg(reinterpret_cast<const uint4*>(bt_row) + i);
             }
-            if (qid_row) {
-              const int4 q4 = __ldg(reinterpret_cast<const int4*>(qid_row + c4 * 4));     // the same for every thread
-              qid[0] = q4.x; qid[1] = q4.y; qid[2] = q4.z; qid[3] = q4.w;
+            if (p.ids) {
+              const int* idw = p.ids + static_cast<long long>(batch % p.mask_n) * p.bias_ld;
+              kid = __ldg(idw + kr);
+              qid_row = idw + qbase + h * 32;
             }
           }
+          tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int c = c4 * 4 + 2 * e;
-            // P = exp2(S * scale_log2 - lse); dS = P * scale * (dP - delta): packed pairs, two exp2
-            float a0, a1;
-            f2_unpack(f2_fma(f2_pack(__uint_as_float(rs[c]), __uint_as_float(rs[c + 1])), sc2, nl2[e]), a0, a1);
+          for (int c4 = 0; c4 < 8; ++c4) {
+            const float4 ls = lse4[c4];
+            const uint64_t nl2[2] = {f2_pack(-ls.x, -ls.y), f2_pack(-ls.z, -ls.w)};
+            float badd[4] = {0.f, 0.f, 0.f, 0.f};
+            int qid[4] = {0, 0, 0, 0};
             if constexpr (BIAS) {
-              float add0 = badd[2 * e], add1 = badd[2 * e + 1];
-              if (mask_col) {          // general additive mask: entry (q, kvrow); a warp's loads cover one line per column
-                add0 += (c < qlim) ? __ldg(mask_col + static_cast<long long>(c) * p.bias_ld) : 0.f;
-                add1 += (c + 1 < qlim) ? __ldg(mask_col + static_cast<long long>(c + 1) * p.bias_ld) : 0.f;
+              if (bt_row) {
+                const uint4 u = bt4[c4 >> 1];
+                const float2 f0 = unpack_bf16x2((c4 & 1) ? u.z : u.x), f1 = unpack_bf16x2((c4 & 1) ? u.w : u.y);
+                badd[0] = f0.x; badd[1] = f0.y; badd[2] = f1.x; badd[3] = f1.y;
               }
-              a0 = fmaf(add0, LOG2E, a0);
-              a1 = fmaf(add1, LOG2E, a1);
-              if (qid_row) {           // keys of another group than the query's carry no probability
-                if (qid[2 * e] != kid) a0 = -INFINITY;
-                if (qid[2 * e + 1] != kid) a1 = -INFINITY;
+              if (qid_row) {
+                const int4 q4 = __ldg(reinterpret_cast<const int4*>(qid_row + c4 * 4));     // the same for every thread
+                qid[0] = q4.x; qid[1] = q4.y; qid[2] = q4.z; qid[3] = q4.w;
               }
             }
-            float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
-            if (boundary) {
-              const int q = qbase + h * 32 + c;
-              if (kvrow >= sk_eff || (p.causal && kvrow > q + shift)) p0 = 0.f;
-              if (kvrow >= sk_eff || (p.causal && kvrow > q + 1 + shift)) p1 = 0.f;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int c = c4 * 4 + 2 * e;
+              // P = exp2(S * scale_log2 - lse): one packed FMA, two exp2
+              float a0, a1;
+              f2_unpack(f2_fma(f2_pack(__uint_as_float(rs[c]), __uint_as_float(rs[c + 1])), sc2, nl2[e]), a0, a1);
+              if constexpr (BIAS) {
+                float add0 = badd[2 * e], add1 = badd[2 * e + 1];
+                if (mask_col) {          // general additive mask: entry (q, kvrow); a warp's loads cover one line per column
+                  add0 += (c < qlim) ? __ldg(mask_col + static_cast<long long>(c) * p.bias_ld) : 0.f;
+                  add1 += (c + 1 < qlim) ? __ldg(mask_col + static_cast<long long>(c + 1) * p.bias_ld) : 0.f;
+                }
+                a0 = fmaf(add0, LOG2E, a0);
+                a1 = fmaf(add1, LOG2E, a1);
+                if (qid_row) {           // keys of another group than the query's carry no probability
+                  if (qid[2 * e] != kid) a0 = -INFINITY;
+                  if (qid[2 * e + 1] != kid) a1 = -INFINITY;
+                }
+              }
+              pr[h * 32 + c] = fast_exp2(a0);
+              pr[h * 32 + c + 1] = fast_exp2(a1);
             }
-            const uint64_t p2 = f2_pack(p0, p1);
-            float dp0 = __uint_as_float(rd[c]), dp1 = __uint_as_float(rd[c + 1]);
+          }
+          if (boundary) {
+            // the first query column that may see this key
+            const int first = (kvrow >= sk_eff ? 0x3fffffff : p.causal ? kvrow - shift : -0x3fffffff) - (qbase + h * 32);
+#pragma unroll
+            for (int c = 0; c < 32; ++c)
+              if (c < first) pr[h * 32 + c] = 0.f;
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float p0 = pr[h * 32 + 2 * i], p1 = pr[h * 32 + 2 * i + 1];
             if constexpr (DROP) {
-              // O = (D * P / (1 - p)) V: dV takes the dropped probabilities, dP the dropped upstream gradient
-              const int q = qbase + h * 32 + c;
+              // O = (D * P / (1 - p)) V: dV takes the dropped probabilities
+              const int q = qbase + h * 32 + 2 * i;
               const bool k0 = drop_keep(bh_key, q, kvrow, p.drop_threshold), k1 = drop_keep(bh_key, q + 1, kvrow, p.drop_threshold);
-              dp0 = k0 ? dp0 * p.drop_scale : 0.f;
-              dp1 = k1 ? dp1 * p.drop_scale : 0.f;
+              keep[h] |= (k0 ? 1u : 0u) << (2 * i) | (k1 ? 2u : 0u) << (2 * i);
               p0 = k0 ? p0 * p.drop_scale : 0.f;
               p1 = k1 ? p1 * p.drop_scale : 0.f;
             }
+            pk[i] = pack_bf16x2(p0, p1);
+          }
+          // both halves of S are read before P^T covers columns of the first: h = 0 writes columns 0-15, which it has read
+          tmem_st_32x32b_x16(tm_s + h * 16, pk);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(gbar(g, B_PT_FULL));
+      }
+      if (prev) {
+        // dQ^T of the previous iteration [lane = head-dim index, columns = query rows] from the dP columns; its products
+        // (and dK's) are done, so nothing reads dS^T any more. The block is staged as [query row][head dim] fp32 and added
+        // into dq_accum by bulk tensor reductions (the adds happen at L2).
+        const int pi = it - 2, phead = kv_head * rep + pi / n_q, pq = (q_start + pi % n_q) * BWD_BQ;
+        good = good && mbar_wait(gbar(g, B_DQ_FULL), (j - 1) & 1, abort_flag, 0x2e);
+        if (issuer) tma_store_wait_read<0>();          // the staging buffer is free again
+        if (!vote(good)) { ok = false; break; }
+        tc_fence_after();
+        {
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32b_x32(tm_dp, r0);
+          tmem_ld_32x32b_x32(tm_dp + 32, r1);
+          tmem_ld_wait();
+          tc_fence_before();
+          mbar_arrive(gbar(g, B_DP_FREE));
+          if (rloc < p.dh) {
+            float* dst = dq_stage + rloc;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) dst[c * p.dh] = __uint_as_float(r0[c]);
+            dst += half_rows;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) dst[c * p.dh] = __uint_as_float(r1[c]);
+          }
+        }
+        fence_async_smem();
+        if (g == 0) named_bar_sync<2, 128>(); else named_bar_sync<3, 128>();
+        if (issuer) {
+          // the half that may lie where dS^T goes leaves first
+          if (pq + 32 < p.sq) tma_reduce_add_4d(&tmDQ, dq_stage + half_rows, 0, phead, pq + 32, batch);
+          tma_store_commit();
+          tma_reduce_add_4d(&tmDQ, dq_stage, 0, phead, pq, batch);
+          tma_store_commit();
+        }
+      }
+      if (!cur) break;
+      good = good && mbar_wait(gbar(g, B_DP_FULL), j & 1, abort_flag, 0x2d);
+      if (issuer) tma_store_wait_read<1>();
+      if (!vote(good)) { ok = false; break; }
+      tc_fence_after();
+      // dS^T = P^T * scale * (dP^T - delta)
+      const uint64_t ps2 = f2_pack(p.scale, p.scale);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t rd[32];
+        tmem_ld_32x32b_x32(tm_dp + h * 32, rd);
+        const float4* del4 = reinterpret_cast<const float4*>(s_delta + st * 64 + h * 32);
+        float* dbias_col = nullptr;          // bias gradient at (first query column of this half, this thread's key)
+        const int qlim = p.sq - (qbase + h * 32);
+        if constexpr (BIAS) {
+          if (kvrow < p.sk && p.dbias)
+            dbias_col = p.dbias + static_cast<long long>(head) * p.sq * p.bias_ld + static_cast<long long>(qbase + h * 32) * p.bias_ld + kvrow;
+        }
+        tmem_ld_wait();
+#pragma unroll
+        for (int c4 = 0; c4 < 8; ++c4) {
+          const float4 dl = del4[c4];
+          const uint64_t nd2[2] = {f2_pack(-dl.x, -dl.y), f2_pack(-dl.z, -dl.w)};
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int c = c4 * 4 + 2 * e;
+            float dp0 = __uint_as_float(rd[c]), dp1 = __uint_as_float(rd[c + 1]);
+            if constexpr (DROP) {        // dP takes the dropped upstream gradient
+              dp0 = (keep[h] >> c) & 1u ? dp0 * p.drop_scale : 0.f;
+              dp1 = (keep[h] >> (c + 1)) & 1u ? dp1 * p.drop_scale : 0.f;
+            }
+            const uint64_t p2 = f2_pack(pr[h * 32 + c], pr[h * 32 + c + 1]);
             const uint64_t t2 = f2_add(f2_pack(dp0, dp1), nd2[e]);
-            float d0, d1;
-            f2_unpack(f2_mul(f2_mul(p2, ps2), t2), d0, d1);
             if constexpr (BIAS) {
               // gradient of the additive term = P * (dP - delta) (dS without the score scale), summed over the batch:
               // consecutive lanes hold consecutive keys, so each atomic add covers one 128-byte line per warp
@@ -881,59 +999,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 if (c + 1 < qlim) atomicAdd(dbias_col + static_cast<long long>(c + 1) * p.bias_ld, g1);
               }
             }
-            rs[c] = __float_as_uint(p0); rs[c + 1] = __float_as_uint(p1);
+            float d0, d1;
+            f2_unpack(f2_mul(f2_mul(p2, ps2), t2), d0, d1);
             rd[c] = __float_as_uint(d0); rd[c + 1] = __float_as_uint(d1);
           }
         }
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
-          uint4 u, w;
-          u.x = pack_bf16x2(__uint_as_float(rs[ch * 8 + 0]), __uint_as_float(rs[ch * 8 + 1]));
-          u.y = pack_bf16x2(__uint_as_float(rs[ch * 8 + 2]), __uint_as_float(rs[ch * 8 + 3]));
-          u.z = pack_bf16x2(__uint_as_float(rs[ch * 8 + 4]), __uint_as_float(rs[ch * 8 + 5]));
-          u.w = pack_bf16x2(__uint_as_float(rs[ch * 8 + 6]), __uint_as_float(rs[ch * 8 + 7]));
+          uint4 w;
           w.x = pack_bf16x2(__uint_as_float(rd[ch * 8 + 0]), __uint_as_float(rd[ch * 8 + 1]));
           w.y = pack_bf16x2(__uint_as_float(rd[ch * 8 + 2]), __uint_as_float(rd[ch * 8 + 3]));
           w.z = pack_bf16x2(__uint_as_float(rd[ch * 8 + 4]), __uint_as_float(rd[ch * 8 + 5]));
           w.w = pack_bf16x2(__uint_as_float(rd[ch * 8 + 6]), __uint_as_float(rd[ch * 8 + 7]));
-          const int piece = ((h * 4 + ch) ^ (rloc & 7)) << 4;
-          *reinterpret_cast<uint4*>(pt_row + piece) = u;
-          *reinterpret_cast<uint4*>(dst_row + piece) = w;
+          *reinterpret_cast<uint4*>(dst_row + (((h * 4 + ch) ^ (rloc & 7)) << 4)) = w;
         }
       }
       tc_fence_before();
-      mbar_arrive(gbar(g, B_DP_FREE));
       fence_async_smem();
-      mbar_arrive(gbar(g, B_PT_FULL));
       mbar_arrive(gbar(g, B_DS_FULL));
-      // dQ^T [lane = head-dim index, columns = query rows] comes back in the S columns once dK / dQ MMAs are done; by
-      // then nothing reads P^T / dS^T any more, so the region is reused to stage the block as [query row][head dim] fp32,
-      // which ONE bulk tensor reduction adds into dq_accum (the adds happen at L2).
-      good = mbar_wait(gbar(g, B_DQ_FULL), j & 1, abort_flag, 0x2e);
-      const bool v2 = g == 0 ? named_bar_all<2, 128>(good) : named_bar_all<3, 128>(good);
-      if (!v2) { ok = false; break; }
-      tc_fence_after();
-      {
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32b_x32(tm_s, r0);
-        tmem_ld_32x32b_x32(tm_s + 32, r1);
-        tmem_ld_wait();
-        tc_fence_before();
-        mbar_arrive(gbar(g, B_S_FREE));
-        if (rloc < p.dh) {
-          float* dst = dq_stage + rloc;
-#pragma unroll
-          for (int c = 0; c < 32; ++c) dst[c * p.dh] = __uint_as_float(r0[c]);
-#pragma unroll
-          for (int c = 0; c < 32; ++c) dst[(32 + c) * p.dh] = __uint_as_float(r1[c]);
-        }
-      }
-      fence_async_smem();
-      if (g == 0) named_bar_sync<2, 128>(); else named_bar_sync<3, 128>();
-      if (issuer) {
-        tma_reduce_add_4d(&tmDQ, dq_stage, 0, head, qbase, batch);
-        tma_store_commit();
-      }
     }
     if (issuer) tma_store_wait<0>();                  // every reduction of this group has been performed
     // final: dK, dV from TMEM (group g takes 64 of the 128 head-dim columns)
@@ -1152,8 +1235,11 @@ static int launch_fwd(const gv_attn_args* a, cudaStream_t stream) {
     cudaError_t e = ensure_max_dynamic_smem(smem_once, kern, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  dim3 grid((a->sq + FWD_BM - 1) / FWD_BM, a->hq, a->b);
-  kern<<<grid, FWD_THREADS, smem, stream>>>(tmQ, tmK, tmV, p);
+  const int q_tiles = (a->sq + FWD_BM - 1) / FWD_BM;
+  p.tile_group = tile_group(a->causal, q_tiles, a->hq * a->b, 512);
+  const long long blocks = static_cast<long long>(q_tiles) * a->hq * a->b;
+  if (blocks > 0x7fffffff) return 2317;
+  kern<<<static_cast<unsigned>(blocks), FWD_THREADS, smem, stream>>>(tmQ, tmK, tmV, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1220,13 +1306,13 @@ extern "C" int gv_attn_bwd(const gv_attn_args* a, gv_stream_t s) {
   if (rc) return rc;
   CUtensorMap tmDQ;
   {
-    // fp32 accumulator [b, sq, hq, dh] contiguous; one reduction covers 64 query rows of one head
+    // fp32 accumulator [b, sq, hq, dh] contiguous; one reduction covers 32 query rows of one head
     EncodeTiledFn fn = attn_encode_fn();
     if (fn == nullptr) return 1001;
     if (reinterpret_cast<uintptr_t>(a->dq_accum) & 15) return 2307;
     cuuint64_t dims[4] = {(cuuint64_t)a->dh, (cuuint64_t)a->hq, (cuuint64_t)a->sq, (cuuint64_t)a->b};
     cuuint64_t strides[3] = {(cuuint64_t)a->dh * 4, (cuuint64_t)a->hq * a->dh * 4, (cuuint64_t)a->sq * a->hq * a->dh * 4};
-    cuuint32_t box[4] = {(cuuint32_t)a->dh, 1, (cuuint32_t)BWD_BQ, 1};
+    cuuint32_t box[4] = {(cuuint32_t)a->dh, 1, (cuuint32_t)(BWD_BQ / 2), 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = fn(&tmDQ, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->dq_accum, dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1250,7 +1336,11 @@ extern "C" int gv_attn_bwd(const gv_attn_args* a, gv_stream_t s) {
   p.bias_t = reinterpret_cast<const bf16*>(a->bias_t); p.mask = a->mask; p.ids = a->ids; p.dbias = a->dbias;
   p.mask_n = a->mask_n > 0 ? a->mask_n : 1; p.bias_ld = a->bias_ld;
   fill_dropout(p, a);
-  dim3 grid((a->sk + BWD_BKV - 1) / BWD_BKV, a->hk, a->b);
+  const int kv_tiles = (a->sk + BWD_BKV - 1) / BWD_BKV;
+  p.tile_group = tile_group(a->causal, kv_tiles, a->hk * a->b, 256);
+  const long long blocks64 = static_cast<long long>(kv_tiles) * a->hk * a->b;
+  if (blocks64 > 0x7fffffff) return 2317;
+  const dim3 grid(static_cast<unsigned>(blocks64));
   auto launch = [&](auto kern, PerDeviceOnce& once) -> cudaError_t {
     cudaError_t e = ensure_max_dynamic_smem(once, kern, BwdSmem::TOTAL);
     if (e != cudaSuccess) return e;

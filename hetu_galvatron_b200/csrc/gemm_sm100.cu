@@ -1244,11 +1244,15 @@ static bool narrow_tiles(const gv_gemm_args* a) {
   return a->N <= 128 || static_cast<long>((a->M + BM - 1) / BM) * ((a->N + 255) / 256) < num_sms();
 }
 
-// Pairs per tile of the split kernel for this product, 1 = no split. The estimate counts waves of tiles: microseconds per
-// 64-deep k-block are 0.36 for a pair's 256 x 256 tile and 0.2 for a CTA's 128 x 128 tile (both measured at 8192 deep and
-// more), plus what joining the sums costs. Splitting pays where the last wave is nearly empty (75 tiles on 74 pairs: 2
-// waves, or 5 quarter waves) or where there is less than one wave of tiles; it must promise 7 %, since the estimate is no
-// better. GV_GEMM_SPLIT = 2 .. 4 forces that split (numerics tests), 1 turns it off.
+// Pairs per tile of the split kernel for this product, 1 = no split. Splitting pays where the last wave of tiles is nearly
+// empty or where there is less than one wave. The estimate is waves x (k-blocks x microseconds + per wave) + per launch:
+//   256 x 256 tiles on pairs              0.36, 0, 5
+//   128 x 128 tiles on single CTAs        0.205, 3, 3
+//   split in two / in three or four       0.36, 1, 6 / 0.38, 3, 6  on 33 / 22 / 15 clusters at once (132 / 132 / 120 SMs)
+// fitted to 26 shapes from 512 x 512 x 2816 to 8192 x 1600 x 50304; a split must promise 8 %, which on all of them kept it to
+// those where it is not the slower one. Measured us, unsplit -> chosen split: 3840 x 1280 x 8192 96.5 -> 77.6 (two),
+// 1024 x 2816 x 8192 60.2 -> 45.7 (three), 384 x 768 x 9216 31.0 -> 22.7 (four), 2048 x 1536 x 151936 992 -> 806 (two).
+// GV_GEMM_SPLIT = 2 .. 4 forces that split (numerics tests), 1 turns it off.
 static int split_plan(const gv_gemm_args* a) {
   static const int forced = [] {
     const char* e = getenv("GV_GEMM_SPLIT");
@@ -1257,21 +1261,21 @@ static int split_plan(const gv_gemm_args* a) {
   if (forced == 1 || a->rope_cols > 0 || a->swiglu_out || a->M <= 0 || a->N <= 0 || a->K <= 0) return 1;
   const int kb = (a->K + BK - 1) / BK;
   if (forced) return kb >= forced ? forced : 1;
-  if (pair_mode() != 1 || kb < 16) return 1;
+  if (pair_mode() != 1 || kb < 40) return 1;
   const long tiles = static_cast<long>((a->M + 255) / 256) * ((a->N + 255) / 256);
   const long sms = num_sms();
   const bool on_pairs = !narrow_tiles(a) && tiles >= sms / 2;
   const long small = static_cast<long>((a->M + BM - 1) / BM) * ((a->N + BM - 1) / BM);
-  double best = on_pairs ? static_cast<double>((tiles + sms / 2 - 1) / (sms / 2)) * kb * 0.36
-                         : static_cast<double>((small + sms - 1) / sms) * kb * 0.2;
+  double best = on_pairs ? static_cast<double>((tiles + sms / 2 - 1) / (sms / 2)) * kb * 0.36 + 5.0
+                         : static_cast<double>((small + sms - 1) / sms) * (kb * 0.205 + 3.0) + 3.0;
   if (!on_pairs && !narrow_tiles(a)) return 1;       // 128 x 256 tiles on single CTAs: one and a half waves, left alone
-  best *= 0.93;
+  best *= 0.92;
   int S = 1;
   for (int s = 2; s <= MAX_SPLIT; ++s) {
     if (kb / s < 8) break;
     const int c = split_clusters(s);
     if (c <= 0) continue;
-    const double t = static_cast<double>((tiles + c - 1) / c) * ((kb + s - 1) / s) * 0.36 + 3.0 + s;
+    const double t = static_cast<double>((tiles + c - 1) / c) * ((kb + s - 1) / s * (s == 2 ? 0.36 : 0.38) + (s == 2 ? 1.0 : 3.0)) + 6.0;
     if (t < best) { best = t; S = s; }
   }
   return S;
