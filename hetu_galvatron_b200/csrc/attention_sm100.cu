@@ -19,6 +19,9 @@
 #include "include/gv_host.h"
 #include "include/gv_ptx.cuh"
 
+#ifndef GV_POLL_NS
+#define GV_POLL_NS 20
+#endif
 namespace gv {
 
 int num_sms();
@@ -472,14 +475,18 @@ constexpr int BWD_BKV = 128;  // KV rows per CTA
 constexpr int BWD_BQ = 64;    // query rows per inner block
 constexpr int BWD_DH = 128;   // head dim is padded to 128 inside the kernel
 constexpr int BWD_THREADS = 64 + 256;
-constexpr int BWD_QSTAGES = 3;
+// Rings of query blocks in shared memory. Q of an iteration is needed from S to dK, its last product, dO only from dP to dV; with
+// three stages of both, S of the next iteration waited for its Q (730 of 6100 clk a round), with four of Q and two of dO it does
+// not, in the same 96 KB.
+constexpr int BWD_QSTAGES = 4, BWD_DOSTAGES = 2;
 
 // Two (kv tile, q block) iterations are in flight per CTA: epilogue group 0 (warps 2-5) owns the even iterations,
 // group 1 (warps 6-9) the odd ones, each with its own accumulators in TMEM, so the tensor cores work for one group while
 // the other does its exponentials. Within a group the steps of neighbouring iterations overlap too: P is computed as soon as
 // S is there and goes back to TMEM, where it is the A operand of dV += P^T dO (no shared memory, no fence); S of the next
-// iteration follows that product, so the group finds it ready when it has written dS; and the dQ block of an iteration is
-// read back between P and dS of the next one, when its products have long finished.
+// iteration follows that product, so the group finds it ready; and dP is multiplied while the group computes P. Clocks of a
+// round of one group (two iterations of the CTA) at 8192 tokens, 32 / 8 heads: 6910 with P before the dQ block and with lse and
+// delta loaded after the ring slot came free, 6530 with them loaded before, 6100 with the dQ block first.
 // TMEM (512 columns): group g: S^T at g*128, overwritten by P^T (bf16, 32 columns); dP^T at g*128 + 64, overwritten by dQ^T;
 // dV at 256, dK at 384.
 struct BwdSmem {
@@ -493,11 +500,12 @@ struct BwdSmem {
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = K_BYTES;
   static constexpr int OFF_Q = 2 * K_BYTES;                       // [BWD_QSTAGES]
-  static constexpr int OFF_DO = OFF_Q + BWD_QSTAGES * Q_BYTES;    // [BWD_QSTAGES]
-  static constexpr int OFF_R = OFF_DO + BWD_QSTAGES * Q_BYTES;    // [2]
-  static constexpr int OFF_STAT = OFF_R + 2 * R_BYTES;            // lse[3][64], delta[3][64] floats
+  static constexpr int OFF_DO = OFF_Q + BWD_QSTAGES * Q_BYTES;    // [BWD_DOSTAGES]
+  static constexpr int OFF_R = OFF_DO + BWD_DOSTAGES * Q_BYTES;   // [2]
+  static constexpr int OFF_STAT = OFF_R + 2 * R_BYTES;            // lse and delta, [BWD_QSTAGES][64] floats each
   static constexpr int OFF_BAR = OFF_STAT + 2 * BWD_QSTAGES * 64 * 4;
-  static constexpr int TOTAL = OFF_BAR + 256 + 1024;
+  static constexpr int BAR_BYTES = 320;
+  static constexpr int TOTAL = OFF_BAR + BAR_BYTES + 704;         // the kernel checks that the base needs no more alignment
 };
 static_assert(BwdSmem::TOTAL <= 232448, "attention backward shared memory budget");
 static_assert(BWD_BQ * BWD_DH * 4 <= BwdSmem::R_BYTES, "dQ staging fits the group region");
@@ -538,18 +546,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   constexpr bool BIAS = MODE == MODE_BIAS, DROP = MODE == MODE_DROP;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* s_lse = reinterpret_cast<float*>(smem + S::OFF_STAT);  // [3][64]
-  float* s_delta = s_lse + BWD_QSTAGES * 64;                     // [3][64]
+  if (static_cast<int>(smem - smem_raw) + S::OFF_BAR + S::BAR_BYTES > S::TOTAL) {  // dynamic smem base less aligned than assumed
+    if (threadIdx.x == 0) record_error((0x20u << 16) | 2u, static_cast<unsigned>(smem - smem_raw));
+    return;
+  }
+  float* s_lse = reinterpret_cast<float*>(smem + S::OFF_STAT);  // [BWD_QSTAGES][64]
+  float* s_delta = s_lse + BWD_QSTAGES * 64;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::OFF_BAR);
   uint64_t* kv_full = bars + 0;
-  uint64_t* qdo_full = bars + 1;    // [3]
-  uint64_t* qdo_empty = bars + 4;   // [3]
-  uint64_t* stat_full = bars + 7;   // [3]
-  // per group g (7 barriers each, starting at 10 + 7 g)
-  auto gbar = [&](int g, int which) { return bars + 10 + 7 * g + which; };
-  enum { B_S_FULL = 0, B_DP_FULL, B_PT_FULL, B_DS_FULL, B_DQ_FULL, B_PV_DONE, B_DP_FREE };
-  uint64_t* all_done = bars + 24;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
+  uint64_t* q_full = bars + 1;      // [BWD_QSTAGES]
+  uint64_t* q_empty = bars + 5;     // [BWD_QSTAGES]
+  uint64_t* stat_full = bars + 9;   // [BWD_QSTAGES]
+  uint64_t* do_full = bars + 13;    // [BWD_DOSTAGES]
+  uint64_t* do_empty = bars + 15;   // [BWD_DOSTAGES]
+  // per group g (8 barriers each, starting at 17 + 8 g)
+  auto gbar = [&](int g, int which) { return bars + 17 + 8 * g + which; };
+  enum { B_S_FULL = 0, B_DP_FULL, B_PT_FULL, B_DS_FULL, B_DQ_FULL, B_DK_DONE, B_PV_DONE, B_DP_FREE };
+  uint64_t* all_done = bars + 33;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 34);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -575,9 +589,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int i = 0; i < BWD_QSTAGES; ++i) {
-      mbar_init(&qdo_full[i], 1);
-      mbar_init(&qdo_empty[i], 1);
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
       mbar_init(&stat_full[i], 32);
+    }
+    for (int i = 0; i < BWD_DOSTAGES; ++i) {
+      mbar_init(&do_full[i], 1);
+      mbar_init(&do_empty[i], 1);
     }
     for (int g = 0; g < 2; ++g) {
       mbar_init(gbar(g, B_S_FULL), 1);
@@ -585,6 +603,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(gbar(g, B_PT_FULL), 128);
       mbar_init(gbar(g, B_DS_FULL), 128);
       mbar_init(gbar(g, B_DQ_FULL), 1);
+      mbar_init(gbar(g, B_DK_DONE), 1);
       mbar_init(gbar(g, B_PV_DONE), 1);
       mbar_init(gbar(g, B_DP_FREE), 128);
     }
@@ -607,7 +626,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    // ---------------- producer: K, V once; then (Q, dO, lse, delta) per iteration into a 3-deep ring ----------------
+    // ---------------- producer: K, V once; then Q, lse, delta and dO of each iteration into their rings ----------------
     bool ok = true;
     if (lane == 0 && n_iter > 0) {
       // head sizes up to 64 fill one 64-wide panel of every operand: the second panel is neither loaded nor multiplied
@@ -621,24 +640,35 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int st = it % BWD_QSTAGES, use = it / BWD_QSTAGES;
       const int head = kv_head * rep + it / n_q;
       const int qb = q_start + it % n_q;
-      if (!mbar_wait(&qdo_empty[st], (use & 1) ^ 1, abort_flag, 0x21)) { ok = false; break; }
-      if (lane == 0) {
-        mbar_expect_tx(&qdo_full[st], 2 * panels * (BWD_BQ * 128));
-        for (int c = 0; c < panels; ++c) {
-          tma_load_4d(smem + S::OFF_Q + st * S::Q_BYTES + c * (BWD_BQ * 128), &tmQ, &qdo_full[st], c * 64, head,
-                      qb * BWD_BQ, batch);
-          tma_load_4d(smem + S::OFF_DO + st * S::Q_BYTES + c * (BWD_BQ * 128), &tmDO, &qdo_full[st], c * 64, head,
-                      qb * BWD_BQ, batch);
-        }
-      }
-      // per-row statistics of the block (plain loads: tiny)
+      // per-row statistics of the block (plain loads: tiny), on their way while the ring stage is still in use. Both are
+      // stored negated, ready to add; -inf -> P = 0 for padded rows
       const long long base = (static_cast<long long>(batch) * p.hq + head) * p.sq + qb * BWD_BQ;
-      for (int i = lane; i < BWD_BQ; i += 32) {
-        const bool in = qb * BWD_BQ + i < p.sq;
-        s_lse[st * 64 + i] = in ? p.lse[base + i] * LOG2E : INFINITY;  // +inf -> P = 0 for padded rows
-        s_delta[st * 64 + i] = in ? p.delta[base + i] : 0.f;
+      float lse[2], delta[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const bool in = qb * BWD_BQ + lane + 32 * h < p.sq;
+        lse[h] = in ? -p.lse[base + lane + 32 * h] * LOG2E : -INFINITY;
+        delta[h] = in ? -p.delta[base + lane + 32 * h] : 0.f;
+      }
+      if (!mbar_wait(&q_empty[st], (use & 1) ^ 1, abort_flag, 0x21)) { ok = false; break; }
+      if (lane == 0) {
+        mbar_expect_tx(&q_full[st], panels * (BWD_BQ * 128));
+        for (int c = 0; c < panels; ++c)
+          tma_load_4d(smem + S::OFF_Q + st * S::Q_BYTES + c * (BWD_BQ * 128), &tmQ, &q_full[st], c * 64, head, qb * BWD_BQ, batch);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        s_lse[st * 64 + lane + 32 * h] = lse[h];
+        s_delta[st * 64 + lane + 32 * h] = delta[h];
       }
       mbar_arrive(&stat_full[st]);
+      const int ds = it % BWD_DOSTAGES;
+      if (!mbar_wait(&do_empty[ds], ((it / BWD_DOSTAGES) & 1) ^ 1, abort_flag, 0x23)) { ok = false; break; }
+      if (lane == 0) {
+        mbar_expect_tx(&do_full[ds], panels * (BWD_BQ * 128));
+        for (int c = 0; c < panels; ++c)
+          tma_load_4d(smem + S::OFF_DO + ds * S::Q_BYTES + c * (BWD_BQ * 128), &tmDO, &do_full[ds], c * 64, head, qb * BWD_BQ, batch);
+      }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer: one thread multiplexing the two groups' pipelines ----------------
@@ -675,7 +705,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         umma_commit<1>(gbar(g, B_S_FULL));
       };
       auto issue_dp = [&](int it) {
-        const int g = it & 1, st = it % BWD_QSTAGES;
+        const int g = it & 1, st = it % BWD_DOSTAGES;
         const uint64_t dod = do_kmaj0 + st * Q_STEP;
 #pragma unroll
         for (int kk = 0; kk < BWD_DH / 16; ++kk) {
@@ -688,7 +718,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       };
       // dV += P^T dO (reduction over the 64 query rows: 8 columns of P^T hold 16 of them)
       auto issue_dv = [&](int it) {
-        const int g = it & 1, st = it % BWD_QSTAGES;
+        const int g = it & 1, st = it % BWD_DOSTAGES;
         const uint64_t dod = do_mnmaj0 + st * Q_STEP;
 #pragma unroll
         for (int kk = 0; kk < BWD_BQ / 16; ++kk)
@@ -709,6 +739,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const uint64_t db = dsd_mn + static_cast<uint64_t>((kk * 2048) >> 4);
           umma_f16_ss<1>(tmem_base + g * 128 + 64, da, db, idesc_dq, kk != 0 ? 1u : 0u);
         }
+        umma_commit<1>(gbar(g, B_DQ_FULL));
 #pragma unroll
         for (int kk = 0; kk < BWD_BQ / 16; ++kk) {
           const uint64_t da = dsd + static_cast<uint64_t>((kk * 32) >> 4);
@@ -716,9 +747,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           umma_f16_ss<1>(tmem_base + TM_DK, da, db, idesc_dv, (dk_started || kk != 0) ? 1u : 0u);
         }
         dk_started = true;
-        // one commit for both: the group overwrites dS^T once it has seen the dQ block
-        umma_commit<1>(gbar(g, B_DQ_FULL));
-        umma_commit<1>(&qdo_empty[st]);
+        umma_commit<1>(gbar(g, B_DK_DONE));
+        umma_commit<1>(&q_empty[st]);
       };
       bool ok = n_iter == 0 || mbar_wait(kv_full, 0, abort_flag, 0x22);
       // next iteration to issue per kind: S and dP in global order (a ring stage must not be probed two uses ahead),
@@ -738,26 +768,31 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             progress = true;
           }
           it = next_dv[g];
-          if (it < n_iter && next_s > it && mbar_test(gbar(g, B_PT_FULL), (it >> 1) & 1)) {
+          if (it < n_iter && next_s > it && mbar_test(gbar(g, B_PT_FULL), (it >> 1) & 1) &&
+              (next_dp > it || mbar_test(&do_full[it % BWD_DOSTAGES], (it / BWD_DOSTAGES) & 1))) {
             tc_fence_after();
             issue_dv(it);
             next_dv[g] += 2;
+            if (next_dp > it) umma_commit<1>(&do_empty[it % BWD_DOSTAGES]);       // whichever of dV and dP comes second
             progress = true;
           }
         }
         if (next_dp < next_s) {
           const int it = next_dp, g = it & 1, j = it >> 1;
           // the group's dQ block of its previous iteration has left these columns
-          if (j == 0 || (next_c[g] >= it && mbar_test(gbar(g, B_DP_FREE), (j - 1) & 1))) {
+          bool ready = mbar_test(&do_full[it % BWD_DOSTAGES], (it / BWD_DOSTAGES) & 1);
+          if (ready && j > 0) ready = next_c[g] >= it && mbar_test(gbar(g, B_DP_FREE), (j - 1) & 1);
+          if (ready) {
             tc_fence_after();
             issue_dp(it);
             ++next_dp;
+            if (next_dv[g] > it) umma_commit<1>(&do_empty[it % BWD_DOSTAGES]);
             progress = true;
           }
         }
         if (next_s < n_iter) {
           const int it = next_s, g = it & 1, j = it >> 1, st = it % BWD_QSTAGES;
-          bool ready = mbar_test(&qdo_full[st], (it / BWD_QSTAGES) & 1);
+          bool ready = mbar_test(&q_full[st], (it / BWD_QSTAGES) & 1);
           // dV of the group's previous iteration has read P^T out of these columns
           if (ready && j > 0) ready = next_dv[g] >= it && mbar_test(gbar(g, B_PV_DONE), (j - 1) & 1);
           if (ready) {
@@ -770,7 +805,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (progress) {
           idle = 0;
           t0 = 0;
-        } else if ((++idle & 0x3ff) == 0) {
+        } else if (__nanosleep(GV_POLL_NS), (++idle & 0x3ff) == 0) {
           if (*abort_flag) { ok = false; break; }
           const uint64_t now = global_timer_ns();
           if (t0 == 0) {
@@ -800,8 +835,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const bool issuer = (threadIdx.x == 64 + g * 128);   // first thread of the group issues its dQ bulk reductions
     auto vote = [&](bool good) { return g == 0 ? named_bar_all<2, 128>(good) : named_bar_all<3, 128>(good); };
     bool ok = true;
-    // One round: P of iteration `it`, the dQ block of the group's previous iteration, dS of `it`; the last round only has
-    // the dQ block. A wait that gave up is carried to the next vote, which all 128 threads reach: the loop is only left
+    // One round: the dQ block of the group's previous iteration (which frees the columns for dP), P of iteration `it` while
+    // dP is multiplied, dS of `it`; the last round only has the dQ block. A wait that gave up is carried to the next vote, which all 128 threads reach: the loop is only left
     // right after one, and the .sync.aligned TMEM accesses stay warp-uniform.
     for (int it = g; it < n_iter + 2; it += 2) {
       const bool cur = it < n_iter, prev = it >= 2 + g;
@@ -816,12 +851,56 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       bool good = true;
       float pr[64];                    // probabilities of this thread's key at the 64 query columns, before dropout
       uint32_t keep[2] = {0u, 0u};     // DROP: which of them survive
-      if (cur) {
-        good = mbar_wait(gbar(g, B_S_FULL), j & 1, abort_flag, 0x2b);
+      if (prev) {
+        // dQ^T of the previous iteration [lane = head-dim index, columns = query rows] from the dP columns. The block is staged as [query row][head dim] fp32 and added
+        // into dq_accum by bulk tensor reductions (the adds happen at L2).
+        const int pi = it - 2, phead = kv_head * rep + pi / n_q, pq = (q_start + pi % n_q) * BWD_BQ;
+        good = good && mbar_wait(gbar(g, B_DQ_FULL), (j - 1) & 1, abort_flag, 0x2e);
+        if (issuer) tma_store_wait_read<0>();          // the staging buffer is free again
+        if (!vote(good)) { ok = false; break; }
+        tc_fence_after();
+        {
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32b_x32(tm_dp, r0);
+          tmem_ld_32x32b_x32(tm_dp + 32, r1);
+          tmem_ld_wait();
+          tc_fence_before();
+          mbar_arrive(gbar(g, B_DP_FREE));
+          float* dst = dq_stage + rloc;
+          if (p.dh == BWD_DH) {                        // immediate offsets
+#pragma unroll
+            for (int c = 0; c < 32; ++c) dst[c * BWD_DH] = __uint_as_float(r0[c]);
+          } else if (rloc < p.dh) {
+#pragma unroll
+            for (int c = 0; c < 32; ++c) dst[c * p.dh] = __uint_as_float(r0[c]);
+          }
+          good = mbar_wait(gbar(g, B_DK_DONE), (j - 1) & 1, abort_flag, 0x2c);    // nothing reads dS^T any more
+          if (p.dh == BWD_DH) {
+#pragma unroll
+            for (int c = 0; c < 32; ++c) dst[S::OFF_DS_IN_R / 4 + c * BWD_DH] = __uint_as_float(r1[c]);
+          } else if (rloc < p.dh) {
+            dst += half_rows;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) dst[c * p.dh] = __uint_as_float(r1[c]);
+          }
+        }
+        fence_async_smem();
+        if (!vote(good)) { ok = false; break; }
+        if (issuer) {
+          // the half that may lie where dS^T goes leaves first
+          if (pq + 32 < p.sq) tma_reduce_add_4d(&tmDQ, dq_stage + half_rows, 0, phead, pq + 32, batch);
+          tma_store_commit();
+          tma_reduce_add_4d(&tmDQ, dq_stage, 0, phead, pq, batch);
+          tma_store_commit();
+        }
+      }
+      if (!cur) break;
+      {
+        good = good && mbar_wait(gbar(g, B_S_FULL), j & 1, abort_flag, 0x2b);
         good = good && mbar_wait(&stat_full[st], (it / BWD_QSTAGES) & 1, abort_flag, 0x2a);
         good = __all_sync(0xffffffffu, good);
       }
-      if (cur && good) {
+      if (good) {
         tc_fence_after();
         const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
 #pragma unroll
@@ -857,7 +936,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
             const float4 ls = lse4[c4];
-            const uint64_t nl2[2] = {f2_pack(-ls.x, -ls.y), f2_pack(-ls.z, -ls.w)};
+            const uint64_t nl2[2] = {f2_pack(ls.x, ls.y), f2_pack(ls.z, ls.w)};
             float badd[4] = {0.f, 0.f, 0.f, 0.f};
             int qid[4] = {0, 0, 0, 0};
             if constexpr (BIAS) {
@@ -921,42 +1000,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc_fence_before();
         mbar_arrive(gbar(g, B_PT_FULL));
       }
-      if (prev) {
-        // dQ^T of the previous iteration [lane = head-dim index, columns = query rows] from the dP columns; its products
-        // (and dK's) are done, so nothing reads dS^T any more. The block is staged as [query row][head dim] fp32 and added
-        // into dq_accum by bulk tensor reductions (the adds happen at L2).
-        const int pi = it - 2, phead = kv_head * rep + pi / n_q, pq = (q_start + pi % n_q) * BWD_BQ;
-        good = good && mbar_wait(gbar(g, B_DQ_FULL), (j - 1) & 1, abort_flag, 0x2e);
-        if (issuer) tma_store_wait_read<0>();          // the staging buffer is free again
-        if (!vote(good)) { ok = false; break; }
-        tc_fence_after();
-        {
-          uint32_t r0[32], r1[32];
-          tmem_ld_32x32b_x32(tm_dp, r0);
-          tmem_ld_32x32b_x32(tm_dp + 32, r1);
-          tmem_ld_wait();
-          tc_fence_before();
-          mbar_arrive(gbar(g, B_DP_FREE));
-          if (rloc < p.dh) {
-            float* dst = dq_stage + rloc;
-#pragma unroll
-            for (int c = 0; c < 32; ++c) dst[c * p.dh] = __uint_as_float(r0[c]);
-            dst += half_rows;
-#pragma unroll
-            for (int c = 0; c < 32; ++c) dst[c * p.dh] = __uint_as_float(r1[c]);
-          }
-        }
-        fence_async_smem();
-        if (g == 0) named_bar_sync<2, 128>(); else named_bar_sync<3, 128>();
-        if (issuer) {
-          // the half that may lie where dS^T goes leaves first
-          if (pq + 32 < p.sq) tma_reduce_add_4d(&tmDQ, dq_stage + half_rows, 0, phead, pq + 32, batch);
-          tma_store_commit();
-          tma_reduce_add_4d(&tmDQ, dq_stage, 0, phead, pq, batch);
-          tma_store_commit();
-        }
-      }
-      if (!cur) break;
       good = good && mbar_wait(gbar(g, B_DP_FULL), j & 1, abort_flag, 0x2d);
       if (issuer) tma_store_wait_read<1>();
       if (!vote(good)) { ok = false; break; }
@@ -978,7 +1021,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int c4 = 0; c4 < 8; ++c4) {
           const float4 dl = del4[c4];
-          const uint64_t nd2[2] = {f2_pack(-dl.x, -dl.y), f2_pack(-dl.z, -dl.w)};
+          const uint64_t nd2[2] = {f2_pack(dl.x, dl.y), f2_pack(dl.z, dl.w)};
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int c = c4 * 4 + 2 * e;
