@@ -123,23 +123,13 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __r
   }
 }
 
-__device__ __forceinline__ float gelu_f(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 0.5f * x * (1.0f + tanhf(k0 * (x + k1 * x * x * x)));
-}
-__device__ __forceinline__ float gelu_grad_f(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float t = tanhf(k0 * (x + k1 * x * x * x));
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * k0 * (1.f + 3.f * k1 * x * x);
-}
-
 __global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long long nvec) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < nvec;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float a[8], o[8];
     unpack8e(reinterpret_cast<const uint4*>(x)[i], a);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = gelu_f(a[e]);
+    for (int e = 0; e < 8; ++e) o[e] = gelu_tanh(a[e]);
     reinterpret_cast<uint4*>(y)[i] = pack8e(o);
   }
 }
@@ -151,7 +141,7 @@ __global__ void gelu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restr
     unpack8e(reinterpret_cast<const uint4*>(x)[i], a);
     unpack8e(reinterpret_cast<const uint4*>(dy)[i], d);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = d[e] * gelu_grad_f(a[e]);
+    for (int e = 0; e < 8; ++e) o[e] = d[e] * gelu_tanh_grad(a[e]);
     reinterpret_cast<uint4*>(dx)[i] = pack8e(o);
   }
 }
@@ -349,6 +339,72 @@ __global__ void lse_merge_kernel(float* __restrict__ acc, float* __restrict__ ls
   for (int c = lane; c < dh; c += 32) a[c] = a[c] * wa + __bfloat162float(o[c]) * wb;
   __syncwarp();
   if (update_lse && lane == 0) lse_acc[li] = ln;
+}
+
+// ------------------------------------------------------------------ head statistics
+// Joins the statistics that the head GEMM's epilogue left per 256 columns (stats [rows, tiles, 2]: max, sum of exp) into one
+// (max, sum) per row, one warp per row, and finishes the loss where this shard holds the whole vocabulary. `target` was written
+// where the label lies in this shard; elsewhere it becomes 0. Replaces a dozen element-wise launches on [rows] and [rows, tiles].
+__global__ void xent_merge_kernel(const float2* __restrict__ stats, int tiles, const long long* __restrict__ labels, long long vocab_start,
+                                  long long vocab_rows, long long ignore_index, float* __restrict__ row_max, float* __restrict__ row_sum,
+                                  float* __restrict__ target, float* __restrict__ lse, float* __restrict__ loss, long long rows) {
+  const int lane = threadIdx.x & 31;
+  const long long row = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
+  if (row >= rows) return;
+  float m = -INFINITY, l = 0.f;
+  for (int t = lane; t < tiles; t += 32) {
+    const float2 v = __ldg(stats + row * tiles + t);
+    const float n = fmaxf(m, v.x);
+    l = (m == -INFINITY ? 0.f : l * expf(m - n)) + v.y * expf(v.x - n);
+    m = n;
+  }
+  const float wm = warp_max_e(m);
+  const float wl = warp_sum_e(m == -INFINITY ? 0.f : l * expf(m - wm));
+  if (lane != 0) return;
+  const long long lab = labels[row];
+  const bool kept = lab != ignore_index, here = kept && lab >= vocab_start && lab < vocab_start + vocab_rows;
+  const float tg = here ? target[row] : 0.f;
+  row_max[row] = wm;
+  row_sum[row] = wl;
+  if (!here) target[row] = 0.f;
+  const float ls = logf(wl) + wm;
+  if (lse != nullptr) lse[row] = ls;
+  if (loss != nullptr) loss[row] = kept ? ls - tg : 0.f;
+}
+
+// ------------------------------------------------------------------ head padding
+// Copies between heads of `narrow` columns and heads of `wide` columns (a multiple of 8, the surplus zero) for up to five
+// tensors [b, s, h, .] of any strides, one block per (element, row): GPT-2 XL's heads of 50 columns around the attention
+// kernels, whose TMA needs a multiple of 8. PAD: narrow -> wide, else wide -> narrow. HBM-bound: the wide side moves 16 bytes
+// per thread, the narrow side, only 4-byte aligned, four times 4 bytes of neighbouring threads. 8192 rows x 32 heads x 50: one
+// strided copy per tensor took 39 us, three tensors now share a launch.
+template <bool PAD>
+__global__ void pad_heads_kernel(const gv_pad_heads_args a) {
+  const int t = blockIdx.y;
+  const int units = a.wide >> 3, total = a.h[t] * units, narrow = a.narrow;
+  const long long rows = static_cast<long long>(a.b) * a.s[t];
+  for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
+    const long long bi = row / a.s[t], si = row - bi * a.s[t];
+    const bf16* src = reinterpret_cast<const bf16*>(a.src[t]) + bi * a.src_stride[t][0] + si * a.src_stride[t][1];
+    bf16* dst = reinterpret_cast<bf16*>(a.dst[t]) + bi * a.dst_stride[t][0] + si * a.dst_stride[t][1];
+    for (int i = threadIdx.x; i < total; i += blockDim.x) {
+      const int hd = i / units, c = (i - hd * units) * 8;
+      const bf16* sp = src + hd * a.src_stride[t][2] + c;
+      bf16* dp = dst + hd * a.dst_stride[t][2] + c;
+      if (PAD) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = c + 2 * e < narrow ? *reinterpret_cast<const uint32_t*>(sp + 2 * e) : 0u;
+        *reinterpret_cast<uint4*>(dp) = make_uint4(w[0], w[1], w[2], w[3]);
+      } else {
+        const uint4 u = *reinterpret_cast<const uint4*>(sp);
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (c + 2 * e < narrow) *reinterpret_cast<uint32_t*>(dp + 2 * e) = w[e];
+      }
+    }
+  }
 }
 
 // ------------------------------------------------------------------ optimizer
@@ -620,6 +676,39 @@ extern "C" int gv_cast_bf16_to_f32(const void* in, float* out, long long n, floa
   if (n <= 0) return 0;
   cast_bf16_f32_kernel<<<grid_for(n / 4 + 4, 256), 256, 0, (cudaStream_t)s>>>((const bf16*)in, out, n, scale,
                                                                               accumulate);
+  return (int)cudaGetLastError();
+}
+
+extern "C" int gv_xent_merge(const float* stats, int tiles, const long long* labels, long long vocab_start, long long vocab_rows,
+                             long long ignore_index, float* row_max, float* row_sum, float* target, float* lse, float* loss,
+                             long long rows, gv_stream_t st) {
+  if (rows <= 0) return 0;
+  if (tiles <= 0 || (reinterpret_cast<uintptr_t>(stats) & 7)) return 2207;
+  xent_merge_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, (cudaStream_t)st>>>(reinterpret_cast<const float2*>(stats), tiles, labels, vocab_start,
+                                                                             vocab_rows, ignore_index, row_max, row_sum, target, lse, loss, rows);
+  return (int)cudaGetLastError();
+}
+
+extern "C" int gv_pad_heads(const gv_pad_heads_args* a, int pad, gv_stream_t st) {
+  if (a->count < 1 || a->count > 5 || a->b <= 0) return 2310;
+  if (a->narrow <= 0 || a->narrow % 2 || a->wide % 8 || a->wide < a->narrow) return 2311;
+  long long rows = 0;
+  int units = 0;
+  for (int t = 0; t < a->count; ++t) {
+    const uintptr_t n = reinterpret_cast<uintptr_t>(pad ? a->src[t] : a->dst[t]), w = reinterpret_cast<uintptr_t>(pad ? a->dst[t] : a->src[t]);
+    const long long* ns = pad ? a->src_stride[t] : a->dst_stride[t];
+    const long long* ws = pad ? a->dst_stride[t] : a->src_stride[t];
+    if ((n & 3) || (w & 15) || ((ns[0] | ns[1] | ns[2]) & 1) || ((ws[0] | ws[1] | ws[2]) & 7)) return 2312;
+    if (a->s[t] <= 0 || a->h[t] <= 0) return 2313;
+    const long long r = static_cast<long long>(a->b) * a->s[t];
+    rows = r > rows ? r : rows;
+    units = a->h[t] * (a->wide / 8) > units ? a->h[t] * (a->wide / 8) : units;
+  }
+  const int threads = units >= 256 ? 256 : (units + 31) / 32 * 32;
+  const long long cap = static_cast<long long>(num_sms()) * 16;
+  const dim3 grid(static_cast<unsigned>(rows < cap ? rows : cap), static_cast<unsigned>(a->count));
+  if (pad) pad_heads_kernel<true><<<grid, threads, 0, (cudaStream_t)st>>>(*a);
+  else pad_heads_kernel<false><<<grid, threads, 0, (cudaStream_t)st>>>(*a);
   return (int)cudaGetLastError();
 }
 

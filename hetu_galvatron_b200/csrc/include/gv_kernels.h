@@ -52,6 +52,10 @@ typedef struct {
   // silu(gate) * up. Needs K-major A and B, bf16 C, no bias / residual / activation / accumulate.
   void* swiglu_out;
   int swiglu_ld;
+  // GELU beside the projection (NULL = off): C receives the projection (+ bias) and gelu_out [M, gelu_ld >= N] (bf16) gelu (tanh
+  // form) of the stored values. Needs K-major A and B, bf16 C, no residual / activation / accumulate / rotary columns / gated activation.
+  void* gelu_out;
+  int gelu_ld;
   // Scratch for a split reduction (NULL: the reduction is not split): gv_gemm_workspace_bytes of the same arguments,
   // 16-byte aligned, uninitialised, in use until the launch has finished.
   void* workspace;
@@ -137,6 +141,13 @@ int gv_xent_loss_grad(void* logits, const long long* labels, const float* row_ma
                       long long rows, int vocab_local, long long ld, long long vocab_start, long long ignore_index,
                       gv_stream_t stream);
 
+// Joins gv_gemm_xent's mode-1 statistics [rows, tiles, 2] into row_max / row_sum [rows]; target[row] becomes 0 where the label is
+// ignored or not in [vocab_start, vocab_start + vocab_rows). lse = log(sum) + max and loss = lse - target (0 for ignored rows)
+// are optional; loss is the cross entropy when this shard is the whole vocabulary.
+int gv_xent_merge(const float* stats, int tiles, const long long* labels, long long vocab_start, long long vocab_rows,
+                  long long ignore_index, float* row_max, float* row_sum, float* target, float* lse, float* loss, long long rows,
+                  gv_stream_t stream);
+
 // ---- optimizer ----------------------------------------------------------------------
 // Fused AdamW on a flat shard: fp32 master/m/v, fp32 or bf16 grads, bf16 parameter write-back.
 // grad_scale multiplies the gradient first (1/world, loss scale, clip coefficient pointer optional).
@@ -212,6 +223,18 @@ typedef struct {
 } gv_attn_args;
 int gv_attn_fwd(const gv_attn_args* args, gv_stream_t stream);
 int gv_attn_bwd(const gv_attn_args* args, gv_stream_t stream);
+
+// Copies `count` (1 to 5) bf16 tensors [b, s, h, .] between heads of `narrow` (even) and `wide` (a multiple of 8, not smaller)
+// columns: pad != 0 narrow -> wide with zeros behind, else wide -> narrow. Strides in elements of (b, s, h), unit inner stride;
+// wide sides 16-byte aligned with strides of multiples of 8, narrow sides 4-byte aligned with even strides.
+typedef struct {
+  const void* src[5];
+  void* dst[5];
+  long long src_stride[5][3], dst_stride[5][3];
+  int s[5], h[5];
+  int count, b, narrow, wide;
+} gv_pad_heads_args;
+int gv_pad_heads(const gv_pad_heads_args* args, int pad, gv_stream_t stream);
 
 // Log-sum-exp merge of a partial attention result into fp32 accumulators (ring / context-parallel attention):
 // acc fp32 [b, s, h, dh] contiguous, lse_acc fp32 [b, h, s]; partial o_blk bf16 [b, sb, h, dh] (element strides

@@ -474,6 +474,25 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   return d;
 }
 
+// 1 / (1 + exp(-x)) without the branch per element of an IEEE division: a reciprocal with one Newton step, which is left out
+// where the denominator has overflowed (its reciprocal is 0).
+__device__ __forceinline__ float sigmoid_nb(float x) {
+  const float d = 1.f + __expf(-x);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  const float z = fmaf(y, fmaf(-d, y, 1.f), y);
+  return d < 1e38f ? z : y;
+}
+// GELU, tanh form: x (1 + tanh u) / 2 = x sigmoid(2 u) with u = sqrt(2 / pi) (x + 0.044715 x^3), and its derivative. The sigmoid
+// has no cancellation where tanh u is close to -1 (at x = -4 the tanh form is off by 1e-3 of the value) and no branch.
+__device__ __forceinline__ float gelu_tanh(float x) {
+  return x * sigmoid_nb(1.5957691216057308f * fmaf(0.044715f * x * x, x, x));
+}
+__device__ __forceinline__ float gelu_tanh_grad(float x) {
+  const float s = sigmoid_nb(1.5957691216057308f * fmaf(0.044715f * x * x, x, x));
+  return fmaf(x * s * (1.f - s), 1.5957691216057308f * fmaf(0.134145f * x, x, 1.f), s);
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);

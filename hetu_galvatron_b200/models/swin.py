@@ -218,7 +218,7 @@ class SwinLayerBlock(nn.Module):
             h = h + self._drop_path(A.linear(self._attention(qkv, b).contiguous(), self.wo, self.bo, cfg=row), ctx, b)
         else:
             h = A.linear(self._attention(qkv, b).contiguous(), self.wo, self.bo, residual=h, cfg=row)
-        m = A.gelu(A.linear(self.ln2(h), self.w1, self.b1, cfg=col))
+        m = A.linear_gelu(self.ln2(h), self.w1, self.b1, cfg=col)
         h = A.linear(m, self.w2, self.b2, residual=h, cfg=row)
         if self.merge:
             R, C = self.res, self.C

@@ -426,10 +426,13 @@ class MLP(nn.Module):
         if (self.cfg.act == "swiglu" and st.weight_tp == 1 and self.b_up is None and A.SAVE_SWIGLU_ACT
                 and A.swiglu_epilogue_supported(x, self.w_up)):
             return A.swiglu_mlp(x, self.w_up, self.w_down, residual)     # activation in the up-projection's epilogue
-        up = A.linear(x, self.w_up, self.b_up, None, st.linear_cfg("col"))
         if self.cfg.act == "swiglu":
+            up = A.linear(x, self.w_up, self.b_up, None, st.linear_cfg("col"))
             return A.swiglu_linear(up, self.w_down, residual, st.linear_cfg("row"))
-        act = torch.relu(up) if self.cfg.act == "relu" else A.gelu(up)          # relu: the original T5 feed-forward
+        if self.cfg.act == "relu":                                              # the original T5 feed-forward
+            act = torch.relu(A.linear(x, self.w_up, self.b_up, None, st.linear_cfg("col")))
+        else:
+            act = A.linear_gelu(x, self.w_up, self.b_up, st.linear_cfg("col"))
         return A.linear(act, self.w_down, self.b_down, residual, st.linear_cfg("row"))
 
 

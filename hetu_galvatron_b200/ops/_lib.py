@@ -57,6 +57,7 @@ class GemmArgs(Structure):
         ("rope_cols", c_int), ("rope_dh", c_int), ("rope_inv_freq", c_void_p), ("rope_pos", c_void_p),
         ("rope_pos_div", c_int), ("rope_pos_mod", c_int), ("rope_pos_offset", c_int),
         ("swiglu_out", c_void_p), ("swiglu_ld", c_int),
+        ("gelu_out", c_void_p), ("gelu_ld", c_int),
         ("workspace", c_void_p), ("workspace_bytes", c_longlong),
     ]
 
@@ -107,10 +108,19 @@ PROTOTYPES = {
     "gv_embedding_bwd": [_P] * 3 + [_L, _I, _L, _L, _P],
     "gv_xent_stats": [_P] * 5 + [_L, _I, _L, _L, _P],
     "gv_xent_loss_grad": [_P] * 6 + [_F, _P, _L, _I, _L, _L, _L, _P],
+    "gv_xent_merge": [_P, _I, _P, _L, _L, _L] + [_P] * 5 + [_L, _P],
     "gv_adamw": [_P, _P, _P, _P, _I, _P, _L] + [_F] * 8 + [_P, _P],
     "gv_sumsq_accum": [_P, _I, _L, _P, _P],
     "gv_lse_merge": [_P] * 4 + [_I] * 6 + [_L, _L, _L, _P],
 }
+
+
+class PadHeadsArgs(Structure):
+    _fields_ = [("src", c_void_p * 5), ("dst", c_void_p * 5), ("src_stride", (c_longlong * 3) * 5), ("dst_stride", (c_longlong * 3) * 5),
+                ("s", c_int * 5), ("h", c_int * 5), ("count", c_int), ("b", c_int), ("narrow", c_int), ("wide", c_int)]
+
+
+PROTOTYPES["gv_pad_heads"] = [POINTER(PadHeadsArgs), _I, _P]
 
 
 def available() -> bool:

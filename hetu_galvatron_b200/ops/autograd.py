@@ -30,7 +30,8 @@ import torch
 
 from ..parallel import collectives as C
 from . import functional as Fn
-from .gemm import gemm, head_xent_grad, head_xent_stats, head_xent_supported, swiglu_epilogue_supported
+from .gemm import (gelu_epilogue_supported, gemm, head_xent_grad, head_xent_loss, head_xent_stats, head_xent_supported,
+                   swiglu_epilogue_supported)
 
 
 # --------------------------------------------------------------------------- helpers
@@ -277,6 +278,37 @@ class GeluFn(torch.autograd.Function):
 
 def gelu(x):
     return GeluFn.apply(x)
+
+
+class LinearGeluFn(torch.autograd.Function):
+    """gelu(x W^T + b) of an un-sharded layer with the activation computed in the projection's epilogue (no separate pass over
+    [tokens, ffn]); the projection is kept for the backward pass."""
+
+    @staticmethod
+    def forward(ctx, x, W, bias):
+        lead = x.shape[:-1]
+        x2 = x.reshape(-1, x.shape[-1])
+        act = torch.empty(x2.shape[0], W.shape[0], dtype=x2.dtype, device=x2.device)
+        up = gemm(x2, W, bias=bias, gelu_out=act)
+        ctx.lead = lead
+        ctx.save_for_backward(x2, W, bias, up)
+        return act.view(*lead, W.shape[0])
+
+    @staticmethod
+    def backward(ctx, dact):
+        x2, W, bias, up = ctx.saved_tensors
+        dy = Fn.gelu_bwd(dact.reshape(-1, W.shape[0]), up)
+        dx = gemm(dy, W, b_mn=True).view(*ctx.lead, W.shape[1]) if ctx.needs_input_grad[0] else None
+        dW = _wgrad(W, dy, x2)
+        db = None if bias is None else _vec_grad(bias, lambda buf: Fn.colsum_accum(dy, buf))
+        return dx, dW, db
+
+
+def linear_gelu(x, W, bias=None, cfg: LinearCfg = LinearCfg()):
+    """gelu(linear(x)): in one kernel for un-sharded layers of bf16 CUDA operands, else one after the other."""
+    if (cfg.mode == "plain" or C.group_size(cfg.group) == 1) and gelu_epilogue_supported(x, W, bias):
+        return LinearGeluFn.apply(x, W, bias)
+    return gelu(linear(x, W, bias, None, cfg))
 
 
 # --------------------------------------------------------------------------- normalisation
@@ -635,6 +667,11 @@ class LMHeadLossFn(torch.autograd.Function):
         if fused:
             # statistics straight from the GEMM's fp32 accumulators; no [tokens, vocab] tensor is ever written
             logits = None
+            if n == 1:
+                ctx.cfg, ctx.n, ctx.fused, ctx.x_shape = cfg, n, fused, x.shape
+                loss, lse = head_xent_loss(xg, W, labels, cfg.vocab_start, cfg.ignore_index)
+                ctx.save_for_backward(x2, W, labels, lse)
+                return loss
             mx, se, tg = head_xent_stats(xg, W, labels, cfg.vocab_start, cfg.ignore_index)
         else:
             logits = gemm(xg, W, out_dtype=torch.float32 if (cfg.fp32_logits or not x.is_cuda) else None)
@@ -651,7 +688,7 @@ class LMHeadLossFn(torch.autograd.Function):
         ctx.cfg, ctx.n, ctx.fused = cfg, n, fused
         ctx.x_shape = x.shape
         if fused:
-            ctx.save_for_backward(x2, W, labels, mx, se)
+            ctx.save_for_backward(x2, W, labels, torch.log(se) + mx)
         else:
             ctx.save_for_backward(x2, W, labels, logits, mx, se, tg)
         return loss
@@ -660,12 +697,10 @@ class LMHeadLossFn(torch.autograd.Function):
     def backward(ctx, dloss):
         cfg, n = ctx.cfg, ctx.n
         if ctx.fused:
-            x2, W, labels, mx, se = ctx.saved_tensors
+            x2, W, labels, lse = ctx.saved_tensors
             xg = C.all_gather_first_dim(x2, cfg.group) if (cfg.mode == "col_sp" and n > 1) else x2
-            keep = (labels != cfg.ignore_index).to(torch.float32)
-            # the head GEMM runs once more; its epilogue turns each fp32 logit into its gradient
-            dlog = head_xent_grad(xg, W, labels, torch.log(se) + mx, dloss.reshape(-1).float() * keep, cfg.vocab_start,
-                                  cfg.ignore_index)
+            # the head GEMM runs once more; its epilogue turns each fp32 logit into its gradient (0 in ignored rows)
+            dlog = head_xent_grad(xg, W, labels, lse, dloss.reshape(-1), cfg.vocab_start, cfg.ignore_index)
         else:
             x2, W, labels, logits, mx, se, tg = ctx.saved_tensors
             Fn.xent_loss_grad_(logits, labels, mx, se, tg, 1.0, cfg.vocab_start, cfg.ignore_index,

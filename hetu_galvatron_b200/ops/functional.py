@@ -476,8 +476,35 @@ def _pads_to_native(q) -> bool:
     return q.dtype == torch.bfloat16 and q.shape[-1] % 8 != 0 and q.shape[-1] < 128
 
 
-def _pad_last(t, dh: int):
-    return torch.nn.functional.pad(t, (0, (dh + 7) // 8 * 8 - dh))
+def _copy_heads(srcs, dsts, narrow: int, pad: bool) -> bool:
+    """One launch that copies [b, s, h, .] tensors between heads of ``narrow`` and of a multiple of 8 columns; False when a
+    tensor is not even-strided and 4-byte aligned (nothing has been copied then)."""
+    for t in (srcs if pad else dsts):
+        sb, ss, sh, inner = t.stride()
+        if inner != 1 or (sb | ss | sh) % 2 or t.data_ptr() % 4 or narrow % 2 or t.dtype != torch.bfloat16:
+            return False
+    a = _lib.PadHeadsArgs(count=len(srcs), b=srcs[0].shape[0], narrow=narrow, wide=(dsts if pad else srcs)[0].shape[-1])
+    for i, (x, y) in enumerate(zip(srcs, dsts)):
+        a.src[i], a.dst[i], a.s[i], a.h[i] = x.data_ptr(), y.data_ptr(), x.shape[1], x.shape[2]
+        a.src_stride[i][:], a.dst_stride[i][:] = x.stride()[:3], y.stride()[:3]
+    _lib.check(_lib.lib().gv_pad_heads(a, int(pad), _s()), "gv_pad_heads")
+    return True
+
+
+def _pad_heads(ts, dh: int):
+    wide = (dh + 7) // 8 * 8
+    if all(t.is_cuda and t.numel() for t in ts):
+        out = [torch.empty(*t.shape[:-1], wide, dtype=t.dtype, device=t.device) for t in ts]
+        if _copy_heads(ts, out, dh, True):
+            return out
+    return [F.pad(t, (0, wide - dh)) for t in ts]
+
+
+def _unpad_heads(srcs, dsts) -> None:
+    if all(t.is_cuda and t.numel() for t in dsts) and _copy_heads(srcs, dsts, dsts[0].shape[-1], False):
+        return
+    for x, y in zip(srcs, dsts):
+        y.copy_(x[..., :y.shape[-1]])
 
 
 def attention_fwd(q, k, v, causal: bool, scale: float | None = None, out: torch.Tensor | None = None, kv_lens=None,
@@ -493,14 +520,13 @@ def attention_fwd(q, k, v, causal: bool, scale: float | None = None, out: torch.
     if _native(q) and _pads_to_native(q):
         # head sizes that are not a multiple of 8 (GPT-2 XL: 50): zero columns change neither the scores nor the output
         dh = q.shape[-1]
-        qp, kp, vp = (_pad_last(t, dh) for t in (q, k, v))
+        qp, kp, vp = _pad_heads((q, k, v), dh)
         if _attn.supported(qp, kp, vp):
             o, lse = _attn.fwd(qp, kp, vp, causal, scale, None, kv_lens, dropout)
-            o = o[..., :dh]
             if out is not None:
-                out.copy_(o)
-                o = out
-            return o, lse
+                _unpad_heads((o,), (out,))
+                return out, lse
+            return o[..., :dh], lse
     o, lse = attention_reference(q, k, v, causal, scale, kv_lens, dropout)
     if out is not None:
         out.copy_(o)
@@ -521,13 +547,13 @@ def attention_bwd(dout, q, k, v, o, lse, causal: bool, scale: float | None = Non
         return _attn.bwd(dout, q, k, v, o, lse, causal, scale, dq, dk, dv, kv_lens, dq_rope, dropout)
     if _native(q) and _pads_to_native(q):
         dh = q.shape[-1]
-        qp, kp, vp, op, dop = (_pad_last(t, dh) for t in (q, k, v, o, dout))
+        qp, kp, vp, op, dop = _pad_heads((q, k, v, o, dout), dh)
         if _attn.supported(qp, kp, vp):
-            gq, gk, gv = (g[..., :dh] for g in _attn.bwd(dop, qp, kp, vp, op, lse, causal, scale, None, None, None, kv_lens, None, dropout))
+            grads = _attn.bwd(dop, qp, kp, vp, op, lse, causal, scale, None, None, None, kv_lens, None, dropout)
             if dq is not None:
-                dq.copy_(gq); dk.copy_(gk); dv.copy_(gv)
+                _unpad_heads(grads, (dq, dk, dv))
                 return dq, dk, dv
-            return gq, gk, gv
+            return tuple(g[..., :dh] for g in grads)
     b, sq, hq, dh = q.shape
     sk, hk = k.shape[1], k.shape[2]
     rep = hq // hk

@@ -54,11 +54,13 @@ def _workspace_bytes(M: int, N: int, K: int) -> int:
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,
          out_dtype: torch.dtype | None = None, bias: torch.Tensor | None = None,
          residual: torch.Tensor | None = None, accumulate: bool = False, gelu: bool = False,
-         alpha: float = 1.0, rope: "RopeEpilogue | None" = None, swiglu_out: torch.Tensor | None = None) -> torch.Tensor:
+         alpha: float = 1.0, rope: "RopeEpilogue | None" = None, swiglu_out: torch.Tensor | None = None,
+         gelu_out: torch.Tensor | None = None) -> torch.Tensor:
     """See module docstring. ``a`` is ``[M,K]`` (or ``[K,M]`` when ``a_mn``), ``b`` is ``[N,K]`` (or ``[K,N]``).
     ``rope``: rotate the leading q / k head columns of the output in the epilogue (see ``RopeEpilogue``).
     ``swiglu_out`` [M, N / 2] bf16: ``b`` is [gate rows | up rows]; besides the projection itself the epilogue stores
-    silu(gate) * up there (see ``swiglu_epilogue_supported``)."""
+    silu(gate) * up there (see ``swiglu_epilogue_supported``). ``gelu_out`` [M, N] bf16: the epilogue also stores gelu of the
+    projection there (see ``gelu_epilogue_supported``)."""
     a = _row_major_2d(a)
     b = _row_major_2d(b)
     if a_mn:
@@ -96,6 +98,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             args.rope_inv_freq = rope.inv_freq.data_ptr()
             args.rope_pos = _lib.p(rope.positions) or None
             args.rope_pos_div, args.rope_pos_mod, args.rope_pos_offset = rope.pos_div, 0, rope.pos_offset
+        elif gelu_out is not None:
+            args.gelu_out, args.gelu_ld = gelu_out.data_ptr(), gelu_out.stride(0)
         elif swiglu_out is None:
             need = _workspace_bytes(M, N, K)
             if need:
@@ -106,7 +110,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
                     pass                    # no room for the partial sums: the product runs unsplit
         _lib.check(_lib.lib().gv_gemm_bf16(args, _lib.stream_ptr()), "gv_gemm_bf16")
         return out
-    if rope is not None or swiglu_out is not None:
+    if rope is not None or swiglu_out is not None or gelu_out is not None:
         raise _lib.KernelError("gemm: the rotary / gated-activation epilogues need the native kernel (bf16 CUDA operands)")
     if a.is_cuda and a.dtype == torch.bfloat16 and not _lib_fallback_allowed():
         raise _lib.KernelError(f"gemm: shape/stride not supported by the sm_100a kernel: M={M} N={N} K={K}")
@@ -137,6 +141,11 @@ def swiglu_epilogue_supported(x: torch.Tensor, w_up: torch.Tensor) -> bool:
             and w_up.stride(1) == 1 and w_up.stride(0) % 8 == 0 and w_up.data_ptr() % 16 == 0)
 
 
+def gelu_epilogue_supported(x: torch.Tensor, W: torch.Tensor, bias) -> bool:
+    """The GELU epilogue wants bf16 CUDA operands in natural storage, row lengths of multiples of 8."""
+    return (_use_native(x, W, bias) and W.dim() == 2 and W.shape[0] % 8 == 0 and W.shape[1] % 8 == 0 and x.numel() > 0)
+
+
 def head_xent_supported(x: torch.Tensor, W: torch.Tensor) -> bool:
     """The cross-entropy epilogues need bf16 CUDA operands in their natural (K-major) storage."""
     return (_use_native(x, W) and x.dim() == 2 and W.dim() == 2 and x.shape[1] == W.shape[1] and x.shape[1] % 8 == 0
@@ -153,26 +162,38 @@ def _head_args(x, W, C):
                          accumulate=0, act=0, alpha=1.0)
 
 
-def head_xent_stats(x: torch.Tensor, W: torch.Tensor, labels: torch.Tensor, vocab_start: int = 0, ignore_index: int = -100):
-    """Language-model head forward without logits: per row (max, sum exp(logit - max), target logit or 0) over this
-    rank's vocabulary shard ``W`` [V_local, K], computed in the epilogue of the head GEMM from its fp32 accumulators."""
+def _head_stats(x, W, labels, vocab_start: int, ignore_index: int, finish: bool):
     M, N = x.shape[0], W.shape[0]
     tiles = (N + 255) // 256
     stats = torch.empty(M, tiles, 2, dtype=torch.float32, device=x.device)
-    target = torch.zeros(M, dtype=torch.float32, device=x.device)
+    rows = torch.empty(5, M, dtype=torch.float32, device=x.device)          # max, sum, target, log-sum-exp, loss
     labels = labels.reshape(-1).to(torch.int64).contiguous()
+    mx, se, target, lse, loss = rows.unbind(0)
     xa = _lib.XentArgs(mode=1, labels=labels.data_ptr(), vocab_start=int(vocab_start), ignore_index=int(ignore_index),
                        stats=stats.data_ptr(), target=target.data_ptr(), lse=0, gscale=0)
     _lib.check(_lib.lib().gv_gemm_xent(_head_args(x, W, None), xa, _lib.stream_ptr()), "gv_gemm_xent(stats)")
-    mx = stats[:, :, 0].max(dim=1).values
-    se = (stats[:, :, 1] * torch.exp(stats[:, :, 0] - mx.unsqueeze(1))).sum(dim=1)
-    return mx, se, target
+    _lib.check(_lib.lib().gv_xent_merge(stats.data_ptr(), tiles, labels.data_ptr(), int(vocab_start), N, int(ignore_index), mx.data_ptr(),
+                                        se.data_ptr(), target.data_ptr(), lse.data_ptr() if finish else 0,
+                                        loss.data_ptr() if finish else 0, M, _lib.stream_ptr()), "gv_xent_merge")
+    return mx, se, target, lse, loss
+
+
+def head_xent_stats(x: torch.Tensor, W: torch.Tensor, labels: torch.Tensor, vocab_start: int = 0, ignore_index: int = -100):
+    """Language-model head forward without logits: per row (max, sum exp(logit - max), target logit or 0) over this
+    rank's vocabulary shard ``W`` [V_local, K], computed in the epilogue of the head GEMM from its fp32 accumulators."""
+    return _head_stats(x, W, labels, vocab_start, ignore_index, False)[:3]
+
+
+def head_xent_loss(x: torch.Tensor, W: torch.Tensor, labels: torch.Tensor, vocab_start: int = 0, ignore_index: int = -100):
+    """(loss, log-sum-exp) per row where ``W`` is the whole vocabulary; ignored rows have loss 0."""
+    _, _, _, lse, loss = _head_stats(x, W, labels, vocab_start, ignore_index, True)
+    return loss, lse
 
 
 def head_xent_grad(x: torch.Tensor, W: torch.Tensor, labels: torch.Tensor, lse: torch.Tensor, gscale: torch.Tensor,
                    vocab_start: int = 0, ignore_index: int = -100) -> torch.Tensor:
     """d loss / d logits (bf16 [M, V_local]) from recomputed logits: (softmax - onehot) * gscale[row], written by the
-    epilogue of the head GEMM; ``lse`` is the log-sum-exp over the whole vocabulary."""
+    epilogue of the head GEMM; ``lse`` is the log-sum-exp over the whole vocabulary. Rows with an ignored label give 0."""
     M, N = x.shape[0], W.shape[0]
     out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
     labels = labels.reshape(-1).to(torch.int64).contiguous()

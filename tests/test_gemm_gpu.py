@@ -307,3 +307,69 @@ def test_gated_activation_extremes():
     v = x[:, :1].double()
     ref = v * torch.sigmoid(v) * v
     assert ((act.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(27, 40, 64), (300, 264, 128), (6939, 1280, 64), (8192, 5120, 72)])
+def test_gelu_epilogue(M, N, K):
+    """Projection and its GELU from one launch: the projection bit-equal to the plain one, the activation that of the stored
+    values in 64 bits; 128-wide tiles, 256-wide tiles and pairs, tails of rows and columns, far negative and positive values."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16, generator=g)
+    w = torch.randn(N, K, device="cuda", dtype=torch.bfloat16, generator=g)
+    bias = torch.randn(N, device="cuda", dtype=torch.bfloat16, generator=g)
+    act = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    up = gemm(x, w, bias=bias, gelu_out=act)
+    assert torch.equal(up, gemm(x, w, bias=bias))
+    v = up.double()
+    z = 2 * (2 / torch.pi) ** 0.5 * (v + 0.044715 * v ** 3)
+    ref = v * torch.sigmoid(z)              # = v (1 + tanh(z / 2)) / 2, which loses everything to cancellation left of -5
+    # one rounding to bf16; in fp32 exp(-z) carries |z| roundings of its argument, |z| < 90 where the result does not vanish
+    assert ((act.double() - ref).abs() <= (2.0 ** -8 + 1e-4) * ref.abs() + 1e-30).all()
+    assert _lib.read_error() is None
+
+
+@pytest.mark.parametrize("rows,V,vocab_start", [(1, 40, 0), (33, 1000, 0), (300, 8192 + 264, 512)])
+def test_head_statistics_merge(rows, V, vocab_start):
+    """Loss and log-sum-exp from the merged tile statistics, with ignored labels and labels outside the shard."""
+    from hetu_galvatron_b200.ops.gemm import head_xent_grad, head_xent_loss, head_xent_stats
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, 64, device="cuda", dtype=torch.bfloat16, generator=g)
+    w = torch.randn(V, 64, device="cuda", dtype=torch.bfloat16, generator=g)
+    labels = torch.randint(0, vocab_start + V + 7, (rows,), device="cuda", generator=g)
+    labels[::5] = -100
+    logits = x.double() @ w.double().t()
+    lse = torch.logsumexp(logits, 1)
+    local = labels - vocab_start
+    here = (labels != -100) & (local >= 0) & (local < V)
+    tg = torch.where(here, logits.gather(1, local.clamp(0, V - 1)[:, None])[:, 0], torch.zeros_like(lse))
+    mx, se, t = head_xent_stats(x, w, labels, vocab_start)
+    assert torch.allclose(torch.log(se.double()) + mx.double(), lse, atol=2e-5 * lse.abs().max().item())
+    assert torch.allclose(t.double(), tg, atol=1e-4)
+    loss, l = head_xent_loss(x, w, labels, vocab_start)
+    assert torch.allclose(l.double(), lse, atol=2e-5 * lse.abs().max().item())
+    assert torch.allclose(loss.double(), torch.where(labels != -100, lse - tg, torch.zeros_like(lse)), atol=2e-4)
+    d = head_xent_grad(x, w, labels, l, torch.ones(rows, device="cuda"), vocab_start)
+    assert (d[labels == -100] == 0).all()
+
+
+@pytest.mark.parametrize("dh,s,hq,hk", [(50, 33, 3, 3), (2, 5, 1, 1), (74, 130, 4, 2), (25, 40, 2, 2)])
+def test_heads_padded_around_attention(dh, s, hq, hk):
+    """Head sizes that are no multiple of 8, as strided views of a packed projection: forward and backward against 64 bits."""
+    from hetu_galvatron_b200.ops import autograd as A
+    g = torch.Generator(device="cuda").manual_seed(dh)
+    b = 2
+    qkv = torch.randn(s * b, (hq + 2 * hk) * dh + (-(hq + 2 * hk) * dh) % 8, device="cuda", dtype=torch.bfloat16, generator=g)[:, :(hq + 2 * hk) * dh]
+    qkv = qkv.contiguous().requires_grad_()
+    do = torch.randn(s * b, hq * dh, device="cuda", dtype=torch.bfloat16, generator=g)
+    o = A.packed_attention(qkv, A.AttnCfg(batch=b, hq=hq, hk=hk, dh=dh, causal=True))
+    grad, = torch.autograd.grad(o, qkv, do)
+    x = qkv.detach().double().requires_grad_()
+    v = x.view(s, b, hq + 2 * hk, dh).permute(1, 2, 0, 3)
+    q, k, vv = v[:, :hq], v[:, hq:hq + hk].repeat_interleave(hq // hk, 1), v[:, hq + hk:].repeat_interleave(hq // hk, 1)
+    sc = (q @ k.transpose(-1, -2)) / dh ** 0.5
+    p = sc.masked_fill(~torch.ones(s, s, dtype=torch.bool, device="cuda").tril(), float("-inf")).softmax(-1)
+    ref = (p @ vv).permute(2, 0, 1, 3).reshape(s * b, hq * dh)
+    rg, = torch.autograd.grad(ref, x, do.double())
+    for got, want in ((o, ref), (grad, rg)):
+        # bf16 probabilities, score gradients and results
+        assert ((got.double() - want).norm() / want.norm()).item() < 1e-2
