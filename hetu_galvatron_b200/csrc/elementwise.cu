@@ -198,19 +198,73 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const bf
   }
 }
 
+// Adds eight bf16 gradients to eight fp32 sums in global memory: two vector reductions (16-byte aligned sums) instead of eight
+// scalar ones, which were what the scatter waited for: 8192 tokens of 4096 columns 199 -> 73 us.
+__device__ __forceinline__ void red_add8(float* dst, const uint4& u, bool aligned) {
+  float a[8];
+  unpack8e(u, a);
+  if (aligned) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a[0]), "f"(a[1]), "f"(a[2]), "f"(a[3]) : "memory");
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4), "f"(a[4]), "f"(a[5]), "f"(a[6]), "f"(a[7]) : "memory");
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) atomicAdd(dst + e, a[e]);
+  }
+}
+
 __global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__ dout,
                                      float* __restrict__ dtable, long long tokens, int hidden, long long vocab_start,
                                      long long vocab_rows) {
   const int vec = hidden >> 3;
+  const bool aligned = (reinterpret_cast<uintptr_t>(dtable) & 15) == 0;
   for (long long t = blockIdx.x; t < tokens; t += gridDim.x) {
     const long long id = ids[t] - vocab_start;
     if (id < 0 || id >= vocab_rows) continue;
     float* dst = dtable + id * hidden;
+    for (int i = threadIdx.x; i < vec; i += blockDim.x) red_add8(dst + i * 8, reinterpret_cast<const uint4*>(dout + t * hidden)[i], aligned);
+  }
+}
+
+// Gradient of a table with a bf16 gradient buffer: the rows of one id are summed in fp32 in `sums` (one row per token, zeroed) at
+// the id's first-come token, which `owner` (one entry per table row, -1) remembers; then each owner's sum is rounded into the
+// buffer once. The sums of a whole [vocab, hidden] table need not be cleared, converted and added: 8192 tokens, 32000 x 4096
+// 500 -> 137 us.
+__global__ void embedding_sum_rows_kernel(const long long* __restrict__ ids, const bf16* __restrict__ dout, int* __restrict__ owner,
+                                          float* __restrict__ sums, long long tokens, int hidden, long long vocab_start,
+                                          long long vocab_rows) {
+  __shared__ int s_owner;
+  const int vec = hidden >> 3;
+  for (long long t = blockIdx.x; t < tokens; t += gridDim.x) {
+    const long long id = ids[t] - vocab_start;
+    if (id < 0 || id >= vocab_rows) continue;          // the same for the whole block
+    if (threadIdx.x == 0) {
+      const int was = atomicCAS(owner + id, -1, static_cast<int>(t));
+      s_owner = was < 0 ? static_cast<int>(t) : was;
+    }
+    __syncthreads();
+    float* dst = sums + static_cast<long long>(s_owner) * hidden;
+    for (int i = threadIdx.x; i < vec; i += blockDim.x) red_add8(dst + i * 8, reinterpret_cast<const uint4*>(dout + t * hidden)[i], true);
+    __syncthreads();
+  }
+}
+
+__global__ void embedding_add_rows_kernel(const long long* __restrict__ ids, const int* __restrict__ owner, const float* __restrict__ sums,
+                                          bf16* __restrict__ dtable, long long tokens, int hidden, long long vocab_start,
+                                          long long vocab_rows) {
+  const int vec = hidden >> 3;
+  for (long long t = blockIdx.x; t < tokens; t += gridDim.x) {
+    const long long id = ids[t] - vocab_start;
+    if (id < 0 || id >= vocab_rows || owner[id] != static_cast<int>(t)) continue;
+    uint4* dst = reinterpret_cast<uint4*>(dtable + id * hidden);
+    const float4* src = reinterpret_cast<const float4*>(sums + t * hidden);
     for (int i = threadIdx.x; i < vec; i += blockDim.x) {
+      const float4 x = src[2 * i], y = src[2 * i + 1];
+      const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
       float a[8];
-      unpack8e(reinterpret_cast<const uint4*>(dout + t * hidden)[i], a);
+      unpack8e(dst[i], a);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) atomicAdd(dst + i * 8 + e, a[e]);
+      for (int e = 0; e < 8; ++e) a[e] += __bfloat162float(__float2bfloat16(v[e]));     // the sum is rounded before it is added
+      dst[i] = pack8e(a);
     }
   }
 }
@@ -614,6 +668,22 @@ extern "C" int gv_embedding_bwd(const long long* ids, const void* dout, float* d
   int grid = (int)(tokens < (long long)num_sms() * 16 ? tokens : (long long)num_sms() * 16);
   embedding_bwd_kernel<<<grid, 128, 0, (cudaStream_t)s>>>(ids, (const bf16*)dout, dtable, tokens, hidden, vocab_start,
                                                           vocab_rows);
+  return (int)cudaGetLastError();
+}
+
+extern "C" int gv_embedding_bwd_bf16(const long long* ids, const void* dout, void* dtable, int* owner, float* sums, long long tokens,
+                                     int hidden, long long vocab_start, long long vocab_rows, gv_stream_t s) {
+  if (tokens <= 0 || vocab_rows <= 0) return 0;
+  if (hidden % 8) return 2205;
+  if (tokens > 0x7fffffff || ((reinterpret_cast<uintptr_t>(dtable) | reinterpret_cast<uintptr_t>(sums) | reinterpret_cast<uintptr_t>(dout)) & 15))
+    return 2208;
+  cudaStream_t st = (cudaStream_t)s;
+  cudaError_t e = cudaMemsetAsync(owner, 0xff, sizeof(int) * static_cast<size_t>(vocab_rows), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(sums, 0, sizeof(float) * static_cast<size_t>(tokens) * hidden, st);
+  if (e != cudaSuccess) return (int)e;
+  const int grid = (int)(tokens < (long long)num_sms() * 16 ? tokens : (long long)num_sms() * 16);
+  embedding_sum_rows_kernel<<<grid, 128, 0, st>>>(ids, (const bf16*)dout, owner, sums, tokens, hidden, vocab_start, vocab_rows);
+  embedding_add_rows_kernel<<<grid, 128, 0, st>>>(ids, owner, sums, (bf16*)dtable, tokens, hidden, vocab_start, vocab_rows);
   return (int)cudaGetLastError();
 }
 

@@ -128,6 +128,11 @@ int gv_embedding_fwd(const long long* ids, const void* table, const int* pos_ids
 int gv_embedding_bwd(const long long* ids, const void* dout, float* dtable_accum, long long tokens, int hidden,
                      long long vocab_start, long long vocab_rows, gv_stream_t stream);
 
+// The same into a bf16 table gradient (16-byte aligned): the rows of an id are summed in fp32, rounded, and added once.
+// owner: int32 [vocab_rows], sums: fp32 [tokens, hidden] (16-byte aligned), both uninitialised scratch.
+int gv_embedding_bwd_bf16(const long long* ids, const void* dout, void* dtable, int* owner, float* sums, long long tokens, int hidden,
+                          long long vocab_start, long long vocab_rows, gv_stream_t stream);
+
 // ---- cross entropy over (a vocab shard of) logits -------------------------------------
 // Pass 1: per-row partial statistics over the local vocab shard: row_max, row_sumexp (relative to row_max),
 //         target_logit (0 if the label is not in this shard).

@@ -17,7 +17,8 @@ _LIB = None
 
 # Kernel launches per library call (for launch accounting in benchmarks).
 KERNELS_PER_CALL = {"gv_attn_bwd": 3, "gv_read_error": 0, "gv_norm_bwd_scratch_elems": 0, "gv_rmsnorm_bwd": 2,
-                    "gv_layernorm_bwd": 2, "gv_device_sm_count": 0, "gv_gemm_workspace_bytes": 0}
+                    "gv_layernorm_bwd": 2, "gv_device_sm_count": 0, "gv_gemm_workspace_bytes": 0,
+                    "gv_embedding_bwd_bf16": 2}
 LAUNCH_COUNT = 0
 
 
@@ -106,6 +107,7 @@ PROTOTYPES = {
     "gv_colsum_accum": [_P, _P, _L, _I, _P],
     "gv_embedding_fwd": [_P] * 5 + [_L, _I, _L, _L, _P],
     "gv_embedding_bwd": [_P] * 3 + [_L, _I, _L, _L, _P],
+    "gv_embedding_bwd_bf16": [_P] * 5 + [_L, _I, _L, _L, _P],
     "gv_xent_stats": [_P] * 5 + [_L, _I, _L, _L, _P],
     "gv_xent_loss_grad": [_P] * 6 + [_F, _P, _L, _I, _L, _L, _L, _P],
     "gv_xent_merge": [_P, _I, _P, _L, _L, _L] + [_P] * 5 + [_L, _P],

@@ -617,9 +617,7 @@ class EmbeddingFn(torch.autograd.Function):
                 if mg.dtype == torch.float32:
                     Fn.embedding_bwd(idx, dout, mg.view(tbl.shape), start)
                 else:
-                    tmp = torch.zeros(tbl.shape, dtype=torch.float32, device=tbl.device)
-                    Fn.embedding_bwd(idx, dout, tmp, start)
-                    mg.view(tbl.shape).add_(tmp.to(mg.dtype))
+                    Fn.embedding_bwd_bf16(idx, dout, mg.view(tbl.shape), start)
 
             def fresh():
                 tmp = torch.zeros(tbl.shape, dtype=torch.float32, device=tbl.device)

@@ -273,6 +273,27 @@ def embedding_bwd(ids: torch.Tensor, dout: torch.Tensor, dtable_accum: torch.Ten
     dtable_accum.index_add_(0, local[mask], d)
 
 
+def embedding_bwd_bf16(ids: torch.Tensor, dout: torch.Tensor, dtable: torch.Tensor, vocab_start: int = 0) -> None:
+    """Adds the table gradient, summed per id in fp32, to the bf16 gradient buffer ``dtable`` [rows, hidden]. Summing per token
+    pays while the tokens are fewer than half of the table's rows (its scratch is [tokens, hidden], not [rows, hidden])."""
+    hidden = dtable.shape[1]
+    flat = ids.reshape(-1)
+    if (_native(dout) and dtable.dtype == torch.bfloat16 and hidden % 8 == 0 and 0 < 2 * flat.numel() <= dtable.shape[0]
+            and dtable.is_contiguous() and dtable.data_ptr() % 16 == 0):
+        flat = flat.to(torch.int64).contiguous()
+        dout = dout.contiguous()
+        if dout.data_ptr() % 16 == 0:
+            owner = torch.empty(dtable.shape[0], dtype=torch.int32, device=dout.device)
+            sums = torch.empty(flat.numel(), hidden, dtype=torch.float32, device=dout.device)
+            rc = _lib.lib().gv_embedding_bwd_bf16(_vp(flat), _vp(dout), _vp(dtable), _vp(owner), _vp(sums), flat.numel(), hidden,
+                                                  vocab_start, dtable.shape[0], _s())
+            _lib.check(rc, "gv_embedding_bwd_bf16")
+            return
+    tmp = torch.zeros(dtable.shape, dtype=torch.float32, device=dtable.device)
+    embedding_bwd(ids, dout, tmp, vocab_start)
+    dtable.add_(tmp.to(dtable.dtype))
+
+
 # ----------------------------------------------------------------------------- cross entropy
 def xent_stats(logits: torch.Tensor, labels: torch.Tensor, vocab_start: int = 0):
     """Per-row (max, sum exp(x - max), target logit or 0) over this rank's vocab shard."""

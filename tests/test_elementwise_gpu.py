@@ -211,3 +211,27 @@ def test_adamw_and_sumsq():
     gb = torch.randn(n, device=DEV).bfloat16()
     Fn.sumsq_accum(gb, out)
     assert abs(out.item() - gb.float().pow(2).sum().item()) / out.item() < 1e-3
+
+
+@pytest.mark.parametrize("tokens,V,H,vocab_start", [(1, 2, 8, 0), (300, 1000, 264, 0), (300, 1000, 264, 500), (700, 4000, 1600, 0), (600, 1000, 64, 0)])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_embedding_gradient_buffers(tokens, V, H, vocab_start, offset):
+    """Gradients of repeated, missing and foreign ids added to fp32 and bf16 buffers, at bases that are and are not 16-byte aligned
+    (the last size has too many tokens for the per-token sums), against sums in 64 bits."""
+    g = torch.Generator(device=DEV).manual_seed(tokens + V)
+    ids = torch.randint(0, vocab_start + V + 3, (tokens,), device=DEV, generator=g)
+    ids[::3] = vocab_start + 1                        # a third of the tokens is one id
+    dout = torch.randn(tokens, H, device=DEV, dtype=torch.bfloat16, generator=g)
+    local = ids - vocab_start
+    inside = (local >= 0) & (local < V)
+    total = torch.zeros(V, H, dtype=torch.float64, device=DEV).index_add_(0, local[inside], dout[inside].double())
+    size = torch.zeros(V, H, dtype=torch.float64, device=DEV).index_add_(0, local[inside], dout[inside].double().abs())
+    for dtype in (torch.float32, torch.bfloat16):
+        buf = torch.randn(V * H + 8, device=DEV, generator=g).to(dtype)[offset:offset + V * H].view(V, H)
+        old = buf.clone()
+        (Fn.embedding_bwd if dtype == torch.float32 else Fn.embedding_bwd_bf16)(ids, dout, buf, vocab_start)
+        ref = old.double() + total
+        # fp32 sums of up to `tokens` terms; in bf16 one rounding of the sum and one of the result
+        bound = tokens * 2.0 ** -23 * (size + old.double().abs()) + (0 if dtype == torch.float32 else 2.0 ** -8 * (total.abs() + ref.abs()))
+        assert ((buf.double() - ref).abs() <= bound + 1e-12).all()
+        assert torch.equal(buf[size.sum(1) == 0], old[size.sum(1) == 0])
