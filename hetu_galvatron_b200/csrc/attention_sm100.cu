@@ -416,6 +416,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_arrive(p_full);
     }
     // epilogue
+    // the last product, by way of the one before it: the softmax may be two products ahead, where the last one's parity alone
+    // would still match that of the phase before the previous one
+    if (ok && n_blocks > 1) ok = mbar_wait(pv_done, n_blocks & 1, abort_flag, 0x1a);
     if (ok && n_blocks > 0) ok = mbar_wait(pv_done, (n_blocks - 1) & 1, abort_flag, 0x1a);
     tc_fence_after();
     const float inv_l = l > 0.f ? 1.f / l : 0.f;

@@ -186,3 +186,18 @@ def test_attention_with_bias_mask_and_group_ids(b, s, h, dh, mask_n, with_bias, 
         hidden = (ids[:, :, None] != ids[:, None, :]).all(dim=0)       # hidden in every window position
         if hidden.any():
             assert grads[3].float()[:, hidden].abs().max().item() == 0.0
+
+
+@pytest.mark.parametrize("b,s,hq,hk,dh,causal", [(1, 16384, 16, 4, 128, True), (2, 4096, 16, 16, 64, True), (4, 333, 8, 8, 64, False)])
+def test_forward_repeats_bit_for_bit(b, s, hq, hk, dh, causal):
+    """The output of a tile is read when its last product is done, however far the softmax has run ahead: thousands of tiles, short
+    and long, give the same bits again and again."""
+    from hetu_galvatron_b200.ops import _lib, attention as AT
+    g = torch.Generator(device="cuda").manual_seed(s)
+    q = torch.randn(b, s, hq, dh, device="cuda", dtype=torch.bfloat16, generator=g)
+    k, v = (torch.randn(b, s, hk, dh, device="cuda", dtype=torch.bfloat16, generator=g) for _ in range(2))
+    first, lse = AT.fwd(q, k, v, causal, dh ** -0.5)
+    for _ in range(24):
+        o, l = AT.fwd(q, k, v, causal, dh ** -0.5)
+        assert torch.equal(o, first) and torch.equal(l, lse)
+    assert _lib.read_error() is None
