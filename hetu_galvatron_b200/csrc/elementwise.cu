@@ -46,37 +46,52 @@ static inline int grid_for(long long work_items, int threads, int ctas_per_sm = 
 }
 
 // ------------------------------------------------------------------ RoPE
-// One thread rotates 8 consecutive pairs (i, i + dh/2) of one (token, head).
+// One thread rotates 8 consecutive pairs (i, i + dh/2) in a run of heads of one token: the angles do not depend on the head, so
+// they are computed once per run. HBM-bound with runs of four heads: 8192 x 32 heads of 128 in place took 39 us with sincosf for
+// every head and now takes 24 (L2 cold).
+constexpr int ROPE_RUN = 4;
 __global__ void rope_kernel(bf16* __restrict__ x, const int* __restrict__ pos, const float* __restrict__ inv_freq,
                             long long tokens, int heads, int dh, long long ld, int pos_div, int pos_mod,
                             int pos_offset, int inverse) {
   const int half = dh >> 1;
   const int vec_per_head = half >> 3;
-  const long long total = tokens * heads * vec_per_head;
+  const int runs = (heads + ROPE_RUN - 1) / ROPE_RUN, per_token = runs * vec_per_head;
+  const long long total = tokens * per_token;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
        idx += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int vi = static_cast<int>(idx % vec_per_head);
-    const long long th = idx / vec_per_head;
-    const int h = static_cast<int>(th % heads);
-    const long long t = th / heads;
+    const long long t = idx / per_token;
+    const int rest = static_cast<int>(idx - t * per_token);
+    const int vi = rest % vec_per_head, h0 = rest / vec_per_head * ROPE_RUN;
     const float p = pos ? static_cast<float>(pos[t])
                         : static_cast<float>(static_cast<int>((t / pos_div) % pos_mod) + pos_offset);
-    bf16* base = x + t * ld + static_cast<long long>(h) * dh + vi * 8;
-    uint4 u1 = *reinterpret_cast<uint4*>(base);
-    uint4 u2 = *reinterpret_cast<uint4*>(base + half);
-    float a[8], b[8], oa[8], ob[8];
-    unpack8e(u1, a);
-    unpack8e(u2, b);
+    float s[8], c[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      float s, c;
-      sincosf(p * __ldg(inv_freq + vi * 8 + e), &s, &c);
-      if (inverse) s = -s;
-      oa[e] = a[e] * c - b[e] * s;
-      ob[e] = b[e] * c + a[e] * s;
+      sincos_any(p * __ldg(inv_freq + vi * 8 + e), s[e], c[e]);
+      if (inverse) s[e] = -s[e];
     }
-    *reinterpret_cast<uint4*>(base) = pack8e(oa);
-    *reinterpret_cast<uint4*>(base + half) = pack8e(ob);
+    bf16* base = x + t * ld + static_cast<long long>(h0) * dh + vi * 8;
+    uint4 u1[ROPE_RUN], u2[ROPE_RUN];
+#pragma unroll
+    for (int r = 0; r < ROPE_RUN; ++r) {
+      if (h0 + r >= heads) break;
+      u1[r] = *reinterpret_cast<uint4*>(base + r * dh);
+      u2[r] = *reinterpret_cast<uint4*>(base + r * dh + half);
+    }
+#pragma unroll
+    for (int r = 0; r < ROPE_RUN; ++r) {
+      if (h0 + r >= heads) break;
+      float a[8], b[8], oa[8], ob[8];
+      unpack8e(u1[r], a);
+      unpack8e(u2[r], b);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        oa[e] = a[e] * c[e] - b[e] * s[e];
+        ob[e] = b[e] * c[e] + a[e] * s[e];
+      }
+      *reinterpret_cast<uint4*>(base + r * dh) = pack8e(oa);
+      *reinterpret_cast<uint4*>(base + r * dh + half) = pack8e(ob);
+    }
   }
 }
 
@@ -93,7 +108,7 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
     unpack8e(*reinterpret_cast<const uint4*>(g), a);
     unpack8e(*reinterpret_cast<const uint4*>(g + f), b);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = a[e] / (1.f + __expf(-a[e])) * b[e];
+    for (int e = 0; e < 8; ++e) o[e] = a[e] * sigmoid_nb(a[e]) * b[e];
     *reinterpret_cast<uint4*>(out + r * f + c) = pack8e(o);
   }
 }
@@ -113,7 +128,7 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __r
     unpack8e(*reinterpret_cast<const uint4*>(dout + r * f + c), d);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float sg = 1.f / (1.f + __expf(-a[e]));
+      const float sg = sigmoid_nb(a[e]);
       const float silu = a[e] * sg;
       da[e] = d[e] * b[e] * (sg + silu * (1.f - sg));
       db[e] = d[e] * silu;
@@ -605,7 +620,7 @@ extern "C" int gv_rope(void* x, const int* pos, const float* inv_freq, long long
                        long long ld, int pos_div, int pos_mod, int pos_offset, int inverse, gv_stream_t s) {
   if (tokens <= 0) return 0;
   if (dh % 16 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15)) return 2201;
-  const long long total = tokens * heads * (dh / 16);
+  const long long total = tokens * ((heads + ROPE_RUN - 1) / ROPE_RUN) * (dh / 16);
   rope_kernel<<<grid_for(total, 256), 256, 0, (cudaStream_t)s>>>((bf16*)x, pos, inv_freq, tokens, heads, dh, ld,
                                                                  pos_div > 0 ? pos_div : 1,
                                                                  pos_mod > 0 ? pos_mod : 0x7fffffff, pos_offset,
@@ -734,6 +749,11 @@ extern "C" int gv_sumsq_accum(const void* x, int is_bf16, long long n, float* ou
   else
     sumsq_kernel<false><<<grid, 256, 0, (cudaStream_t)s>>>(x, n, out);
   return (int)cudaGetLastError();
+}
+
+extern "C" int gv_zero(void* ptr, long long bytes, gv_stream_t s) {
+  if (bytes <= 0) return 0;
+  return (int)cudaMemsetAsync(ptr, 0, static_cast<size_t>(bytes), (cudaStream_t)s);
 }
 
 extern "C" int gv_cast_f32_to_bf16(const float* in, void* out, long long n, float scale, gv_stream_t s) {

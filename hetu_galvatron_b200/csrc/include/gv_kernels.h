@@ -161,6 +161,8 @@ int gv_adamw(float* master, float* m, float* v, const void* grad, int grad_is_bf
              float grad_scale, const float* clip_coef, gv_stream_t stream);
 // sum of squares of a flat buffer accumulated into out[0] (fp32, atomic)
 int gv_sumsq_accum(const void* x, int is_bf16, long long n, float* out, gv_stream_t stream);
+// clears `bytes` bytes
+int gv_zero(void* ptr, long long bytes, gv_stream_t stream);
 // casts / scaling
 int gv_cast_f32_to_bf16(const float* in, void* out, long long n, float scale, gv_stream_t stream);
 int gv_cast_bf16_to_f32(const void* in, float* out, long long n, float scale, int accumulate, gv_stream_t stream);

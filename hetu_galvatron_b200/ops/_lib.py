@@ -17,7 +17,7 @@ _LIB = None
 
 # Kernel launches per library call (for launch accounting in benchmarks).
 KERNELS_PER_CALL = {"gv_attn_bwd": 3, "gv_read_error": 0, "gv_norm_bwd_scratch_elems": 0, "gv_rmsnorm_bwd": 2,
-                    "gv_layernorm_bwd": 2, "gv_device_sm_count": 0, "gv_gemm_workspace_bytes": 0,
+                    "gv_layernorm_bwd": 2, "gv_device_sm_count": 0, "gv_gemm_workspace_bytes": 0, "gv_zero": 0,
                     "gv_embedding_bwd_bf16": 2}
 LAUNCH_COUNT = 0
 
@@ -113,6 +113,7 @@ PROTOTYPES = {
     "gv_xent_merge": [_P, _I, _P, _L, _L, _L] + [_P] * 5 + [_L, _P],
     "gv_adamw": [_P, _P, _P, _P, _I, _P, _L] + [_F] * 8 + [_P, _P],
     "gv_sumsq_accum": [_P, _I, _L, _P, _P],
+    "gv_zero": [_P, _L, _P],
     "gv_lse_merge": [_P] * 4 + [_I] * 6 + [_L, _L, _L, _P],
 }
 

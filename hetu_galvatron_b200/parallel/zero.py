@@ -421,7 +421,7 @@ class ParamBucket:
             self._fused_clear_grad()
             self.fused.shard_valid = False
         elif self.grad_flat is not None:
-            self.grad_flat.zero_()
+            Fn.zero_(self.grad_flat)
         if self.dp_type != "ddp" or self.d == 1:
             self.grad_shard = None if self.d > 1 else self.grad_flat
         self.reduced = False

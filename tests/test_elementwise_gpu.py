@@ -235,3 +235,22 @@ def test_embedding_gradient_buffers(tokens, V, H, vocab_start, offset):
         bound = tokens * 2.0 ** -23 * (size + old.double().abs()) + (0 if dtype == torch.float32 else 2.0 ** -8 * (total.abs() + ref.abs()))
         assert ((buf.double() - ref).abs() <= bound + 1e-12).all()
         assert torch.equal(buf[size.sum(1) == 0], old[size.sum(1) == 0])
+
+
+@pytest.mark.parametrize("tokens,heads,dh", [(1, 1, 16), (33, 3, 64), (70, 9, 128), (300, 4, 80)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_rope_runs_of_heads(tokens, heads, dh, inverse):
+    """In-place rotation of a strided view, head counts that are no multiple of a run, positions on both sides of the limit of the
+    branch-free sines, against the rotation in 64 bits of the same fp32 angles."""
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    buf = torch.randn(tokens, heads + 2, dh, device=DEV, dtype=torch.bfloat16, generator=g)
+    old = buf.double()
+    pos = torch.randint(0, 200000, (tokens,), device=DEV, dtype=torch.int32, generator=g)
+    freq = 1.0 / (10000.0 ** (torch.arange(0, dh, 2, device=DEV).float() / dh))
+    Fn.rope_(buf[:, :heads], freq, positions=pos, inverse=inverse)
+    ang = (pos.float()[:, None] * freq[None]).double()[:, None]
+    a, b, sn = old[:, :heads, :dh // 2], old[:, :heads, dh // 2:], ang.sin() * (-1 if inverse else 1)
+    ref = torch.cat([a * ang.cos() - b * sn, b * ang.cos() + a * sn], -1)
+    # one rounding to bf16, sines to 1e-7
+    assert ((buf[:, :heads].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6 * (a.abs() + b.abs() + 1).repeat(1, 1, 2)).all()
+    assert torch.equal(buf[:, heads:].double(), old[:, heads:])
