@@ -165,9 +165,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* v_full = bars + 3;    // [2]
   uint64_t* kv_empty = bars + 5;  // [2]
   uint64_t* s_full = bars + 7;    // [2]
-  uint64_t* p_full = bars + 9;
-  uint64_t* pv_done = bars + 10;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  // one per score buffer: a warp that is a block ahead of another must not arrive in its place
+  uint64_t* p_full = bars + 9;    // [2]
+  uint64_t* pv_done = bars + 11;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   if (static_cast<int>(smem - smem_raw) + S::OFF_BAR + 128 > S::TOTAL) {  // dynamic smem base less aligned than assumed
@@ -197,8 +198,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&v_full[i], 1);
       mbar_init(&kv_empty[i], 1);
       mbar_init(&s_full[i], 1);
+      mbar_init(&p_full[i], 128);
     }
-    mbar_init(p_full, 128);
     mbar_init(pv_done, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -272,7 +273,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           issue_s(jn);
         }
         if (!mbar_wait(&v_full[j & 1], (j >> 1) & 1, abort_flag, 0x16)) { ok = false; break; }
-        if (!mbar_wait(p_full, j & 1, abort_flag, 0x17)) { ok = false; break; }
+        if (!mbar_wait(&p_full[j & 1], (j >> 1) & 1, abort_flag, 0x17)) { ok = false; break; }
         tc_fence_after();
         const uint64_t v_desc = v_desc0 + static_cast<uint64_t>((j & 1) * (S::KV_BYTES >> 4));
 #pragma unroll
@@ -413,7 +414,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         l = la + lb;
       }
       tc_fence_before();
-      mbar_arrive(p_full);
+      mbar_arrive(&p_full[j & 1]);
     }
     // epilogue
     // the last product, by way of the one before it: the softmax may be two products ahead, where the last one's parity alone

@@ -201,3 +201,21 @@ def test_forward_repeats_bit_for_bit(b, s, hq, hk, dh, causal):
         o, l = AT.fwd(q, k, v, causal, dh ** -0.5)
         assert torch.equal(o, first) and torch.equal(l, lse)
     assert _lib.read_error() is None
+
+
+def test_windowed_forward_repeats_bit_for_bit():
+    """The same with bias and group ids, whose loads let the warps of a tile drift a block apart: no warp's probabilities may be
+    taken for written before they are."""
+    from hetu_galvatron_b200.ops import _lib, attention as AT
+    g = torch.Generator(device="cuda").manual_seed(0)
+    qkv = torch.randn(256, 144, 3, 6, 32, device="cuda", dtype=torch.bfloat16, generator=g)
+    bias = torch.randn(6, 144, 144, device="cuda", generator=g).bfloat16()
+    ids = torch.randint(0, 4, (64, 144), device="cuda", generator=g)
+    add = AT.Additive(144, 144, bias, None, ids)
+    q, k, v = qkv.unbind(2)
+    first, lse = AT.fwd(q, k, v, False, 32 ** -0.5, additive=add)
+    assert torch.isfinite(first.float()).all()
+    for _ in range(60):
+        o, l = AT.fwd(q, k, v, False, 32 ** -0.5, additive=add)
+        assert torch.equal(o, first) and torch.equal(l, lse)
+    assert _lib.read_error() is None
