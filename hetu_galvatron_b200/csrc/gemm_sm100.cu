@@ -1288,7 +1288,8 @@ extern "C" int gv_gemm_bf16(const gv_gemm_args* a, gv_stream_t s) {
   using namespace gv;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(s);
   if (a->M <= 0 || a->N <= 0 || a->K <= 0) return 0;
-  if ((a->K % 8) || (a->lda % 8) || (a->ldb % 8) || (a->ldc % (a->c_f32 ? 4 : 8))) return 2001;
+  // K only counts rows of operands that are both stored along M and N: any number of them (zeros are read beyond the last)
+  if ((a->K % 8 && !(a->a_mn_major && a->b_mn_major)) || (a->lda % 8) || (a->ldb % 8) || (a->ldc % (a->c_f32 ? 4 : 8))) return 2001;
   if ((reinterpret_cast<uintptr_t>(a->A) | reinterpret_cast<uintptr_t>(a->B) | reinterpret_cast<uintptr_t>(a->C)) & 15)
     return 2002;
   if (a->a_mn_major && (a->M % 8)) return 2003;

@@ -80,7 +80,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     elif out.shape != (M, N):
         out = out.view(M, N)
     native = _use_native(a, b, bias, residual) and out.dtype in (torch.bfloat16, torch.float32) \
-        and K % 8 == 0 and out.stride(1) == 1
+        and (K % 8 == 0 or a_mn and b_mn) and out.stride(1) == 1
     if native and (a_mn and M % 8 or b_mn and N % 8 or out.stride(0) % 8):
         native = False
     if native:
@@ -206,6 +206,6 @@ def head_xent_grad(x: torch.Tensor, W: torch.Tensor, labels: torch.Tensor, lse: 
 
 
 def _lib_fallback_allowed() -> bool:
-    # Odd shapes (K or leading dimensions not multiples of 8) only occur in tiny unit-test models;
+    # Odd shapes (leading dimensions, or K of a K-major operand, not multiples of 8) only occur in tiny unit-test models;
     # they take the PyTorch path instead of failing.
     return True

@@ -373,3 +373,20 @@ def test_heads_padded_around_attention(dh, s, hq, hk):
     for got, want in ((o, ref), (grad, rg)):
         # bf16 probabilities, score gradients and results
         assert ((got.double() - want).norm() / want.norm()).item() < 1e-2
+
+
+@pytest.mark.parametrize("M,N,K", [(72, 40, 1), (136, 264, 67), (1280, 592, 6939), (5120, 1280, 3003), (192, 768, 9217)])
+def test_weight_gradient_of_any_row_count(M, N, K):
+    """Operands stored along M and N reduce over any number of rows (of the last, smaller batch of an epoch): fp32 accumulation into
+    a gradient buffer on single CTAs, pairs and split reductions, against 64 bits."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    dy = torch.randn(K, M, device="cuda", dtype=torch.bfloat16, generator=g)
+    x = torch.randn(K, N, device="cuda", dtype=torch.bfloat16, generator=g)
+    buf = torch.randn(M, N, device="cuda", generator=g)
+    ref = buf.double() + dy.double().t() @ x.double()
+    size = buf.double().abs() + dy.double().abs().t() @ x.double().abs()
+    before = _lib.launch_count()
+    gemm(dy, x, a_mn=True, b_mn=True, out=buf, accumulate=True)
+    assert _lib.launch_count() == before + 1                 # the kernel, not the library
+    assert ((buf.double() - ref).abs() <= (K + 4) * 2.0 ** -23 * size).all()
+    assert _lib.read_error() is None
