@@ -16,6 +16,7 @@
 // two epilogue warpgroups write P^T back to TMEM and dS^T to shared memory, dV += P^T dO, dK += dS^T Q,
 // dQ^T = K^T dS^T is read back from TMEM and added into an fp32 dQ buffer with bulk reductions.
 // Every operand is consumed in the layout it has in shared memory (K-major or MN-major descriptors).
+#include "include/gv_attn_order.h"
 #include "include/gv_kernels.h"
 #include "include/gv_host.h"
 #include "include/gv_ptx.cuh"
@@ -167,8 +168,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* s_full = bars + 7;    // [2]
   // one per score buffer: a warp that is a block ahead of another must not arrive in its place
   uint64_t* p_full = bars + 9;    // [2]
-  uint64_t* pv_done = bars + 11;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  uint64_t* pv_done = bars + 11;  // [PV_BARRIERS], see pv_phase
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11 + PV_BARRIERS);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   if (static_cast<int>(smem - smem_raw) + S::OFF_BAR + 128 > S::TOTAL) {  // dynamic smem base less aligned than assumed
@@ -200,7 +201,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 128);
     }
-    mbar_init(pv_done, 1);
+    for (int i = 0; i < PV_BARRIERS; ++i) mbar_init(&pv_done[i], 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
@@ -215,6 +216,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  auto wait_pv = [&](int block, unsigned int site) {    // until P V of this block has been added to O
+    const PvPhase ph = pv_phase(block);
+    return mbar_wait(&pv_done[ph.barrier], ph.parity, abort_flag, site);
+  };
 
   if (warp == 0) {
     if (elect_one() && n_blocks > 0) {
@@ -268,7 +273,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const int jn = j + 1;
           if (!mbar_wait(&k_full[jn & 1], (jn >> 1) & 1, abort_flag, 0x14)) { ok = false; break; }
           // the buffer still holds P of two blocks ago until its product with V is done
-          if (j > 0 && !mbar_wait(pv_done, (j - 1) & 1, abort_flag, 0x15)) { ok = false; break; }
+          if (j > 0 && !wait_pv(j - 1, 0x15)) { ok = false; break; }
           tc_fence_after();
           issue_s(jn);
         }
@@ -282,7 +287,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           umma_f16_ts(tmem_base + TM_O, tmem_base + TM_S + (j & 1) * FWD_BN + kk * 8, db, idesc_pv, (j | kk) != 0 ? 1u : 0u);
         }
         umma_commit<1>(&kv_empty[j & 1]);
-        umma_commit<1>(pv_done);
+        umma_commit<1>(&pv_done[pv_phase(j).barrier]);
       }
     }
   } else {
@@ -365,7 +370,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const bool need = mx > m_used + 8.f;
         if (__any_sync(0xffffffffu, need)) {
           // only now does it matter that the previous block's product has been added to O
-          bool done = mbar_wait(pv_done, (j - 1) & 1, abort_flag, 0x19);
+          const bool done = wait_pv(j - 1, 0x19);
           if (!__all_sync(0xffffffffu, done)) { ok = false; break; }
           tc_fence_after();
           const float m_new = fmaxf(m_used, mx);
@@ -417,10 +422,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_arrive(&p_full[j & 1]);
     }
     // epilogue
-    // the last product, by way of the one before it: the softmax may be two products ahead, where the last one's parity alone
-    // would still match that of the phase before the previous one
-    if (ok && n_blocks > 1) ok = mbar_wait(pv_done, n_blocks & 1, abort_flag, 0x1a);
-    if (ok && n_blocks > 0) ok = mbar_wait(pv_done, (n_blocks - 1) & 1, abort_flag, 0x1a);
+    if (ok && n_blocks > 0) ok = wait_pv(n_blocks - 1, 0x1a);
     tc_fence_after();
     const float inv_l = l > 0.f ? 1.f / l : 0.f;
     if (qrow < p.sq && ok) {

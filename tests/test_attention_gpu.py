@@ -190,8 +190,8 @@ def test_attention_with_bias_mask_and_group_ids(b, s, h, dh, mask_n, with_bias, 
 
 @pytest.mark.parametrize("b,s,hq,hk,dh,causal", [(1, 16384, 16, 4, 128, True), (2, 4096, 16, 16, 64, True), (4, 333, 8, 8, 64, False)])
 def test_forward_repeats_bit_for_bit(b, s, hq, hk, dh, causal):
-    """The output of a tile is read when its last product is done, however far the softmax has run ahead: thousands of tiles, short
-    and long, give the same bits again and again."""
+    """Thousands of tiles, short and long, give the same bits again and again. (That no wait can miss its phase is walked through in
+    test_protocol_sim.py; here the tiles just run.)"""
     from hetu_galvatron_b200.ops import _lib, attention as AT
     g = torch.Generator(device="cuda").manual_seed(s)
     q = torch.randn(b, s, hq, dh, device="cuda", dtype=torch.bfloat16, generator=g)

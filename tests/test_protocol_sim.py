@@ -7,13 +7,12 @@ import subprocess
 
 import pytest
 
-SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "hetu_galvatron_b200", "csrc", "sim",
-                   "flag_protocol_sim.cpp")
+SIM = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "hetu_galvatron_b200", "csrc", "sim")
 
 
-def _build(tmp, tsan):
+def _build(tmp, tsan, source="flag_protocol_sim.cpp"):
     exe = os.path.join(tmp, "sim_tsan" if tsan else "sim")
-    cmd = ["g++", "-std=c++17", "-O1", "-g", "-pthread"] + (["-fsanitize=thread"] if tsan else []) + [SRC, "-o", exe]
+    cmd = ["g++", "-std=c++17", "-O1", "-g", "-pthread"] + (["-fsanitize=thread"] if tsan else []) + [os.path.join(SIM, source), "-o", exe]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         if tsan:
@@ -126,3 +125,21 @@ def test_mailbox_checker_sees_a_buffer_reused_under_its_readers(sim):
     rc, out, _ = _run(sim, "--ranks", 4, "--epochs", 50, "--mode", "mailbox", "--drop-rank", 2, "--drop-epoch", 20,
                       "--budget-us", 50000, timeout=60)
     assert rc == 0 and out["mismatches"] == 0 and out["timeouts"] == 3 and out["error"]["site"] in (0x17, 0x18)
+
+
+@pytest.fixture(scope="module")
+def attention_order(tmp_path_factory):
+    return _build(str(tmp_path_factory.mktemp("attention_order")), False, "attention_order_sim.cpp")
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 3, 4, 5, 8])
+def test_attention_forward_waits_in_every_interleaving(attention_order, blocks):
+    """However a softmax warp is held up, each wait for a product finds its phase, and O is read when its products are done."""
+    rc, out, _ = _run(attention_order, "--blocks", blocks)
+    assert rc == 0 and out["stuck"] == 0 and out["early"] == 0 and out["states"] > 50, out
+
+
+def test_attention_checker_sees_a_phase_that_has_passed(attention_order):
+    """One barrier for all products: the last wait misses its phase by way of the product before, and passes too early without."""
+    assert _run(attention_order, "--blocks", 4, "--schedule", "single")[1]["stuck"] > 0
+    assert _run(attention_order, "--blocks", 4, "--schedule", "direct")[1]["early"] > 0
