@@ -437,15 +437,17 @@ class AttnCfg:
 
 
 def _qkv_views(qkv: torch.Tensor, cfg: AttnCfg):
-    """q, k, v [batch, s, heads, dh] as views of the contiguous packed projection."""
-    tokens, ld = qkv.shape
+    """q, k, v [batch, s, heads, dh] as views of the packed projection. The forward pass makes it contiguous; what a saved-tensor
+    hook hands back in the backward pass need not be."""
+    tokens, width = qkv.shape
     b, hq, hk, dh = cfg.batch, cfg.hq, cfg.hk, cfg.dh
-    s, at, strides = tokens // b, qkv.storage_offset(), (ld, b * ld, dh, 1)
-    if s * b != tokens or (hq + 2 * hk) * dh != ld:
+    ld, inner = (width, 1) if qkv.is_contiguous() else qkv.stride()
+    s, at, head, strides = tokens // b, qkv.storage_offset(), dh * inner, (ld, b * ld, dh * inner, inner)
+    if s * b != tokens or (hq + 2 * hk) * dh != width:
         raise ValueError("packed projection %s does not hold %d + 2 x %d heads of %d for whole sequences of %d elements"
                          % (tuple(qkv.shape), hq, hk, dh, b))
-    return (qkv.as_strided((b, s, hq, dh), strides, at), qkv.as_strided((b, s, hk, dh), strides, at + hq * dh),
-            qkv.as_strided((b, s, hk, dh), strides, at + (hq + hk) * dh))
+    return (qkv.as_strided((b, s, hq, dh), strides, at), qkv.as_strided((b, s, hk, dh), strides, at + hq * head),
+            qkv.as_strided((b, s, hk, dh), strides, at + (hq + hk) * head))
 
 
 def _rope_packed_(qkv: torch.Tensor, cfg: AttnCfg, inv_freq, positions, inverse: bool):
