@@ -105,6 +105,16 @@ __device__ __forceinline__ float4 bf16x4_to_f4(uint32_t lo, uint32_t hi) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
+// Four columns of the bias, the first a multiple of four. A bias that does not start on 8 bytes (a view into a larger buffer) is
+// read element by element.
+__device__ __forceinline__ float4 epi_bias4(const __nv_bfloat16* b) {
+  if ((reinterpret_cast<uintptr_t>(b) & 7) == 0) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(b));
+    return bf16x4_to_f4(u.x, u.y);
+  }
+  return make_float4(__bfloat162float(b[0]), __bfloat162float(b[1]), __bfloat162float(b[2]), __bfloat162float(b[3]));
+}
+
 __device__ __forceinline__ bool epi_has_old(const GemmDev& p) { return p.residual != nullptr || p.accumulate; }
 
 // The residual, or without one the old C, of a chunk. Column groups that N cuts are read by epi_store itself.
@@ -160,10 +170,7 @@ __device__ __forceinline__ void epi_store(const GemmDev& p, const float4* stage,
     float4 v[8];
     epi_fetch(stage, lane, v);
     float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.bias != nullptr) {
-      const uint2 u = __ldg(reinterpret_cast<const uint2*>(p.bias + col));
-      b = bf16x4_to_f4(u.x, u.y);
-    }
+    if (p.bias != nullptr) b = epi_bias4(p.bias + col);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       v[i].x = v[i].x * p.alpha + b.x; v[i].y = v[i].y * p.alpha + b.y;
@@ -269,11 +276,9 @@ __device__ __forceinline__ void epi_pack32(const GemmDev& p, const uint32_t (&r)
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
   if (p.bias != nullptr) {
     if (col0 + 32 <= p.N) {
-      const uint2* bp = reinterpret_cast<const uint2*>(p.bias + col0);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const uint2 u = __ldg(bp + j);
-        const float4 b = bf16x4_to_f4(u.x, u.y);
+        const float4 b = epi_bias4(p.bias + col0 + 4 * j);
         v[4 * j] += b.x; v[4 * j + 1] += b.y; v[4 * j + 2] += b.z; v[4 * j + 3] += b.w;
       }
     } else {

@@ -25,7 +25,8 @@ int gv_read_error(unsigned int out[4]);
 //   c_f32 = 0: C is bf16 [M, ldc]; c_f32 = 1: C is fp32 [M, ldc]
 //   accumulate != 0: C += result (used to accumulate weight gradients over micro-batches)
 //   act: 0 none, 1 GELU(tanh) applied after bias
-// Requirements: lda, ldb, ldc multiples of 8, K too unless both operands are MN-major; all base pointers 16-byte aligned.
+// Requirements: lda, ldb, ldc multiples of 8, K too unless both operands are MN-major; all base pointers 16-byte aligned
+// but the bias, which may start anywhere.
 typedef struct {
   const void* A;
   const void* B;

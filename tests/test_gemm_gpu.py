@@ -90,6 +90,31 @@ def test_gemm_epilogue_edges(M, N, K, f32):
     assert _lib.read_error() is None
 
 
+@pytest.mark.parametrize("M,N,K", [(33, 6, 8), (33, 24, 64), (130, 40, 64), (300, 264, 128)])
+@pytest.mark.parametrize("offset", [1, 2, 4])
+def test_gemm_bias_at_any_address(M, N, K, offset):
+    """A bias that is a view into a larger buffer, aligned to 2, 4 or 8 bytes: each of the epilogues that add one, against the
+    same bias in an allocation of its own."""
+    g = torch.Generator(device="cuda").manual_seed(M * N + offset)
+    rnd = lambda *s: torch.randn(*s, device="cuda", dtype=torch.bfloat16, generator=g)
+    a, b, bias = rnd(M, K), rnd(N, K), rnd(N + 8)[offset:offset + N]
+    ld = (N + 7) // 8 * 8
+    assert bias.data_ptr() % 16 == 2 * offset
+
+    def outputs(bias):
+        bf = torch.zeros(M, ld, device="cuda", dtype=torch.bfloat16)
+        f32, acc, act = torch.zeros(M, ld, device="cuda"), torch.ones(M, ld, device="cuda"), torch.zeros_like(bf)
+        gemm(a, b, out=bf[:, :N], bias=bias)
+        gemm(a, b, out=f32[:, :N], bias=bias)
+        gemm(a, b, out=acc[:, :N], bias=bias, accumulate=True)
+        up = gemm(a, b, bias=bias, gelu_out=act[:, :N]) if N % 8 == 0 else bf
+        return bf, f32, acc, act, up
+
+    for got, ref in zip(outputs(bias), outputs(bias.clone())):
+        assert torch.equal(got, ref)
+    assert _lib.read_error() is None
+
+
 def test_gemm_linear_grads_match_torch():
     torch.manual_seed(2)
     M, N, K = 1024, 768, 512
