@@ -411,6 +411,9 @@ __global__ void lse_merge_kernel(float* __restrict__ acc, float* __restrict__ ls
 }
 
 // ------------------------------------------------------------------ head statistics
+// A tile without a finite maximum has nothing to add, unless its sum is NaN (logits that are NaN or infinite): then so is the row's.
+__device__ __forceinline__ float scaled_sum(float sum, float max, float new_max) { return sum * (max == -INFINITY ? 0.f : expf(max - new_max)); }
+
 // Joins the statistics that the head GEMM's epilogue left per 256 columns (stats [rows, tiles, 2]: max, sum of exp) into one
 // (max, sum) per row, one warp per row, and finishes the loss where this shard holds the whole vocabulary. `target` was written
 // where the label lies in this shard; elsewhere it becomes 0. Replaces a dozen element-wise launches on [rows] and [rows, tiles].
@@ -424,11 +427,11 @@ __global__ void xent_merge_kernel(const float2* __restrict__ stats, int tiles, c
   for (int t = lane; t < tiles; t += 32) {
     const float2 v = __ldg(stats + row * tiles + t);
     const float n = fmaxf(m, v.x);
-    l = (m == -INFINITY ? 0.f : l * expf(m - n)) + v.y * expf(v.x - n);
+    l = scaled_sum(l, m, n) + scaled_sum(v.y, v.x, n);
     m = n;
   }
   const float wm = warp_max_e(m);
-  const float wl = warp_sum_e(m == -INFINITY ? 0.f : l * expf(m - wm));
+  const float wl = warp_sum_e(scaled_sum(l, m, wm));
   if (lane != 0) return;
   const long long lab = labels[row];
   const bool kept = lab != ignore_index, here = kept && lab >= vocab_start && lab < vocab_start + vocab_rows;

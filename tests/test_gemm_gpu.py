@@ -415,3 +415,22 @@ def test_weight_gradient_of_any_row_count(M, N, K):
     assert _lib.launch_count() == before + 1                 # the kernel, not the library
     assert ((buf.double() - ref).abs() <= (K + 4) * 2.0 ** -23 * size).all()
     assert _lib.read_error() is None
+@pytest.mark.parametrize("rows,tiles", [(1, 1), (9, 40), (300, 70)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_head_statistics_of_bad_weights(rows, tiles, bad):
+    """A tile of the vocabulary whose weights have gone NaN or infinite shows in the loss of every row, wherever the tile is among
+    those that a lane joins."""
+    from hetu_galvatron_b200.ops.gemm import head_xent_loss, head_xent_stats
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, 64, device="cuda", dtype=torch.bfloat16, generator=g)
+    w = torch.randn(256 * tiles, 64, device="cuda", dtype=torch.bfloat16, generator=g)
+    x[:, 0] = 1.0
+    labels = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    for tile in sorted({0, tiles // 2, tiles - 1}):
+        broken = w.clone()
+        broken[256 * tile:256 * (tile + 1), 0] = bad              # the logits of these columns
+        loss, lse = head_xent_loss(x, broken, labels)
+        _, se, _ = head_xent_stats(x, broken, labels)
+        assert not torch.isfinite(loss).any() and not torch.isfinite(lse).any() and not torch.isfinite(se).any()
+
+
