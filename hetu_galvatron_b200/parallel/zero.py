@@ -428,7 +428,8 @@ class ParamBucket:
 
     # ------------------------------------------------------------------ optimizer
     def grad_sumsq(self, out: torch.Tensor, tp_size: int) -> None:
-        """Adds this bucket's share of the squared global gradient norm (already divided by d^2) into out[0]."""
+        """Adds this bucket's share of the squared global gradient norm (already divided by d^2) into out[0]: zero before, or the
+        sum of few others, since fp32 adds of many partial sums to a large one lose bits."""
         if self.numel == 0 or self.grad_shard is None:
             return
         if self.d == 1 and not self.skip_params and not (self.dup_params and tp_size > 1):
@@ -762,10 +763,11 @@ class ZeroEngine:
 
     def grad_norm(self) -> torch.Tensor:
         dev = next((b.device for b in self.buckets if b.numel), torch.device("cpu"))
-        total = torch.zeros(1, dtype=torch.float32, device=dev)
-        for b in self.buckets:
+        parts = torch.zeros(max(len(self.buckets), 1), dtype=torch.float32, device=dev)      # one sum per bucket
+        for i, b in enumerate(self.buckets):
             tp = b.tp_group.size if b.tp_group is not None else 1
-            b.grad_sumsq(total, tp)
+            b.grad_sumsq(parts[i:i + 1], tp)
+        total = parts.sum(0, keepdim=True)
         if dist.is_initialized() and dist.get_world_size() > 1:
             dist.all_reduce(total, group=self.world_group)
         return total.sqrt()

@@ -1,4 +1,4 @@
-"""The autograd functions of ops/autograd.py on the CPU path."""
+"""The autograd functions of ops/autograd.py and the gradient norm over their buffers, on the CPU path."""
 import pytest
 import torch
 
@@ -26,3 +26,17 @@ def test_packed_attention_under_saved_tensor_hooks(layout):
         o = A.packed_attention(x * 1.0, cfg)
     got, = torch.autograd.grad(o, x, do)
     assert torch.equal(got, want)
+
+
+def test_gradient_norm_keeps_the_bits_of_small_buckets():
+    """Each bucket's squares are summed on their own: 64 buckets of norm one beside one of norm 4096 are not rounded away one by
+    one (fp32 resolves 2 at 4096^2)."""
+    from hetu_galvatron_b200.parallel.zero import ParamBucket, ZeroEngine
+    engine = ZeroEngine()
+    for i in range(65):
+        b = engine.add_bucket(ParamBucket("b%d" % i, [torch.nn.Parameter(torch.zeros(4))], None))
+        b._ensure_grad()
+        b.grad_flat[0] = 4096.0 if i == 0 else 1.0
+        b.grad_shard = b.grad_flat
+    exact = (4096.0 ** 2 + 64) ** 0.5
+    assert abs(engine.grad_norm().item() - exact) < 2.0 ** -23 * 2 * exact
