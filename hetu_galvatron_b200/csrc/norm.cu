@@ -38,9 +38,11 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 // take two or four warps and one barrier per sum. One row per warp team and CTA slot (no grid stride): the scheduler refills the SM.
 // L2 flushed, 8192 x 4096 RMSNorm: 41.0 us with one row per 256-thread CTA and its two barriers, 30.7 us now (134 MB, of which
 // about 4 us are the launch); 36864 x 192: 75.8 -> 14.3 us.
+// KEEP32: a residual whose sum with x is not stored. Nothing rounds that sum then: both addends stay in registers as they came
+// and are added in fp32 wherever the row is used.
 constexpr int FWD_THREADS = 256;
 
-template <bool LAYER, int WARPS, int VPL>
+template <bool LAYER, int WARPS, int VPL, bool KEEP32>
 __global__ void __launch_bounds__(FWD_THREADS)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                 const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
@@ -72,7 +74,24 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     const int i = t + j * 32 * WARPS;
     raw[j] = (row_ok && i < nvec) ? __ldcs(reinterpret_cast<const uint4*>(x + off) + i) : make_uint4(0u, 0u, 0u, 0u);
   }
-  if (res) {
+  uint4 raw_res[KEEP32 ? VPL : 1];
+  if constexpr (KEEP32) {
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) {
+      const int i = t + j * 32 * WARPS;
+      raw_res[j] = (row_ok && i < nvec) ? __ldcs(reinterpret_cast<const uint4*>(res + off) + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+  auto values = [&](int j, float (&v)[8]) {          // vector j of the row; zero beyond its end
+    unpack8(raw[j], v);
+    if constexpr (KEEP32) {
+      float r[8];
+      unpack8(raw_res[j], r);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] += r[e];
+    }
+  };
+  if (!KEEP32 && res) {
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
       const int i = t + j * 32 * WARPS;
@@ -83,7 +102,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] += r[e];
         raw[j] = pack8(v);           // the residual stream is carried in bf16; normalise what is actually stored
-        if (h_out) reinterpret_cast<uint4*>(h_out + off)[i] = raw[j];
+        reinterpret_cast<uint4*>(h_out + off)[i] = raw[j];
       }
     }
   }
@@ -93,7 +112,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
       float v[8];
-      unpack8(raw[j], v);            // vectors beyond the row are zero
+      values(j, v);
 #pragma unroll
       for (int e = 0; e < 8; ++e) s += v[e];
     }
@@ -103,8 +122,11 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 #pragma unroll
   for (int j = 0; j < VPL; ++j) {
     float v[8];
-    unpack8(raw[j], v);
+    values(j, v);
     const float m = (t + j * 32 * WARPS < nvec) ? mean : 0.f;
+    // RMSNorm: one chain per vector, since 64 adds in a row lose more than the 16 of a narrower share (rstd of 4096 columns
+    // 4.9e-8 off against 4.4e-8). LayerNorm's variance is taken about the mean and loses nothing to it.
+    float sv = LAYER ? s2 : 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) sv += (v[e] - m) * (v[e] - m);
     s2 = LAYER ? sv : s2 + sv;
@@ -120,14 +142,11 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     const int i = t + j * 32 * WARPS;
     if (i < nvec) {
       float v[8], wv[8];
-      unpack8(raw[j], v);
+      values(j, v);
       unpack8(__ldg(reinterpret_cast<const uint4*>(w) + i), wv);
       if (LAYER) {
         float bv[8];
         unpack8(__ldg(reinterpret_cast<const uint4*>(b) + i), bv);
-    // RMSNorm: one chain per vector, since 64 adds in a row lose more than the 16 of a narrower share (rstd of 4096 columns
-    // 4.9e-8 off against 4.4e-8). LayerNorm's variance is taken about the mean and loses nothing to it.
-    float sv = LAYER ? s2 : 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = (v[e] - mean) * rstd * wv[e] + bv[e];
       } else {
@@ -326,19 +345,26 @@ typedef __nv_bfloat16 bf16;
 
 // Rows of up to 512 / 1024 / 2048 columns: one warp each (2, 4 or 8 vectors per lane); up to 4096 two warps, up to 8192 four.
 // Sixteen vectors per lane would need no barrier at 4096 columns either, but 147 registers leave one CTA per SM.
-template <bool LAYER>
-static int launch_norm_fwd(const void* x, const void* res, const void* w, const void* b, void* y, void* h_out, float* mean,
+template <bool LAYER, bool KEEP32>
+static int launch_norm_fwd_rows(const void* x, const void* res, const void* w, const void* b, void* y, void* h_out, float* mean,
                            float* rstd, int rows, int cols, float eps, cudaStream_t s) {
   auto go = [&](auto kern, int teams) {
     kern<<<(rows + teams - 1) / teams, FWD_THREADS, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)w, (const bf16*)b,
                                                             (bf16*)y, (bf16*)h_out, mean, rstd, rows, cols, eps);
     return (int)cudaGetLastError();
   };
-  if (cols <= 512) return go(norm_fwd_kernel<LAYER, 1, 2>, 8);
-  if (cols <= 1024) return go(norm_fwd_kernel<LAYER, 1, 4>, 8);
-  if (cols <= 2048) return go(norm_fwd_kernel<LAYER, 1, 8>, 8);
-  if (cols <= 4096) return go(norm_fwd_kernel<LAYER, 2, 8>, 4);
-  return go(norm_fwd_kernel<LAYER, 4, 8>, 2);
+  if (cols <= 512) return go(norm_fwd_kernel<LAYER, 1, 2, KEEP32>, 8);
+  if (cols <= 1024) return go(norm_fwd_kernel<LAYER, 1, 4, KEEP32>, 8);
+  if (cols <= 2048) return go(norm_fwd_kernel<LAYER, 1, 8, KEEP32>, 8);
+  if (cols <= 4096) return go(norm_fwd_kernel<LAYER, 2, 8, KEEP32>, 4);
+  return go(norm_fwd_kernel<LAYER, 4, 8, KEEP32>, 2);
+}
+
+template <bool LAYER>
+static int launch_norm_fwd(const void* x, const void* res, const void* w, const void* b, void* y, void* h_out, float* mean,
+                           float* rstd, int rows, int cols, float eps, cudaStream_t s) {
+  if (res != nullptr && h_out == nullptr) return launch_norm_fwd_rows<LAYER, true>(x, res, w, b, y, h_out, mean, rstd, rows, cols, eps, s);
+  return launch_norm_fwd_rows<LAYER, false>(x, res, w, b, y, h_out, mean, rstd, rows, cols, eps, s);
 }
 
 struct BwdShape { int threads, v, grid; };

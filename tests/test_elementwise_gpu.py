@@ -78,6 +78,32 @@ def test_rmsnorm_statistics_in_fp32(cols):
     assert (rstd.double() - ref).norm() <= 4.6e-8 * ref.norm()
 
 
+@pytest.mark.parametrize("layer", [False, True])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (5, 1032), (17, 2056), (3, 8184)])
+def test_norm_of_a_sum_that_is_not_stored(rows, cols, layer):
+    """The C entry points with a residual and no buffer for the sum: the norm is that of the unrounded sum."""
+    from hetu_galvatron_b200.ops import _lib
+    g = torch.Generator(device=DEV).manual_seed(rows + cols)
+    mk = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    x, res, w, b = mk(rows, cols), mk(rows, cols), mk(cols), mk(cols)
+    y, mean, rstd = torch.empty_like(x), torch.empty(rows, device=DEV), torch.empty(rows, device=DEV)
+    p = lambda t: t.data_ptr()
+    if layer:
+        rc = _lib.lib().gv_layernorm_fwd(p(x), p(res), p(w), p(b), p(y), 0, p(mean), p(rstd), rows, cols, 1e-5, _lib.stream_ptr())
+    else:
+        rc = _lib.lib().gv_rmsnorm_fwd(p(x), p(res), p(w), p(y), 0, p(rstd), rows, cols, 1e-5, _lib.stream_ptr())
+    assert rc == 0
+    h = x.double() + res.double()
+    mu = h.mean(-1, keepdim=True) if layer else 0.0
+    r = ((h - mu).pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt()
+    ref = (h - mu) * r * w.double() + (b.double() if layer else 0.0)
+    # one rounding to bf16 (2^-8 of the value at most) and a few fp32 ones, which turn one result in some thousand to the other
+    # side; with the sum rounded first about a third of them would differ
+    assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * (1 + h.abs().max() * r) * (w.double().abs() + 1)).all()
+    assert (y != ref.bfloat16()).float().mean() < 0.01
+    assert ((rstd.double() - r[:, 0]).abs() <= 1e-6 * r[:, 0]).all()
+
+
 def test_norm_weight_gradients_are_bitwise_repeatable():
     """The weight (and bias) gradient is reduced in two stages in a fixed order, without atomics: same bits every run."""
     torch.manual_seed(1)
