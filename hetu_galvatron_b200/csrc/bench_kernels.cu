@@ -3,6 +3,7 @@
 // single-CTA form and in the cta_group::2 pair form. Operands sit in (zeroed) shared memory, the accumulator in
 // tensor memory; nothing else runs, so the figure is the tensor pipe's cost of one instruction. The attention and
 // GEMM tile shapes were chosen from this table (an N = 64 instruction costs 48 cycles, not 32).
+// gv_eval_math evaluates the kernels' element-wise functions in fp32, for their checks against 64 bits.
 // The reference has no GPU code of its own and therefore no counterpart of this file.
 #include "include/gv_kernels.h"
 #include "include/gv_host.h"
@@ -76,6 +77,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128, 1) probe_pair(l
   if (threadIdx.x < 32) { tc_fence_after(); tmem_dealloc<2>(tmem_base, 512); }
 }
 
+__global__ void eval_math_kernel(int which, const float* __restrict__ x, float* __restrict__ y, long long n) {
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const float v = x[i];
+    float s = 0.f, c = 0.f, r = 0.f;
+    if (which <= 1) sincos_any(v, s, c);
+    switch (which) {
+      case 0: r = s; break;
+      case 1: r = c; break;
+      case 2: r = gate_sigmoid(v); break;
+      case 3: r = gate_silu(v); break;
+      case 4: r = v / (1.f + __expf(-v)); break;
+      case 5: r = gelu_tanh(v); break;
+      case 6: r = gelu_tanh_grad(v); break;
+      default: r = 1.f / (1.f + __expf(-v)); break;
+    }
+    y[i] = r;
+  }
+}
 
 template <int N, int M>
 static int launch_single(long long* out, int reps, cudaStream_t s) {
@@ -118,6 +138,16 @@ extern "C" int gv_bench_mma_issue(int pair, int m, int n, int reps, long long* o
     if (m == 128 && n == 256) return launch_pair<256, 128>(out_dev, reps, s);
   }
   return 2602;
+}
+
+// y[i] = f(x[i]) in fp32; which: 0 sine, 1 cosine (as rotated with), 2 sigmoid, 3 silu (of a gate), 4 silu by an IEEE division,
+// 5 GELU, 6 its derivative, 7 sigmoid by a division.
+extern "C" int gv_eval_math(int which, const float* x, float* y, long long n, gv_stream_t stream) {
+  if (which < 0 || which > 7) return 2603;
+  if (n <= 0) return 0;
+  const long long blocks = (n + 255) / 256;
+  eval_math_kernel<<<static_cast<unsigned>(blocks < 1184 ? blocks : 1184), 256, 0, (cudaStream_t)stream>>>(which, x, y, n);
+  return static_cast<int>(cudaGetLastError());
 }
 
 GV_DEFINE_ERROR_READER(gv_read_error_bench)

@@ -108,7 +108,7 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
     unpack8e(*reinterpret_cast<const uint4*>(g), a);
     unpack8e(*reinterpret_cast<const uint4*>(g + f), b);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = a[e] * sigmoid_nb(a[e]) * b[e];
+    for (int e = 0; e < 8; ++e) o[e] = gate_silu(a[e]) * b[e];
     *reinterpret_cast<uint4*>(out + r * f + c) = pack8e(o);
   }
 }
@@ -128,7 +128,7 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __r
     unpack8e(*reinterpret_cast<const uint4*>(dout + r * f + c), d);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float sg = sigmoid_nb(a[e]);
+      const float sg = gate_sigmoid(a[e]);
       const float silu = a[e] * sg;
       da[e] = d[e] * b[e] * (sg + silu * (1.f - sg));
       db[e] = d[e] * silu;

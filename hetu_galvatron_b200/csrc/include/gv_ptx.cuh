@@ -506,6 +506,27 @@ __device__ __forceinline__ float sigmoid_nb(float x) {
   const float z = fmaf(y, fmaf(-d, y, 1.f), y);
   return d < 1e38f ? z : y;
 }
+// The gate of SwiGLU: 1 / (1 + exp(-x)) and x / (1 + exp(-x)) as exact as with a division, which x * sigmoid_nb(x) is not: the
+// quotient by the approximate reciprocal, corrected by its remainder, has the same bits for every bf16 x. The reciprocal is
+// taken of a quarter of the denominator, so that it stays among the normal numbers while the denominator is finite. Where it
+// is not, or x is infinite, the correction is NaN and the plain product right.
+struct GateTerms { float d, y; };        // 1 + exp(-x) and its approximate reciprocal
+__device__ __forceinline__ GateTerms gate_terms(float x) {
+  const float t = __expf(-x);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaf(t, 0.25f, 0.25f)));
+  return {1.f + t, 0.25f * y};
+}
+__device__ __forceinline__ float gate_sigmoid(float x) {
+  const GateTerms g = gate_terms(x);
+  const float z = fmaf(g.y, fmaf(-g.d, g.y, 1.f), g.y);
+  return z == z ? z : g.y;
+}
+__device__ __forceinline__ float gate_silu(float x) {
+  const GateTerms g = gate_terms(x);
+  const float q = x * g.y, r = fmaf(fmaf(-g.d, q, x), g.y, q);
+  return r == r ? r : q;
+}
 // GELU, tanh form: x (1 + tanh u) / 2 = x sigmoid(2 u) with u = sqrt(2 / pi) (x + 0.044715 x^3), and its derivative. The sigmoid
 // has no cancellation where tanh u is close to -1 (at x = -4 the tanh form is off by 1e-3 of the value) and no branch.
 __device__ __forceinline__ float gelu_tanh(float x) {

@@ -114,6 +114,7 @@ PROTOTYPES = {
     "gv_adamw": [_P, _P, _P, _P, _I, _P, _L] + [_F] * 8 + [_P, _P],
     "gv_sumsq_accum": [_P, _I, _L, _P, _P],
     "gv_zero": [_P, _L, _P],
+    "gv_eval_math": [_I, _P, _P, _L, _P],
     "gv_lse_merge": [_P] * 4 + [_I] * 6 + [_L, _L, _L, _P],
 }
 

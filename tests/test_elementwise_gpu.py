@@ -290,3 +290,32 @@ def test_rope_runs_of_heads(tokens, heads, dh, inverse):
     # one rounding to bf16, sines to 1e-7
     assert ((buf[:, :heads].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6 * (a.abs() + b.abs() + 1).repeat(1, 1, 2)).all()
     assert torch.equal(buf[:, heads:].double(), old[:, heads:])
+
+
+def _eval(which, x):
+    from hetu_galvatron_b200.ops import _lib
+    y = torch.empty_like(x)
+    _lib.check(_lib.lib().gv_eval_math(which, x.data_ptr(), y.data_ptr(), x.numel(), _lib.stream_ptr()), "gv_eval_math")
+    return y
+
+
+def _all_bf16():
+    """Every finite bf16 number, in fp32."""
+    x = torch.arange(-32768, 32768, device=DEV).to(torch.int16).view(torch.bfloat16).float()
+    return x[torch.isfinite(x)]
+
+
+def test_gates_are_as_exact_as_divisions():
+    """Over every bf16 gate silu is what an IEEE division gives, and sigmoid no further from 64 bits."""
+    x = torch.cat([_all_bf16(), torch.tensor([float("inf"), float("-inf"), float("nan")], device=DEV)])
+    assert torch.equal(_eval(3, x).nan_to_num(nan=7.0), _eval(4, x).nan_to_num(nan=7.0))
+    x = x[x > -88]                                   # below, 1 + exp(-x) overflows
+    x = x[torch.isfinite(x)]
+    ref = torch.sigmoid(x.double())
+    err = lambda y, r: (y.double() - r).abs() / r.abs()
+    # CUDA's bound for __expf: 2 + floor(1.173 |x|) units; one rounding of the sum, one of the quotient
+    bound = (4 + 1.173 * x.abs()) * 2.0 ** -23
+    sig, sig_div = err(_eval(2, x), ref), err(_eval(7, x), ref)
+    assert (sig <= bound).all() and sig.max() <= sig_div.max() * (1 + 2.0 ** -20) and sig.mean() <= sig_div.mean() * (1 + 1e-4)
+    big = (x.double() * ref).abs() > 2.0 ** -126
+    assert (err(_eval(3, x), x.double() * ref) <= bound)[big].all()
