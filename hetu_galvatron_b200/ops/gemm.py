@@ -8,6 +8,7 @@ transpose (reference: megatron/core/tensor_parallel/layers.py:417,462,534).
 from __future__ import annotations
 
 import functools
+import warnings
 
 import torch
 
@@ -49,6 +50,23 @@ class RopeEpilogue:
 def _workspace_bytes(M: int, N: int, K: int) -> int:
     """Scratch of a split reduction for a product of these sizes (at most 38 MB); 0: not split."""
     return _lib.lib().gv_gemm_workspace_bytes(_lib.GemmArgs(M=M, N=N, K=K))
+
+
+# Products (device, M, N, K) whose scratch once did not fit. They stay unsplit: a product that was split or not as memory happened
+# to be free would change its last bits from call to call, and each failed allocation first empties the allocator's cache.
+_NO_SCRATCH: set = set()
+
+
+def _split_scratch(M: int, N: int, K: int, device) -> "torch.Tensor | None":
+    need = _workspace_bytes(M, N, K)
+    if not need or (device.index, M, N, K) in _NO_SCRATCH:
+        return None
+    try:
+        return torch.empty(need, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        _NO_SCRATCH.add((device.index, M, N, K))
+        warnings.warn("no room for %.0f MB of partial sums: products of %d x %d x %d run unsplit from now on" % (need / 1e6, M, N, K))
+        return None
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,
@@ -101,13 +119,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         elif gelu_out is not None:
             args.gelu_out, args.gelu_ld = gelu_out.data_ptr(), gelu_out.stride(0)
         elif swiglu_out is None:
-            need = _workspace_bytes(M, N, K)
-            if need:
-                try:
-                    scratch = torch.empty(need, dtype=torch.uint8, device=a.device)
-                    args.workspace, args.workspace_bytes = scratch.data_ptr(), need
-                except torch.cuda.OutOfMemoryError:
-                    pass                    # no room for the partial sums: the product runs unsplit
+            scratch = _split_scratch(M, N, K, a.device)
+            if scratch is not None:
+                args.workspace, args.workspace_bytes = scratch.data_ptr(), scratch.numel()
         _lib.check(_lib.lib().gv_gemm_bf16(args, _lib.stream_ptr()), "gv_gemm_bf16")
         return out
     if rope is not None or swiglu_out is not None or gelu_out is not None:

@@ -214,6 +214,31 @@ assert all(torch.equal(gemm(a, w, out_dtype=torch.float32), first) for _ in rang
         assert v < 1e-2, (k, v, res)
 
 
+def test_products_without_room_for_scratch_stay_unsplit(monkeypatch):
+    """An allocation of the partial sums that fails (once, made up on the host) costs one warning; from then on the product repeats
+    its bits whether or not there is room again."""
+    import importlib
+    G = importlib.import_module("hetu_galvatron_b200.ops.gemm")
+    M, N, K = 384, 768, 9216
+    assert G._workspace_bytes(M, N, K) > 0
+    a, b = (torch.randn(n, K, device="cuda", dtype=torch.bfloat16, generator=torch.Generator(device="cuda").manual_seed(n)) for n in (M, N))
+    empty, failed = torch.empty, []
+
+    def full(*args, **kw):
+        if kw.get("dtype") == torch.uint8 and not failed:
+            failed.append(args)
+            raise torch.cuda.OutOfMemoryError("out of memory")
+        return empty(*args, **kw)
+
+    monkeypatch.setattr(G, "_NO_SCRATCH", set())
+    monkeypatch.setattr(torch, "empty", full)
+    with pytest.warns(UserWarning, match="unsplit"):
+        first = gemm(a, b, out_dtype=torch.float32)
+    assert failed and torch.equal(gemm(a, b, out_dtype=torch.float32), first)
+    ref = a.double() @ b.double().t()
+    assert ((first.double() - ref).abs() <= (K + 4) * 2.0 ** -23 * (a.double().abs() @ b.double().abs().t())).all()
+
+
 @pytest.mark.parametrize("M,V,K,vocab_start", [(256, 1000, 256, 0), (300, 4096, 512, 4096), (8192, 32000, 1024, 0), (128, 264, 64, 0)])
 def test_lm_head_cross_entropy_epilogues(M, V, K, vocab_start):
     """Head GEMM whose epilogue computes the cross-entropy statistics (no logits stored), and its backward twin whose
