@@ -104,6 +104,54 @@ def test_norm_of_a_sum_that_is_not_stored(rows, cols, layer):
     assert ((rstd.double() - r[:, 0]).abs() <= 1e-6 * r[:, 0]).all()
 
 
+@pytest.mark.parametrize("branch", [False, True])
+@pytest.mark.parametrize("grads", ["fp32", "bf16", "mixed", "autograd"])
+def test_layernorm_gradient_buffers(grads, branch):
+    """Weight and bias gradients added straight into fp32 buffers, through a scratch pair into others, or handed to autograd; with
+    and without the residual branch's gradient; twice, so that the second adds to the first."""
+    from hetu_galvatron_b200.ops import autograd as A
+    g = torch.Generator(device=DEV).manual_seed(3)
+    mk = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    x, w, b = mk(37, 264).requires_grad_(), mk(264).requires_grad_(), mk(264).requires_grad_()
+    dy, dres = mk(37, 264), mk(37, 264)
+    if grads != "autograd":
+        for p, dtype in ((w, torch.bfloat16 if grads == "bf16" else torch.float32), (b, torch.float32 if grads == "fp32" else torch.bfloat16)):
+            p.main_grad, p.hooked = torch.zeros(264, device=DEV, dtype=dtype), 0
+            p.grad_ready_hook = lambda q: setattr(q, "hooked", q.hooked + 1)
+    xd, wd, bd = (t.detach().double().requires_grad_() for t in (x, w, b))
+    ref = torch.nn.functional.layer_norm(xd, (264,), wd, bd, 1e-5)
+    outs, refs = ([ref, xd], [dy.double(), dres.double()]) if branch else ([ref], [dy.double()])
+    want = torch.autograd.grad(outs, (xd, wd, bd), refs)
+    for times in (1, 2):
+        if branch:
+            y, h = A.layernorm_branch(x, w, b)
+            got = torch.autograd.grad([y, h], (x, w, b), [dy, dres], allow_unused=True)
+        else:
+            got = torch.autograd.grad(A.layernorm(x, w, b), (x, w, b), dy, allow_unused=True)
+        assert ((got[0].double() - want[0]).abs() <= 2.0 ** -8 * want[0].abs() + 1e-4).all()
+        for p, t, r in ((w, got[1], want[1]), (b, got[2], want[2])):
+            if grads == "autograd":
+                assert ((t.double() - r).abs() <= 2.0 ** -8 * r.abs() + 1e-4).all()
+            else:
+                assert t is None and p.hooked == times
+                # fp32 sums of 37 terms; into bf16 one rounding of each sum and one of each addition
+                bound = 1e-4 + (0 if p.main_grad.dtype == torch.float32 else times * 2.0 ** -7 * r.abs())
+                assert ((p.main_grad.double() - times * r).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype,n", [(torch.bfloat16, 5), (torch.float32, (1 << 18) - 1), (torch.float32, 1 << 18), (torch.bfloat16, (1 << 19) + 3)])
+def test_clearing_buffers(dtype, n):
+    """Gradient buffers on both sides of the size from which they are cleared by memset, at an offset of one element: all of the
+    view and nothing else."""
+    buf = torch.ones(n + 2, device=DEV, dtype=dtype)
+    buf[1] = float("nan")
+    Fn.zero_(buf[1:n + 1])
+    assert (buf[1:n + 1] == 0).all() and buf[0] == 1 and buf[n + 1] == 1
+    wide = torch.ones(4, n, device=DEV, dtype=dtype)
+    Fn.zero_(wide[:, :n - 1])                      # not contiguous
+    assert (wide[:, :n - 1] == 0).all() and (wide[:, n - 1] == 1).all()
+
+
 def test_norm_weight_gradients_are_bitwise_repeatable():
     """The weight (and bias) gradient is reduced in two stages in a fixed order, without atomics: same bits every run."""
     torch.manual_seed(1)

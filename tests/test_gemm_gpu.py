@@ -378,6 +378,41 @@ def test_gelu_epilogue(M, N, K):
     assert _lib.read_error() is None
 
 
+@pytest.mark.parametrize("lead,f,h,bias", [((27,), 40, 64, True), ((5, 60), 264, 128, False), ((8192,), 5120, 72, True)])
+@pytest.mark.parametrize("main_grad", [None, torch.float32, torch.bfloat16])
+def test_linear_gelu_gradients(lead, f, h, bias, main_grad):
+    """gelu(x W^T + b) as one Function against 64 bits of the same bf16 inputs: input gradient, and weight and bias gradients handed
+    to autograd or added to gradient buffers; upstream gradients may be expanded or transposed views."""
+    from hetu_galvatron_b200.ops import autograd as A
+    g = torch.Generator(device="cuda").manual_seed(f)
+    rnd = lambda *s: torch.randn(*s, device="cuda", dtype=torch.bfloat16, generator=g)
+    x, W = rnd(*lead, h).requires_grad_(), (rnd(f, h) * h ** -0.5).requires_grad_()
+    b = rnd(f).requires_grad_() if bias else None
+    params = [W] + ([b] if bias else [])
+    for dout in (rnd(*lead, f), rnd(f).expand(*lead, f), rnd(f, *lead).movedim(0, -1)):
+        xd, Wd, bd = (None if t is None else t.detach().double().requires_grad_() for t in (x, W, b))
+        # the gradient of the GELU is taken at the stored (rounded) projection
+        up = xd @ Wd.t() + (0 if bd is None else bd)
+        up = up + (up.detach().to(torch.bfloat16).double() - up.detach())
+        ref = torch.nn.functional.gelu(up, approximate="tanh")
+        want = torch.autograd.grad(ref, [xd, Wd] + ([bd] if bias else []), dout.double())
+        if main_grad is not None:
+            for p in params:
+                p.main_grad, p.hooked = torch.zeros(p.shape, device="cuda", dtype=main_grad), 0
+                p.grad_ready_hook = lambda q: setattr(q, "hooked", q.hooked + 1)
+        y = A.linear_gelu(x, W, b)
+        assert type(y.grad_fn).__name__.startswith("LinearGeluFn")
+        got = torch.autograd.grad(y, [x] + params, dout, allow_unused=True)
+        if main_grad is not None:
+            assert all(p.hooked == 1 for p in params) and all(t is None for t in got[1:])
+            got = [got[0]] + [p.main_grad for p in params]
+        assert y.shape == ref.shape and (y.double() - ref).norm() <= 4e-3 * ref.norm()
+        for t, r in zip(got, want):
+            # dact, gelu' and the result rounded to bf16 (2^-9 each, at random): about 0.3 % of the norm; sums of one sign less
+            assert t.shape == r.shape and (t.double() - r).norm() <= 6e-3 * r.norm()
+    assert _lib.read_error() is None
+
+
 @pytest.mark.parametrize("rows,V,vocab_start", [(1, 40, 0), (33, 1000, 0), (300, 8192 + 264, 512)])
 def test_head_statistics_merge(rows, V, vocab_start):
     """Loss and log-sum-exp from the merged tile statistics, with ignored labels and labels outside the shard."""
@@ -444,6 +479,36 @@ def test_weight_gradient_of_any_row_count(M, N, K):
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 def test_head_statistics_of_bad_weights(rows, tiles, bad):
     """A tile of the vocabulary whose weights have gone NaN or infinite shows in the loss of every row, wherever the tile is among
+@pytest.mark.parametrize("dh", [50, 25])
+@pytest.mark.parametrize("form", ["heads first", "odd rows", "expanded gradient"])
+def test_padded_heads_of_other_strides(dh, form):
+    """q, k, v stored [b, h, s, dh], with a row stride that is no multiple of two elements, and an upstream gradient that is an
+    expanded view, against the same values in contiguous tensors."""
+    from hetu_galvatron_b200.ops import autograd as A
+    g = torch.Generator(device="cuda").manual_seed(dh)
+    b, sq, sk, hq, hk = 2, 37, 70, 4, 2
+
+    def rnd(s, h):
+        if form == "heads first":
+            return torch.randn(b, h, s, dh, device="cuda", dtype=torch.bfloat16, generator=g).transpose(1, 2)
+        if form == "odd rows":
+            return torch.randn(b, s, h * dh + 1, device="cuda", dtype=torch.bfloat16, generator=g)[..., :h * dh].unflatten(-1, (h, dh))
+        return torch.randn(b, s, h, dh, device="cuda", dtype=torch.bfloat16, generator=g)
+
+    q, k, v = rnd(sq, hq), rnd(sk, hk), rnd(sk, hk)
+    do = rnd(1, 1)[:1].expand(b, sq, hq, dh) if form == "expanded gradient" else rnd(sq, hq)
+    res = []
+    for copy in (lambda t: t.detach(), lambda t: t.contiguous().clone()):
+        qkv = [copy(t).requires_grad_() for t in (q, k, v)]
+        o, lse = A.attention(*qkv, False)
+        res.append((o.detach(), lse) + torch.autograd.grad(o, qkv, copy(do)))
+    # dq is summed by reductions in any order: fp32 sums, then one rounding
+    for i, (got, want) in enumerate(zip(*res)):
+        assert torch.equal(got, want) if i < 2 else (got.float() - want.float()).norm() <= 1e-3 * want.float().norm()
+    ref = torch.nn.functional.scaled_dot_product_attention(*(t.double().transpose(1, 2).repeat_interleave(hq // t.shape[2], 1) for t in (q, k, v)))
+    assert (res[0][0].double() - ref.transpose(1, 2)).norm() <= 1e-2 * ref.norm()
+
+
     those that a lane joins."""
     from hetu_galvatron_b200.ops.gemm import head_xent_loss, head_xent_stats
     g = torch.Generator(device="cuda").manual_seed(rows)
