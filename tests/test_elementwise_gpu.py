@@ -335,7 +335,7 @@ def test_rope_runs_of_heads(tokens, heads, dh, inverse):
     ang = (pos.float()[:, None] * freq[None]).double()[:, None]
     a, b, sn = old[:, :heads, :dh // 2], old[:, :heads, dh // 2:], ang.sin() * (-1 if inverse else 1)
     ref = torch.cat([a * ang.cos() - b * sn, b * ang.cos() + a * sn], -1)
-    # one rounding to bf16, sines to 1e-7
+    # one rounding to bf16 and one in the products; the sines themselves are checked in fp32 below
     assert ((buf[:, :heads].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6 * (a.abs() + b.abs() + 1).repeat(1, 1, 2)).all()
     assert torch.equal(buf[:, heads:].double(), old[:, heads:])
 
@@ -367,3 +367,35 @@ def test_gates_are_as_exact_as_divisions():
     assert (sig <= bound).all() and sig.max() <= sig_div.max() * (1 + 2.0 ** -20) and sig.mean() <= sig_div.mean() * (1 + 1e-4)
     big = (x.double() * ref).abs() > 2.0 ** -126
     assert (err(_eval(3, x), x.double() * ref) <= bound)[big].all()
+
+
+def test_sines_in_fp32():
+    """Sine and cosine of the rotation: 6.4e-8 of 64 bits up to 65536 (dense values, both sides of every multiple of pi / 4 there, the
+    ends of the range), CUDA's 2 units beyond."""
+    g = torch.Generator(device=DEV).manual_seed(0)
+    dense = torch.cat([torch.rand(1 << 22, device=DEV, generator=g) * s for s in (1.0, 10.0, 1000.0, 65536.0)])
+    edges = (torch.arange(83443, device=DEV, dtype=torch.float64) * (torch.pi / 4)).float()
+    edges = torch.cat([edges, torch.nextafter(edges, torch.zeros_like(edges)), torch.nextafter(edges, torch.full_like(edges, 1e9))])
+    top = torch.tensor([65536.0, 65535.996, 65536.004, 1e-30, 0.0, 3e5, 1e9, 3e38], device=DEV)
+    x = torch.cat([dense, edges, top])
+    x = torch.cat([x, -x])
+    near = x.abs() <= 65536.0
+    for which, f in ((0, torch.sin), (1, torch.cos)):
+        err = (_eval(which, x).double() - f(x.double())).abs()
+        assert err[near].max() <= 6.5e-8 and err[~near].max() <= 2.0 ** -23
+
+
+def test_gelu_in_fp32():
+    """GELU and its derivative over every bf16 number up to 2^40, against 64 bits."""
+    x = _all_bf16()
+    x = x[x.abs() < 2.0 ** 40]
+    v = x.double()
+    c = 2 * (2 / torch.pi) ** 0.5
+    z = c * (v + 0.044715 * v ** 3)
+    s = torch.sigmoid(z)
+    # the argument is off by three roundings, exp(-z) by CUDA's bound of 2 + 1.173 |z| units besides, where the result does not vanish
+    unit = (8 + 4.2 * z.abs().clamp(max=90)) * 2.0 ** -23
+    assert ((_eval(5, x).double() - v * s).abs() <= unit * (v * s).abs() + 1e-30).all()
+    a, b = v * s * (1 - s) * c * (1 + 0.134145 * v * v), s
+    ok = v.abs() < 2.0 ** 15
+    assert ((_eval(6, x).double() - (a + b)).abs() <= 3 * unit * (a.abs() + b) + 1e-30)[ok].all()

@@ -338,7 +338,7 @@ def test_rotary_epilogue_positions(M, dh, largest):
     ang = (pos.float()[:, None] * freq[None]).double()[:, None]
     a, b = h[:, :3, :dh // 2], h[:, :3, dh // 2:]
     ref = torch.cat([a * ang.cos() - b * ang.sin(), b * ang.cos() + a * ang.sin()], -1)
-    # bf16 rounding of the result, fp32 sums of 64 products, sines to 1e-7
+    # bf16 rounding of the result, fp32 sums of 64 products (the sines are checked in fp32 in test_elementwise_gpu.py)
     bound = 2.0 ** -8 * ref.abs() + 1e-5 * (a.abs() + b.abs() + 1).repeat(1, 1, 2)
     assert ((y[:, :3] - ref).abs() <= bound).all()
     assert ((y[:, 3] - h[:, 3]).abs() <= 2.0 ** -8 * h[:, 3].abs() + 1e-5).all()
@@ -437,6 +437,25 @@ def test_head_statistics_merge(rows, V, vocab_start):
     assert (d[labels == -100] == 0).all()
 
 
+@pytest.mark.parametrize("rows,tiles", [(1, 1), (9, 40), (300, 70)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_head_statistics_of_bad_weights(rows, tiles, bad):
+    """A tile of the vocabulary whose weights have gone NaN or infinite shows in the loss of every row, wherever the tile is among
+    those that a lane joins."""
+    from hetu_galvatron_b200.ops.gemm import head_xent_loss, head_xent_stats
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, 64, device="cuda", dtype=torch.bfloat16, generator=g)
+    w = torch.randn(256 * tiles, 64, device="cuda", dtype=torch.bfloat16, generator=g)
+    x[:, 0] = 1.0
+    labels = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    for tile in sorted({0, tiles // 2, tiles - 1}):
+        broken = w.clone()
+        broken[256 * tile:256 * (tile + 1), 0] = bad              # the logits of these columns
+        loss, lse = head_xent_loss(x, broken, labels)
+        _, se, _ = head_xent_stats(x, broken, labels)
+        assert not torch.isfinite(loss).any() and not torch.isfinite(lse).any() and not torch.isfinite(se).any()
+
+
 @pytest.mark.parametrize("dh,s,hq,hk", [(50, 33, 3, 3), (2, 5, 1, 1), (74, 130, 4, 2), (25, 40, 2, 2)])
 def test_heads_padded_around_attention(dh, s, hq, hk):
     """Head sizes that are no multiple of 8, as strided views of a packed projection: forward and backward against 64 bits."""
@@ -460,25 +479,6 @@ def test_heads_padded_around_attention(dh, s, hq, hk):
         assert ((got.double() - want).norm() / want.norm()).item() < 1e-2
 
 
-@pytest.mark.parametrize("M,N,K", [(72, 40, 1), (136, 264, 67), (1280, 592, 6939), (5120, 1280, 3003), (192, 768, 9217)])
-def test_weight_gradient_of_any_row_count(M, N, K):
-    """Operands stored along M and N reduce over any number of rows (of the last, smaller batch of an epoch): fp32 accumulation into
-    a gradient buffer on single CTAs, pairs and split reductions, against 64 bits."""
-    g = torch.Generator(device="cuda").manual_seed(K)
-    dy = torch.randn(K, M, device="cuda", dtype=torch.bfloat16, generator=g)
-    x = torch.randn(K, N, device="cuda", dtype=torch.bfloat16, generator=g)
-    buf = torch.randn(M, N, device="cuda", generator=g)
-    ref = buf.double() + dy.double().t() @ x.double()
-    size = buf.double().abs() + dy.double().abs().t() @ x.double().abs()
-    before = _lib.launch_count()
-    gemm(dy, x, a_mn=True, b_mn=True, out=buf, accumulate=True)
-    assert _lib.launch_count() == before + 1                 # the kernel, not the library
-    assert ((buf.double() - ref).abs() <= (K + 4) * 2.0 ** -23 * size).all()
-    assert _lib.read_error() is None
-@pytest.mark.parametrize("rows,tiles", [(1, 1), (9, 40), (300, 70)])
-@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
-def test_head_statistics_of_bad_weights(rows, tiles, bad):
-    """A tile of the vocabulary whose weights have gone NaN or infinite shows in the loss of every row, wherever the tile is among
 @pytest.mark.parametrize("dh", [50, 25])
 @pytest.mark.parametrize("form", ["heads first", "odd rows", "expanded gradient"])
 def test_padded_heads_of_other_strides(dh, form):
@@ -509,18 +509,18 @@ def test_padded_heads_of_other_strides(dh, form):
     assert (res[0][0].double() - ref.transpose(1, 2)).norm() <= 1e-2 * ref.norm()
 
 
-    those that a lane joins."""
-    from hetu_galvatron_b200.ops.gemm import head_xent_loss, head_xent_stats
-    g = torch.Generator(device="cuda").manual_seed(rows)
-    x = torch.randn(rows, 64, device="cuda", dtype=torch.bfloat16, generator=g)
-    w = torch.randn(256 * tiles, 64, device="cuda", dtype=torch.bfloat16, generator=g)
-    x[:, 0] = 1.0
-    labels = torch.zeros(rows, dtype=torch.int64, device="cuda")
-    for tile in sorted({0, tiles // 2, tiles - 1}):
-        broken = w.clone()
-        broken[256 * tile:256 * (tile + 1), 0] = bad              # the logits of these columns
-        loss, lse = head_xent_loss(x, broken, labels)
-        _, se, _ = head_xent_stats(x, broken, labels)
-        assert not torch.isfinite(loss).any() and not torch.isfinite(lse).any() and not torch.isfinite(se).any()
-
-
+@pytest.mark.parametrize("M,N,K", [(72, 40, 1), (136, 264, 67), (1280, 592, 6939), (5120, 1280, 3003), (192, 768, 9217)])
+def test_weight_gradient_of_any_row_count(M, N, K):
+    """Operands stored along M and N reduce over any number of rows (of the last, smaller batch of an epoch): fp32 accumulation into
+    a gradient buffer on single CTAs, pairs and split reductions, against 64 bits."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    dy = torch.randn(K, M, device="cuda", dtype=torch.bfloat16, generator=g)
+    x = torch.randn(K, N, device="cuda", dtype=torch.bfloat16, generator=g)
+    buf = torch.randn(M, N, device="cuda", generator=g)
+    ref = buf.double() + dy.double().t() @ x.double()
+    size = buf.double().abs() + dy.double().abs().t() @ x.double().abs()
+    before = _lib.launch_count()
+    gemm(dy, x, a_mn=True, b_mn=True, out=buf, accumulate=True)
+    assert _lib.launch_count() == before + 1                 # the kernel, not the library
+    assert ((buf.double() - ref).abs() <= (K + 4) * 2.0 ** -23 * size).all()
+    assert _lib.read_error() is None
