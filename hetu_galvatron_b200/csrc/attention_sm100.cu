@@ -21,9 +21,6 @@
 #include "include/gv_host.h"
 #include "include/gv_ptx.cuh"
 
-#ifndef GV_POLL_NS
-#define GV_POLL_NS 20
-#endif
 namespace gv {
 
 int num_sms();
@@ -802,7 +799,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (progress) {
           idle = 0;
           t0 = 0;
-        } else if (__nanosleep(GV_POLL_NS), (++idle & 0x3ff) == 0) {
+        } else if (__nanosleep(20), (++idle & 0x3ff) == 0) {
           if (*abort_flag) { ok = false; break; }
           const uint64_t now = global_timer_ns();
           if (t0 == 0) {
@@ -833,8 +830,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     auto vote = [&](bool good) { return g == 0 ? named_bar_all<2, 128>(good) : named_bar_all<3, 128>(good); };
     bool ok = true;
     // One round: the dQ block of the group's previous iteration (which frees the columns for dP), P of iteration `it` while
-    // dP is multiplied, dS of `it`; the last round only has the dQ block. A wait that gave up is carried to the next vote, which all 128 threads reach: the loop is only left
-    // right after one, and the .sync.aligned TMEM accesses stay warp-uniform.
+    // dP is multiplied, dS of `it`; the last round only has the dQ block. A wait that gave up is carried to the next vote, which
+    // all 128 threads reach: the loop is only left right after one, and the .sync.aligned TMEM accesses stay warp-uniform.
     for (int it = g; it < n_iter + 2; it += 2) {
       const bool cur = it < n_iter, prev = it >= 2 + g;
       if (!cur && !prev) break;
@@ -849,8 +846,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       float pr[64];                    // probabilities of this thread's key at the 64 query columns, before dropout
       uint32_t keep[2] = {0u, 0u};     // DROP: which of them survive
       if (prev) {
-        // dQ^T of the previous iteration [lane = head-dim index, columns = query rows] from the dP columns. The block is staged as [query row][head dim] fp32 and added
-        // into dq_accum by bulk tensor reductions (the adds happen at L2).
+        // dQ^T of the previous iteration [lane = head-dim index, columns = query rows] from the dP columns. The block is staged as
+        // [query row][head dim] fp32 and added into dq_accum by bulk tensor reductions (the adds happen at L2).
         const int pi = it - 2, phead = kv_head * rep + pi / n_q, pq = (q_start + pi % n_q) * BWD_BQ;
         good = good && mbar_wait(gbar(g, B_DQ_FULL), (j - 1) & 1, abort_flag, 0x2e);
         if (issuer) tma_store_wait_read<0>();          // the staging buffer is free again
