@@ -1258,7 +1258,10 @@ static int split_plan(const gv_gemm_args* a) {
   if (forced == 1 || a->rope_cols > 0 || a->swiglu_out || a->gelu_out || a->M <= 0 || a->N <= 0 || a->K <= 0) return 1;
   const int kb = (a->K + BK - 1) / BK;
   if (forced) return kb >= forced ? forced : 1;
-  if (pair_mode() != 1 || kb < 96) return 1;      // shorter ones gain 2 us at most (512 x 512 x 4096: 18.7 -> 16.6)
+  // Not fitted below 96 k-blocks, where the join weighs as much as what it saves. Forced splits, us unsplit / in two / three / four:
+  // 2999 x 3584 x 3584 68 / 76 / 93 / 115, 2048 x 1024 x 5120 29 / 31 / 37 / 41, 1024 x 2816 x 4096 39 / 37 / 35 / 41,
+  // 3840 x 1280 x 5120 64 / 55 / 59 / 63, 512 x 512 x 5632 29 / 27 / 25 / 23: some there would gain up to a fifth and are left.
+  if (pair_mode() != 1 || kb < 96) return 1;
   const long tiles = static_cast<long>((a->M + 255) / 256) * ((a->N + 255) / 256);
   const long sms = num_sms();
   const bool on_pairs = !narrow_tiles(a) && tiles >= sms / 2;
