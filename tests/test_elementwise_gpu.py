@@ -37,8 +37,9 @@ def test_rmsnorm(rows, cols):
 
 
 # edges of the row layouts: one vector, a lane short of and past a warp's share, each step of vectors per thread and of warps per
-# row, the widest row; single rows, odd rows, more rows than ring stages of every CTA
-NORM_EDGES = [(1, 8), (3, 248), (2, 264), (5, 1032), (131, 2048), (17, 2056), (9, 4104), (3, 8184), (4099, 768), (2500, 3584)]
+# row, the widest row; single rows, odd rows, more rows than ring stages of every CTA; the last ones with more rows than are few
+NORM_EDGES = [(1, 8), (3, 248), (2, 264), (5, 1032), (131, 2048), (17, 2056), (9, 4104), (3, 8184), (4099, 768), (2500, 3584),
+              (1201, 520), (1201, 1032), (1201, 2048), (1201, 2056), (1201, 4104), (1201, 8184), (149, 4096)]
 
 
 @pytest.mark.parametrize("layer", [False, True])
@@ -79,7 +80,7 @@ def test_rmsnorm_statistics_in_fp32(cols):
 
 
 @pytest.mark.parametrize("layer", [False, True])
-@pytest.mark.parametrize("rows,cols", [(1, 8), (5, 1032), (17, 2056), (3, 8184)])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (5, 1032), (17, 2056), (3, 8184), (1201, 4104)])
 def test_norm_of_a_sum_that_is_not_stored(rows, cols, layer):
     """The C entry points with a residual and no buffer for the sum: the norm is that of the unrounded sum."""
     from hetu_galvatron_b200.ops import _lib
@@ -321,7 +322,7 @@ def test_embedding_gradient_buffers(tokens, V, H, vocab_start, offset):
         assert torch.equal(buf[size.sum(1) == 0], old[size.sum(1) == 0])
 
 
-@pytest.mark.parametrize("tokens,heads,dh", [(1, 1, 16), (33, 3, 64), (70, 9, 128), (300, 4, 80)])
+@pytest.mark.parametrize("tokens,heads,dh", [(1, 1, 16), (33, 3, 64), (70, 9, 128), (300, 4, 80), (4099, 1, 64), (2000, 7, 64)])
 @pytest.mark.parametrize("inverse", [False, True])
 def test_rope_runs_of_heads(tokens, heads, dh, inverse):
     """In-place rotation of a strided view, head counts that are no multiple of a run, positions on both sides of the limit of the
