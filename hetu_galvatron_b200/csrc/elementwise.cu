@@ -48,8 +48,9 @@ static inline int grid_for(long long work_items, int threads, int ctas_per_sm = 
 // ------------------------------------------------------------------ RoPE
 // One thread rotates 8 consecutive pairs (i, i + dh/2) in a run of heads of one token: the angles do not depend on the head, so
 // they are computed once per run. HBM-bound with runs of four heads: 8192 x 32 heads of 128 in place took 39 us with sincosf for
-// every head and now takes 24 (L2 cold).
-constexpr int ROPE_RUN = 4;
+// every head and now takes 24 (L2 cold). Runs of one head where there is no other to share with, or too few for a block per SM:
+// 65536 x 1 x 64 11.5 -> 9.5 us, 512 x 4 x 128 6.9 -> 5.4.
+template <int ROPE_RUN>
 __global__ void rope_kernel(bf16* __restrict__ x, const int* __restrict__ pos, const float* __restrict__ inv_freq,
                             long long tokens, int heads, int dh, long long ld, int pos_div, int pos_mod,
                             int pos_offset, int inverse) {
@@ -623,11 +624,13 @@ extern "C" int gv_rope(void* x, const int* pos, const float* inv_freq, long long
                        long long ld, int pos_div, int pos_mod, int pos_offset, int inverse, gv_stream_t s) {
   if (tokens <= 0) return 0;
   if (dh % 16 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15)) return 2201;
-  const long long total = tokens * ((heads + ROPE_RUN - 1) / ROPE_RUN) * (dh / 16);
-  rope_kernel<<<grid_for(total, 256), 256, 0, (cudaStream_t)s>>>((bf16*)x, pos, inv_freq, tokens, heads, dh, ld,
-                                                                 pos_div > 0 ? pos_div : 1,
-                                                                 pos_mod > 0 ? pos_mod : 0x7fffffff, pos_offset,
-                                                                 inverse);
+  auto go = [&](auto kern, int run) {
+    const long long total = tokens * ((heads + run - 1) / run) * (dh / 16);
+    kern<<<grid_for(total, 256), 256, 0, (cudaStream_t)s>>>((bf16*)x, pos, inv_freq, tokens, heads, dh, ld, pos_div > 0 ? pos_div : 1,
+                                                            pos_mod > 0 ? pos_mod : 0x7fffffff, pos_offset, inverse);
+  };
+  if (heads == 1 || tokens * heads * (dh / 16) <= 256ll * num_sms()) go(rope_kernel<1>, 1);
+  else go(rope_kernel<4>, 4);
   return (int)cudaGetLastError();
 }
 
