@@ -269,8 +269,10 @@ __device__ __forceinline__ void epi_put64(const uint32_t (&w)[32], float4* stage
   }
 }
 
-// alpha, bias and GELU on one row's 32 columns, rounded to bf16 pairs. The bias is the same for all lanes: broadcast loads.
-__device__ __forceinline__ void epi_pack32(const GemmDev& p, const uint32_t (&r)[32], int col0, uint32_t* w) {
+// alpha, bias, GELU and (RES) the residual on one row's 32 columns, rounded to bf16 pairs. The bias is the same for all lanes:
+// broadcast loads.
+template <bool RES = false>
+__device__ __forceinline__ void epi_pack32(const GemmDev& p, const uint32_t (&r)[32], int col0, uint32_t* w, const uint4* res = nullptr) {
   float v[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
@@ -291,8 +293,35 @@ __device__ __forceinline__ void epi_pack32(const GemmDev& p, const uint32_t (&r)
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
   }
+  if constexpr (RES) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 a = bf16x4_to_f4(res[j].x, res[j].y), b = bf16x4_to_f4(res[j].z, res[j].w);
+      v[8 * j] += a.x; v[8 * j + 1] += a.y; v[8 * j + 2] += a.z; v[8 * j + 3] += a.w;
+      v[8 * j + 4] += b.x; v[8 * j + 5] += b.y; v[8 * j + 6] += b.z; v[8 * j + 7] += b.w;
+    }
+  }
 #pragma unroll
   for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+}
+
+// The residual of one row's 32 columns, one row per lane (zeros beyond N).
+__device__ __forceinline__ void epi_load_res32(const GemmDev& p, int row, int col0, uint4 (&o)[4]) {
+  if (row >= p.M || col0 >= p.N) return;
+  const __nv_bfloat16* rp = p.residual + static_cast<size_t>(row) * p.ldr + col0;
+  if (col0 + 32 <= p.N) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = reinterpret_cast<const uint4*>(rp)[j];
+  } else {
+    const unsigned short* up = reinterpret_cast<const unsigned short*>(rp);
+    const int n = p.N - col0;
+    uint32_t w[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      w[i] = (2 * i < n ? up[2 * i] : 0u) | (2 * i + 1 < n ? static_cast<uint32_t>(up[2 * i + 1]) << 16 : 0u);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+  }
 }
 
 // Rotary embedding (non-interleaved halves) on two 32-column chunks of one output row that sit half a head apart:
@@ -540,6 +569,30 @@ __device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr,
         tmem_ld_32x32b_x32(t_addr + (c + h) * 32, r);
         tmem_ld_wait();
         epi_pack32(p, r, n0 + (c + h) * 32, w + 16 * h);
+      }
+      epi_put64(w, stage, lane, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.M, p.N, row0, n0 + c * 32);
+    }
+    return true;
+  }
+  // Residual and bf16 output: the residual comes one row per lane, like the accumulators, a chunk ahead, and is added before the
+  // chunk is rounded and staged. The store below moves twice the staging bytes: 36864 x 192 x 768 39.0 -> 32.8 us, 8192 x 1025 x 512
+  // 41.0 -> 33.9, 8192 x 1600 x 1600 58.4 -> 51.3 (34.8, 36.8 and 57.4 with the whole epilogue one row per lane). 128-wide tiles run where
+  // tiles are few, and there the time to the first store counts: 300 x 257 x 200 with a bias 12.4 us below, 14.2 this way.
+  if (BN == 256 && !SPLIT && p.residual != nullptr && !p.accumulate && !p.c_f32) {
+    uint4 res[4];
+    epi_load_res32(p, row, n0 + c0 * 32, res);
+    if (!wait()) return false;
+#pragma unroll 1
+    for (int c = c0; c < c0 + CHUNKS; c += 2) {
+      if (n0 + c * 32 >= p.N) break;
+      uint32_t w[32];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        __syncwarp();
+        tmem_ld_32x32b_x32(t_addr + (c + h) * 32, r);
+        tmem_ld_wait();
+        epi_pack32<true>(p, r, n0 + (c + h) * 32, w + 16 * h, res);
+        if (c + h + 1 < c0 + CHUNKS) epi_load_res32(p, row, n0 + (c + h + 1) * 32, res);
       }
       epi_put64(w, stage, lane, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.M, p.N, row0, n0 + c * 32);
     }

@@ -90,6 +90,27 @@ def test_gemm_epilogue_edges(M, N, K, f32):
     assert _lib.read_error() is None
 
 
+@pytest.mark.parametrize("M,N,K", [(19000, 200, 64), (19001, 333, 72), (2500, 2046, 136), (40, 257, 64)])
+@pytest.mark.parametrize("act", [False, True])
+def test_gemm_residual_into_bf16(M, N, K, act):
+    """The residual added before the bf16 rounding, on pairs and on narrow tiles, with tails of rows and
+    columns; in place, too: the residual's own buffer is the output."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    rnd = lambda *s: torch.randn(*s, device="cuda", dtype=torch.bfloat16, generator=g)
+    ld = (N + 7) // 8 * 8 + 8
+    a, b, bias, buf = rnd(M, K), rnd(N, K), rnd(ld)[:N], rnd(M, ld)
+    x = a.double() @ b.double().t() + bias.double()
+    ref = (torch.nn.functional.gelu(x, approximate="tanh") if act else x) + buf[:, :N].double()
+    size = a.double().abs() @ b.double().abs().t() + x.abs() + buf[:, :N].double().abs() + 1
+    old = buf.clone()
+    out = torch.empty_like(buf)
+    gemm(a, b, out=out[:, :N], bias=bias, gelu=act, residual=buf[:, :N])
+    assert ((out[:, :N].double() - ref).abs() <= (K + 16) * 2.0 ** -23 * size + 2.0 ** -8 * ref.abs()).all()
+    gemm(a, b, out=buf[:, :N], bias=bias, gelu=act, residual=buf[:, :N])
+    assert torch.equal(buf[:, :N], out[:, :N]) and torch.equal(buf[:, N:], old[:, N:])
+    assert _lib.read_error() is None
+
+
 @pytest.mark.parametrize("M,N,K", [(33, 6, 8), (33, 24, 64), (130, 40, 64), (300, 264, 128)])
 @pytest.mark.parametrize("offset", [1, 2, 4])
 def test_gemm_bias_at_any_address(M, N, K, offset):
