@@ -269,7 +269,7 @@ __device__ __forceinline__ void epi_put64(const uint32_t (&w)[32], float4* stage
   }
 }
 
-// alpha, bias, GELU and (RES) the residual on one row's 32 columns, rounded to bf16 pairs. The bias is the same for all lanes:
+// alpha, bias, GELU and (RES) the residual or old C on one row's 32 columns, rounded to bf16 pairs. The bias is the same for all lanes:
 // broadcast loads.
 template <bool RES = false>
 __device__ __forceinline__ void epi_pack32(const GemmDev& p, const uint32_t (&r)[32], int col0, uint32_t* w, const uint4* res = nullptr) {
@@ -305,10 +305,11 @@ __device__ __forceinline__ void epi_pack32(const GemmDev& p, const uint32_t (&r)
   for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
 }
 
-// The residual of one row's 32 columns, one row per lane (zeros beyond N).
+// 32 columns of the residual, or without one of the old C in bf16, one row per lane (zeros beyond N).
 __device__ __forceinline__ void epi_load_res32(const GemmDev& p, int row, int col0, uint4 (&o)[4]) {
   if (row >= p.M || col0 >= p.N) return;
-  const __nv_bfloat16* rp = p.residual + static_cast<size_t>(row) * p.ldr + col0;
+  const __nv_bfloat16* rp = p.residual != nullptr ? p.residual + static_cast<size_t>(row) * p.ldr + col0
+                                                  : reinterpret_cast<const __nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + col0;
   if (col0 + 32 <= p.N) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) o[j] = reinterpret_cast<const uint4*>(rp)[j];
@@ -574,11 +575,11 @@ __device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr,
     }
     return true;
   }
-  // Residual and bf16 output: the residual comes one row per lane, like the accumulators, a chunk ahead, and is added before the
+  // Residual or accumulation, and bf16 output: what is added comes one row per lane, like the accumulators, a chunk ahead, and is added before the
   // chunk is rounded and staged. The store below moves twice the staging bytes: 36864 x 192 x 768 39.0 -> 32.8 us, 8192 x 1025 x 512
   // 41.0 -> 33.9, 8192 x 1600 x 1600 58.4 -> 51.3 (34.8, 36.8 and 57.4 with the whole epilogue one row per lane). 128-wide tiles run where
   // tiles are few, and there the time to the first store counts: 300 x 257 x 200 with a bias 12.4 us below, 14.2 this way.
-  if (BN == 256 && !SPLIT && p.residual != nullptr && !p.accumulate && !p.c_f32) {
+  if (BN == 256 && !SPLIT && !p.c_f32 && (p.residual != nullptr) != (p.accumulate != 0)) {
     uint4 res[4];
     epi_load_res32(p, row, n0 + c0 * 32, res);
     if (!wait()) return false;

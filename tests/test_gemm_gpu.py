@@ -93,8 +93,8 @@ def test_gemm_epilogue_edges(M, N, K, f32):
 @pytest.mark.parametrize("M,N,K", [(19000, 200, 64), (19001, 333, 72), (2500, 2046, 136), (40, 257, 64)])
 @pytest.mark.parametrize("act", [False, True])
 def test_gemm_residual_into_bf16(M, N, K, act):
-    """The residual added before the bf16 rounding, on pairs and on narrow tiles, with tails of rows and
-    columns; in place, too: the residual's own buffer is the output."""
+    """The residual added before the bf16 rounding, on pairs and on narrow tiles, with tails of rows and columns; in place, too: the
+    residual's own buffer is the output; and the same bits by accumulation into a bf16 buffer."""
     g = torch.Generator(device="cuda").manual_seed(M + N)
     rnd = lambda *s: torch.randn(*s, device="cuda", dtype=torch.bfloat16, generator=g)
     ld = (N + 7) // 8 * 8 + 8
@@ -108,6 +108,9 @@ def test_gemm_residual_into_bf16(M, N, K, act):
     assert ((out[:, :N].double() - ref).abs() <= (K + 16) * 2.0 ** -23 * size + 2.0 ** -8 * ref.abs()).all()
     gemm(a, b, out=buf[:, :N], bias=bias, gelu=act, residual=buf[:, :N])
     assert torch.equal(buf[:, :N], out[:, :N]) and torch.equal(buf[:, N:], old[:, N:])
+    acc = old.clone()
+    gemm(a, b, out=acc[:, :N], bias=bias, gelu=act, accumulate=True)
+    assert torch.equal(acc, buf)
     assert _lib.read_error() is None
 
 
