@@ -219,3 +219,23 @@ def test_windowed_forward_repeats_bit_for_bit():
         o, l = AT.fwd(q, k, v, False, 32 ** -0.5, additive=add)
         assert torch.equal(o, first) and torch.equal(l, lse)
     assert _lib.read_error() is None
+
+
+def test_more_sequences_than_a_grid_dimension():
+    """Tiles of equal length are found by grid dimensions up to 65535 sequences and by their number beyond; forward and backward
+    against 64 bits."""
+    from hetu_galvatron_b200.ops import _lib, attention as AT
+    g = torch.Generator(device="cuda").manual_seed(0)
+    b, s, h, dh = 65537, 3, 2, 8
+    q, k, v, do = (torch.randn(b, s, h, dh, device="cuda", dtype=torch.bfloat16, generator=g) for _ in range(4))
+    o, lse = AT.fwd(q, k, v, False, dh ** -0.5)
+    grads = AT.bwd(do, q, k, v, o, lse, False, dh ** -0.5)
+    x = [t.double().transpose(1, 2).requires_grad_() for t in (q, k, v)]
+    ref = ((x[0] @ x[1].transpose(-1, -2)) * dh ** -0.5).softmax(-1) @ x[2]
+    want = torch.autograd.grad(ref, x, do.double().transpose(1, 2))
+    # bf16 probabilities, score gradients and results
+    for got, r in zip((o, *grads), (ref, *want)):
+        r = r.transpose(1, 2)
+        assert (got.double() - r).norm() <= 1e-2 * r.norm()
+        assert (got[-1].double() - r[-1]).norm() <= 3e-2 * r[-1].norm()      # the last sequence, beyond the dimension
+    assert _lib.read_error() is None
