@@ -8,8 +8,11 @@
 // ring. S = Q K^T lands in TMEM (double buffered), four softmax warps (one row per thread) turn it into
 // bf16 P in the same columns, O += P V reads P from there and accumulates in TMEM with lazy rescaling (O is only
 // rescaled when the running row maximum grew by more than 2^8, and only then does the softmax wait for the
-// previous product). Two CTAs fit per SM so one CTA's softmax overlaps the other's MMAs. With P in swizzled shared
-// memory behind one wait per block, 16384 tokens, 32 / 8 heads of 128, took 2200 us; now 2046 us.
+// previous product). Two CTAs fit per SM so one CTA's softmax overlaps the other's MMAs. K and V have rings of their own: a
+// stage of K is free as soon as S is there, a softmax and a product before V's, and with one barrier for both the load of K came
+// too late for the next S. 16384 tokens, 32 / 8 heads of 128: 2200 us with P in swizzled shared memory behind one wait per block,
+// 2046 with P in TMEM, 1705 with separate rings (4096 tokens, 32 heads, two sequences: 322 -> 252; 64-wide heads, 2048 tokens:
+// 80 -> 74).
 //
 // Backward: one CTA = 128 KV rows of one (batch, kv head); it loops over the query heads of its group and
 // over 64-row query blocks, holding dK and dV in TMEM. Per block: S^T = K Q^T, dP^T = V dO^T (TMEM),
@@ -181,12 +184,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* q_full = bars + 0;
   uint64_t* k_full = bars + 1;    // [2]
   uint64_t* v_full = bars + 3;    // [2]
-  uint64_t* kv_empty = bars + 5;  // [2]
-  uint64_t* s_full = bars + 7;    // [2]
+  uint64_t* k_empty = bars + 5;   // [2], K is free once S is there, V a softmax and a product later
+  uint64_t* v_empty = bars + 7;   // [2]
+  uint64_t* s_full = bars + 9;    // [2]
   // one per score buffer: a warp that is a block ahead of another must not arrive in its place
-  uint64_t* p_full = bars + 9;    // [2]
-  uint64_t* pv_done = bars + 11;  // [PV_BARRIERS], see pv_phase
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11 + PV_BARRIERS);
+  uint64_t* p_full = bars + 11;   // [2]
+  uint64_t* pv_done = bars + 13;  // [PV_BARRIERS], see pv_phase
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13 + PV_BARRIERS);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   if (static_cast<int>(smem - smem_raw) + S::OFF_BAR + 128 > S::TOTAL) {  // dynamic smem base less aligned than assumed
@@ -213,7 +217,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1);
       mbar_init(&v_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
+      mbar_init(&k_empty[i], 1);
+      mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 128);
     }
@@ -245,12 +250,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tma_load_4d(smem + S::OFF_Q + c * (FWD_BM * 128), &tmQ, q_full, c * 64, head, q0, batch);
       for (int j = 0; j < n_blocks; ++j) {
         const int st = j & 1;
-        if (!mbar_wait(&kv_empty[st], ((j >> 1) & 1) ^ 1, abort_flag, 0x11)) break;
+        if (!mbar_wait(&k_empty[st], ((j >> 1) & 1) ^ 1, abort_flag, 0x11)) break;
         mbar_expect_tx(&k_full[st], S::KV_BYTES);
 #pragma unroll
         for (int c = 0; c < S::PANELS; ++c)
           tma_load_4d(smem + S::OFF_K + st * S::KV_BYTES + c * (FWD_BN * 128), &tmK, &k_full[st], c * 64, kv_head,
                       j * FWD_BN, batch);
+        if (!mbar_wait(&v_empty[st], ((j >> 1) & 1) ^ 1, abort_flag, 0x1b)) break;
         mbar_expect_tx(&v_full[st], S::KV_BYTES);
 #pragma unroll
         for (int c = 0; c < S::PANELS; ++c)
@@ -278,6 +284,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           umma_f16_ss<1>(d_tmem, da, db, idesc_s, kk != 0 ? 1u : 0u);
         }
         umma_commit<1>(&s_full[j & 1]);
+        umma_commit<1>(&k_empty[j & 1]);
       };
       bool ok = mbar_wait(q_full, 0, abort_flag, 0x12) && mbar_wait(&k_full[0], 0, abort_flag, 0x13);
       if (ok) {
@@ -302,7 +309,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const uint64_t db = v_desc + static_cast<uint64_t>((kk * 2048) >> 4);
           umma_f16_ts(tmem_base + TM_O, tmem_base + TM_S + (j & 1) * FWD_BN + kk * 8, db, idesc_pv, (j | kk) != 0 ? 1u : 0u);
         }
-        umma_commit<1>(&kv_empty[j & 1]);
+        umma_commit<1>(&v_empty[j & 1]);
         umma_commit<1>(&pv_done[pv_phase(j).barrier]);
       }
     }
