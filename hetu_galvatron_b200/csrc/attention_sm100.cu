@@ -17,7 +17,8 @@
 // Backward: one CTA = 128 KV rows of one (batch, kv head); it loops over the query heads of its group and
 // over 64-row query blocks, holding dK and dV in TMEM. Per block: S^T = K Q^T, dP^T = V dO^T (TMEM),
 // two epilogue warpgroups write P^T back to TMEM and dS^T to shared memory, dV += P^T dO, dK += dS^T Q,
-// dQ^T = K^T dS^T is read back from TMEM and added into an fp32 dQ buffer with bulk reductions.
+// dQ^T = K^T dS^T is read back from TMEM by a third warpgroup and added into an fp32 dQ buffer, four rows a time. Three threads
+// issue the products, each the kinds that follow one another.
 // Every operand is consumed in the layout it has in shared memory (K-major or MN-major descriptors).
 #include "include/gv_attn_order.h"
 #include "include/gv_kernels.h"
@@ -494,41 +495,51 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 constexpr int BWD_BKV = 128;  // KV rows per CTA
 constexpr int BWD_BQ = 64;    // query rows per inner block
 constexpr int BWD_DH = 128;   // head dim is padded to 128 inside the kernel
-constexpr int BWD_THREADS = 64 + 256;
+constexpr int BWD_THREADS = 512;
 // Rings of query blocks in shared memory. Q of an iteration is needed from S to dK, its last product, dO only from dP to dV; with
 // three stages of both, S of the next iteration waited for its Q (730 of 6100 clk a round), with four of Q and two of dO it does
 // not, in the same 96 KB.
-constexpr int BWD_QSTAGES = 4, BWD_DOSTAGES = 2;
+constexpr int BWD_QSTAGES = 4, BWD_DOSTAGES = 4;
 
 // Two (kv tile, q block) iterations are in flight per CTA: epilogue group 0 (warps 2-5) owns the even iterations,
 // group 1 (warps 6-9) the odd ones, each with its own accumulators in TMEM, so the tensor cores work for one group while
 // the other does its exponentials. Within a group the steps of neighbouring iterations overlap too: P is computed as soon as
 // S is there and goes back to TMEM, where it is the A operand of dV += P^T dO (no shared memory, no fence); S of the next
-// iteration follows that product, so the group finds it ready; and dP is multiplied while the group computes P. Clocks of a
-// round of one group (two iterations of the CTA) at 8192 tokens, 32 / 8 heads: 6910 with P before the dQ block and with lse and
-// delta loaded after the ring slot came free, 6530 with them loaded before, 6100 with the dQ block first.
+// iteration follows that product, so the group finds it ready; dP is multiplied while the group computes P; and dQ leaves by way
+// of warps of its own while the group goes on.
+// Clocks of an iteration at 8192 tokens, 32 / 8 heads of 128: 3050 with one issuing thread that polled for every kind of product
+// (1900 of them for its tests of barriers) and the groups staging dQ in shared memory for bulk reductions; 2720 with three
+// issuing threads and warps for dQ, which then waited 1170 for the reductions to have read the staging buffer; 2340 with the
+// additions straight from registers. The tensor cores need 1740 (N = 64 products run at two thirds of their rate), the additions
+// 1770 of the dQ warps: an SM gets rid of about 21 bytes of them a clock, whatever their form.
+// us with delta, clearing and conversion, before -> now: 16384 tokens, 32 / 8 heads of 128, 6075 -> 5010 to 5250; 4096 tokens, 32
+// heads, two sequences, 972 -> 820 to 850; 2999 tokens, 28 / 4 heads, 584 -> 445; 2048 tokens, 16 heads of 64, four sequences,
+// 272 -> 209; 512 keys with padding, 16 heads of 80, 16 sequences, 191 -> 166; 1024 tokens with dropout, 32 heads of 56, 8 sequences,
+// 465 -> 384.
 // TMEM (512 columns): group g: S^T at g*128, overwritten by P^T (bf16, 32 columns); dP^T at g*128 + 64, overwritten by dQ^T;
 // dV at 256, dK at 384.
 struct BwdSmem {
   static constexpr int K_BYTES = BWD_BKV * BWD_DH * 2;   // 32 KB, 2 panels of [128 x 128 B]
   static constexpr int Q_BYTES = BWD_BQ * BWD_DH * 2;    // 16 KB, 2 panels of [64 x 128 B]
   static constexpr int DS_BYTES = BWD_BKV * BWD_BQ * 2;  // 16 KB, 1 panel of [128 x 128 B]
-  // per group: 16 KB for the dQ block [64][dh] fp32 on its way out, then dS^T; a head size above 64 makes the block 32 KB,
-  // and its second half of the rows goes where the (consumed) dS^T was
-  static constexpr int OFF_DS_IN_R = 32 * BWD_DH * 4;
-  static constexpr int R_BYTES = OFF_DS_IN_R + DS_BYTES;
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = K_BYTES;
   static constexpr int OFF_Q = 2 * K_BYTES;                       // [BWD_QSTAGES]
   static constexpr int OFF_DO = OFF_Q + BWD_QSTAGES * Q_BYTES;    // [BWD_DOSTAGES]
-  static constexpr int OFF_R = OFF_DO + BWD_DOSTAGES * Q_BYTES;   // [2]
-  static constexpr int OFF_STAT = OFF_R + 2 * R_BYTES;            // lse and delta, [BWD_QSTAGES][64] floats each
+  static constexpr int OFF_DS = OFF_DO + BWD_DOSTAGES * Q_BYTES;  // [2] one per group
+  static constexpr int OFF_STAT = OFF_DS + 2 * DS_BYTES;          // lse and delta, [BWD_QSTAGES][64] floats each
   static constexpr int OFF_BAR = OFF_STAT + 2 * BWD_QSTAGES * 64 * 4;
   static constexpr int BAR_BYTES = 320;
   static constexpr int TOTAL = OFF_BAR + BAR_BYTES + 704;         // the kernel checks that the base needs no more alignment
 };
 static_assert(BwdSmem::TOTAL <= 232448, "attention backward shared memory budget");
-static_assert(BWD_BQ * BWD_DH * 4 <= BwdSmem::R_BYTES, "dQ staging fits the group region");
+
+// dq_accum holds the rows of one head of one batch element in groups of four: a group is [head dim][4 rows], so that a thread with one
+// column of dQ^T adds its four rows as one piece. The last group of a sequence has its sq % 4 rows, [head dim][rows]. First element
+// of a group:
+__device__ __forceinline__ long long dq_group(long long head_of_batch, int group, int sq, int dh) {
+  return (head_of_batch * sq + 4 * static_cast<long long>(group)) * dh;
+}
 
 struct BwdParams {
   const float* lse;
@@ -538,7 +549,7 @@ struct BwdParams {
   float drop_scale;
   unsigned long long drop_seed;
   int drop_head_offset;
-  float* dq_accum;  // fp32 [b, sq, hq, dh] contiguous
+  float* dq_accum;  // fp32, b * hq * sq * dh elements, see dq_group
   bf16* dk;
   bf16* dv;
   int b, sq, sk, hq, hk, dh;
@@ -557,11 +568,15 @@ struct BwdParams {
   int mask_n, bias_ld;
 };
 
+// Registers of the roles: the issuing warps (0-3) and the dQ warps (4-7) give up what the two groups (8-15) need. The sum over
+// the four warpgroups must not exceed what the block is launched with (see launch).
+constexpr int BWD_REGS_ISSUE = 72, BWD_REGS_DRAIN = 88, BWD_REGS_GROUP = 176;
+static_assert(BWD_REGS_ISSUE + BWD_REGS_DRAIN + 2 * BWD_REGS_GROUP <= 4 * 128, "register split");
+
 template <int MODE>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                const __grid_constant__ CUtensorMap tmDQ, BwdParams p) {
+                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, BwdParams p) {
   using S = BwdSmem;
   constexpr bool BIAS = MODE == MODE_BIAS, DROP = MODE == MODE_DROP;
   extern __shared__ uint8_t smem_raw[];
@@ -578,12 +593,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* q_empty = bars + 5;     // [BWD_QSTAGES]
   uint64_t* stat_full = bars + 9;   // [BWD_QSTAGES]
   uint64_t* do_full = bars + 13;    // [BWD_DOSTAGES]
-  uint64_t* do_empty = bars + 15;   // [BWD_DOSTAGES]
-  // per group g (8 barriers each, starting at 17 + 8 g)
-  auto gbar = [&](int g, int which) { return bars + 17 + 8 * g + which; };
+  uint64_t* do_empty = bars + 17;   // [BWD_DOSTAGES]
+  // per group g (8 barriers each, starting at 21 + 8 g)
+  auto gbar = [&](int g, int which) { return bars + 21 + 8 * g + which; };
   enum { B_S_FULL = 0, B_DP_FULL, B_PT_FULL, B_DS_FULL, B_DQ_FULL, B_DK_DONE, B_PV_DONE, B_DP_FREE };
-  uint64_t* all_done = bars + 33;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 34);
+  uint64_t* all_done = bars + 37;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 38);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -600,6 +615,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   // a tile made of padding keys only receives no gradient: no iterations, zeros are written
   const int n_q = kv0 >= sk_eff ? 0 : max(0, n_qblocks_total - q_start);
   const int n_iter = n_q * rep;  // iterations: (head in group, q block)
+  // (head of the group, query block) of an iteration, carried along instead of divided out each time (the groups divide: they do
+  // it while they wait, and with dropout the kernel is 6 % slower when they carry it, too)
+  struct At {
+    int rep, q;
+    __device__ __forceinline__ void advance(int by, int n_q) {
+      q += by;
+      while (q >= n_q) { q -= n_q; ++rep; }
+    }
+  };
   const int panels = p.dh <= 64 ? 1 : 2;     // 64-wide head-dim panels that hold data
   const int ksteps = panels * 4;             // 16-wide contraction steps over the head dim (S^T, dP^T)
   constexpr uint32_t TMEM_COLS = 512;
@@ -626,14 +650,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(gbar(g, B_PV_DONE), 1);
       mbar_init(gbar(g, B_DP_FREE), 128);
     }
-    mbar_init(all_done, 1);
+    mbar_init(all_done, 2);            // dV's and dK's issuers
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmDO);
-    tma_prefetch_desc(&tmDQ);
   }
   if (warp == 1) {
     tmem_alloc<1>(tmem_slot, TMEM_COLS);
@@ -644,222 +667,159 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    // ---------------- producer: K, V once; then Q, lse, delta and dO of each iteration into their rings ----------------
-    bool ok = true;
-    if (lane == 0 && n_iter > 0) {
-      // head sizes up to 64 fill one 64-wide panel of every operand: the second panel is neither loaded nor multiplied
-      mbar_expect_tx(kv_full, 2 * panels * (BWD_BKV * 128));
-      for (int c = 0; c < panels; ++c) {
-        tma_load_4d(smem + S::OFF_K + c * (BWD_BKV * 128), &tmK, kv_full, c * 64, kv_head, kv0, batch);
-        tma_load_4d(smem + S::OFF_V + c * (BWD_BKV * 128), &tmV, kv_full, c * 64, kv_head, kv0, batch);
+  // (each warpgroup sets its registers in its own branch: where branches join again the compiler counts on the fewest)
+  if (warp < 4) {
+    reg_dealloc<BWD_REGS_ISSUE>();
+    if (warp == 0) {
+      // ---------------- producer: K, V once; then Q, lse, delta and dO of each iteration into their rings ----------------
+      bool ok = true;
+      if (lane == 0 && n_iter > 0) {
+        // head sizes up to 64 fill one 64-wide panel of every operand: the second panel is neither loaded nor multiplied
+        mbar_expect_tx(kv_full, 2 * panels * (BWD_BKV * 128));
+        for (int c = 0; c < panels; ++c) {
+          tma_load_4d(smem + S::OFF_K + c * (BWD_BKV * 128), &tmK, kv_full, c * 64, kv_head, kv0, batch);
+          tma_load_4d(smem + S::OFF_V + c * (BWD_BKV * 128), &tmV, kv_full, c * 64, kv_head, kv0, batch);
+        }
       }
-    }
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const int st = it % BWD_QSTAGES, use = it / BWD_QSTAGES;
-      const int head = kv_head * rep + it / n_q;
-      const int qb = q_start + it % n_q;
-      // per-row statistics of the block (plain loads: tiny), on their way while the ring stage is still in use. Both are
-      // stored negated, ready to add; -inf -> P = 0 for padded rows
-      const long long base = (static_cast<long long>(batch) * p.hq + head) * p.sq + qb * BWD_BQ;
-      float lse[2], delta[2];
+      At at = {0, 0};
+      for (int it = 0; it < n_iter && ok; ++it, at.advance(1, n_q)) {
+        const int st = it % BWD_QSTAGES, use = it / BWD_QSTAGES;
+        const int head = kv_head * rep + at.rep;
+        const int qb = q_start + at.q;
+        // per-row statistics of the block (plain loads: tiny), on their way while the ring stage is still in use. Both are
+        // stored negated, ready to add; -inf -> P = 0 for padded rows
+        const long long base = (static_cast<long long>(batch) * p.hq + head) * p.sq + qb * BWD_BQ;
+        float lse[2], delta[2];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const bool in = qb * BWD_BQ + lane + 32 * h < p.sq;
-        lse[h] = in ? -p.lse[base + lane + 32 * h] * LOG2E : -INFINITY;
-        delta[h] = in ? -p.delta[base + lane + 32 * h] : 0.f;
-      }
-      if (!mbar_wait(&q_empty[st], (use & 1) ^ 1, abort_flag, 0x21)) { ok = false; break; }
-      if (lane == 0) {
-        mbar_expect_tx(&q_full[st], panels * (BWD_BQ * 128));
-        for (int c = 0; c < panels; ++c)
-          tma_load_4d(smem + S::OFF_Q + st * S::Q_BYTES + c * (BWD_BQ * 128), &tmQ, &q_full[st], c * 64, head, qb * BWD_BQ, batch);
-      }
+        for (int h = 0; h < 2; ++h) {
+          const bool in = qb * BWD_BQ + lane + 32 * h < p.sq;
+          lse[h] = in ? -p.lse[base + lane + 32 * h] * LOG2E : -INFINITY;
+          delta[h] = in ? -p.delta[base + lane + 32 * h] : 0.f;
+        }
+        if (!mbar_wait(&q_empty[st], (use & 1) ^ 1, abort_flag, 0x21)) { ok = false; break; }
+        if (lane == 0) {
+          mbar_expect_tx(&q_full[st], panels * (BWD_BQ * 128));
+          for (int c = 0; c < panels; ++c)
+            tma_load_4d(smem + S::OFF_Q + st * S::Q_BYTES + c * (BWD_BQ * 128), &tmQ, &q_full[st], c * 64, head, qb * BWD_BQ, batch);
+        }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        s_lse[st * 64 + lane + 32 * h] = lse[h];
-        s_delta[st * 64 + lane + 32 * h] = delta[h];
+        for (int h = 0; h < 2; ++h) {
+          s_lse[st * 64 + lane + 32 * h] = lse[h];
+          s_delta[st * 64 + lane + 32 * h] = delta[h];
+        }
+        mbar_arrive(&stat_full[st]);
+        const int ds = it % BWD_DOSTAGES;
+        if (!mbar_wait(&do_empty[ds], ((it / BWD_DOSTAGES) & 1) ^ 1, abort_flag, 0x23)) { ok = false; break; }
+        if (lane == 0) {
+          mbar_expect_tx(&do_full[ds], panels * (BWD_BQ * 128));
+          for (int c = 0; c < panels; ++c)
+            tma_load_4d(smem + S::OFF_DO + ds * S::Q_BYTES + c * (BWD_BQ * 128), &tmDO, &do_full[ds], c * 64, head, qb * BWD_BQ, batch);
+        }
       }
-      mbar_arrive(&stat_full[st]);
-      const int ds = it % BWD_DOSTAGES;
-      if (!mbar_wait(&do_empty[ds], ((it / BWD_DOSTAGES) & 1) ^ 1, abort_flag, 0x23)) { ok = false; break; }
-      if (lane == 0) {
-        mbar_expect_tx(&do_full[ds], panels * (BWD_BQ * 128));
-        for (int c = 0; c < panels; ++c)
-          tma_load_4d(smem + S::OFF_DO + ds * S::Q_BYTES + c * (BWD_BQ * 128), &tmDO, &do_full[ds], c * 64, head, qb * BWD_BQ, batch);
-      }
-    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer: one thread multiplexing the two groups' pipelines ----------------
-    if (elect_one()) {
+    } else if (elect_one()) {
+      // ---------------- MMA issuers: one thread each for S (warp 1), for dP and dV (warp 2) and for dQ and dK (warp 3) ----------------
+      // Every thread takes the iterations in order and waits for what its next product needs, so that the tensor cores get
+      // whatever is ready first. One thread that polled for all five kinds spent 1900 of 3050 clk an iteration on its tests, and
+      // those, not the tensor cores (1740 clk), set the pace.
       constexpr uint32_t idesc_st = make_idesc_bf16(BWD_BKV, BWD_BQ, 0, 0);   // S^T, dP^T: A=K/V (K-major), B=Q/dO (K-major)
       // dV, dK: A=P^T/dS^T (K-major), B=dO/Q (MN-major); 64 output columns are enough for head sizes up to 64
       const uint32_t idesc_dv = panels == 1 ? make_idesc_bf16(BWD_BKV, 64, 0, 1) : make_idesc_bf16(BWD_BKV, BWD_DH, 0, 1);
       constexpr uint32_t idesc_dq = make_idesc_bf16(BWD_DH, BWD_BQ, 1, 1);    // dQ^T: A=K (MN-major), B=dS^T (MN-major)
-      // Base descriptors, built once (an operand advances by adding (bytes >> 4)): K and V as K-major A operands, K
-      // again as the MN-major A operand of dQ^T; Q / dO per ring stage as K-major B (S^T, dP^T) and MN-major B (dK, dV);
-      // dS^T per group as K-major A (dK) and as MN-major B (dQ^T). P^T, the A operand of dV, is read from TMEM.
-      const uint64_t k_kmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_K), 0, 1024);
-      const uint64_t v_kmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_V), 0, 1024);
-      const uint64_t k_mnmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_K), BWD_BKV * 128, 1024);
-      const uint64_t q_kmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_Q), 0, 1024);
-      const uint64_t do_kmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_DO), 0, 1024);
-      const uint64_t q_mnmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_Q), BWD_BQ * 128, 1024);
-      const uint64_t do_mnmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_DO), BWD_BQ * 128, 1024);
-      const uint64_t dst_kmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_R + S::OFF_DS_IN_R), 0, 1024);
-      const uint64_t dst_mnmaj0 = make_smem_desc_sw128(smem_u32(smem + S::OFF_R + S::OFF_DS_IN_R), BWD_BKV * 128, 1024);
-      constexpr uint64_t Q_STEP = S::Q_BYTES >> 4, R_STEP = S::R_BYTES >> 4;
-      bool dv_started = false, dk_started = false;
-      // S^T = K Q^T and dP^T = V dO^T of iteration `it` into its group's accumulators
-      auto issue_s = [&](int it) {
-        const int g = it & 1, st = it % BWD_QSTAGES;
-        const uint64_t qd = q_kmaj0 + st * Q_STEP;
+      constexpr uint64_t Q_STEP = S::Q_BYTES >> 4, DS_STEP = S::DS_BYTES >> 4;
+      // S^T or dP^T of an iteration: rows of K or V times rows of a Q or dO stage
+      auto issue_st = [&](uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc) {
 #pragma unroll
         for (int kk = 0; kk < BWD_DH / 16; ++kk) {
           if (kk >= ksteps) break;
-          const uint64_t da = k_kmaj + static_cast<uint64_t>(((kk >> 2) * (BWD_BKV * 128) + (kk & 3) * 32) >> 4);
-          const uint64_t db = qd + static_cast<uint64_t>(((kk >> 2) * (BWD_BQ * 128) + (kk & 3) * 32) >> 4);
-          umma_f16_ss<1>(tmem_base + g * 128, da, db, idesc_st, kk != 0 ? 1u : 0u);
+          const uint64_t da = a_desc + static_cast<uint64_t>(((kk >> 2) * (BWD_BKV * 128) + (kk & 3) * 32) >> 4);
+          const uint64_t db = b_desc + static_cast<uint64_t>(((kk >> 2) * (BWD_BQ * 128) + (kk & 3) * 32) >> 4);
+          umma_f16_ss<1>(d_tmem, da, db, idesc_st, kk != 0 ? 1u : 0u);
         }
-        umma_commit<1>(gbar(g, B_S_FULL));
-      };
-      auto issue_dp = [&](int it) {
-        const int g = it & 1, st = it % BWD_DOSTAGES;
-        const uint64_t dod = do_kmaj0 + st * Q_STEP;
-#pragma unroll
-        for (int kk = 0; kk < BWD_DH / 16; ++kk) {
-          if (kk >= ksteps) break;
-          const uint64_t da = v_kmaj + static_cast<uint64_t>(((kk >> 2) * (BWD_BKV * 128) + (kk & 3) * 32) >> 4);
-          const uint64_t db = dod + static_cast<uint64_t>(((kk >> 2) * (BWD_BQ * 128) + (kk & 3) * 32) >> 4);
-          umma_f16_ss<1>(tmem_base + g * 128 + 64, da, db, idesc_st, kk != 0 ? 1u : 0u);
-        }
-        umma_commit<1>(gbar(g, B_DP_FULL));
-      };
-      // dV += P^T dO (reduction over the 64 query rows: 8 columns of P^T hold 16 of them)
-      auto issue_dv = [&](int it) {
-        const int g = it & 1, st = it % BWD_DOSTAGES;
-        const uint64_t dod = do_mnmaj0 + st * Q_STEP;
-#pragma unroll
-        for (int kk = 0; kk < BWD_BQ / 16; ++kk)
-          umma_f16_ts(tmem_base + TM_DV, tmem_base + g * 128 + kk * 8, dod + static_cast<uint64_t>((kk * 2048) >> 4), idesc_dv,
-                      (dv_started || kk != 0) ? 1u : 0u);
-        dv_started = true;
-        umma_commit<1>(gbar(g, B_PV_DONE));
-      };
-      // dK += dS^T Q ; dQ^T = K^T dS^T into the group's dP columns (the group has read dP by then)
-      auto issue_c = [&](int it) {
-        const int g = it & 1, st = it % BWD_QSTAGES;
-        const uint64_t dsd = dst_kmaj0 + g * R_STEP, dsd_mn = dst_mnmaj0 + g * R_STEP, qd = q_mnmaj0 + st * Q_STEP;
-#pragma unroll
-        for (int kk = 0; kk < BWD_BKV / 16; ++kk) {
-          // A = K as [M = dh, K = kv]: MN-major, dh panels 128 rows * 128 B apart, 16 kv rows per step;
-          // B = dS^T as [N = q, K = kv]: MN-major, a single 64-wide panel
-          const uint64_t da = k_mnmaj + static_cast<uint64_t>((kk * 2048) >> 4);
-          const uint64_t db = dsd_mn + static_cast<uint64_t>((kk * 2048) >> 4);
-          umma_f16_ss<1>(tmem_base + g * 128 + 64, da, db, idesc_dq, kk != 0 ? 1u : 0u);
-        }
-        umma_commit<1>(gbar(g, B_DQ_FULL));
-#pragma unroll
-        for (int kk = 0; kk < BWD_BQ / 16; ++kk) {
-          const uint64_t da = dsd + static_cast<uint64_t>((kk * 32) >> 4);
-          const uint64_t db = qd + static_cast<uint64_t>((kk * 2048) >> 4);
-          umma_f16_ss<1>(tmem_base + TM_DK, da, db, idesc_dv, (dk_started || kk != 0) ? 1u : 0u);
-        }
-        dk_started = true;
-        umma_commit<1>(gbar(g, B_DK_DONE));
-        umma_commit<1>(&q_empty[st]);
       };
       bool ok = n_iter == 0 || mbar_wait(kv_full, 0, abort_flag, 0x22);
-      // next iteration to issue per kind: S and dP in global order (a ring stage must not be probed two uses ahead),
-      // the others in order within each group
-      int next_s = 0, next_dp = 0, next_dv[2] = {0, 1}, next_c[2] = {0, 1};
-      uint32_t idle = 0;
-      uint64_t t0 = 0;
-      while (ok && (next_c[0] < n_iter || next_c[1] < n_iter)) {
-        bool progress = false;
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          int it = next_c[g];
-          if (it < n_iter && next_dp > it && next_dv[g] > it && mbar_test(gbar(g, B_DS_FULL), (it >> 1) & 1)) {
-            tc_fence_after();
-            issue_c(it);
-            next_c[g] += 2;
-            progress = true;
-          }
-          it = next_dv[g];
-          if (it < n_iter && next_s > it && mbar_test(gbar(g, B_PT_FULL), (it >> 1) & 1) &&
-              (next_dp > it || mbar_test(&do_full[it % BWD_DOSTAGES], (it / BWD_DOSTAGES) & 1))) {
-            tc_fence_after();
-            issue_dv(it);
-            next_dv[g] += 2;
-            if (next_dp > it) umma_commit<1>(&do_empty[it % BWD_DOSTAGES]);       // whichever of dV and dP comes second
-            progress = true;
-          }
-        }
-        if (next_dp < next_s) {
-          const int it = next_dp, g = it & 1, j = it >> 1;
-          // the group's dQ block of its previous iteration has left these columns
-          bool ready = mbar_test(&do_full[it % BWD_DOSTAGES], (it / BWD_DOSTAGES) & 1);
-          if (ready && j > 0) ready = next_c[g] >= it && mbar_test(gbar(g, B_DP_FREE), (j - 1) & 1);
-          if (ready) {
-            tc_fence_after();
-            issue_dp(it);
-            ++next_dp;
-            if (next_dv[g] > it) umma_commit<1>(&do_empty[it % BWD_DOSTAGES]);
-            progress = true;
-          }
-        }
-        if (next_s < n_iter) {
-          const int it = next_s, g = it & 1, j = it >> 1, st = it % BWD_QSTAGES;
-          bool ready = mbar_test(&q_full[st], (it / BWD_QSTAGES) & 1);
+      if (warp == 1) {
+        const uint64_t k_desc = make_smem_desc_sw128(smem_u32(smem + S::OFF_K), 0, 1024);
+        const uint64_t q_desc = make_smem_desc_sw128(smem_u32(smem + S::OFF_Q), 0, 1024);
+        for (int it = 0; it < n_iter && ok; ++it) {
+          const int g = it & 1, j = it >> 1, st = it % BWD_QSTAGES;
+          ok = mbar_wait(&q_full[st], (it / BWD_QSTAGES) & 1, abort_flag, 0x24);
           // dV of the group's previous iteration has read P^T out of these columns
-          if (ready && j > 0) ready = next_dv[g] >= it && mbar_test(gbar(g, B_PV_DONE), (j - 1) & 1);
-          if (ready) {
-            tc_fence_after();
-            issue_s(it);
-            ++next_s;
-            progress = true;
-          }
+          if (j > 0) ok = ok && mbar_wait(gbar(g, B_PV_DONE), (j - 1) & 1, abort_flag, 0x25);
+          if (!ok) break;
+          tc_fence_after();
+          issue_st(tmem_base + g * 128, k_desc, q_desc + st * Q_STEP);
+          umma_commit<1>(gbar(g, B_S_FULL));
         }
-        if (progress) {
-          idle = 0;
-          t0 = 0;
-        } else if (__nanosleep(20), (++idle & 0x3ff) == 0) {
-          if (*abort_flag) { ok = false; break; }
-          const uint64_t now = global_timer_ns();
-          if (t0 == 0) {
-            t0 = now;
-          } else if (now - t0 > GV_WAIT_NS) {
-            *abort_flag = 1;
-            record_error((0x30u << 16) | 1u, static_cast<unsigned>(next_s), static_cast<unsigned>(next_c[0]));
-            ok = false;
-            break;
-          }
+      } else if (warp == 2) {
+        const uint64_t v_desc = make_smem_desc_sw128(smem_u32(smem + S::OFF_V), 0, 1024);
+        const uint64_t do_kmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_DO), 0, 1024);
+        const uint64_t do_mnmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_DO), BWD_BQ * 128, 1024);
+        for (int it = 0; it < n_iter && ok; ++it) {
+          const int g = it & 1, j = it >> 1, st = it % BWD_DOSTAGES;
+          ok = mbar_wait(&do_full[st], (it / BWD_DOSTAGES) & 1, abort_flag, 0x26);
+          // the group's dQ block of its previous iteration has left these columns
+          if (j > 0) ok = ok && mbar_wait(gbar(g, B_DP_FREE), (j - 1) & 1, abort_flag, 0x27);
+          if (!ok) break;
+          tc_fence_after();
+          issue_st(tmem_base + g * 128 + 64, v_desc, do_kmaj + st * Q_STEP);
+          umma_commit<1>(gbar(g, B_DP_FULL));
+          // dV += P^T dO (reduction over the 64 query rows: 8 columns of P^T, read from TMEM, hold 16 of them)
+          if (!mbar_wait(gbar(g, B_PT_FULL), j & 1, abort_flag, 0x28)) break;
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < BWD_BQ / 16; ++kk)
+            umma_f16_ts(tmem_base + TM_DV, tmem_base + g * 128 + kk * 8, do_mnmaj + st * Q_STEP + static_cast<uint64_t>((kk * 2048) >> 4),
+                        idesc_dv, (it | kk) != 0 ? 1u : 0u);
+          umma_commit<1>(gbar(g, B_PV_DONE));
+          umma_commit<1>(&do_empty[st]);
         }
+        umma_commit<1>(all_done);
+      } else {
+        // K again as the MN-major A operand of dQ^T; Q per ring stage as the MN-major B of dK; dS^T per group as K-major A (dK) and as
+        // MN-major B (dQ^T)
+        const uint64_t k_desc = make_smem_desc_sw128(smem_u32(smem + S::OFF_K), BWD_BKV * 128, 1024);
+        const uint64_t q_desc = make_smem_desc_sw128(smem_u32(smem + S::OFF_Q), BWD_BQ * 128, 1024);
+        const uint64_t ds_kmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_DS), 0, 1024);
+        const uint64_t ds_mnmaj = make_smem_desc_sw128(smem_u32(smem + S::OFF_DS), BWD_BKV * 128, 1024);
+        for (int it = 0; it < n_iter && ok; ++it) {
+          const int g = it & 1, j = it >> 1, st = it % BWD_QSTAGES;
+          ok = mbar_wait(&q_full[st], (it / BWD_QSTAGES) & 1, abort_flag, 0x29) && mbar_wait(gbar(g, B_DS_FULL), j & 1, abort_flag, 0x20);
+          if (!ok) break;
+          tc_fence_after();
+          // dQ^T = K^T dS^T into the group's dP columns (the group has read dP by then)
+#pragma unroll
+          for (int kk = 0; kk < BWD_BKV / 16; ++kk) {
+            // A = K as [M = dh, K = kv]: MN-major, dh panels 128 rows * 128 B apart, 16 kv rows per step;
+            // B = dS^T as [N = q, K = kv]: MN-major, a single 64-wide panel
+            umma_f16_ss<1>(tmem_base + g * 128 + 64, k_desc + static_cast<uint64_t>((kk * 2048) >> 4),
+                           ds_mnmaj + g * DS_STEP + static_cast<uint64_t>((kk * 2048) >> 4), idesc_dq, kk != 0 ? 1u : 0u);
+          }
+          umma_commit<1>(gbar(g, B_DQ_FULL));
+          // dK += dS^T Q
+#pragma unroll
+          for (int kk = 0; kk < BWD_BQ / 16; ++kk)
+            umma_f16_ss<1>(tmem_base + TM_DK, ds_kmaj + g * DS_STEP + static_cast<uint64_t>((kk * 32) >> 4),
+                           q_desc + st * Q_STEP + static_cast<uint64_t>((kk * 2048) >> 4), idesc_dv, (it | kk) != 0 ? 1u : 0u);
+          umma_commit<1>(gbar(g, B_DK_DONE));
+          umma_commit<1>(&q_empty[st]);
+        }
+        umma_commit<1>(all_done);
       }
-      umma_commit<1>(all_done);
     }
-  } else {
+  } else if (warp >= 8) {
+    reg_alloc<BWD_REGS_GROUP>();
     // ---------------- two epilogue groups: thread = one KV row (TMEM lane), all 64 query columns of its block ----------------
-    const int g = (warp - 2) >> 2;      // group 0: warps 2-5, group 1: warps 6-9
+    const int g = (warp - 8) >> 2;      // group 0: warps 8-11, group 1: warps 12-15
     const int quarter = warp & 3;       // TMEM lane group
     const int rloc = quarter * 32 + lane;
     const int kvrow = kv0 + rloc;
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t tm_s = tmem_base + lane_off + g * 128, tm_dp = tm_s + 64;
-    uint8_t* region = smem + S::OFF_R + g * S::R_BYTES;
-    uint8_t* dst_row = region + S::OFF_DS_IN_R + rloc * 128;
-    const int half_rows = p.dh <= 64 ? 32 * p.dh : S::OFF_DS_IN_R / 4;   // floats between the two halves of a dQ block
-    float* dq_stage = reinterpret_cast<float*>(region);
-    const bool issuer = (threadIdx.x == 64 + g * 128);   // first thread of the group issues its dQ bulk reductions
-    auto vote = [&](bool good) { return g == 0 ? named_bar_all<2, 128>(good) : named_bar_all<3, 128>(good); };
+    uint8_t* dst_row = smem + S::OFF_DS + g * S::DS_BYTES + rloc * 128;
     bool ok = true;
-    // One round: the dQ block of the group's previous iteration (which frees the columns for dP), P of iteration `it` while
-    // dP is multiplied, dS of `it`; the last round only has the dQ block. A wait that gave up is carried to the next vote, which
-    // all 128 threads reach: the loop is only left right after one, and the .sync.aligned TMEM accesses stay warp-uniform.
-    for (int it = g; it < n_iter + 2; it += 2) {
-      const bool cur = it < n_iter, prev = it >= 2 + g;
-      if (!cur && !prev) break;
+    // One round: P of iteration `it` while dP is multiplied, then dS. A wait that gave up is its whole warp's result, so that the
+    // .sync.aligned TMEM accesses stay warp-uniform; the other warps' waits see the abort flag.
+    for (int it = g; it < n_iter; it += 2) {
       const int j = it >> 1, st = it % BWD_QSTAGES;
       const int head = kv_head * rep + it / n_q;
       const int qb = q_start + it % n_q;
@@ -867,59 +827,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t bh_key = DROP ? drop_key(p.drop_seed, batch, head + p.drop_head_offset) : 0u;
       const bool boundary = (kv0 + BWD_BKV > sk_eff) || (p.causal && (kv0 + BWD_BKV - 1 > qbase + shift));
       const int kr = min(kvrow, p.sk - 1);
-      bool good = true;
       float pr[64];                    // probabilities of this thread's key at the 64 query columns, before dropout
       uint32_t keep[2] = {0u, 0u};     // DROP: which of them survive
-      if (prev) {
-        // dQ^T of the previous iteration [lane = head-dim index, columns = query rows] from the dP columns. The block is staged as
-        // [query row][head dim] fp32 and added into dq_accum by bulk tensor reductions (the adds happen at L2).
-        const int pi = it - 2, phead = kv_head * rep + pi / n_q, pq = (q_start + pi % n_q) * BWD_BQ;
-        good = good && mbar_wait(gbar(g, B_DQ_FULL), (j - 1) & 1, abort_flag, 0x2e);
-        if (issuer) tma_store_wait_read<0>();          // the staging buffer is free again
-        if (!vote(good)) { ok = false; break; }
-        tc_fence_after();
-        {
-          uint32_t r0[32], r1[32];
-          tmem_ld_32x32b_x32(tm_dp, r0);
-          tmem_ld_32x32b_x32(tm_dp + 32, r1);
-          tmem_ld_wait();
-          tc_fence_before();
-          mbar_arrive(gbar(g, B_DP_FREE));
-          float* dst = dq_stage + rloc;
-          if (p.dh == BWD_DH) {                        // immediate offsets
-#pragma unroll
-            for (int c = 0; c < 32; ++c) dst[c * BWD_DH] = __uint_as_float(r0[c]);
-          } else if (rloc < p.dh) {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) dst[c * p.dh] = __uint_as_float(r0[c]);
-          }
-          good = mbar_wait(gbar(g, B_DK_DONE), (j - 1) & 1, abort_flag, 0x2c);    // nothing reads dS^T any more
-          if (p.dh == BWD_DH) {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) dst[S::OFF_DS_IN_R / 4 + c * BWD_DH] = __uint_as_float(r1[c]);
-          } else if (rloc < p.dh) {
-            dst += half_rows;
-#pragma unroll
-            for (int c = 0; c < 32; ++c) dst[c * p.dh] = __uint_as_float(r1[c]);
-          }
-        }
-        fence_async_smem();
-        if (!vote(good)) { ok = false; break; }
-        if (issuer) {
-          // the half that may lie where dS^T goes leaves first
-          if (pq + 32 < p.sq) tma_reduce_add_4d(&tmDQ, dq_stage + half_rows, 0, phead, pq + 32, batch);
-          tma_store_commit();
-          tma_reduce_add_4d(&tmDQ, dq_stage, 0, phead, pq, batch);
-          tma_store_commit();
-        }
-      }
-      if (!cur) break;
+      bool good = mbar_wait(gbar(g, B_S_FULL), j & 1, abort_flag, 0x2b);
+      good = good && mbar_wait(&stat_full[st], (it / BWD_QSTAGES) & 1, abort_flag, 0x2a);
+      if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
       {
-        good = good && mbar_wait(gbar(g, B_S_FULL), j & 1, abort_flag, 0x2b);
-        good = good && mbar_wait(&stat_full[st], (it / BWD_QSTAGES) & 1, abort_flag, 0x2a);
-        good = __all_sync(0xffffffffu, good);
-      }
-      if (good) {
         tc_fence_after();
         const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
 #pragma unroll
@@ -1019,9 +932,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc_fence_before();
         mbar_arrive(gbar(g, B_PT_FULL));
       }
-      good = good && mbar_wait(gbar(g, B_DP_FULL), j & 1, abort_flag, 0x2d);
-      if (issuer) tma_store_wait_read<1>();
-      if (!vote(good)) { ok = false; break; }
+      good = mbar_wait(gbar(g, B_DP_FULL), j & 1, abort_flag, 0x2d);
+      if (j > 0) good = good && mbar_wait(gbar(g, B_DK_DONE), (j - 1) & 1, abort_flag, 0x2c);    // nothing reads the last dS^T any more
+      if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
       tc_fence_after();
       // dS^T = P^T * scale * (dP^T - delta)
       const uint64_t ps2 = f2_pack(p.scale, p.scale);
@@ -1080,7 +993,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       fence_async_smem();
       mbar_arrive(gbar(g, B_DS_FULL));
     }
-    if (issuer) tma_store_wait<0>();                  // every reduction of this group has been performed
     // final: dK, dV from TMEM (group g takes 64 of the 128 head-dim columns)
     if (ok && n_iter > 0) ok = mbar_wait(all_done, 0, abort_flag, 0x2f);
     tc_fence_after();
@@ -1119,6 +1031,41 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               *reinterpret_cast<uint4*>(dv_row + col) = w;
             }
           }
+        }
+      }
+    }
+  } else {
+    reg_dealloc<BWD_REGS_DRAIN>();
+    // ---------------- dQ: warps 4-7 add each block into dq_accum while the groups go on with P of the next ----------------
+    // dQ^T of an iteration [lane = head-dim index, columns = query rows] comes from its group's dP columns, which are free once it
+    // has been read. Four neighbouring rows of a lane are one 16-byte addition at L2, those of a warp 512 bytes in a row (see
+    // dq_group).
+    const int quarter = warp & 3, rloc = quarter * 32 + lane;
+    At at = {0, 0};
+    for (int it = 0; it < n_iter; ++it, at.advance(1, n_q)) {
+      const int g = it & 1, head = kv_head * rep + at.rep, q0 = (q_start + at.q) * BWD_BQ;
+      const uint32_t tm_dq = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + g * 128 + 64;
+      const bool good = mbar_wait(gbar(g, B_DQ_FULL), (it >> 1) & 1, abort_flag, 0x2e);
+      if (!__all_sync(0xffffffffu, good)) break;
+      tc_fence_after();
+      uint32_t r[64];
+      tmem_ld_32x32b_x32(tm_dq, r);
+      tmem_ld_32x32b_x32(tm_dq + 32, r + 32);
+      tmem_ld_wait();
+      tc_fence_before();
+      mbar_arrive(gbar(g, B_DP_FREE));
+      if (rloc < p.dh) {
+        float* dst = p.dq_accum + dq_group(batch * static_cast<long long>(p.hq) + head, q0 >> 2, p.sq, p.dh);
+        const int rows = min(BWD_BQ, p.sq - q0);       // of the block that exist
+        float* to = dst + 4 * rloc;
+#pragma unroll
+        for (int c = 0; c < BWD_BQ; c += 4, to += 4 * p.dh)
+          if (c + 4 <= rows)
+            red_add_v4(to, __uint_as_float(r[c]), __uint_as_float(r[c + 1]), __uint_as_float(r[c + 2]), __uint_as_float(r[c + 3]));
+        if (rows & 3) {                                // the last group of a sequence: 1 to 3 rows
+#pragma unroll
+          for (int c = 0; c < BWD_BQ; ++c)
+            if (c >= (rows & ~3) && c < rows) atomicAdd(dst + (rows & ~3) * p.dh + rloc * (rows & 3) + (c & 3), __uint_as_float(r[c]));
         }
       }
     }
@@ -1163,63 +1110,62 @@ __global__ void attn_delta_kernel(const bf16* __restrict__ o, const bf16* __rest
   }
 }
 
-// dq (bf16, strided) = dq_accum (fp32 [b, sq, hq, dh])
-__global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, int b, int sq, int hq,
-                                       int dh, long long sb, long long ss, long long sh) {
-  const int vec = dh >> 3;
-  const long long total = static_cast<long long>(b) * sq * hq * vec;
+// dq (bf16, strided) = dq_accum, optionally (ROPE) with the inverse rotary rotation of the query gradient folded in (the forward pass
+// rotated q; the gradient w.r.t. the un-rotated projection is the transposed rotation of dq). One thread converts four rows of 8
+// columns, with ROPE of the first half of a head together with their partners in the second half.
+template <bool ROPE>
+__global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, int b, int sq, int hq, int dh,
+                                       long long sb, long long ss, long long sh, const float* __restrict__ inv_freq,
+                                       const int* __restrict__ pos, int pos_offset) {
+  constexpr int PARTS = ROPE ? 2 : 1;
+  const int span = dh / PARTS, vec = span >> 3, groups = (sq + 3) >> 2;
+  const long long total = static_cast<long long>(b) * hq * groups * vec;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int v = static_cast<int>(i % vec);
-    const long long row = i / vec;  // (b, s, h)
-    const int h = static_cast<int>(row % hq);
-    const int s = static_cast<int>((row / hq) % sq);
-    const int bb = static_cast<int>(row / (static_cast<long long>(hq) * sq));
-    const float4 x = *reinterpret_cast<const float4*>(acc + row * dh + v * 8);
-    const float4 y = *reinterpret_cast<const float4*>(acc + row * dh + v * 8 + 4);
-    uint4 u;
-    u.x = pack_bf16x2(x.x, x.y); u.y = pack_bf16x2(x.z, x.w);
-    u.z = pack_bf16x2(y.x, y.y); u.w = pack_bf16x2(y.z, y.w);
-    *reinterpret_cast<uint4*>(dq + bb * sb + s * ss + h * sh + v * 8) = u;
-  }
-}
-
-// dq (bf16, strided) = R^T(dq_accum): the fp32 -> bf16 conversion with the inverse rotary rotation of the query
-// gradient folded in (the forward pass rotated q; the gradient w.r.t. the un-rotated projection is the transposed
-// rotation of dq). One thread converts 8 columns of the first half of a head and their partners in the second half.
-__global__ void attn_dq_convert_rope_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, int b, int sq, int hq,
-                                            int dh, long long sb, long long ss, long long sh,
-                                            const float* __restrict__ inv_freq, const int* __restrict__ pos, int pos_offset) {
-  const int half = dh >> 1;
-  const int vec = half >> 3;
-  const long long total = static_cast<long long>(b) * sq * hq * vec;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int v = static_cast<int>(i % vec);
-    const long long row = i / vec;  // (b, s, h)
-    const int h = static_cast<int>(row % hq);
-    const int s = static_cast<int>((row / hq) % sq);
-    const int bb = static_cast<int>(row / (static_cast<long long>(hq) * sq));
-    const float p = pos ? static_cast<float>(pos[static_cast<long long>(s) * b + bb]) : static_cast<float>(s + pos_offset);
-    const float* src = acc + row * dh + v * 8;
-    float x1[8], x2[8], o1[8], o2[8];
-    *reinterpret_cast<float4*>(x1) = *reinterpret_cast<const float4*>(src);
-    *reinterpret_cast<float4*>(x1 + 4) = *reinterpret_cast<const float4*>(src + 4);
-    *reinterpret_cast<float4*>(x2) = *reinterpret_cast<const float4*>(src + half);
-    *reinterpret_cast<float4*>(x2 + 4) = *reinterpret_cast<const float4*>(src + half + 4);
+    const long long r = i / vec;           // (b, h, group)
+    const int g = static_cast<int>(r % groups);
+    const long long bh = r / groups;
+    const int h = static_cast<int>(bh % hq), bb = static_cast<int>(bh / hq);
+    const int rows = min(4, sq - 4 * g);
+    const float* src = acc + dq_group(bh, g, sq, dh);
+    float x[PARTS][8][4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float sn, cs;
-      sincosf(p * __ldg(inv_freq + v * 8 + e), &sn, &cs);
-      o1[e] = x1[e] * cs + x2[e] * sn;      // transposed rotation: sin -> -sin
-      o2[e] = x2[e] * cs - x1[e] * sn;
+    for (int part = 0; part < PARTS; ++part)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int d = part * span + v * 8 + e;
+        if (rows == 4) {
+          *reinterpret_cast<float4*>(x[part][e]) = *reinterpret_cast<const float4*>(src + 4 * d);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) x[part][e][k] = k < rows ? src[rows * d + k] : 0.f;
+        }
+      }
+    bf16* dst = dq + bb * sb + 4 * g * ss + h * sh + v * 8;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k >= rows) break;
+      if constexpr (ROPE) {
+        const int s = 4 * g + k;
+        const float p = pos ? static_cast<float>(pos[static_cast<long long>(s) * b + bb]) : static_cast<float>(s + pos_offset);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          float sn, cs;
+          sincosf(p * __ldg(inv_freq + v * 8 + e), &sn, &cs);
+          const float a = x[0][e][k], c = x[1][e][k];
+          x[0][e][k] = a * cs + c * sn;      // transposed rotation: sin -> -sin
+          x[1][e][k] = c * cs - a * sn;
+        }
+      }
+#pragma unroll
+      for (int part = 0; part < PARTS; ++part) {
+        uint4 u;
+        u.x = pack_bf16x2(x[part][0][k], x[part][1][k]); u.y = pack_bf16x2(x[part][2][k], x[part][3][k]);
+        u.z = pack_bf16x2(x[part][4][k], x[part][5][k]); u.w = pack_bf16x2(x[part][6][k], x[part][7][k]);
+        *reinterpret_cast<uint4*>(dst + k * ss + part * span) = u;
+      }
     }
-    uint4 u, w;
-    u.x = pack_bf16x2(o1[0], o1[1]); u.y = pack_bf16x2(o1[2], o1[3]); u.z = pack_bf16x2(o1[4], o1[5]); u.w = pack_bf16x2(o1[6], o1[7]);
-    w.x = pack_bf16x2(o2[0], o2[1]); w.y = pack_bf16x2(o2[2], o2[3]); w.z = pack_bf16x2(o2[4], o2[5]); w.w = pack_bf16x2(o2[6], o2[7]);
-    bf16* dst = dq + bb * sb + s * ss + h * sh + v * 8;
-    *reinterpret_cast<uint4*>(dst) = u;
-    *reinterpret_cast<uint4*>(dst + half) = w;
   }
 }
 
@@ -1367,27 +1313,7 @@ extern "C" int gv_attn_bwd(const gv_attn_args* a, gv_stream_t s) {
   if (rc) return rc;
   rc = make_tmap_bshd(&tmV, a->v, a->b, a->sk, a->hk, a->dh, a->v_stride_b, a->v_stride_s, a->v_stride_h, BWD_BKV);
   if (rc) return rc;
-  CUtensorMap tmDQ;
-  {
-    // fp32 accumulator [b, sq, hq, dh] contiguous; one reduction covers 32 query rows of one head
-    EncodeTiledFn fn = attn_encode_fn();
-    if (fn == nullptr) return 1001;
-    if (reinterpret_cast<uintptr_t>(a->dq_accum) & 15) return 2307;
-    cuuint64_t dims[4] = {(cuuint64_t)a->dh, (cuuint64_t)a->hq, (cuuint64_t)a->sq, (cuuint64_t)a->b};
-    cuuint64_t strides[3] = {(cuuint64_t)a->dh * 4, (cuuint64_t)a->hq * a->dh * 4, (cuuint64_t)a->sq * a->hq * a->dh * 4};
-    cuuint32_t box[4] = {(cuuint32_t)a->dh, 1, (cuuint32_t)(BWD_BQ / 2), 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = fn(&tmDQ, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->dq_accum, dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r == CUDA_ERROR_INVALID_CONTEXT) {   // see make_tmap_bshd
-      bind_context_of(a->dq_accum);
-      r = fn(&tmDQ, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->dq_accum, dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    }
-    if (r != CUDA_SUCCESS) return 1000 + static_cast<int>(r);
-  }
+  if (reinterpret_cast<uintptr_t>(a->dq_accum) & 15) return 2307;
   BwdParams p;
   p.lse = a->lse; p.delta = a->delta; p.dq_accum = a->dq_accum;
   p.dk = reinterpret_cast<bf16*>(a->dk); p.dv = reinterpret_cast<bf16*>(a->dv);
@@ -1404,10 +1330,19 @@ extern "C" int gv_attn_bwd(const gv_attn_args* a, gv_stream_t s) {
   const long long blocks64 = static_cast<long long>(kv_tiles) * a->hk * a->b;
   if (blocks64 > 0x7fffffff) return 2317;
   const dim3 grid = tile_grid(a->causal, kv_tiles, a->hk, a->b, p.tile_group);
+  // A register split that asks for more than the launch brings would wait for good.
+  auto enough_registers = [](auto kern) {
+    cudaFuncAttributes attr;
+    return cudaFuncGetAttributes(&attr, kern) == cudaSuccess &&
+           4 * attr.numRegs >= BWD_REGS_ISSUE + BWD_REGS_DRAIN + 2 * BWD_REGS_GROUP;
+  };
+  static const bool registers_ok = enough_registers(attn_bwd_kernel<MODE_PLAIN>) && enough_registers(attn_bwd_kernel<MODE_BIAS>) &&
+                                   enough_registers(attn_bwd_kernel<MODE_DROP>);
+  if (!registers_ok) return 2318;
   auto launch = [&](auto kern, PerDeviceOnce& once) -> cudaError_t {
     cudaError_t e = ensure_max_dynamic_smem(once, kern, BwdSmem::TOTAL);
     if (e != cudaSuccess) return e;
-    kern<<<grid, BWD_THREADS, BwdSmem::TOTAL, stream>>>(tmQ, tmK, tmV, tmDO, tmDQ, p);
+    kern<<<grid, BWD_THREADS, BwdSmem::TOTAL, stream>>>(tmQ, tmK, tmV, tmDO, p);
     return cudaSuccess;
   };
   static PerDeviceOnce once_plain, once_bias, once_drop;
@@ -1419,18 +1354,15 @@ extern "C" int gv_attn_bwd(const gv_attn_args* a, gv_stream_t s) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
   {
-    const long long total = static_cast<long long>(a->b) * a->sq * a->hq * (a->dh / 8);
+    const bool rope = a->dq_rope_inv_freq != nullptr && a->dh % 16 == 0;
+    const long long total = static_cast<long long>(a->b) * a->hq * ((a->sq + 3) / 4) * (a->dh / (rope ? 16 : 8));
     long long blocks = (total + 255) / 256;
     const long long cap = static_cast<long long>(num_sms()) * 8;
     if (blocks > cap) blocks = cap;
-    if (a->dq_rope_inv_freq != nullptr && a->dh % 16 == 0)
-      attn_dq_convert_rope_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(
-          a->dq_accum, reinterpret_cast<bf16*>(a->dq), a->b, a->sq, a->hq, a->dh, a->dq_stride_b, a->dq_stride_s,
-          a->dq_stride_h, a->dq_rope_inv_freq, a->dq_rope_pos, a->dq_rope_pos_offset);
-    else
-      attn_dq_convert_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(
-          a->dq_accum, reinterpret_cast<bf16*>(a->dq), a->b, a->sq, a->hq, a->dh, a->dq_stride_b, a->dq_stride_s,
-          a->dq_stride_h);
+    auto convert = rope ? attn_dq_convert_kernel<true> : attn_dq_convert_kernel<false>;
+    convert<<<static_cast<int>(blocks), 256, 0, stream>>>(a->dq_accum, reinterpret_cast<bf16*>(a->dq), a->b, a->sq, a->hq, a->dh,
+                                                          a->dq_stride_b, a->dq_stride_s, a->dq_stride_h, a->dq_rope_inv_freq,
+                                                          a->dq_rope_pos, a->dq_rope_pos_offset);
   }
   return static_cast<int>(cudaGetLastError());
 }

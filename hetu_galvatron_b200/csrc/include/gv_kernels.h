@@ -182,7 +182,7 @@ typedef struct {
   void* dq;       // bf16 output
   void* dk;       // bf16 output
   void* dv;       // bf16 output
-  float* dq_accum;  // fp32 scratch [b, sq, hq, dh], zeroed by the launcher
+  float* dq_accum;  // fp32 scratch of b * sq * hq * dh elements in the kernel's own order, zeroed by the launcher
   float* delta;     // fp32 scratch [b, hq, sq]
   int b, sq, sk, hq, hk, dh;
   long long q_stride_b, q_stride_s, q_stride_h;

@@ -73,6 +73,45 @@ def test_attention_bwd(b, sq, sk, hq, hk, dh, causal):
     assert _rel(dv, vf.grad) < 3e-2
 
 
+@pytest.mark.parametrize("dh,causal", [(8, False), (64, True), (72, False), (128, True)])
+@pytest.mark.parametrize("sq", [1, 2, 3, 5, 63, 66, 127, 196])
+def test_query_gradient_of_any_number_of_rows(sq, dh, causal):
+    """dQ is summed in groups of four rows, with a group of sq % 4 at the end of a sequence; two sequences and grouped heads, so that one
+    block's rows must not reach the next one's. bf16 operands and results, fp32 sums of at most 196 terms: 8 bits and some."""
+    b, hq, hk = 2, 4, 2
+    sk = sq if causal else 70
+    q, k, v = (t.clone() for t in _mk(b, sq, sk, hq, hk, dh))
+    o, lse = Fn.attention_fwd(q, k, v, causal, dh ** -0.5)
+    dout = torch.randn_like(o)
+    got = Fn.attention_bwd(dout, q, k, v, o, lse, causal, dh ** -0.5)
+    torch.cuda.synchronize()
+    assert _lib.read_error() is None
+    ref = [t.double().detach().requires_grad_(True) for t in (q, k, v)]
+    Fn.attention_reference(*ref, causal, dh ** -0.5)[0].backward(dout.double())
+    for g, r in zip(got, ref):
+        assert ((g.double() - r.grad).norm() / r.grad.norm().clamp(min=1e-3)).item() < 1e-2
+
+
+@pytest.mark.parametrize("s,dh", [(5, 16), (66, 64), (131, 128)])
+def test_query_gradient_rotated_back_in_the_conversion(s, dh):
+    b, h = 2, 2
+    inv_freq = Fn.rope_inv_freq(dh, 10000.0, "cuda")
+    q, k, v = (t.clone() for t in _mk(b, s, s, h, h, dh))
+    o, lse = Fn.attention_fwd(q, k, v, True, dh ** -0.5)
+    dout = torch.randn_like(o)
+    plain = Fn.attention_bwd(dout, q, k, v, o, lse, True, dh ** -0.5)[0]
+    # positions in sequence-major token order, not in step with the rows
+    pos = (torch.arange(s * b, device="cuda") * 7 % 50).to(torch.int32)
+    rotated = Fn.attention_bwd(dout, q, k, v, o, lse, True, dh ** -0.5, dq=torch.empty_like(q), dk=torch.empty_like(k), dv=torch.empty_like(v),
+                               dq_rope=(inv_freq, pos, 0))[0]
+    ang = pos.view(s, b).t().double().unsqueeze(-1) * inv_freq.double()
+    cos, sin = ang.cos().unsqueeze(2), ang.sin().unsqueeze(2)
+    x1, x2 = plain.double().chunk(2, dim=-1)
+    want = torch.cat([x1 * cos + x2 * sin, x2 * cos - x1 * sin], dim=-1)
+    # two roundings to bf16 against one
+    assert ((rotated.double() - want).norm() / want.norm()).item() < 6e-3
+
+
 def test_attention_is_repeatable():
     """Forward, dK and dV have a fixed accumulation order (bitwise equal across runs); dQ is summed over KV tiles by
     fp32 reduce-adds whose order depends on CTA scheduling, so it is only equal up to fp32 rounding."""
