@@ -18,6 +18,7 @@
 #include "include/gv_kernels.h"
 #include "include/gv_host.h"
 #include "include/gv_ptx.cuh"
+#include "include/gv_tile_share.h"
 
 namespace gv {
 
@@ -63,6 +64,11 @@ struct GemmDev {
   const float* rope_inv_freq;  // [rope_dh / 2]
   const int* rope_pos;         // [M] explicit positions, or NULL: position = (row / div) % mod + offset
   int rope_pos_div, rope_pos_mod, rope_pos_offset;
+  // tiles that several CTA pairs share (0 = none; pair kernel only), the room for their partial sums and what marks this launch there
+  int share_tiles, share_each;
+  float4* share_parts;
+  unsigned long long* share_counts;
+  unsigned long long share_nonce;
 };
 
 template <int BN>
@@ -866,12 +872,136 @@ struct SplitExchange {
   }
 };
 
-template <bool SPLIT> struct ExchangeOf { using type = NoExchange; };
-template <> struct ExchangeOf<true> { using type = SplitExchange; };
+// What the pairs do with a tile: every tile goes to one pair; SPLIT: the pairs of a cluster share all; SHARE: all pairs share the first.
+enum { PAIR_WHOLE = 0, PAIR_SPLIT = 1, PAIR_SHARE = 2 };
+template <int MODE> struct ExchangeOf { using type = NoExchange; };
+template <> struct ExchangeOf<PAIR_SPLIT> { using type = SplitExchange; };
 
-// SPLIT: S pairs of the cluster share each tile; otherwise the cluster is one pair and S and ws are unused.
-template <bool A_MN, bool B_MN, int EPI, bool SPLIT>
+struct WholeTiles {
+  int tile, step, num_tiles, kb;
+  __device__ __forceinline__ WholeTiles(const TileShare& s, int pair, int num_pairs, int tiles) : tile(pair), step(num_pairs), num_tiles(tiles), kb(s.kb) {}
+  __device__ __forceinline__ bool next(Segment& g) {
+    g.tile = tile; g.kb0 = 0; g.kb1 = kb;
+    tile += step;
+    return g.tile < num_tiles;
+  }
+};
+
+// Shared tiles (see gv_tile_share.h): the pairs of a tile each multiply a range of its k-blocks. Chunk by chunk (32 x 32, per warp),
+// whoever comes last joins the sums and stores the result; nobody has to wait for another pair, so nothing depends on which CTAs run
+// at the same time. A warp that is not last leaves its sums in global memory (they stay in L2) and counts itself in. Each pair
+// starts at another chunk, so that pairs that arrive together share the joining: one warp that joined all four chunks of four pairs read
+// 48 KB in a chain of loads, 18 us a tile against 10. The sums are added in the pairs' order whoever adds them: results repeat bit for bit.
+// A counter holds the launch's number in its upper 56 bits: whatever else the uninitialised room held counts as nobody, and the
+// last warp clears it for a launch that is replayed with the same number.
+constexpr int SHARE_POLLS = 3;                   // of a chunk's counter before its sums are left too: 0.7 us each, as long as a peer is late
+
+struct ShareJoin {
+  const GemmDev& p;
+  int pair, lo, n, lane, warp_slot;              // pairs lo .. lo + n - 1 share the tile; warp_slot: of this CTA and warp, in the room of a pair
+  uint32_t t_addr;
+  int c0;                                        // the warp's first chunk
+  unsigned long long* count;                     // [4] of this tile, CTA and warp
+
+  __device__ __forceinline__ float4* part(int q, int i) const {
+    return p.share_parts + (static_cast<size_t>(q) * 16 + warp_slot) * (4 * SPLIT_CHUNK) + i * SPLIT_CHUNK + lane;
+  }
+  __device__ __forceinline__ int arrived(unsigned long long v) const { return (v & ~0xFFull) == p.share_nonce ? static_cast<int>(v & 0xFF) : 0; }
+  __device__ __forceinline__ int peek(int i) const { return arrived(*reinterpret_cast<volatile unsigned long long*>(count + i)); }
+  __device__ __forceinline__ bool count_in(int i) const {        // one lane; true: the last one
+    unsigned long long seen = *reinterpret_cast<volatile unsigned long long*>(count + i);
+    for (;;) {
+      const unsigned long long was = atomicCAS(count + i, seen, p.share_nonce | static_cast<unsigned long long>(arrived(seen) + 1));
+      if (was == seen) return arrived(seen) == n - 1;
+      seen = was;
+    }
+  }
+  __device__ __forceinline__ void leave(int i) const {
+    uint32_t r[32];
+    __syncwarp();
+    tmem_ld_32x32b_x32(t_addr + (c0 + i) * 32, r);
+    tmem_ld_wait();
+    float4* dst = part(pair, i);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      __stcg(dst + j * 32, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
+                                       __uint_as_float(r[4 * j + 3])));
+  }
+  __device__ __forceinline__ void finish(int i, int row0, int n0, float4* stage) const {
+    EpiOld old;
+    const int col0 = n0 + (c0 + i) * 32;
+    if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(count + i) = 0;
+    __threadfence();
+    __syncwarp();
+    float sum[32];
+    uint32_t r[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) sum[j] = 0.f;
+#pragma unroll 1
+    for (int q = lo; q < lo + n; ++q) {
+      if (q == pair) {
+        tmem_ld_32x32b_x32(t_addr + (c0 + i) * 32, r);
+        tmem_ld_wait();
+      } else {
+        const float4* src = part(q, i);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 v = __ldcg(src + j * 32);
+          r[4 * j] = __float_as_uint(v.x); r[4 * j + 1] = __float_as_uint(v.y);
+          r[4 * j + 2] = __float_as_uint(v.z); r[4 * j + 3] = __float_as_uint(v.w);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 32; ++j) sum[j] += __uint_as_float(r[j]);
+    }
+    if (col0 >= p.N) return;
+    if (epi_has_old(p)) epi_load_old(p, row0, col0, lane, old);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(sum[j]);
+    epi_stage(r, stage, lane);
+    epi_store(p, stage, row0, col0, lane, old);
+  }
+  __device__ __forceinline__ void run(int row0, int n0, float4* stage) const {
+    // this pair's order: chunks rot, rot + 1, ...; the last `own` of them are those that it expects to join
+    const int rot = (pair - lo) * 4 / n, own = n == 2 ? 2 : 1;
+#pragma unroll 1
+    for (int phase = 0; phase < 2; ++phase) {
+      const int first = phase ? 4 - own : 0, many = phase ? own : 4 - own;
+      // lane j looks after chunk (rot + first + j) % 4
+      const int mine = (rot + first + lane) & 3;
+      bool last = false;
+      if (lane < many) {
+        last = peek(mine) == n - 1;
+        if (phase)
+          for (int t = 0; t < SHARE_POLLS && !last; ++t) last = peek(mine) == n - 1;
+      }
+      const unsigned skip = __ballot_sync(0xffffffffu, last);
+#pragma unroll 1
+      for (int j = 0; j < many; ++j)
+        if (!(skip >> j & 1)) leave((rot + first + j) & 3);
+      __threadfence();
+      __syncwarp();
+      if (lane < many && !last) last = count_in(mine);
+      const unsigned join = __ballot_sync(0xffffffffu, last);
+#pragma unroll 1
+      for (int j = 0; j < many; ++j)
+        if (join >> j & 1) finish((rot + first + j) & 3, row0, n0, stage);
+    }
+  }
+};
+
+__device__ __forceinline__ void share_join(const GemmDev& p, const TileShare& s, int tile, int pair, uint32_t cta, uint32_t t_addr, int quarter,
+                                           int half, int lane, int row0, int n0, float4* stage) {
+  const int slot = cta * 8 + quarter * 2 + half;
+  const ShareJoin j = {p, pair, tile * s.each, s.each, lane, slot, t_addr, half * 4, p.share_counts + (tile * 16 + slot) * 4};
+  j.run(row0, n0, stage);
+}
+
+// PAIR_SPLIT: S pairs of the cluster share each tile; otherwise the cluster is one pair and S and ws are unused.
+template <bool A_MN, bool B_MN, int EPI, int MODE>
 __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmDev& p, int S, float4* ws) {
+  constexpr bool SPLIT = MODE == PAIR_SPLIT;
+  using Walk = typename std::conditional<MODE == PAIR_SHARE, SegmentWalk, WholeTiles>::type;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + P_BAR_OFFSET);   // used in CTA 0 only
@@ -892,8 +1022,10 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
   const int num_tiles = num_m * num_n;
   const int all_kb = (p.K + BK - 1) / BK;
   const int split = static_cast<int>(cta_rank >> 1);
-  const int kb0 = SPLIT ? static_cast<int>(static_cast<long long>(all_kb) * split / S) : 0;
-  const int kb1 = SPLIT ? static_cast<int>(static_cast<long long>(all_kb) * (split + 1) / S) : all_kb;
+  // a split product's k-blocks of every tile; otherwise all of them, but for the shared tiles
+  const int kb_lo = SPLIT ? static_cast<int>(static_cast<long long>(all_kb) * split / S) : 0;
+  const int kb_n = SPLIT ? static_cast<int>(static_cast<long long>(all_kb) * (split + 1) / S) - kb_lo : all_kb;
+  const TileShare share = {p.share_tiles, p.share_each, kb_n};
   constexpr uint32_t TMEM_COLS = 2 * TN;
 
   if (threadIdx.x == 0) {
@@ -929,13 +1061,14 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      Walk walk(share, pair, num_pairs, num_tiles);
+      for (Segment seg; ok && walk.next(seg);) {
         int tm, tn;
-        tile_coords(tile, num_m, num_n, tm, tn);
+        tile_coords(seg.tile, num_m, num_n, tm, tn);
         const int m0 = tm * TM + static_cast<int>(cta) * BM;      // this CTA's rows of A and of the output
         // this CTA's 128 rows of B (columns of the output); gated mode: CTA 0 stages the gate rows, CTA 1 the up rows
         const int nb0 = EPI == EPI_SWIGLU ? tn * 128 + static_cast<int>(cta) * p.swiglu_f : tn * TN + static_cast<int>(cta) * BM;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = kb_lo + seg.kb0; kb < kb_lo + seg.kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, 5)) { ok = false; break; }
           uint8_t* sA = smem + stage * P_STAGE_BYTES;
           uint8_t* sB = sA + P_HALF_BYTES;
@@ -971,17 +1104,18 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
       const uint64_t b_desc0 = B_MN ? make_smem_desc_sw128(smem_u32(smem) + P_HALF_BYTES, BK * 128, 1024)
                                     : make_smem_desc_sw128(smem_u32(smem) + P_HALF_BYTES, 0, 1024);
       constexpr uint64_t A_STEP = A_MN ? (2048 >> 4) : (32 >> 4), B_STEP = B_MN ? (2048 >> 4) : (32 >> 4);
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      Walk walk(share, pair, num_pairs, num_tiles);
+      for (Segment seg; ok && walk.next(seg);) {
         if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, 6)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TN;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag, 7)) { ok = false; break; }
           tc_fence_after();
           const uint64_t so = static_cast<uint64_t>(stage) * (P_STAGE_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            umma_f16_ss<2>(d_tmem, a_desc0 + so + k * A_STEP, b_desc0 + so + k * B_STEP, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+            umma_f16_ss<2>(d_tmem, a_desc0 + so + k * A_STEP, b_desc0 + so + k * B_STEP, idesc, (kb != seg.kb0 || k != 0) ? 1u : 0u);
           umma_commit_pair(&empty_bar[stage], leader);   // frees this stage in both CTAs once these MMAs retire
           if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
         }
@@ -997,17 +1131,23 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
     float4* stage_buf = reinterpret_cast<float4*>(smem + P_EPI_OFFSET + (warp - 2) * EPI_STAGE_BYTES);
     int acc = 0;
     uint32_t acc_phase = 0;
-    typename ExchangeOf<SPLIT>::type ex;
+    typename ExchangeOf<MODE>::type ex;
     if constexpr (SPLIT)
       ex = {ws + (static_cast<size_t>(pair) * 2 + cta) * 2 * S * SPLIT_PART, joined, abort_flag, S, split, cta, {0u, 0u}};
-    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+    Walk walk(share, pair, num_pairs, num_tiles);
+    for (Segment seg; walk.next(seg);) {
       int tm, tn;
-      tile_coords(tile, num_m, num_n, tm, tn);
+      tile_coords(seg.tile, num_m, num_n, tm, tn);
       const uint32_t t_addr = tmem_base + acc * TN + (static_cast<uint32_t>(quarter * 32) << 16);
       const int row0 = tm * TM + static_cast<int>(cta) * BM + quarter * 32;
-      const bool ok = epilogue_tile<TN, EPI>(p, t_addr, row0, tn, half, quarter, lane, acc, stage_buf, [&] {
-        return epilogue_wait(&acc_full[acc], acc_phase, abort_flag, 8);
-      }, ex);
+      auto wait = [&] { return epilogue_wait(&acc_full[acc], acc_phase, abort_flag, 8); };
+      bool ok;
+      if (MODE == PAIR_SHARE && seg.kb1 - seg.kb0 < kb_n) {
+        ok = wait();
+        if (ok) share_join(p, share, seg.tile, pair, cta, t_addr, quarter, half, lane, row0, tn * TN, stage_buf);
+      } else {
+        ok = epilogue_tile<TN, EPI>(p, t_addr, row0, tn, half, quarter, lane, acc, stage_buf, wait, ex);
+      }
       if (!ok) break;
       __syncwarp();
       tc_fence_before();
@@ -1028,14 +1168,20 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
 template <bool A_MN, bool B_MN, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmDev p) {
-  pair_body<A_MN, B_MN, EPI, false>(tmA, tmB, p, 1, nullptr);
+  pair_body<A_MN, B_MN, EPI, PAIR_WHOLE>(tmA, tmB, p, 1, nullptr);
+}
+
+template <bool A_MN, bool B_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+gemm_bf16_share_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmDev p) {
+  pair_body<A_MN, B_MN, EPI_LINEAR, PAIR_SHARE>(tmA, tmB, p, 1, nullptr);
 }
 
 // Launched with clusters of 2 S CTAs.
 template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmDev p, int S, float4* ws) {
-  pair_body<A_MN, B_MN, EPI_LINEAR, true>(tmA, tmB, p, S, ws);
+  pair_body<A_MN, B_MN, EPI_LINEAR, PAIR_SPLIT>(tmA, tmB, p, S, ws);
 }
 
 // ----------------------------------------------------------------------------------
@@ -1127,6 +1273,20 @@ static void fill_rope(GemmDev& p, const gv_gemm_args* a) {
   p.rope_pos_offset = a->rope_pos_offset;
 }
 
+// Counters of the shared tiles (per tile, CTA of the pair, epilogue warp and chunk), then the partial sums of each pair.
+static long long share_count_bytes(const TileShare& s) { return static_cast<long long>(s.tiles) * 2 * 8 * 4 * 8; }
+static long long share_bytes(const TileShare& s) {
+  return s.tiles ? share_count_bytes(s) + static_cast<long long>(s.tiles) * s.each * 2 * SPLIT_PART * 16 : 0;
+}
+static void fill_share(GemmDev& p, const gv_gemm_args* a, const TileShare& s) {
+  static std::atomic<unsigned long long> launches{0};
+  p.share_tiles = s.tiles; p.share_each = s.each;
+  p.share_counts = reinterpret_cast<unsigned long long*>(a->workspace);
+  p.share_parts = s.tiles ? reinterpret_cast<float4*>(reinterpret_cast<char*>(a->workspace) + share_count_bytes(s)) : nullptr;
+  // an odd multiplier makes different launches' numbers differ in all bits; zero is what the last warp leaves
+  p.share_nonce = s.tiles ? (launches.fetch_add(1, std::memory_order_relaxed) * 2 + 1) * 0x9E3779B97F4A7C15ull << 8 : 0;
+}
+
 template <int BN, bool A_MN, bool B_MN, int EPI = EPI_LINEAR>
 static int launch_gemm(const gv_gemm_args* a, cudaStream_t stream, const gv_xent_args* x = nullptr) {
   CUtensorMap tmA, tmB;
@@ -1152,6 +1312,7 @@ static int launch_gemm(const gv_gemm_args* a, cudaStream_t stream, const gv_xent
   fill_xent(p, x, BN);
   fill_rope(p, a);
   fill_swiglu(p, a);
+  fill_share(p, a, {0, 1, 0});
   auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, EPI>;
   constexpr int smem = GemmSmem<BN>::TOTAL;
   static PerDeviceOnce smem_once;
@@ -1189,6 +1350,7 @@ static int fill_pair(const gv_gemm_args* a, const gv_xent_args* x, CUtensorMap& 
   fill_xent(p, x, 256);
   fill_rope(p, a);
   fill_swiglu(p, a);
+  fill_share(p, a, {0, 1, 0});
   return 0;
 }
 
@@ -1213,6 +1375,19 @@ static int resident_clusters(Kernel kern, int ctas) {
   return n;
 }
 
+// CTA pairs that the device holds at once (the four layouts need the same resources).
+static int gemm_pairs() {
+  static std::atomic<int> n{0};
+  int v = n.load(std::memory_order_relaxed);
+  if (v == 0) {
+    auto kern = gemm_bf16_share_kernel<false, false>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_TOTAL) != cudaSuccess) cudaGetLastError();
+    v = resident_clusters(kern, 2);
+    n.store(v, std::memory_order_relaxed);
+  }
+  return v;
+}
+
 template <bool A_MN, bool B_MN, int EPI = EPI_LINEAR>
 static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv_xent_args* x = nullptr) {
   CUtensorMap tmA, tmB;
@@ -1230,6 +1405,23 @@ static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv
   if (max_pairs == 0) max_pairs = resident_clusters(kern, 2);
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
   kern<<<2 * pairs, GEMM_THREADS, P_SMEM_TOTAL, stream>>>(tmA, tmB, p);
+  return static_cast<int>(cudaGetLastError());
+}
+
+template <bool A_MN, bool B_MN>
+static int launch_gemm_share(const gv_gemm_args* a, cudaStream_t stream, const TileShare& share) {
+  CUtensorMap tmA, tmB;
+  GemmDev p;
+  const int rc = fill_pair<A_MN, B_MN>(a, nullptr, tmA, tmB, p);
+  if (rc) return rc;
+  fill_share(p, a, share);
+  auto kern = gemm_bf16_share_kernel<A_MN, B_MN>;
+  static PerDeviceOnce smem_once;
+  {
+    cudaError_t e = ensure_max_dynamic_smem(smem_once, kern, P_SMEM_TOTAL);
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  kern<<<2 * gemm_pairs(), GEMM_THREADS, P_SMEM_TOTAL, stream>>>(tmA, tmB, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1295,6 +1487,39 @@ static bool narrow_tiles(const gv_gemm_args* a) {
   return a->N <= 128 || static_cast<long>((a->M + BM - 1) / BM) * ((a->N + 255) / 256) < num_sms();
 }
 
+constexpr double SHARE_COSTS_US = 11.0;
+
+// The shared tiles' time, of the time of a whole tile.
+static double shared_part(const TileShare& s) { return static_cast<double>((s.kb + s.each - 1) / s.each) / s.kb; }
+
+static bool runs_on_pairs(const gv_gemm_args* a) {
+  const long tiles = static_cast<long>((a->M + 255) / 256) * ((a->N + 255) / 256);
+  if (pair_mode() == 0) return false;
+  return pair_mode() == 2 || ((a->swiglu_out || !narrow_tiles(a)) && tiles >= num_sms() / 2);
+}
+
+// Tiles of this product that CTA pairs share (none: every tile goes to one pair): those of a last wave that is at most half full. The
+// rest of that wave's time, at 0.36 us a k-block, must be more than what leaving and joining the sums costs; with fewer k-blocks the
+// joining is also longer than the whole tile that it should hide behind. Measured us, whole -> shared: 8192 x 1280 x 5120 88 -> 77,
+// 8192 x 1600 x 6400 142 -> 125, 1280 x 5120 x 8192 102 -> 90, 2999 x 3584 x 18944 309 -> 282, 2999 x 3584 x 3584 (would save 13 us)
+// 61.6 -> 57.5; 8192 x 1600 x 1600 (7 us) 40.5 -> 44.9, 4608 x 3584 x 2999 (8 us) 88 -> 92, 8192 x 1280 x 1280 (5 us) 28.8 -> 33.
+// A last wave that is more than half full, cut into even ranges over all pairs, lost 10 to 40 us: parts of two tiles a pair, joined late.
+// GV_GEMM_SHARE = 0 turns it off, 2 shares whenever a wave is not full (numerics tests).
+static TileShare share_plan(const gv_gemm_args* a) {
+  static const int mode = [] {
+    const char* e = getenv("GV_GEMM_SHARE");
+    return e && e[0] >= '0' && e[0] <= '2' ? e[0] - '0' : 1;
+  }();
+  const TileShare none = {0, 1, 0};
+  if (mode == 0 || a->rope_cols > 0 || a->swiglu_out || a->gelu_out || a->M <= 0 || a->N <= 0 || a->K <= 0 || !runs_on_pairs(a)) return none;
+  const long tiles = static_cast<long>((a->M + 255) / 256) * ((a->N + 255) / 256);
+  const int all = gemm_pairs(), left = static_cast<int>(tiles % all), kb = (a->K + BK - 1) / BK;
+  if ((mode != 2 && tiles < all)) return none;
+  const TileShare s = share_of(left, all, kb);
+  if (mode == 2 || s.tiles == 0) return s;
+  return (1.0 - shared_part(s)) * kb * 0.36 > SHARE_COSTS_US ? s : none;
+}
+
 // Pairs per tile of the split kernel for this product, 1 = no split. Splitting pays where the last wave of tiles is nearly
 // empty or where there is less than one wave. The estimate is waves x (k-blocks x microseconds + per wave) + per launch:
 //   256 x 256 tiles on pairs              0.36, 0, 5
@@ -1323,6 +1548,8 @@ static int split_plan(const gv_gemm_args* a) {
   double best = on_pairs ? static_cast<double>((tiles + sms / 2 - 1) / (sms / 2)) * kb * 0.36 + 5.0
                          : static_cast<double>((small + sms - 1) / sms) * (kb * 0.205 + 3.0) + 3.0;
   if (!on_pairs && !narrow_tiles(a)) return 1;       // 128 x 256 tiles on single CTAs: one and a half waves, left alone
+  const TileShare share = share_plan(a);
+  if (share.tiles) best = (static_cast<double>(tiles / gemm_pairs()) + shared_part(share)) * kb * 0.36 + 7.0;
   best *= 0.92;
   int S = 1;
   for (int s = 2; s <= MAX_SPLIT; ++s) {
@@ -1369,8 +1596,7 @@ extern "C" int gv_gemm_bf16(const gv_gemm_args* a, gv_stream_t s) {
     if (a->a_mn_major || a->b_mn_major || a->bias || a->residual || a->act || a->accumulate || a->c_f32 || a->rope_cols ||
         (a->N % 256) || (a->swiglu_ld % 8) || (reinterpret_cast<uintptr_t>(a->swiglu_out) & 15))
       return 2007;
-    const long pair_tiles = static_cast<long>((a->M + 255) / 256) * (a->N / 256);
-    if (pair_mode() != 0 && (pair_mode() == 2 || pair_tiles >= num_sms() / 2)) return launch_gemm_pair<false, false, EPI_SWIGLU>(a, stream);
+    if (runs_on_pairs(a)) return launch_gemm_pair<false, false, EPI_SWIGLU>(a, stream);
     return launch_gemm<256, false, false, EPI_SWIGLU>(a, stream);
   }
   const int key = (a->a_mn_major ? 2 : 0) | (a->b_mn_major ? 1 : 0);
@@ -1386,18 +1612,27 @@ extern "C" int gv_gemm_bf16(const gv_gemm_args* a, gv_stream_t s) {
       }
     }
   }
-  const bool narrow = narrow_tiles(a);
-  // K-major operands and enough 256 x 256 tiles for every SM pair: the two-CTA kernel
-  if (pair_mode() != 0) {
-    const long pair_tiles = static_cast<long>((a->M + 255) / 256) * ((a->N + 255) / 256);
-    if (pair_mode() == 2 || (!narrow && pair_tiles >= num_sms() / 2)) {
-      if (a->gelu_out) return launch_gemm_pair<false, false, EPI_GELU>(a, stream);
+  if (a->workspace != nullptr) {
+    const TileShare share = share_plan(a);
+    if (share.tiles) {
+      if (a->workspace_bytes < share_bytes(share) || (reinterpret_cast<uintptr_t>(a->workspace) & 15)) return 2008;
       switch (key) {
-        case 0: return launch_gemm_pair<false, false>(a, stream);
-        case 1: return launch_gemm_pair<false, true>(a, stream);
-        case 2: return launch_gemm_pair<true, false>(a, stream);
-        default: return launch_gemm_pair<true, true>(a, stream);
+        case 0: return launch_gemm_share<false, false>(a, stream, share);
+        case 1: return launch_gemm_share<false, true>(a, stream, share);
+        case 2: return launch_gemm_share<true, false>(a, stream, share);
+        default: return launch_gemm_share<true, true>(a, stream, share);
       }
+    }
+  }
+  const bool narrow = narrow_tiles(a);
+  // enough 256 x 256 tiles for every SM pair: the two-CTA kernel
+  if (runs_on_pairs(a)) {
+    if (a->gelu_out) return launch_gemm_pair<false, false, EPI_GELU>(a, stream);
+    switch (key) {
+      case 0: return launch_gemm_pair<false, false>(a, stream);
+      case 1: return launch_gemm_pair<false, true>(a, stream);
+      case 2: return launch_gemm_pair<true, false>(a, stream);
+      default: return launch_gemm_pair<true, true>(a, stream);
     }
   }
   if (a->gelu_out) return narrow ? launch_gemm<128, false, false, EPI_GELU>(a, stream) : launch_gemm<256, false, false, EPI_GELU>(a, stream);
@@ -1420,7 +1655,7 @@ extern "C" int gv_gemm_bf16(const gv_gemm_args* a, gv_stream_t s) {
 
 extern "C" long long gv_gemm_workspace_bytes(const gv_gemm_args* a) {
   const int S = gv::split_plan(a);
-  return S > 1 ? gv::split_bytes(a, S) : 0;
+  return S > 1 ? gv::split_bytes(a, S) : gv::share_bytes(gv::share_plan(a));
 }
 
 // Language-model head with the cross entropy in the GEMM epilogue. Always runs the 256-column-wide tiles, so the

@@ -48,7 +48,8 @@ class RopeEpilogue:
 
 @functools.lru_cache(maxsize=1024)
 def _workspace_bytes(M: int, N: int, K: int) -> int:
-    """Scratch of a split reduction for a product of these sizes (at most 38 MB); 0: not split."""
+    """Scratch of a product of these sizes whose reductions CTA pairs share, of all tiles or of the last wave's (at most 39 MB); 0: none
+    is shared."""
     return _lib.lib().gv_gemm_workspace_bytes(_lib.GemmArgs(M=M, N=N, K=K))
 
 

@@ -238,6 +238,47 @@ assert all(torch.equal(gemm(a, w, out_dtype=torch.float32), first) for _ in rang
         assert v < 1e-2, (k, v, res)
 
 
+def test_shared_tiles_match_fp32_reference():
+    """Tiles shared by CTA pairs whenever a wave is not full (two to four pairs per tile, tails of M, N and K, fewer k-blocks than pairs),
+    in every layout, with every epilogue of a plain product, and the same bits on every repeat, whatever the scratch held."""
+    import json
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    extra = """
+from hetu_galvatron_b200.ops.gemm import _workspace_bytes
+assert _workspace_bytes(300, 768, 1000) > 0 and _workspace_bytes(256, 512, 64) == 0
+res = {}
+def rel(y, ref):
+    return ((y.float() - ref.float()).norm() / ref.float().norm()).item()
+for M, N, K in [(300, 768, 1000), (1400, 1536, 320), (1200, 1080, 136), (2304, 2304, 64), (5000, 1032, 2048)]:
+    a, w = torch.randn(M, K, device="cuda", dtype=torch.bfloat16), torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.1
+    first = gemm(a, w, out_dtype=torch.float32)
+    for _ in range(4):
+        junk = torch.randint(0, 256, (_workspace_bytes(M, N, K) or 1,), device="cuda", dtype=torch.uint8)
+        del junk                                            # the next call's scratch
+        assert torch.equal(gemm(a, w, out_dtype=torch.float32), first)
+    ref = a.float() @ w.float().t()
+    res["%d fp32" % M] = rel(first, ref)
+    bias = torch.randn(N + 1, device="cuda", dtype=torch.bfloat16)[1:]
+    res["%d gelu" % M] = rel(gemm(a, w, bias=bias, gelu=True), torch.nn.functional.gelu(ref + bias.float(), approximate="tanh"))
+    old = torch.randn(M, N, device="cuda", dtype=torch.bfloat16)
+    res["%d bf16 accumulate" % M] = rel(gemm(a, w, out=old.clone(), accumulate=True), ref + old.float())
+torch.cuda.synchronize()
+res["error"] = _lib.read_error()
+print("SHARED " + json.dumps(res))
+"""
+    env = dict(os.environ, GV_GEMM_SHARE="2", GV_GEMM_PAIR="2", GV_GEMM_SPLIT="1")
+    r = subprocess.run([sys.executable, "-c", PAIR_SCRIPT % root + extra], capture_output=True, text=True, timeout=300, env=env)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
+    for tag in ("PAIR ", "SHARED "):
+        res = json.loads([l for l in r.stdout.splitlines() if l.startswith(tag)][0][len(tag):])
+        assert res.pop("error") is None
+        for k, v in res.items():
+            assert v < 1e-2, (k, v, res)      # bf16 outputs: one or two roundings of 2^-9
+
+
 def test_products_without_room_for_scratch_stay_unsplit(monkeypatch):
     """An allocation of the partial sums that fails (once, made up on the host) costs one warning; from then on the product repeats
     its bits whether or not there is room again."""

@@ -143,3 +143,11 @@ def test_attention_checker_sees_a_phase_that_has_passed(attention_order):
     """One barrier for all products: the last wait misses its phase by way of the product before, and passes too early without."""
     assert _run(attention_order, "--blocks", 4, "--schedule", "single")[1]["stuck"] > 0
     assert _run(attention_order, "--blocks", 4, "--schedule", "direct")[1]["early"] > 0
+
+
+@pytest.mark.parametrize("pairs,tiles,kb", [(74, 300, 24), (72, 150, 24), (74, 75, 300), (7, 60, 24)])
+def test_shared_tiles_cover_every_k_block_once(tmp_path, pairs, tiles, kb):
+    """The parts that the GEMM's CTA pairs take of shared tiles, and how many a tile's last warp counts and reads."""
+    sim = _build(str(tmp_path), False, "tile_share_sim.cpp")
+    rc, out, _ = _run(sim, "--pairs", pairs, "--tiles", tiles, "--kb", kb)
+    assert rc == 0 and out["wrong"] == 0 and out["products"] > 1000 and out["most_pairs_per_tile"] <= 4, out
