@@ -3,6 +3,7 @@
 * ``_lib/libgvkernels.so``  -- the sm_100a CUDA kernel library (plain C ABI, loaded with ctypes)
 * ``_lib/dp_core*.so``      -- the C++ dynamic-programming search core (pybind11 module)
 * ``_lib/data_index*.so``   -- the C++ dataset index builder (pybind11 module)
+* ``_lib/torch_ops*.so``    -- the C++ autograd Functions of the un-sharded hot path (pybind11 module over libtorch)
 
 The reference builds its single native module with setuptools (setup.py:39-44) and a Makefile
 (Makefile:1-16); here nvcc / g++ are called directly so that the built objects stay inside the
@@ -136,8 +137,37 @@ def build_data_index(force: bool = False) -> Path:
     return _build_pybind("data_index", "data_index.cpp", force)
 
 
+def build_torch_ops(force: bool = False) -> Path:
+    """The module that launches the kernels from C++ autograd Functions. Needs the headers and libraries of the installed torch, whose
+    version is part of the stamp."""
+    import pybind11
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    LIB_DIR.mkdir(exist_ok=True)
+    src = CSRC / "torch_ops.cpp"
+    out = LIB_DIR / ("torch_ops" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-march=x86-64-v3",
+             "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+    digest = _hash_sources([src, CSRC / "include" / "gv_kernels.h"], flags + [torch.__version__])
+    stamp = LIB_DIR / "torch_ops.hash"
+    if not force and out.exists() and stamp.exists() and stamp.read_text() == digest:
+        return out
+    paths = ["-I" + str(CSRC)] + [a for p in include_paths("cuda") + [pybind11.get_include(), sysconfig.get_paths()["include"]] for a in ("-isystem", p)]
+    libs = [a for p in library_paths("cuda") for a in ("-L" + p,)]
+    cmd = ["g++", *flags, *paths, str(src), "-o", str(out), *libs, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for torch_ops.cpp:\n{r.stdout}\n{r.stderr}")
+    stamp.write_text(digest)
+    return out
+
+
 def build_all(force: bool = False, verbose: bool = False) -> None:
-    build_cuda(force, verbose)
+    with ThreadPoolExecutor(max_workers=1) as ex:
+        ops = ex.submit(build_torch_ops, force)
+        build_cuda(force, verbose)
+        ops.result()
     if (CSRC / "dp_core.cpp").exists():
         build_dp_core(force)
     if (CSRC / "data_index.cpp").exists():
@@ -148,7 +178,7 @@ def load_pybind(name: str):
     """Import a pybind11 module built by this file (building it first if it is missing)."""
     import importlib.util
 
-    builder = {"dp_core": build_dp_core, "data_index": build_data_index}[name]
+    builder = {"dp_core": build_dp_core, "data_index": build_data_index, "torch_ops": build_torch_ops}[name]
     path = builder()
     spec = importlib.util.spec_from_file_location(name, path)
     mod = importlib.util.module_from_spec(spec)

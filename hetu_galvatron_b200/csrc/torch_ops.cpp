@@ -1,0 +1,825 @@
+// Autograd Functions of the un-sharded hot path in C++: the counterparts of the Functions of the same name in ops/autograd.py, which
+// stay for tensor parallelism, other types and devices, and everything that this file refuses. Same launches in the same order on
+// the same operands; what goes is the host time between them. A Python Function costs 13 us of host time forward and backward before it
+// does anything, and its launch wrappers another 5 to 20 us each: a step of a two-layer model of 1.0 ms of kernels took 4.9 ms.
+//
+// Every entry point returns None where its conditions do not hold (operands that are not plain bf16 CUDA tensors, sizes that the
+// kernels refuse, tensors of a functorch transform or a subclass), and the caller takes the Python Function.
+//
+// Weight gradients follow the main_grad protocol of ops/autograd.py; a gradient buffer that the kernels cannot take is
+// handed to the Python code.
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_cpp_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <atomic>
+#include <cmath>
+#include <limits>
+#include <mutex>
+#include <optional>
+#include <set>
+#include <string>
+#include <tuple>
+
+#include "include/gv_kernels.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+// ------------------------------------------------------------------ launches
+// The kernel library's entry points; the addresses come from the library that Python has loaded.
+#define GV_ENTRIES(X)                                                                                                              \
+  X(gv_gemm_bf16) X(gv_gemm_xent) X(gv_gemm_workspace_bytes) X(gv_xent_merge) X(gv_rmsnorm_fwd) X(gv_rmsnorm_bwd) X(gv_layernorm_fwd) \
+  X(gv_layernorm_bwd) X(gv_norm_bwd_scratch_elems) X(gv_rope) X(gv_swiglu_bwd) X(gv_gelu_bwd) X(gv_colsum_accum) X(gv_attn_fwd) X(gv_attn_bwd)
+struct Entries {
+#define X(name) decltype(&::name) name = nullptr;
+  GV_ENTRIES(X)
+#undef X
+} K;
+
+std::atomic<long long> g_launches{0};
+
+struct LaunchFailure : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
+
+void launched(int rc, const char* what, int kernels = 1) {
+  g_launches.fetch_add(kernels, std::memory_order_relaxed);
+  if (rc != 0) throw LaunchFailure(std::string(what) + " failed to launch (code " + std::to_string(rc) + ")");
+}
+
+gv_stream_t stream() { return reinterpret_cast<gv_stream_t>(at::cuda::getCurrentCUDAStream().stream()); }
+
+// Python functions for what is not done here: (_wgrad, _vec_grad over a ready sum, a product whose scratch did not fit). Never freed:
+// the interpreter may be gone when statics are destroyed.
+py::object *g_wgrad = nullptr, *g_vecgrad = nullptr, *g_no_scratch = nullptr, *g_error = nullptr;
+PyObject *g_main_grad = nullptr, *g_hook = nullptr;
+
+// Runs a Function without the GIL (a launch may wait for the device's queue); a launch that failed raises the package's KernelError.
+template <class F>
+auto no_gil(F f) -> decltype(f()) {
+  std::string what;
+  {
+    py::gil_scoped_release released;
+    try {
+      return f();
+    } catch (const LaunchFailure& e) {
+      what = e.what();
+    }
+  }
+  PyErr_SetString(g_error->ptr(), what.c_str());
+  throw py::error_already_set();
+}
+
+// ------------------------------------------------------------------ conditions
+// A tensor whose address may be taken: no functorch wrapper, no Python subclass, no other layout.
+bool plain(const Tensor& t) {
+  static const c10::DispatchKeySet odd = c10::DispatchKeySet({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                                              c10::DispatchKey::Functionalize, c10::DispatchKey::Python,
+                                                              c10::DispatchKey::PythonTLSSnapshot, c10::DispatchKey::Conjugate,
+                                                              c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor});
+  return t.defined() && t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has_any(odd);
+}
+bool plain16(const Tensor& t) { return plain(t) && t.scalar_type() == at::kBFloat16; }
+// No transform, trace or mode that would have to see the operators of a Python Function.
+bool plain_mode() {
+  static const c10::DispatchKeySet odd = c10::DispatchKeySet({c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::Python,
+                                                              c10::DispatchKey::PythonDispatcher, c10::DispatchKey::Functionalize,
+                                                              c10::DispatchKey::Tracer});
+  return !c10::impl::tls_local_dispatch_key_set().included_.has_any(odd);
+}
+bool aligned(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15) == 0; }
+bool rows_ok(const Tensor& t) { return t.stride(1) == 1 && t.stride(0) % 8 == 0 && aligned(t); }
+// A weight [N, K] that the GEMM takes as stored, in forward, input- and weight-gradient products.
+bool weight_ok(const Tensor& w) {
+  return plain16(w) && w.dim() == 2 && w.size(0) > 0 && w.size(1) > 0 && w.size(0) % 8 == 0 && w.size(1) % 8 == 0 && rows_ok(w);
+}
+bool input_ok(const Tensor& x) { return plain16(x) && x.dim() >= 1 && x.numel() > 0 && x.numel() / x.size(-1) < (1ll << 31); }
+
+void* ptr(const Tensor& t) { return t.defined() ? t.mutable_data_ptr() : nullptr; }
+const void* cptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
+Tensor row_major(const Tensor& t) { return rows_ok(t) ? t : t.contiguous(); }
+Tensor flat2d(const Tensor& t) { return t.reshape({-1, t.size(-1)}); }
+Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
+Tensor empty16(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options()); }
+Tensor empty32(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
+// The gradient of an output, contiguous and aligned for 16-byte loads.
+Tensor ready(const Tensor& t) {
+  Tensor c = t.contiguous();
+  return aligned(c) ? c : c.clone();
+}
+
+// ------------------------------------------------------------------ GEMM
+struct Rope {
+  int cols = 0, dh = 0, pos_div = 1, pos_offset = 0;
+  Tensor inv_freq;
+};
+
+std::mutex g_no_scratch_lock;
+std::set<std::tuple<int, int, int, int>> g_no_scratch_products;     // see ops/gemm.py _NO_SCRATCH
+
+Tensor scratch_for(const gv_gemm_args& a, const Tensor& like) {
+  gv_gemm_args sizes = {};
+  sizes.M = a.M; sizes.N = a.N; sizes.K = a.K;
+  const long long need = K.gv_gemm_workspace_bytes(&sizes);
+  if (need == 0) return Tensor();
+  const auto key = std::make_tuple(static_cast<int>(like.device().index()), a.M, a.N, a.K);
+  {
+    std::lock_guard<std::mutex> lock(g_no_scratch_lock);
+    if (g_no_scratch_products.count(key)) return Tensor();
+  }
+  try {
+    return at::empty({need}, like.options().dtype(at::kByte));
+  } catch (const c10::OutOfMemoryError&) {
+    py::gil_scoped_acquire gil;
+    (*g_no_scratch)(std::get<0>(key), a.M, a.N, a.K, need);
+    return Tensor();
+  }
+}
+
+// out = a b^T with either operand in its transposed storage, as ops/gemm.py gemm.
+void gemm_into(const Tensor& a_, bool a_mn, const Tensor& b_, bool b_mn, const Tensor& out, bool accumulate, const Tensor& bias = Tensor(),
+               const Tensor& residual = Tensor(), const Rope* rope = nullptr, const Tensor& swiglu_out = Tensor(), const Tensor& gelu_out = Tensor()) {
+  const Tensor a = row_major(a_), b = row_major(b_);
+  gv_gemm_args g = {};
+  g.A = cptr(a); g.B = cptr(b); g.C = ptr(out); g.bias = cptr(bias); g.residual = cptr(residual);
+  g.M = static_cast<int>(a.size(a_mn ? 1 : 0)); g.K = static_cast<int>(a.size(a_mn ? 0 : 1)); g.N = static_cast<int>(b.size(b_mn ? 1 : 0));
+  g.lda = static_cast<int>(a.stride(0)); g.ldb = static_cast<int>(b.stride(0)); g.ldc = static_cast<int>(out.stride(0));
+  g.ldr = residual.defined() ? static_cast<int>(residual.stride(0)) : 0;
+  g.a_mn_major = a_mn; g.b_mn_major = b_mn;
+  g.c_f32 = out.scalar_type() == at::kFloat; g.accumulate = accumulate; g.alpha = 1.f;
+  Tensor scratch;
+  if (swiglu_out.defined()) { g.swiglu_out = ptr(swiglu_out); g.swiglu_ld = static_cast<int>(swiglu_out.stride(0)); }
+  if (rope != nullptr) {
+    g.rope_cols = rope->cols; g.rope_dh = rope->dh;
+    g.rope_inv_freq = static_cast<const float*>(cptr(rope->inv_freq));
+    g.rope_pos_div = rope->pos_div; g.rope_pos_offset = rope->pos_offset;
+  } else if (gelu_out.defined()) {
+    g.gelu_out = ptr(gelu_out); g.gelu_ld = static_cast<int>(gelu_out.stride(0));
+  } else if (!swiglu_out.defined()) {
+    scratch = scratch_for(g, a);
+    if (scratch.defined()) { g.workspace = ptr(scratch); g.workspace_bytes = scratch.numel(); }
+  }
+  launched(K.gv_gemm_bf16(&g, stream()), "gv_gemm_bf16");
+}
+
+// x W^T [rows, N]
+Tensor project(const Tensor& x2, const Tensor& W, const Tensor& bias = Tensor(), const Tensor& residual = Tensor(), const Rope* rope = nullptr) {
+  Tensor y = empty16({x2.size(0), W.size(0)}, x2);
+  gemm_into(x2, false, W, false, y, false, bias, residual.defined() ? row_major(flat2d(residual)) : Tensor(), rope);
+  return y;
+}
+// dy W [rows, K]
+Tensor input_grad(const Tensor& dy2, const Tensor& W) {
+  Tensor dx = empty16({dy2.size(0), W.size(1)}, dy2);
+  gemm_into(dy2, false, W, true, dx, false);
+  return dx;
+}
+
+at::DimVector with_last(const at::DimVector& lead, int64_t n) {
+  at::DimVector s(lead);
+  s.push_back(n);
+  return s;
+}
+
+// ------------------------------------------------------------------ parameter gradients
+struct Buffer {
+  Tensor main_grad;        // where the gradient is accumulated; undefined: none
+  py::object hook, param;  // to be called when it has been (hook may be empty); touched with the GIL only
+  bool in_python = false;  // a buffer that the kernels do not take
+};
+
+// What Python has attached to a parameter. Buffers that the kernels take: fp32 or bf16, as long as the parameter, contiguous, aligned.
+Buffer buffer_of(const Tensor& p) {
+  Buffer b;
+  b.param = py::reinterpret_steal<py::object>(THPVariable_Wrap(p));
+  PyObject* mg = PyObject_GetAttr(b.param.ptr(), g_main_grad);
+  if (mg == nullptr) PyErr_Clear();
+  py::object held = py::reinterpret_steal<py::object>(mg);
+  if (mg == nullptr || mg == Py_None) return b;
+  b.in_python = true;
+  if (THPVariable_Check(mg)) {
+    const Tensor& t = THPVariable_Unpack(mg);
+    if (plain(t) && (t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16) && t.is_contiguous() && t.numel() == p.numel() && aligned(t)) {
+      b.main_grad = t;
+      b.in_python = false;
+    }
+  }
+  PyObject* hook = PyObject_GetAttr(b.param.ptr(), g_hook);
+  if (hook == nullptr) PyErr_Clear();
+  else if (hook == Py_None) Py_DECREF(hook);
+  else b.hook = py::reinterpret_steal<py::object>(hook);
+  return b;
+}
+
+template <class F>
+auto in_python(F f) {                       // exceptions of Python code cross the autograd engine as text
+  try {
+    return f();
+  } catch (py::error_already_set& e) {
+    const std::string what = e.what();
+    throw std::runtime_error(what);
+  }
+}
+
+void accumulated(Buffer& b) {
+  if (b.hook) in_python([&] { return b.hook(b.param); });
+}
+
+// dW of y = x W^T: into W.main_grad (nothing is returned then) or a fresh gradient.
+Tensor weight_grad(const Tensor& W, const Tensor& dy2, const Tensor& x2) {
+  Tensor mg;
+  bool py_side = false, hooked = false;
+  {
+    py::gil_scoped_acquire gil;
+    Buffer b = buffer_of(W);
+    mg = b.main_grad; py_side = b.in_python; hooked = static_cast<bool>(b.hook);
+    if (py_side)
+      return in_python([&] {
+        py::object r = (*g_wgrad)(W, dy2, x2);
+        return r.is_none() ? Tensor() : r.cast<Tensor>();
+      });
+  }
+  if (mg.defined()) {
+    gemm_into(dy2, true, x2, true, mg.view({W.size(0), W.size(1)}), true);
+    if (hooked) {
+      py::gil_scoped_acquire gil;
+      Buffer b = buffer_of(W);
+      accumulated(b);
+    }
+    return Tensor();
+  }
+  Tensor dw = at::empty({W.size(0), W.size(1)}, W.options());
+  gemm_into(dy2, true, x2, true, dw, false);
+  return dw;
+}
+
+// The gradient of a vector parameter: `fill(buf)` adds it to an fp32 buffer.
+template <class Fill>
+Tensor vector_grad(const Tensor& p, Fill fill) {
+  Tensor mg;
+  bool py_side = false, hooked = false;
+  {
+    py::gil_scoped_acquire gil;
+    Buffer b = buffer_of(p);
+    mg = b.main_grad; py_side = b.in_python; hooked = static_cast<bool>(b.hook);
+  }
+  if (mg.defined() && mg.scalar_type() == at::kFloat) {
+    fill(mg.view({-1}));
+  } else {
+    Tensor tmp = at::zeros({p.numel()}, p.options().dtype(at::kFloat));
+    fill(tmp);
+    if (py_side) {
+      py::gil_scoped_acquire gil;
+      return in_python([&] {
+        py::object r = (*g_vecgrad)(p, tmp);
+        return r.is_none() ? Tensor() : r.cast<Tensor>();
+      });
+    }
+    if (!mg.defined()) return tmp.to(p.scalar_type()).view(p.sizes());
+    mg.view({-1}).add_(tmp.to(mg.scalar_type()));
+  }
+  if (hooked) {
+    py::gil_scoped_acquire gil;
+    Buffer b = buffer_of(p);
+    accumulated(b);
+  }
+  return Tensor();
+}
+
+Tensor bias_grad(const Tensor& bias, const Tensor& dy2) {
+  return vector_grad(bias, [&](const Tensor& buf) {
+    launched(K.gv_colsum_accum(cptr(dy2), static_cast<float*>(ptr(buf)), dy2.size(0), static_cast<int>(dy2.size(1)), stream()), "gv_colsum_accum");
+  });
+}
+
+// ------------------------------------------------------------------ linear
+struct LinearFn : Function<LinearFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& W, const OptTensor& bias, const OptTensor& residual, const Rope& rope) {
+    const Tensor x2 = flat2d(x);
+    const Tensor y = project(x2, W, opt(bias), opt(residual), rope.cols ? &rope : nullptr);
+    at::DimVector lead(x.sizes().begin(), x.sizes().end() - 1);
+    ctx->saved_data["lead"] = at::IntArrayRef(lead).vec();
+    ctx->saved_data["residual"] = residual.has_value();
+    ctx->save_for_backward({x2, W, opt(bias)});
+    return y.view(with_last(lead, W.size(0)));
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x2 = saved[0], &W = saved[1], &bias = saved[2], &dy = grads[0];
+    const Tensor dy2 = dy.reshape({-1, W.size(0)}).contiguous();
+    Tensor dx, db;
+    if (ctx->needs_input_grad(0)) {
+      const auto lead = ctx->saved_data["lead"].toIntVector();
+      dx = input_grad(dy2, W).view(with_last(at::DimVector(lead.begin(), lead.end()), W.size(1)));
+    }
+    Tensor dW = weight_grad(W, dy2, x2);
+    if (bias.defined()) db = bias_grad(bias, dy2);
+    return {dx, dW, db, ctx->saved_data["residual"].toBool() ? dy : Tensor(), Tensor()};
+  }
+};
+
+bool add_on_ok(const OptTensor& t, int64_t numel) { return !t.has_value() || (plain16(*t) && t->numel() == numel); }
+bool linear_ok(const Tensor& x, const Tensor& W, const OptTensor& bias, const OptTensor& residual) {
+  return plain_mode() && input_ok(x) && weight_ok(W) && x.size(-1) == W.size(1) && add_on_ok(bias, W.size(0)) &&
+         (!bias.has_value() || bias->is_contiguous()) && add_on_ok(residual, x.numel() / x.size(-1) * W.size(0));
+}
+
+py::object linear(const Tensor& x, const Tensor& W, const OptTensor& bias, const OptTensor& residual,
+                  const std::optional<std::tuple<int, int, Tensor, int, int>>& rope) {
+  if (!linear_ok(x, W, bias, residual)) return py::none();
+  Rope r;
+  if (rope.has_value()) {
+    std::tie(r.cols, r.dh, r.inv_freq, r.pos_div, r.pos_offset) = *rope;
+    if (r.cols <= 0 || !plain(r.inv_freq) || r.inv_freq.scalar_type() != at::kFloat || !r.inv_freq.is_contiguous() || r.inv_freq.numel() != r.dh / 2)
+      return py::none();
+  }
+  return py::cast(no_gil([&] { return LinearFn::apply(x, W, bias, residual, r); }));
+}
+
+// ------------------------------------------------------------------ MLP
+struct SwiGLUMLPFn : Function<SwiGLUMLPFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w_up, const Tensor& w_down, const OptTensor& residual) {
+    const Tensor x2 = flat2d(x);
+    const int64_t f = w_up.size(0) / 2;
+    const Tensor act = empty16({x2.size(0), f}, x2), gu = empty16({x2.size(0), 2 * f}, x2);
+    gemm_into(x2, false, w_up, false, gu, false, Tensor(), Tensor(), nullptr, act);
+    const Tensor y = project(act, w_down, Tensor(), opt(residual));
+    at::DimVector lead(x.sizes().begin(), x.sizes().end() - 1);
+    ctx->saved_data["lead"] = at::IntArrayRef(lead).vec();
+    ctx->saved_data["residual"] = residual.has_value();
+    ctx->save_for_backward({x2, w_up, w_down, gu, act});
+    return y.view(with_last(lead, w_down.size(0)));
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x2 = saved[0], &w_up = saved[1], &w_down = saved[2], &act = saved[4], &dy = grads[0];
+    const Tensor gu = ready(saved[3]);
+    const Tensor dy2 = dy.reshape({-1, w_down.size(0)}).contiguous();
+    Tensor da = input_grad(dy2, w_down);
+    Tensor dw_down = weight_grad(w_down, dy2, act);
+    const Tensor dgu = at::empty_like(gu);
+    launched(K.gv_swiglu_bwd(cptr(da), cptr(gu), ptr(dgu), gu.size(0), static_cast<int>(gu.size(1) / 2), stream()), "gv_swiglu_bwd");
+    da.reset();
+    const auto lead = ctx->saved_data["lead"].toIntVector();
+    Tensor dx = input_grad(dgu, w_up).view(with_last(at::DimVector(lead.begin(), lead.end()), w_up.size(1)));
+    Tensor dw_up = weight_grad(w_up, dgu, x2);
+    return {dx, dw_up, dw_down, ctx->saved_data["residual"].toBool() ? dy : Tensor()};
+  }
+};
+
+py::object swiglu_mlp(const Tensor& x, const Tensor& w_up, const Tensor& w_down, const OptTensor& residual) {
+  if (!linear_ok(x, w_up, std::nullopt, std::nullopt) || !weight_ok(w_down) || w_up.size(0) % 256 != 0 || w_down.size(1) * 2 != w_up.size(0) ||
+      !add_on_ok(residual, x.numel() / x.size(-1) * w_down.size(0)))
+    return py::none();
+  return py::cast(no_gil([&] { return SwiGLUMLPFn::apply(x, w_up, w_down, residual); }));
+}
+
+struct LinearGeluFn : Function<LinearGeluFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& W, const OptTensor& bias) {
+    const Tensor x2 = flat2d(x);
+    const Tensor act = empty16({x2.size(0), W.size(0)}, x2), up = empty16({x2.size(0), W.size(0)}, x2);
+    gemm_into(x2, false, W, false, up, false, opt(bias), Tensor(), nullptr, Tensor(), act);
+    at::DimVector lead(x.sizes().begin(), x.sizes().end() - 1);
+    ctx->saved_data["lead"] = at::IntArrayRef(lead).vec();
+    ctx->save_for_backward({x2, W, opt(bias), up});
+    return act.view(with_last(lead, W.size(0)));
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x2 = saved[0], &W = saved[1], &bias = saved[2];
+    const Tensor up = ready(saved[3]), dact = ready(grads[0]);
+    const Tensor dy = at::empty_like(up);
+    launched(K.gv_gelu_bwd(cptr(dact), cptr(up), ptr(dy), up.numel(), stream()), "gv_gelu_bwd");
+    Tensor dx, db;
+    if (ctx->needs_input_grad(0)) {
+      const auto lead = ctx->saved_data["lead"].toIntVector();
+      dx = input_grad(dy, W).view(with_last(at::DimVector(lead.begin(), lead.end()), W.size(1)));
+    }
+    Tensor dW = weight_grad(W, dy, x2);
+    if (bias.defined()) db = bias_grad(bias, dy);
+    return {dx, dW, db};
+  }
+};
+
+py::object linear_gelu(const Tensor& x, const Tensor& W, const OptTensor& bias) {
+  if (!linear_ok(x, W, bias, std::nullopt)) return py::none();
+  return py::cast(no_gil([&] { return LinearGeluFn::apply(x, W, bias); }));
+}
+
+// ------------------------------------------------------------------ norms
+struct NormShape { int rows, cols; };
+NormShape norm_shape(const Tensor& x) { return {static_cast<int>(x.numel() / x.size(-1)), static_cast<int>(x.size(-1))}; }
+Tensor norm_scratch(const NormShape& n, bool layer, const Tensor& like) {
+  return empty32({std::max<int64_t>(K.gv_norm_bwd_scratch_elems(n.rows, n.cols, layer), 1)}, like);
+}
+
+struct RMSNorm {
+  static Tensor fwd(const Tensor& x_, const Tensor& w, double eps, Tensor& rstd) {
+    const Tensor x = x_.contiguous(), y = at::empty_like(x);
+    const NormShape n = norm_shape(x);
+    rstd = empty32({n.rows}, x);
+    launched(K.gv_rmsnorm_fwd(cptr(x), nullptr, cptr(w), ptr(y), nullptr, static_cast<float*>(ptr(rstd)), n.rows, n.cols, static_cast<float>(eps), stream()),
+             "gv_rmsnorm_fwd");
+    return y;
+  }
+  static variable_list bwd(const variable_list& saved, const Tensor& dy_, const Tensor& dres_) {
+    const Tensor x = ready(saved[0]), dy = dy_.contiguous(), dres = dres_.defined() ? dres_.contiguous() : Tensor(), &w = saved[1], &rstd = saved[2];
+    const NormShape n = norm_shape(x);
+    const Tensor dx = at::empty_like(x), scratch = norm_scratch(n, false, x);
+    Tensor dw = vector_grad(w, [&](const Tensor& buf) {
+      launched(K.gv_rmsnorm_bwd(cptr(dy), cptr(x), cptr(w), static_cast<const float*>(cptr(rstd)), cptr(dres), ptr(dx), static_cast<float*>(ptr(buf)),
+                                static_cast<float*>(ptr(scratch)), scratch.numel(), n.rows, n.cols, stream()),
+               "gv_rmsnorm_bwd", 2);
+    });
+    return {dx, dw};
+  }
+};
+
+struct RMSNormFn : Function<RMSNormFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, double eps) {
+    Tensor rstd, y = RMSNorm::fwd(x, w, eps, rstd);
+    ctx->save_for_backward({x, w, rstd});
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    variable_list g = RMSNorm::bwd(ctx->get_saved_variables(), grads[0], Tensor());
+    return {g[0], g[1], Tensor()};
+  }
+};
+
+// (norm(x), x): the gradient of the second output is added in the backward kernel.
+struct RMSNormBranchFn : Function<RMSNormBranchFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, double eps) {
+    Tensor rstd, y = RMSNorm::fwd(x, w, eps, rstd);
+    ctx->save_for_backward({x, w, rstd});
+    ctx->set_materialize_grads(false);
+    return {y, x.view_as(x)};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    if (!grads[0].defined()) return {grads[1], Tensor(), Tensor()};
+    variable_list g = RMSNorm::bwd(ctx->get_saved_variables(), grads[0], grads[1]);
+    return {g[0], g[1], Tensor()};
+  }
+};
+
+struct LayerNorm {
+  static Tensor fwd(const Tensor& x_, const Tensor& w, const Tensor& b, double eps, Tensor& mean, Tensor& rstd) {
+    const Tensor x = x_.contiguous(), y = at::empty_like(x);
+    const NormShape n = norm_shape(x);
+    mean = empty32({n.rows}, x);
+    rstd = empty32({n.rows}, x);
+    launched(K.gv_layernorm_fwd(cptr(x), nullptr, cptr(w), cptr(b), ptr(y), nullptr, static_cast<float*>(ptr(mean)), static_cast<float*>(ptr(rstd)), n.rows,
+                                n.cols, static_cast<float>(eps), stream()),
+             "gv_layernorm_fwd");
+    return y;
+  }
+  static variable_list bwd(const variable_list& saved, const Tensor& dy_, const Tensor& dres_) {
+    const Tensor x = ready(saved[0]), dy = dy_.contiguous(), dres = dres_.defined() ? dres_.contiguous() : Tensor();
+    const Tensor &w = saved[1], &b = saved[2], &mean = saved[3], &rstd = saved[4];
+    const NormShape n = norm_shape(x);
+    const Tensor dx = at::empty_like(x), scratch = norm_scratch(n, true, x);
+    auto run = [&](const Tensor& dw, const Tensor& db) {
+      launched(K.gv_layernorm_bwd(cptr(dy), cptr(x), cptr(w), static_cast<const float*>(cptr(mean)), static_cast<const float*>(cptr(rstd)), cptr(dres), ptr(dx),
+                                  static_cast<float*>(ptr(dw)), static_cast<float*>(ptr(db)), static_cast<float*>(ptr(scratch)), scratch.numel(), n.rows,
+                                  n.cols, stream()),
+               "gv_layernorm_bwd", 2);
+    };
+    Tensor mw, mb;
+    bool hooked = false;
+    {
+      py::gil_scoped_acquire gil;
+      Buffer bw = buffer_of(w), bb = buffer_of(b);
+      mw = bw.main_grad; mb = bb.main_grad;
+      hooked = bw.hook || bb.hook;
+    }
+    if (mw.defined() && mb.defined() && mw.scalar_type() == at::kFloat && mb.scalar_type() == at::kFloat) {
+      run(mw.view({-1}), mb.view({-1}));
+      if (hooked) {
+        py::gil_scoped_acquire gil;
+        for (const Tensor& p : {w, b}) {
+          Buffer buf = buffer_of(p);
+          accumulated(buf);
+        }
+      }
+      return {dx, Tensor(), Tensor()};
+    }
+    const Tensor dwb = at::zeros({2, w.numel()}, w.options().dtype(at::kFloat));
+    run(dwb[0], dwb[1]);
+    Tensor dw = vector_grad(w, [&](const Tensor& buf) { buf.add_(dwb[0]); });
+    Tensor db = vector_grad(b, [&](const Tensor& buf) { buf.add_(dwb[1]); });
+    return {dx, dw, db};
+  }
+};
+
+struct LayerNormFn : Function<LayerNormFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& b, double eps) {
+    Tensor mean, rstd, y = LayerNorm::fwd(x, w, b, eps, mean, rstd);
+    ctx->save_for_backward({x, w, b, mean, rstd});
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    variable_list g = LayerNorm::bwd(ctx->get_saved_variables(), grads[0], Tensor());
+    return {g[0], g[1], g[2], Tensor()};
+  }
+};
+
+struct LayerNormBranchFn : Function<LayerNormBranchFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& b, double eps) {
+    Tensor mean, rstd, y = LayerNorm::fwd(x, w, b, eps, mean, rstd);
+    ctx->save_for_backward({x, w, b, mean, rstd});
+    ctx->set_materialize_grads(false);
+    return {y, x.view_as(x)};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    if (!grads[0].defined()) return {grads[1], Tensor(), Tensor(), Tensor()};
+    variable_list g = LayerNorm::bwd(ctx->get_saved_variables(), grads[0], grads[1]);
+    return {g[0], g[1], g[2], Tensor()};
+  }
+};
+
+bool norm_ok(const Tensor& x, const Tensor& w) {
+  return plain_mode() && input_ok(x) && x.size(-1) % 8 == 0 && x.size(-1) <= 8192 && aligned(x) && plain16(w) && w.is_contiguous() && aligned(w) &&
+         w.numel() == x.size(-1);
+}
+
+py::object rmsnorm(const Tensor& x, const Tensor& w, double eps, bool branch) {
+  if (!norm_ok(x, w)) return py::none();
+  const variable_list out = no_gil([&] { return branch ? RMSNormBranchFn::apply(x, w, eps) : variable_list{RMSNormFn::apply(x, w, eps)}; });
+  return branch ? py::object(py::make_tuple(out[0], out[1])) : py::cast(out[0]);
+}
+
+py::object layernorm(const Tensor& x, const Tensor& w, const Tensor& b, double eps, bool branch) {
+  if (!norm_ok(x, w) || !norm_ok(x, b)) return py::none();
+  const variable_list out = no_gil([&] { return branch ? LayerNormBranchFn::apply(x, w, b, eps) : variable_list{LayerNormFn::apply(x, w, b, eps)}; });
+  return branch ? py::object(py::make_tuple(out[0], out[1])) : py::cast(out[0]);
+}
+
+// ------------------------------------------------------------------ attention
+struct Dropout { double p = 0.0; unsigned long long seed = 0; int head_offset = 0; };
+
+struct Heads {                             // one of q, k, v, o: address, strides of batch, sequence and head in elements
+  const void* at;
+  long long b, s, h;
+};
+Heads heads_of(const Tensor& t) { return {cptr(t), t.stride(0), t.stride(1), t.stride(2)}; }
+Heads heads_at(const Tensor& t, int64_t offset, long long b, long long s, long long h) {
+  return {static_cast<const char*>(cptr(t)) + 2 * offset, b, s, h};
+}
+
+gv_attn_args attention_args(const Heads& q, const Heads& k, const Heads& v, const Heads& o, const Tensor& lse, int b, int sq, int sk, int hq, int hk, int dh,
+                            bool causal, double scale, const Tensor& lens, const Dropout& drop) {
+  gv_attn_args a = {};
+  a.q = q.at; a.k = k.at; a.v = v.at; a.o = const_cast<void*>(o.at); a.lse = static_cast<float*>(ptr(lse));
+  a.b = b; a.sq = sq; a.sk = sk; a.hq = hq; a.hk = hk; a.dh = dh;
+  a.q_stride_b = q.b; a.q_stride_s = q.s; a.q_stride_h = q.h;
+  a.k_stride_b = k.b; a.k_stride_s = k.s; a.k_stride_h = k.h;
+  a.v_stride_b = v.b; a.v_stride_s = v.s; a.v_stride_h = v.h;
+  a.o_stride_b = o.b; a.o_stride_s = o.s; a.o_stride_h = o.h;
+  a.causal = causal; a.scale = static_cast<float>(scale);
+  a.kv_lens = static_cast<const int*>(cptr(lens));
+  if (drop.p > 0.0) { a.dropout_p = static_cast<float>(drop.p); a.dropout_seed = drop.seed; a.dropout_head_offset = drop.head_offset; }
+  return a;
+}
+void set_grads(gv_attn_args& a, const Heads& dout, const Heads& dq, const Heads& dk, const Heads& dv, const Tensor& dq_accum, const Tensor& delta) {
+  a.dout = dout.at; a.dq = const_cast<void*>(dq.at); a.dk = const_cast<void*>(dk.at); a.dv = const_cast<void*>(dv.at);
+  a.dq_accum = static_cast<float*>(ptr(dq_accum)); a.delta = static_cast<float*>(ptr(delta));
+  a.do_stride_b = dout.b; a.do_stride_s = dout.s; a.do_stride_h = dout.h;
+  a.dq_stride_b = dq.b; a.dq_stride_s = dq.s; a.dq_stride_h = dq.h;
+  a.dk_stride_b = dk.b; a.dk_stride_s = dk.s; a.dk_stride_h = dk.h;
+  a.dv_stride_b = dv.b; a.dv_stride_s = dv.s; a.dv_stride_h = dv.h;
+}
+Tensor lengths(const OptTensor& lens, const Tensor& like) {
+  return lens.has_value() ? lens->to(like.options().dtype(at::kInt)).contiguous() : Tensor();
+}
+
+void keep_dropout(AutogradContext* ctx, const Dropout& d) {
+  ctx->saved_data["p"] = d.p;
+  ctx->saved_data["seed"] = static_cast<int64_t>(d.seed);
+  ctx->saved_data["off"] = static_cast<int64_t>(d.head_offset);
+}
+Dropout kept_dropout(AutogradContext* ctx) {
+  return {ctx->saved_data["p"].toDouble(), static_cast<unsigned long long>(ctx->saved_data["seed"].toInt()), static_cast<int>(ctx->saved_data["off"].toInt())};
+}
+
+// Packed projection [s * b, (hq + 2 hk) dh] in sequence-major order; q and k are rotated already where `rope` is set.
+struct Packed {
+  int batch, hq, hk, dh;
+  bool causal, rope;
+  int pos_offset;
+  double scale;
+  int64_t width() const { return static_cast<int64_t>(hq + 2 * hk) * dh; }
+  Heads q(const Tensor& t) const { return heads_at(t, 0, width(), batch * width(), dh); }
+  Heads k(const Tensor& t) const { return heads_at(t, static_cast<int64_t>(hq) * dh, width(), batch * width(), dh); }
+  Heads v(const Tensor& t) const { return heads_at(t, static_cast<int64_t>(hq + hk) * dh, width(), batch * width(), dh); }
+  Heads o(const Tensor& t) const { return heads_at(t, 0, static_cast<long long>(hq) * dh, static_cast<long long>(batch) * hq * dh, dh); }
+};
+
+struct PackedAttentionFn : Function<PackedAttentionFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& qkv_, const OptTensor& inv_freq, const OptTensor& lens_, const Packed& c, const Dropout& drop) {
+    const Tensor qkv = ready(qkv_), lens = lengths(lens_, qkv_);
+    const int64_t tokens = qkv.size(0);
+    const int s = static_cast<int>(tokens / c.batch);
+    const Tensor o = empty16({s, c.batch, c.hq, c.dh}, qkv), lse = empty32({c.batch, c.hq, s}, qkv);
+    const gv_attn_args a = attention_args(c.q(qkv), c.k(qkv), c.v(qkv), c.o(o), lse, c.batch, s, s, c.hq, c.hk, c.dh, c.causal, c.scale, lens, drop);
+    launched(K.gv_attn_fwd(&a, stream()), "gv_attn_fwd");
+    ctx->saved_data["cfg"] = std::vector<int64_t>{c.batch, c.hq, c.hk, c.dh, c.causal, c.rope, c.pos_offset};
+    ctx->saved_data["scale"] = c.scale;
+    keep_dropout(ctx, drop);
+    ctx->save_for_backward({qkv, o, lse, opt(inv_freq), lens});
+    return o.view({tokens, static_cast<int64_t>(c.hq) * c.dh});
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor qkv = ready(saved[0]), o = ready(saved[1]), dout = ready(grads[0]), &lse = saved[2], &inv_freq = saved[3], &lens = saved[4];
+    const auto n = ctx->saved_data["cfg"].toIntVector();
+    const Packed c = {static_cast<int>(n[0]), static_cast<int>(n[1]), static_cast<int>(n[2]), static_cast<int>(n[3]), n[4] != 0, n[5] != 0,
+                      static_cast<int>(n[6]), ctx->saved_data["scale"].toDouble()};
+    const int64_t tokens = qkv.size(0);
+    const int s = static_cast<int>(tokens / c.batch);
+    const Tensor dqkv = at::empty_like(qkv), dq_accum = empty32({c.batch, s, c.hq, c.dh}, qkv), delta = empty32({c.batch, c.hq, s}, qkv);
+    gv_attn_args a = attention_args(c.q(qkv), c.k(qkv), c.v(qkv), c.o(o), lse, c.batch, s, s, c.hq, c.hk, c.dh, c.causal, c.scale, lens, kept_dropout(ctx));
+    set_grads(a, c.o(dout), c.q(dqkv), c.k(dqkv), c.v(dqkv), dq_accum, delta);
+    if (c.rope) { a.dq_rope_inv_freq = static_cast<const float*>(cptr(inv_freq)); a.dq_rope_pos_offset = c.pos_offset; }
+    launched(K.gv_attn_bwd(&a, stream()), "gv_attn_bwd", 3);
+    if (c.rope)
+      launched(K.gv_rope(const_cast<void*>(c.k(dqkv).at), nullptr, static_cast<const float*>(cptr(inv_freq)), tokens, c.hk, c.dh, c.width(), c.batch, 0,
+                         c.pos_offset, 1, stream()),
+               "gv_rope");
+    return {dqkv, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+py::object packed_attention(const Tensor& qkv, int batch, int hq, int hk, int dh, bool causal, bool rope, int pos_offset, std::optional<double> scale,
+                            const OptTensor& inv_freq, const OptTensor& kv_lens, double p, unsigned long long seed, int head_offset) {
+  if (!plain_mode() || !input_ok(qkv) || qkv.dim() != 2 || batch <= 0 || hk <= 0 || hq % hk != 0 || dh % 8 != 0 || dh > 128 || dh <= 0 ||
+      qkv.size(0) % batch != 0 || qkv.size(1) != static_cast<int64_t>(hq + 2 * hk) * dh || (kv_lens.has_value() && (!plain(*kv_lens) || kv_lens->numel() != batch)))
+    return py::none();
+  if (rope && (dh % 16 != 0 || !inv_freq.has_value() || !plain(*inv_freq) || inv_freq->scalar_type() != at::kFloat || !inv_freq->is_contiguous() ||
+               inv_freq->numel() != dh / 2))
+    return py::none();
+  const Packed c = {batch, hq, hk, dh, causal, rope, pos_offset, scale.has_value() ? *scale : 1.0 / std::sqrt(static_cast<double>(dh))};
+  return py::cast(no_gil([&] { return PackedAttentionFn::apply(qkv, inv_freq, kv_lens, c, Dropout{p, seed, head_offset}); }));
+}
+
+bool heads_ok(const Tensor& t) {
+  return plain16(t) && t.dim() == 4 && t.numel() > 0 && t.stride(3) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 && t.stride(2) % 8 == 0 && aligned(t);
+}
+Tensor heads_ready(const Tensor& t) { return heads_ok(t) ? t : ready(t); }
+
+struct AttentionFn : Function<AttentionFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& lens_, bool causal, double scale,
+                               const Dropout& drop) {
+    const int b = q.size(0), sq = q.size(1), hq = q.size(2), dh = q.size(3), sk = k.size(1), hk = k.size(2);
+    const Tensor o = empty16({b, sq, hq, dh}, q), lse = empty32({b, hq, sq}, q), lens = lengths(lens_, q);
+    const gv_attn_args a = attention_args(heads_of(q), heads_of(k), heads_of(v), heads_of(o), lse, b, sq, sk, hq, hk, dh, causal, scale, lens, drop);
+    launched(K.gv_attn_fwd(&a, stream()), "gv_attn_fwd");
+    ctx->saved_data["causal"] = causal;
+    ctx->saved_data["scale"] = scale;
+    keep_dropout(ctx, drop);
+    ctx->save_for_backward({q, k, v, o, lse, lens});
+    ctx->mark_non_differentiable({lse});
+    ctx->set_materialize_grads(false);
+    return {o, lse};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    if (!grads[0].defined()) return variable_list(7);
+    const auto saved = ctx->get_saved_variables();
+    const Tensor q = heads_ready(saved[0]), k = heads_ready(saved[1]), v = heads_ready(saved[2]), o = heads_ready(saved[3]), dout = heads_ready(grads[0]);
+    const Tensor &lse = saved[4], &lens = saved[5];
+    const int b = q.size(0), sq = q.size(1), hq = q.size(2), dh = q.size(3), sk = k.size(1), hk = k.size(2);
+    const Tensor dq = empty16({b, sq, hq, dh}, q), dk = empty16({b, sk, hk, dh}, q), dv = empty16({b, sk, hk, dh}, q);
+    const Tensor dq_accum = empty32({b, sq, hq, dh}, q), delta = empty32({b, hq, sq}, q);
+    gv_attn_args a = attention_args(heads_of(q), heads_of(k), heads_of(v), heads_of(o), lse, b, sq, sk, hq, hk, dh, ctx->saved_data["causal"].toBool(),
+                                    ctx->saved_data["scale"].toDouble(), lens, kept_dropout(ctx));
+    set_grads(a, heads_of(dout), heads_of(dq), heads_of(dk), heads_of(dv), dq_accum, delta);
+    launched(K.gv_attn_bwd(&a, stream()), "gv_attn_bwd", 3);
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+py::object attention(const Tensor& q, const Tensor& k, const Tensor& v, bool causal, std::optional<double> scale, const OptTensor& kv_lens, double p,
+                     unsigned long long seed, int head_offset) {
+  if (!plain_mode() || !heads_ok(q) || !heads_ok(k) || !heads_ok(v) || q.size(3) % 8 != 0 || q.size(3) > 128 || k.size(3) != q.size(3) || v.sizes() != k.sizes() ||
+      k.size(0) != q.size(0) || q.size(2) % k.size(2) != 0 || (kv_lens.has_value() && (!plain(*kv_lens) || kv_lens->numel() != q.size(0))))
+    return py::none();
+  const double sc = scale.has_value() ? *scale : 1.0 / std::sqrt(static_cast<double>(q.size(3)));
+  const variable_list out = no_gil([&] { return AttentionFn::apply(q, k, v, kv_lens, causal, sc, Dropout{p, seed, head_offset}); });
+  return py::make_tuple(out[0], out[1]);
+}
+
+// ------------------------------------------------------------------ language-model head
+gv_gemm_args head_args(const Tensor& x, const Tensor& W, const Tensor& C) {
+  gv_gemm_args g = {};
+  g.A = cptr(x); g.B = cptr(W); g.C = ptr(C);
+  g.M = static_cast<int>(x.size(0)); g.N = static_cast<int>(W.size(0)); g.K = static_cast<int>(x.size(1));
+  g.lda = static_cast<int>(x.stride(0)); g.ldb = static_cast<int>(W.stride(0)); g.ldc = C.defined() ? static_cast<int>(C.stride(0)) : g.N;
+  g.alpha = 1.f;
+  return g;
+}
+
+struct LMHeadLossFn : Function<LMHeadLossFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& W, const Tensor& labels_, int64_t vocab_start, int64_t ignore_index) {
+    const Tensor x2 = flat2d(x), labels = labels_.reshape({-1}).to(at::kLong).contiguous();
+    const int64_t M = x2.size(0), N = W.size(0), tiles = (N + 255) / 256;
+    const Tensor stats = empty32({M, tiles, 2}, x2), rows = empty32({3, M}, x2), lse = empty32({M}, x2), loss = empty32({M}, x2);
+    float* r = static_cast<float*>(ptr(rows));                  // max, sum, target
+    gv_xent_args xa = {};
+    xa.mode = 1; xa.labels = static_cast<const long long*>(cptr(labels)); xa.vocab_start = vocab_start; xa.ignore_index = ignore_index;
+    xa.stats = static_cast<float*>(ptr(stats)); xa.target = r + 2 * M;
+    const gv_gemm_args g = head_args(x2, W, Tensor());
+    launched(K.gv_gemm_xent(&g, &xa, stream()), "gv_gemm_xent(stats)");
+    launched(K.gv_xent_merge(static_cast<const float*>(cptr(stats)), static_cast<int>(tiles), xa.labels, vocab_start, N, ignore_index, r, r + M, r + 2 * M,
+                             static_cast<float*>(ptr(lse)), static_cast<float*>(ptr(loss)), M, stream()),
+             "gv_xent_merge");
+    ctx->saved_data["sizes"] = x.sizes().vec();
+    ctx->saved_data["start"] = vocab_start;
+    ctx->saved_data["ignore"] = ignore_index;
+    ctx->save_for_backward({x2, W, labels, lse});
+    return loss;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor x2 = row_major(saved[0]), W = row_major(saved[1]), labels = saved[2].contiguous(), lse = saved[3].contiguous();
+    const Tensor dloss = grads[0].reshape({-1}).to(at::kFloat).contiguous();
+    const Tensor dlog = empty16({x2.size(0), W.size(0)}, x2);
+    gv_xent_args xa = {};
+    xa.mode = 2; xa.labels = static_cast<const long long*>(cptr(labels));
+    xa.vocab_start = ctx->saved_data["start"].toInt(); xa.ignore_index = ctx->saved_data["ignore"].toInt();
+    xa.lse = static_cast<const float*>(cptr(lse)); xa.gscale = static_cast<const float*>(cptr(dloss));
+    const gv_gemm_args g = head_args(x2, W, dlog);
+    launched(K.gv_gemm_xent(&g, &xa, stream()), "gv_gemm_xent(grad)");
+    Tensor dx = input_grad(dlog, W).view(ctx->saved_data["sizes"].toIntVector());
+    Tensor dW = weight_grad(saved[1], dlog, x2);
+    return {dx, dW, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+py::object lm_head_loss(const Tensor& x, const Tensor& W, const Tensor& labels, int64_t vocab_start, int64_t ignore_index) {
+  if (!plain_mode() || !input_ok(x) || !weight_ok(W) || x.size(-1) != W.size(1) || !plain(labels) || labels.numel() * x.size(-1) != x.numel()) return py::none();
+  const Tensor x2 = flat2d(x.detach());
+  if (!rows_ok(x2)) return py::none();
+  return py::cast(no_gil([&] { return LMHeadLossFn::apply(x, W, labels, vocab_start, ignore_index); }));
+}
+
+// Python sees the nodes under the names that the Python Functions' nodes have.
+template <class Fn>
+void name_node(const char* name) {
+  using namespace torch::autograd;
+  static PyGetSetDef properties[] = {THP_FUNCTION_DEFAULT_PROPERTIES, {nullptr, nullptr, nullptr, nullptr, nullptr}};
+  static PyTypeObject type;
+  _initFunctionPyTypeObject(type, name, properties, nullptr);
+  registerCppFunction(typeid(CppNode<Fn>), &type);
+}
+
+void init(const py::dict& addresses, py::object wgrad, py::object vecgrad, py::object no_scratch, py::object error) {
+#define X(name) K.name = reinterpret_cast<decltype(K.name)>(addresses[#name].cast<uintptr_t>());
+  GV_ENTRIES(X)
+#undef X
+  g_wgrad = new py::object(std::move(wgrad));
+  g_vecgrad = new py::object(std::move(vecgrad));
+  g_no_scratch = new py::object(std::move(no_scratch));
+  g_error = new py::object(std::move(error));
+  g_main_grad = PyUnicode_InternFromString("main_grad");
+  g_hook = PyUnicode_InternFromString("grad_ready_hook");
+  name_node<LinearFn>("LinearFnBackward");
+  name_node<SwiGLUMLPFn>("SwiGLUMLPFnBackward");
+  name_node<LinearGeluFn>("LinearGeluFnBackward");
+  name_node<RMSNormFn>("RMSNormFnBackward");
+  name_node<RMSNormBranchFn>("RMSNormBranchFnBackward");
+  name_node<LayerNormFn>("LayerNormFnBackward");
+  name_node<LayerNormBranchFn>("LayerNormBranchFnBackward");
+  name_node<PackedAttentionFn>("PackedAttentionFnBackward");
+  name_node<AttentionFn>("AttentionFnBackward");
+  name_node<LMHeadLossFn>("LMHeadLossFnBackward");
+}
+
+}  // namespace
+
+PYBIND11_MODULE(torch_ops, m) {
+  m.doc() = "C++ autograd Functions of the un-sharded hot path";
+  m.def("init", &init);
+  m.def("launch_count", [] { return g_launches.load(std::memory_order_relaxed); });
+  m.def("no_scratch_for", [](int device, int M, int N, int K_) {
+    std::lock_guard<std::mutex> lock(g_no_scratch_lock);
+    g_no_scratch_products.insert(std::make_tuple(device, M, N, K_));
+  });
+  m.def("linear", torch::wrap_pybind_function(linear));
+  m.def("swiglu_mlp", torch::wrap_pybind_function(swiglu_mlp));
+  m.def("linear_gelu", torch::wrap_pybind_function(linear_gelu));
+  m.def("rmsnorm", torch::wrap_pybind_function(rmsnorm));
+  m.def("layernorm", torch::wrap_pybind_function(layernorm));
+  m.def("packed_attention", torch::wrap_pybind_function(packed_attention));
+  m.def("attention", torch::wrap_pybind_function(attention));
+  m.def("lm_head_loss", torch::wrap_pybind_function(lm_head_loss));
+}

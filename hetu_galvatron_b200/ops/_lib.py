@@ -7,6 +7,7 @@ PyTorch kernels for bf16 CUDA tensors.
 from __future__ import annotations
 
 import ctypes
+import threading
 from ctypes import POINTER, Structure, c_float, c_int, c_longlong, c_uint, c_ulonglong, c_void_p
 
 import torch
@@ -127,6 +128,12 @@ class PadHeadsArgs(Structure):
 PROTOTYPES["gv_pad_heads"] = [POINTER(PadHeadsArgs), _I, _P]
 
 
+# what csrc/torch_ops.cpp calls
+TORCH_OPS_ENTRIES = ("gv_gemm_bf16", "gv_gemm_xent", "gv_gemm_workspace_bytes", "gv_xent_merge", "gv_rmsnorm_fwd", "gv_rmsnorm_bwd",
+                     "gv_layernorm_fwd", "gv_layernorm_bwd", "gv_norm_bwd_scratch_elems", "gv_rope", "gv_swiglu_bwd", "gv_gelu_bwd",
+                     "gv_colsum_accum", "gv_attn_fwd", "gv_attn_bwd")
+
+
 def available() -> bool:
     """True when the kernel library can be used (a CUDA device is present)."""
     return torch.cuda.is_available()
@@ -154,8 +161,30 @@ def lib():
     return _LIB
 
 
+_TORCH_OPS = None
+_TORCH_OPS_LOCK = threading.Lock()
+
+
+def torch_ops():
+    """The C++ autograd Functions (csrc/torch_ops.cpp), on the same kernel library as ``lib()``; on a machine with a GPU a module that
+    cannot be built is an error."""
+    global _TORCH_OPS
+    if _TORCH_OPS is None:
+        with _TORCH_OPS_LOCK:
+            if _TORCH_OPS is None:
+                import importlib
+
+                autograd, gemm = (importlib.import_module("." + n, __package__) for n in ("autograd", "gemm"))
+                mod = _build.load_pybind("torch_ops")
+                cdll = object.__getattribute__(lib(), "_cdll")
+                mod.init({n: ctypes.cast(getattr(cdll, n), c_void_p).value for n in TORCH_OPS_ENTRIES}, autograd._wgrad, autograd._vec_grad_of_sum,
+                         gemm._scratch_did_not_fit, KernelError)
+                _TORCH_OPS = mod
+    return _TORCH_OPS
+
+
 def launch_count() -> int:
-    return LAUNCH_COUNT
+    return LAUNCH_COUNT + (0 if _TORCH_OPS is None else _TORCH_OPS.launch_count())
 
 
 def stream_ptr() -> int:

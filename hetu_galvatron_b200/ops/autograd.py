@@ -29,6 +29,7 @@ from typing import Any, Optional
 import torch
 
 from ..parallel import collectives as C
+from . import _lib
 from . import functional as Fn
 from .gemm import (gelu_epilogue_supported, gemm, head_xent_grad, head_xent_loss, head_xent_stats, head_xent_supported,
                    swiglu_epilogue_supported)
@@ -70,6 +71,16 @@ def _vec_grad(p: torch.Tensor, fill_accum):
         return tmp.to(p.dtype).view(p.shape)
 
     return _accum_param_grad(p, into, fresh)
+
+
+def _vec_grad_of_sum(p: torch.Tensor, total: torch.Tensor):
+    """``_vec_grad`` of a gradient that has been summed already (fp32)."""
+    return _vec_grad(p, lambda buf: buf.add_(total))
+
+
+# Un-sharded bf16 CUDA operands take the C++ Functions of csrc/torch_ops.cpp, which are the Functions below with less host time between
+# the same launches. They return None for operands that they do not take.
+_native = _lib.torch_ops
 
 
 @dataclass(frozen=True)
@@ -166,6 +177,10 @@ def linear(x, W, bias=None, residual=None, cfg: LinearCfg = LinearCfg(), rope=No
     """``rope`` (a ``gemm.RopeEpilogue``): the projection's epilogue rotates its q / k head columns. This Function's
     backward treats the rotated output as its output, so the consumer's backward must hand back the gradient with the
     inverse rotation applied (``PackedAttentionFn`` does, for ``AttnCfg.rope`` with ``rope_applied``)."""
+    if x.is_cuda and (cfg.mode == "plain" or C.group_size(cfg.group) == 1) and (rope is None or rope.positions is None):
+        y = _native().linear(x, W, bias, residual, None if rope is None else (rope.cols, rope.dh, rope.inv_freq, rope.pos_div, rope.pos_offset))
+        if y is not None:
+            return y
     return LinearFn.apply(x, W, bias, residual, cfg, rope)
 
 
@@ -261,6 +276,10 @@ class SwiGLUMLPFn(torch.autograd.Function):
 
 
 def swiglu_mlp(x, w_up, w_down, residual=None):
+    if x.is_cuda:
+        y = _native().swiglu_mlp(x, w_up, w_down, residual)
+        if y is not None:
+            return y
     return SwiGLUMLPFn.apply(x, w_up, w_down, residual)
 
 
@@ -307,7 +326,8 @@ class LinearGeluFn(torch.autograd.Function):
 def linear_gelu(x, W, bias=None, cfg: LinearCfg = LinearCfg()):
     """gelu(linear(x)): in one kernel for un-sharded layers of bf16 CUDA operands, else one after the other."""
     if (cfg.mode == "plain" or C.group_size(cfg.group) == 1) and gelu_epilogue_supported(x, W, bias):
-        return LinearGeluFn.apply(x, W, bias)
+        y = _native().linear_gelu(x, W, bias)
+        return LinearGeluFn.apply(x, W, bias) if y is None else y
     return gelu(linear(x, W, bias, None, cfg))
 
 
@@ -332,6 +352,10 @@ class RMSNormFn(torch.autograd.Function):
 
 
 def rmsnorm(x, w, eps: float = 1e-5):
+    if x.is_cuda:
+        y = _native().rmsnorm(x, w, eps, False)
+        if y is not None:
+            return y
     return RMSNormFn.apply(x, w, eps)
 
 
@@ -363,6 +387,10 @@ class RMSNormBranchFn(torch.autograd.Function):
 
 
 def rmsnorm_branch(x, w, eps: float = 1e-5):
+    if x.is_cuda:
+        y = _native().rmsnorm(x, w, eps, True)
+        if y is not None:
+            return y
     return RMSNormBranchFn.apply(x, w, eps)
 
 
@@ -396,6 +424,10 @@ class LayerNormFn(torch.autograd.Function):
 
 
 def layernorm(x, w, b, eps: float = 1e-5):
+    if x.is_cuda:
+        y = _native().layernorm(x, w, b, eps, False)
+        if y is not None:
+            return y
     return LayerNormFn.apply(x, w, b, eps)
 
 
@@ -417,6 +449,10 @@ class LayerNormBranchFn(torch.autograd.Function):
 
 
 def layernorm_branch(x, w, b, eps: float = 1e-5):
+    if x.is_cuda:
+        y = _native().layernorm(x, w, b, eps, True)
+        if y is not None:
+            return y
     return LayerNormBranchFn.apply(x, w, b, eps)
 
 
@@ -504,6 +540,12 @@ class PackedAttentionFn(torch.autograd.Function):
 
 def packed_attention(qkv, cfg: AttnCfg, inv_freq=None, positions=None, kv_lens=None):
     """``kv_lens`` int [batch]: keys at or beyond kv_lens[b] are padding (the padding mask of encoder batches)."""
+    if qkv.is_cuda and (not cfg.rope or (cfg.rope_applied and positions is None)):
+        p, seed, head_offset = cfg.dropout or (0.0, 0, 0)
+        o = _native().packed_attention(qkv, cfg.batch, cfg.hq, cfg.hk, cfg.dh, cfg.causal, cfg.rope, cfg.pos_offset, cfg.scale, inv_freq, kv_lens,
+                                       p, seed & 0xFFFFFFFFFFFFFFFF, head_offset)
+        if o is not None:
+            return o
     return PackedAttentionFn.apply(qkv, inv_freq, positions, cfg, kv_lens)
 
 
@@ -526,6 +568,11 @@ class AttentionFn(torch.autograd.Function):
 
 
 def attention(q, k, v, causal: bool = True, scale: float | None = None, kv_lens=None, dropout=None):
+    if q.is_cuda:
+        p, seed, head_offset = dropout or (0.0, 0, 0)
+        out = _native().attention(q, k, v, causal, scale, kv_lens, p, seed & 0xFFFFFFFFFFFFFFFF, head_offset)
+        if out is not None:
+            return out
     return AttentionFn.apply(q, k, v, causal, scale, kv_lens, dropout)
 
 
@@ -715,4 +762,8 @@ class LMHeadLossFn(torch.autograd.Function):
 
 
 def lm_head_loss(x, W, labels, cfg: LossCfg = LossCfg()):
+    if x.is_cuda and not cfg.fp32_logits and C.group_size(cfg.group) == 1:
+        loss = _native().lm_head_loss(x, W, labels, cfg.vocab_start, cfg.ignore_index)
+        if loss is not None:
+            return loss
     return LMHeadLossFn.apply(x, W, labels, cfg)

@@ -65,9 +65,14 @@ def _split_scratch(M: int, N: int, K: int, device) -> "torch.Tensor | None":
     try:
         return torch.empty(need, dtype=torch.uint8, device=device)
     except torch.cuda.OutOfMemoryError:
-        _NO_SCRATCH.add((device.index, M, N, K))
-        warnings.warn("no room for %.0f MB of partial sums: products of %d x %d x %d run unsplit from now on" % (need / 1e6, M, N, K))
+        _scratch_did_not_fit(device.index, M, N, K, need)
         return None
+
+
+def _scratch_did_not_fit(device_index: int, M: int, N: int, K: int, need: int) -> None:
+    _NO_SCRATCH.add((device_index, M, N, K))
+    _lib.torch_ops().no_scratch_for(device_index, M, N, K)
+    warnings.warn("no room for %.0f MB of partial sums: products of %d x %d x %d run unsplit from now on" % (need / 1e6, M, N, K))
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,

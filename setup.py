@@ -1,5 +1,5 @@
-"""Packaging: ``pip install .`` builds the three native libraries in place (sm_100a CUDA kernel library, C++ search
-core, C++ dataset index builder) and installs ``hetu_galvatron_b200`` plus the ``galvatron`` import alias.
+"""Packaging: ``pip install .`` builds the native libraries in place (sm_100a CUDA kernel library, C++ search
+core, C++ dataset index builder, C++ autograd Functions) and installs ``hetu_galvatron_b200`` plus the ``galvatron`` import alias.
 
 The reference's setup (setup.py:39-96) compiles one pybind11 extension with setuptools; here the native build is the
 package's own ``_build`` module (nvcc / g++ called directly, stale builds detected by hash), run as part of ``build_py``

@@ -1,0 +1,281 @@
+"""The C++ autograd Functions against the Python Functions of the same operators: the same launches, so the same bits (dQ, which
+is summed in the order that blocks finish in, within fp32 rounding), for every form of operand that they take, and the Python
+Function for what they do not."""
+import pytest
+import torch
+
+from hetu_galvatron_b200.ops import _lib
+from hetu_galvatron_b200.ops import autograd as A
+from hetu_galvatron_b200.ops import functional as Fn
+from hetu_galvatron_b200.ops.gemm import RopeEpilogue
+
+pytestmark = pytest.mark.gpu
+
+
+def _t(*shape, scale=1.0, dtype=torch.bfloat16):
+    return (torch.randn(*shape, device="cuda") * scale).to(dtype)
+
+
+def _forms(t):
+    """The same values contiguous, in transposed storage, and as columns of a wider matrix."""
+    wide = torch.zeros(t.shape[0], t.shape[1] + 24, dtype=t.dtype, device=t.device)
+    wide[:, 8:-16] = t
+    return [t.clone(), t.t().contiguous().t(), wide[:, 8:-16]]
+
+
+def _grads(params, buffers):
+    out = []
+    for p in params:
+        mg = getattr(p, "main_grad", None)
+        out.append(p.grad if mg is None else mg.clone())
+        p.grad = None
+        if mg is not None:
+            mg.copy_(buffers[p])
+    return out
+
+
+def _buffers(params, kind):
+    start = {}
+    for p in params:
+        if kind is not None:
+            start[p] = torch.randn(p.shape, device="cuda").to(kind)
+            p.main_grad = start[p].clone()
+            p.calls = 0
+            p.grad_ready_hook = lambda q: setattr(q, "calls", q.calls + 1)
+    return start
+
+
+@pytest.mark.parametrize("grads", [None, torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("op", ["linear", "gelu"])
+@pytest.mark.parametrize("bias,residual", [(False, False), (True, True)])
+def test_projections(op, bias, residual, grads):
+    torch.manual_seed(0)
+    rows, n, k = 131, 264, 136
+    w = _t(n, k, scale=0.1).requires_grad_()
+    b = _t(n).requires_grad_() if bias else None
+    params = [p for p in (w, b) if p is not None]
+    start = _buffers(params, grads)
+    base, dy = _t(rows, k), _t(rows, n)
+    for form in _forms(base):
+        for lead in ((rows, k), (1, rows, k)):
+            for dform in _forms(dy):
+                got = []
+                for cpp in (True, False):
+                    x = form.detach().requires_grad_()
+                    r = dy.clone().requires_grad_() if residual else None
+                    h = x.view(lead) if form.is_contiguous() else x
+                    if op == "linear":
+                        y = A.linear(h, w, b, r) if cpp else A.LinearFn.apply(h, w, b, r, A.LinearCfg(), None)
+                    else:
+                        y = A.linear_gelu(h, w, b) if cpp else A.LinearGeluFn.apply(h, w, b)
+                    y.backward(dform.unsqueeze(0) if y.dim() == 3 else dform)
+                    got.append([y.detach(), x.grad, None if r is None or op == "gelu" else r.grad] + _grads(params, start))
+                for i, (a, c) in enumerate(zip(*got)):
+                    if a is None:
+                        assert c is None
+                    elif i < 4:
+                        assert torch.equal(a, c)
+                    else:                                  # the bias: fp32 sums over rows by atomic additions, then at most one rounding to bf16
+                        assert ((a - c).float().norm() / c.float().norm()).item() < 2.0 ** -9
+    if grads is not None:
+        assert all(p.calls > 0 for p in params)
+    assert _lib.read_error() is None
+
+
+def test_input_without_gradient_and_no_grad_mode():
+    x, w = _t(64, 128), _t(256, 128, scale=0.1).requires_grad_()
+    before = _lib.launch_count()
+    y = A.linear(x, w)
+    y.sum().backward()
+    assert _lib.launch_count() == before + 2                   # forward and weight gradient, no input gradient
+    with torch.no_grad():
+        z = A.linear(x, w)
+    assert torch.equal(y.detach(), z) and not z.requires_grad and z.grad_fn is None
+
+
+@pytest.mark.parametrize("dh", [64, 128])
+def test_rotary_projection(dh):
+    x, w = _t(96, 128).requires_grad_(), _t(4 * dh, 128, scale=0.1).requires_grad_()
+    inv = Fn.rope_inv_freq(dh, 10000.0, "cuda")
+    ep = RopeEpilogue(3 * dh, dh, inv, None, 2, 5)
+    got = []
+    for fn in (lambda: A.linear(x, w, rope=ep), lambda: A.LinearFn.apply(x, w, None, None, A.LinearCfg(), ep)):
+        y = fn()
+        got.append((y.detach(),) + torch.autograd.grad(y, (x, w), torch.ones_like(y)))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("grads", [None, torch.float32, torch.bfloat16])
+def test_gated_mlp(grads):
+    torch.manual_seed(1)
+    x, r = _t(3, 50, 136), _t(3, 50, 136)
+    up, down = _t(512, 136, scale=0.1).requires_grad_(), _t(136, 256, scale=0.1).requires_grad_()
+    start = _buffers([up, down], grads)
+    got = []
+    for fn in (A.swiglu_mlp, A.SwiGLUMLPFn.apply):
+        xi, ri = x.clone().requires_grad_(), r.clone().requires_grad_()
+        y = fn(xi, up, down, ri)
+        y.backward(x)
+        got.append([y.detach(), xi.grad, ri.grad] + _grads([up, down], start))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("grads", [None, torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["rms", "layer"])
+@pytest.mark.parametrize("branch", [False, True])
+def test_norms(kind, branch, grads):
+    torch.manual_seed(2)
+    w, b = (1 + _t(264, scale=0.1)).requires_grad_(), _t(264).requires_grad_()
+    params = [w] if kind == "rms" else [w, b]
+    start = _buffers(params, grads)
+    base, dy, dres = _t(70, 264), _t(70, 264), _t(70, 264)
+    cls = getattr(A, ("RMSNorm" if kind == "rms" else "LayerNorm") + ("BranchFn" if branch else "Fn"))
+    op = getattr(A, ("rmsnorm" if kind == "rms" else "layernorm") + ("_branch" if branch else ""))
+    for form in _forms(base):
+        for used in ((True, True), (True, False), (False, True)) if branch else ((True, False),):
+            got = []
+            for fn in (op, cls.apply):
+                x = form.detach().requires_grad_()
+                out = fn(x, *params, 1e-5)
+                y, h = out if branch else (out, None)
+                outs = [t for t, u in ((y, used[0]), (h, used[1])) if u and t is not None]
+                torch.autograd.backward(outs, [dy, dres][:2] if len(outs) == 2 else [dy if used[0] else dres])
+                got.append([y.detach(), x.grad] + _grads(params, start))
+            for i, (p, q) in enumerate(zip(*got)):
+                if i < 2 or used[0]:                       # without a gradient of y the Python side adds zeros where this one adds nothing
+                    assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("rope", [False, True])
+@pytest.mark.parametrize("dropout", [None, (0.2, 123456789012345678901 % (1 << 64), 3)])
+@pytest.mark.parametrize("lens", [None, [40, 77]])
+def test_packed_attention(rope, dropout, lens):
+    torch.manual_seed(3)
+    b, s, hq, hk, dh = 2, 77, 4, 2, 64
+    qkv = _t(s * b, (hq + 2 * hk) * dh)
+    inv = Fn.rope_inv_freq(dh, 10000.0, "cuda") if rope else None
+    cfg = A.AttnCfg(batch=b, hq=hq, hk=hk, dh=dh, causal=lens is None, rope=rope, rope_applied=rope, pos_offset=4, dropout=dropout)
+    kv = None if lens is None else torch.tensor(lens, device="cuda")
+    dout = _t(s * b, hq * dh)
+    for form in _forms(qkv):
+        got = []
+        for fn in (A.packed_attention, lambda q, c, i, p, l: A.PackedAttentionFn.apply(q, i, p, c, l)):
+            x = form.detach().requires_grad_()
+            o = fn(x, cfg, inv, None, kv)
+            o.backward(dout)
+            got.append((o.detach(), x.grad))
+        assert torch.equal(got[0][0], got[1][0])
+        n = hq * dh
+        assert torch.equal(got[0][1][:, n:], got[1][1][:, n:])
+        assert ((got[0][1] - got[1][1]).float().norm() / got[1][1].float().norm()).item() < 1e-3       # bf16 of fp32 sums in another order
+
+
+@pytest.mark.parametrize("dropout", [None, (0.1, 99, 0)])
+def test_attention_over_strided_heads(dropout):
+    torch.manual_seed(4)
+    b, sq, sk, h, dh = 2, 33, 70, 4, 40
+    kv = _t(sk, b, 2, h, dh)
+    q = _t(sq, b, h, dh).transpose(0, 1).requires_grad_()
+    k, v = (kv[:, :, i].transpose(0, 1).detach().requires_grad_() for i in range(2))
+    lens = torch.tensor([70, 20], device="cuda", dtype=torch.int32)
+    do = _t(sq, b, h, dh).transpose(0, 1)
+    got = []
+    for fn in (A.attention, A.AttentionFn.apply):
+        o, lse = fn(q, k, v, False, None, lens, dropout)
+        assert not lse.requires_grad
+        got.append((o.detach(), lse) + torch.autograd.grad(o, (k, v, q), do))
+    assert all(torch.equal(a, b) for a, b in list(zip(*got))[:4])
+    assert ((got[0][4] - got[1][4]).float().norm() / got[1][4].float().norm()).item() < 1e-3
+    with pytest.raises((RuntimeError, AssertionError)):
+        A.attention(q, k, v, False, None, lens[:1])
+
+
+@pytest.mark.parametrize("grads", [None, torch.float32])
+def test_language_model_head(grads):
+    torch.manual_seed(5)
+    x, w = _t(61, 136), _t(1000, 136, scale=0.1).requires_grad_()
+    labels = torch.randint(0, 1000, (61,), device="cuda")
+    labels[::5] = -100
+    start = _buffers([w], grads)
+    got = []
+    for fn in (lambda h: A.lm_head_loss(h, w, labels), lambda h: A.LMHeadLossFn.apply(h, w, labels, A.LossCfg())):
+        h = x.clone().view(1, 61, 136).requires_grad_()
+        loss = fn(h)
+        loss.backward(torch.full((61,), 0.25, device="cuda"))
+        got.append([loss.detach(), h.grad] + _grads([w], start))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+def test_saved_tensors_go_through_hooks():
+    """Hooks that hand back other tensors (here: the same values in transposed storage) see every saved tensor and are believed."""
+    torch.manual_seed(6)
+    w, nw = _t(256, 136, scale=0.1).requires_grad_(), (1 + _t(136, scale=0.1)).requires_grad_()
+    x = _t(40, 136)
+    seen = []
+
+    def pack(t):
+        seen.append(t.shape)
+        return t
+
+    def unpack(t):
+        return t.t().contiguous().t() if t.dim() == 2 else t
+
+    def run():
+        h = x.clone().requires_grad_()
+        y = A.packed_attention(A.linear(A.rmsnorm(h, nw), w), A.AttnCfg(batch=2, hq=2, hk=1, dh=64))
+        return (h.grad,) + torch.autograd.grad(y, (h, w, nw), torch.ones_like(y))
+
+    plain = run()
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        hooked = run()
+    assert len(seen) >= 3 + 2 + 3
+    for a, b in list(zip(plain, hooked))[1:]:
+        assert ((a - b).float().norm() / a.float().norm()).item() < 1e-3
+
+
+def test_weight_changed_in_place_before_backward_is_refused():
+    x, w = _t(32, 64).requires_grad_(), _t(64, 64).requires_grad_()
+    y = A.linear(x, w)
+    with torch.no_grad():
+        w.add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.sum().backward()
+
+
+def test_hook_that_raises_and_buffers_for_the_python_side():
+    x, w = _t(32, 64), _t(64, 64).requires_grad_()
+    w.main_grad = torch.zeros(64, 64, device="cuda")
+
+    def fails(_):
+        raise ValueError("from the hook")
+
+    w.grad_ready_hook = fails
+    with pytest.raises(Exception, match="from the hook"):
+        A.linear(x, w).sum().backward()
+    del w.grad_ready_hook
+    w.main_grad = torch.zeros(64 * 64 + 1, device="cuda")[1:].view(64, 64)         # 4-byte aligned: not for the kernel
+    with pytest.raises(Exception, match="gv_gemm_bf16"):
+        A.linear(x, w).sum().backward()
+
+
+def test_what_is_not_taken_goes_to_the_python_functions():
+    x, w = _t(16, 64), _t(64, 64)
+    ops = _lib.torch_ops()
+    assert ops.linear(x.float(), w.float(), None, None, None) is None
+    assert ops.linear(x, w[:, :60], None, None, None) is None
+    assert ops.linear(x, w[:60], None, None, None) is None
+    assert ops.linear(x[:0], w, None, None, None) is None
+    assert ops.linear(x.cpu(), w, None, None, None) is None
+    assert ops.rmsnorm(x, w[0, :60], 1e-5, False) is None
+    with pytest.raises(Exception):
+        torch.func.vmap(lambda t: A.linear(t, w))(x.view(2, 8, 64))
+    with pytest.raises(Exception):
+        torch.func.jvp(lambda t: A.linear(t, w), (x,), (x,))
+    off = _t(16 * 64 + 1)[1:].view(16, 64)                                          # 2-byte aligned
+    for fn in (lambda: A.linear(off, w), lambda: A.LinearFn.apply(off, w, None, None, A.LinearCfg(), None)):
+        with pytest.raises(_lib.KernelError):
+            fn()
+    with pytest.raises(ValueError):
+        A.linear(x, _t(64, 72))
+    with pytest.raises(_lib.KernelError):
+        A.linear(x, w, rope=RopeEpilogue(48, 64, Fn.rope_inv_freq(64, 1e4, "cuda"), None, 1, 0))       # not a whole head
