@@ -36,6 +36,7 @@ CUDA_SOURCES = [
     "attention_sm100.cu",
     "norm.cu",
     "elementwise.cu",
+    "window_bias.cu",
     "comm_kernels.cu",
     "fused_gemm_sm100.cu",
     "nvlink_bench.cu",

@@ -232,6 +232,12 @@ typedef struct {
 int gv_attn_fwd(const gv_attn_args* args, gv_stream_t stream);
 int gv_attn_bwd(const gv_attn_args* args, gv_stream_t stream);
 
+// Relative-position bias of attention in windows of ws x ws tokens, S = ws^2: from table bf16 [(2 ws - 1)^2, heads] to the `bias` and
+// `bias_t` of gv_attn_args, bf16 [heads, S, ld] with zeros beyond column S, and from their gradient `dbias` fp32 [heads, S, ld] back:
+// dtable fp32 [(2 ws - 1)^2, heads] += the sum over all pairs of tokens with an entry's offset, in a fixed order.
+int gv_window_bias(const void* table, int heads, int ws, int ld, void* bias, void* bias_t, gv_stream_t stream);
+int gv_window_bias_bwd(const float* dbias, int heads, int ws, int ld, float* dtable, gv_stream_t stream);
+
 // Copies `count` (1 to 5) bf16 tensors [b, s, h, .] between heads of `narrow` (even) and `wide` (a multiple of 8, not smaller)
 // columns: pad != 0 narrow -> wide with zeros behind, else wide -> narrow. Strides in elements of (b, s, h), unit inner stride;
 // wide sides 16-byte aligned with strides of multiples of 8, narrow sides 4-byte aligned with even strides.

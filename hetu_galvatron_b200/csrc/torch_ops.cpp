@@ -40,7 +40,8 @@ namespace {
 // The kernel library's entry points; the addresses come from the library that Python has loaded.
 #define GV_ENTRIES(X)                                                                                                              \
   X(gv_gemm_bf16) X(gv_gemm_xent) X(gv_gemm_workspace_bytes) X(gv_xent_merge) X(gv_rmsnorm_fwd) X(gv_rmsnorm_bwd) X(gv_layernorm_fwd) \
-  X(gv_layernorm_bwd) X(gv_norm_bwd_scratch_elems) X(gv_rope) X(gv_swiglu_bwd) X(gv_gelu_bwd) X(gv_colsum_accum) X(gv_attn_fwd) X(gv_attn_bwd)
+  X(gv_layernorm_bwd) X(gv_norm_bwd_scratch_elems) X(gv_rope) X(gv_swiglu_bwd) X(gv_gelu_bwd) X(gv_colsum_accum) X(gv_attn_fwd) X(gv_attn_bwd) \
+  X(gv_window_bias) X(gv_window_bias_bwd)
 struct Entries {
 #define X(name) decltype(&::name) name = nullptr;
   GV_ENTRIES(X)
@@ -718,6 +719,74 @@ py::object attention(const Tensor& q, const Tensor& k, const Tensor& v, bool cau
   return py::make_tuple(out[0], out[1]);
 }
 
+// Attention within windows of one projection [tokens, 3 heads dh] whose rows `perm` sorts by window (`inv` undoes it), with the
+// relative-position bias of `table` and, in shifted windows, group ids [n, ld] of the tokens. q, k and v are read out of the sorted
+// rows and their gradients written into one sorted buffer: as three separate ones they came back through three cleared buffers of
+// the whole projection's size, three copies and two additions. The table's gradient is summed from the kernel's in fp32.
+struct WindowAttentionFn : Function<WindowAttentionFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& qkv, const Tensor& table, const Tensor& perm, const Tensor& inv, const OptTensor& ids_, int ws,
+                        int dh) {
+    const Tensor x = qkv.index_select(0, perm), ids = opt(ids_);
+    const int S = ws * ws, heads = static_cast<int>(table.size(1)), ld = (S + 63) / 64 * 64, windows = static_cast<int>(x.size(0) / S);
+    const Tensor bias = empty16({heads, S, ld}, x), bias_t = empty16({heads, S, ld}, x);
+    launched(K.gv_window_bias(cptr(table), heads, ws, ld, ptr(bias), ptr(bias_t), stream()), "gv_window_bias");
+    const Tensor o = empty16({x.size(0), static_cast<int64_t>(heads) * dh}, x), lse = empty32({windows, heads, S}, x);
+    const gv_attn_args a = args(x, o, lse, bias, bias_t, ids, windows, S, heads, dh, ld);
+    launched(K.gv_attn_fwd(&a, stream()), "gv_attn_fwd");
+    ctx->saved_data["ws"] = static_cast<int64_t>(ws);
+    ctx->saved_data["dh"] = static_cast<int64_t>(dh);
+    ctx->save_for_backward({x, table, o, lse, bias, bias_t, perm, inv, ids});
+    return o.index_select(0, inv);
+  }
+  static Heads part(const Tensor& t, int which, int S, int heads, int dh, int parts) {
+    const long long width = static_cast<long long>(parts) * heads * dh;
+    return heads_at(t, static_cast<int64_t>(which) * heads * dh, S * width, width, dh);
+  }
+  static gv_attn_args args(const Tensor& x, const Tensor& o, const Tensor& lse, const Tensor& bias, const Tensor& bias_t, const Tensor& ids, int windows, int S,
+                           int heads, int dh, int ld) {
+    gv_attn_args a = attention_args(part(x, 0, S, heads, dh, 3), part(x, 1, S, heads, dh, 3), part(x, 2, S, heads, dh, 3), part(o, 0, S, heads, dh, 1), lse,
+                                    windows, S, S, heads, heads, dh, false, 1.0 / std::sqrt(static_cast<double>(dh)), Tensor(), Dropout());
+    a.bias = cptr(bias); a.bias_t = cptr(bias_t); a.bias_ld = ld;
+    if (ids.defined()) { a.ids = static_cast<const int*>(cptr(ids)); a.mask_n = static_cast<int>(ids.size(0)); }
+    return a;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor x = ready(saved[0]), o = ready(saved[2]), lse = saved[3].contiguous(), bias = ready(saved[4]), bias_t = ready(saved[5]);
+    const Tensor &table = saved[1], &perm = saved[6], &inv = saved[7];
+    const Tensor ids = saved[8].defined() ? ready(saved[8]) : Tensor();
+    const int ws = static_cast<int>(ctx->saved_data["ws"].toInt()), dh = static_cast<int>(ctx->saved_data["dh"].toInt());
+    const int S = ws * ws, heads = static_cast<int>(table.size(1)), ld = static_cast<int>(bias.size(2)), windows = static_cast<int>(x.size(0) / S);
+    const Tensor dout = grads[0].index_select(0, perm);
+    const Tensor dx = at::empty_like(x), dq_accum = empty32({windows, S, heads, dh}, x), delta = empty32({windows, heads, S}, x);
+    const Tensor dbias = at::zeros({heads, S, ld}, x.options().dtype(at::kFloat));
+    gv_attn_args a = args(x, o, lse, bias, bias_t, ids, windows, S, heads, dh, ld);
+    set_grads(a, part(dout, 0, S, heads, dh, 1), part(dx, 0, S, heads, dh, 3), part(dx, 1, S, heads, dh, 3), part(dx, 2, S, heads, dh, 3), dq_accum, delta);
+    a.dbias = static_cast<float*>(ptr(dbias));
+    launched(K.gv_attn_bwd(&a, stream()), "gv_attn_bwd", 3);
+    Tensor dtable = vector_grad(table, [&](const Tensor& buf) {
+      launched(K.gv_window_bias_bwd(static_cast<const float*>(cptr(dbias)), heads, ws, ld, static_cast<float*>(ptr(buf)), stream()), "gv_window_bias_bwd");
+    });
+    return {dx.index_select(0, inv), dtable, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+bool rows_of(const Tensor& t, int64_t rows, const Tensor& like) {
+  return plain(t) && t.scalar_type() == at::kLong && t.dim() == 1 && t.numel() == rows && t.device() == like.device();
+}
+
+py::object window_attention(const Tensor& qkv, const Tensor& table, const Tensor& perm, const Tensor& inv, const OptTensor& ids, int ws, int dh) {
+  if (!plain_mode() || !input_ok(qkv) || qkv.dim() != 2 || !plain16(table) || table.dim() != 2 || !table.is_contiguous() || ws <= 0 || ws > 64 || dh <= 0 ||
+      dh % 8 != 0 || dh > 128)
+    return py::none();
+  const int64_t S = static_cast<int64_t>(ws) * ws, ld = (S + 63) / 64 * 64, rows = qkv.size(0), heads = table.size(1);
+  if (heads == 0 || table.size(0) != (2 * ws - 1) * (2 * ws - 1) || qkv.size(1) != 3 * heads * dh || rows % S != 0 || !rows_of(perm, rows, qkv) ||
+      !rows_of(inv, rows, qkv) || (ids.has_value() && (!plain(*ids) || ids->scalar_type() != at::kInt || ids->dim() != 2 || !ids->is_contiguous() ||
+                                                       ids->size(1) != ld || ids->size(0) == 0 || !aligned(*ids))))
+    return py::none();
+  return py::cast(no_gil([&] { return WindowAttentionFn::apply(qkv, table, perm, inv, ids, ws, dh); }));
+}
+
 // ------------------------------------------------------------------ language-model head
 gv_gemm_args head_args(const Tensor& x, const Tensor& W, const Tensor& C) {
   gv_gemm_args g = {};
@@ -801,6 +870,7 @@ void init(const py::dict& addresses, py::object wgrad, py::object vecgrad, py::o
   name_node<LayerNormBranchFn>("LayerNormBranchFnBackward");
   name_node<PackedAttentionFn>("PackedAttentionFnBackward");
   name_node<AttentionFn>("AttentionFnBackward");
+  name_node<WindowAttentionFn>("WindowAttentionFnBackward");
   name_node<LMHeadLossFn>("LMHeadLossFnBackward");
 }
 
@@ -821,5 +891,6 @@ PYBIND11_MODULE(torch_ops, m) {
   m.def("layernorm", torch::wrap_pybind_function(layernorm));
   m.def("packed_attention", torch::wrap_pybind_function(packed_attention));
   m.def("attention", torch::wrap_pybind_function(attention));
+  m.def("window_attention", torch::wrap_pybind_function(window_attention));
   m.def("lm_head_loss", torch::wrap_pybind_function(lm_head_loss));
 }

@@ -1,0 +1,76 @@
+// Relative-position bias of windowed attention (Swin): from the table of offsets to the score terms that the attention kernels read,
+// and from their gradient back to the table's. A window has ws x ws tokens; tokens i and j use table row
+// (y_i - y_j + ws - 1) (2 ws - 1) + x_i - x_j + ws - 1.
+//
+// Bound by launches and latency, not by bytes (a few MB): as index, permutation, two padded copies and their gradients, among them a
+// sort of all ws^4 indices for the table's gradient, these were 17 launches and 120 us of kernels a layer at ws = 12; now two launches,
+// 5 us together at 6 heads and 12 at 48.
+#include "include/gv_kernels.h"
+#include "include/gv_ptx.cuh"
+
+namespace gv {
+int num_sms();
+typedef __nv_bfloat16 bf16;
+
+// Eight columns of a row of both matrices per thread. The table (a few 10 KB) stays in L1, so the scattered reads cost little.
+__global__ void window_bias_kernel(const bf16* __restrict__ table, int heads, int ws, int ld, bf16* __restrict__ bias, bf16* __restrict__ bias_t) {
+  const int S = ws * ws, vecs = ld >> 3, span = 2 * ws - 1;
+  const long long total = static_cast<long long>(heads) * S * vecs;
+  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total; t += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int c0 = static_cast<int>(t % vecs) * 8, row = static_cast<int>(t / vecs % S), h = static_cast<int>(t / vecs / S);
+    const int yr = row / ws, xr = row % ws;
+    alignas(16) bf16 a[8], b[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int c = c0 + e, yc = c / ws, xc = c % ws;
+      const bool in = c < S;
+      const int at = ((yr - yc + ws - 1) * span + xr - xc + ws - 1);     // query `row`, key c
+      a[e] = in ? table[static_cast<long long>(at) * heads + h] : __float2bfloat16(0.f);
+      b[e] = in ? table[static_cast<long long>(span * span - 1 - at) * heads + h] : __float2bfloat16(0.f);   // query c, key `row`
+    }
+    const long long o = (static_cast<long long>(h) * S + row) * ld + c0;
+    *reinterpret_cast<uint4*>(bias + o) = *reinterpret_cast<const uint4*>(a);
+    *reinterpret_cast<uint4*>(bias_t + o) = *reinterpret_cast<const uint4*>(b);
+  }
+}
+
+// One warp per table entry and head sums the pairs of tokens with that offset, always in the same order.
+__global__ void window_bias_bwd_kernel(const float* __restrict__ dbias, int heads, int ws, int ld, float* __restrict__ dtable) {
+  const int S = ws * ws, span = 2 * ws - 1, lane = threadIdx.x & 31;
+  const long long total = static_cast<long long>(span) * span * heads;
+  for (long long t = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5; t < total; t += static_cast<long long>(gridDim.x) * (blockDim.x >> 5)) {
+    const int h = static_cast<int>(t % heads), at = static_cast<int>(t / heads);
+    const int dy = at / span - (ws - 1), dx = at % span - (ws - 1);
+    const int y0 = max(0, -dy), x0 = max(0, -dx), ny = ws - abs(dy), nx = ws - abs(dx);
+    float acc = 0.f;
+    for (int e = lane; e < ny * nx; e += 32) {
+      const int j = (y0 + e / nx) * ws + x0 + e % nx, i = j + dy * ws + dx;
+      acc += dbias[(static_cast<long long>(h) * S + i) * ld + j];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) dtable[t] += acc;
+  }
+}
+
+static int blocks_for(long long threads) {
+  const long long g = (threads + 255) / 256, cap = static_cast<long long>(num_sms()) * 8;
+  return static_cast<int>(g < cap ? g : cap);
+}
+}  // namespace gv
+
+static bool window_args_ok(int heads, int ws, int ld) { return heads > 0 && ws > 0 && ws <= 64 && ld >= ws * ws && ld % 8 == 0; }
+
+extern "C" int gv_window_bias(const void* table, int heads, int ws, int ld, void* bias, void* bias_t, gv_stream_t s) {
+  if (!window_args_ok(heads, ws, ld) || ((reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(bias_t)) & 15)) return 2501;
+  gv::window_bias_kernel<<<gv::blocks_for(static_cast<long long>(heads) * ws * ws * (ld / 8)), 256, 0, reinterpret_cast<cudaStream_t>(s)>>>(
+      reinterpret_cast<const gv::bf16*>(table), heads, ws, ld, reinterpret_cast<gv::bf16*>(bias), reinterpret_cast<gv::bf16*>(bias_t));
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int gv_window_bias_bwd(const float* dbias, int heads, int ws, int ld, float* dtable, gv_stream_t s) {
+  if (!window_args_ok(heads, ws, ld)) return 2501;
+  const long long span = 2 * ws - 1;
+  gv::window_bias_bwd_kernel<<<gv::blocks_for(span * span * heads * 32), 256, 0, reinterpret_cast<cudaStream_t>(s)>>>(dbias, heads, ws, ld, dtable);
+  return static_cast<int>(cudaGetLastError());
+}

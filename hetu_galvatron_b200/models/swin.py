@@ -23,6 +23,7 @@ import torch.nn.functional as F
 
 from ..core.hybrid_model import ModuleSpec
 from ..ops import autograd as A
+from ..ops.attention import additive_ld, pad_rows
 from .transformer import BatchCtx, LayerStrategy, ModelConfig, _det_normal, _shard_cols, _shard_rows
 
 META_DIR = os.path.join(os.path.dirname(__file__), "meta_configs")
@@ -76,6 +77,10 @@ class _LN(nn.Module):
 
     def forward(self, x):
         return A.layernorm(x, self.weight, self.bias, self.eps)
+
+    def branch(self, x):
+        """(norm(x), x): the gradient of the residual branch is added in the norm's backward kernel."""
+        return A.layernorm_branch(x, self.weight, self.bias, self.eps)
 
 
 def _relative_index(ws: int) -> torch.Tensor:
@@ -158,6 +163,7 @@ class SwinLayerBlock(nn.Module):
         self._perm_cache: dict = {}
         if self.shift:
             self.register_buffer("regions", _shift_regions(self.res, self.ws, self.shift).to(device), persistent=False)
+            self.register_buffer("region_rows", pad_rows(self.regions, additive_ld(self.ws ** 2, self.ws ** 2), torch.int32, -1), persistent=False)
         if merge:
             self.ln_merge = _LN(4 * C, cfg, device, dup)
             self.w_merge = nn.Parameter(_det_normal((2 * C, 4 * C), cfg.init_std, seed + 7, device, cfg.dtype))
@@ -190,6 +196,9 @@ class SwinLayerBlock(nn.Module):
         R, ws, hl, dh = self.res, self.ws, self.heads_l, self.dh
         nw, S = R // ws, ws * ws
         perm, inv = self._window_rows(b, qkv.device)
+        o = A.window_attention(qkv, self.rel_table, perm, inv, self.region_rows if self.shift else None, ws, dh)
+        if o is not None:
+            return o
         x = _PermuteRows.apply(qkv, perm, inv).view(b * nw * nw, S, 3, hl, dh)      # [windows, tokens, q|k|v, heads, dh]
         bias = self.rel_table[self.rel_index.view(-1)].view(S, S, hl).permute(2, 0, 1)
         regions = self.regions if self.shift else None  # [nw^2, S]: window w of every image uses regions[w]
@@ -213,12 +222,14 @@ class SwinLayerBlock(nn.Module):
         st, b = self.st, ctx.batch
         col = st.linear_cfg("col")
         row = st.linear_cfg("row")
-        qkv = A.linear(self.ln1(h), self.wqkv, self.bqkv, cfg=col)
+        y, h = self.ln1.branch(h)
+        qkv = A.linear(y, self.wqkv, self.bqkv, cfg=col)
         if self.cfg.drop_path_rate > 0.0 and ctx.extra.get("rng") is not None:
             h = h + self._drop_path(A.linear(self._attention(qkv, b).contiguous(), self.wo, self.bo, cfg=row), ctx, b)
         else:
             h = A.linear(self._attention(qkv, b).contiguous(), self.wo, self.bo, residual=h, cfg=row)
-        m = A.linear_gelu(self.ln2(h), self.w1, self.b1, cfg=col)
+        y, h = self.ln2.branch(h)
+        m = A.linear_gelu(y, self.w1, self.b1, cfg=col)
         h = A.linear(m, self.w2, self.b2, residual=h, cfg=row)
         if self.merge:
             R, C = self.res, self.C

@@ -620,6 +620,13 @@ def biased_attention(q, k, v, bias=None, mask=None, ids=None, scale: float | Non
     return Fn.biased_attention_reference(q, k, v, scale, bias, mask, ids)
 
 
+def window_attention(qkv, table, perm, inv, ids, window: int, dh: int):
+    """Attention within windows of ``window`` x ``window`` tokens: rows of the packed projection ``qkv`` [tokens, 3 heads dh] sorted by
+    window with ``perm`` (and back with ``inv``), relative-position bias from ``table`` [(2 window - 1)^2, heads], group ids ``ids``
+    (``attention.pad_rows`` of [n, window^2], fill -1) or None. One C++ Function for un-sharded bf16 CUDA operands, else None."""
+    return _native().window_attention(qkv, table, perm, inv, ids, window, dh) if qkv.is_cuda else None
+
+
 class RopeFn(torch.autograd.Function):
     """Out-of-place rotary embedding on [tokens, heads, dh] (used by the Ulysses / ring paths)."""
 

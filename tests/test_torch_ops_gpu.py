@@ -279,3 +279,48 @@ def test_what_is_not_taken_goes_to_the_python_functions():
         A.linear(x, _t(64, 72))
     with pytest.raises(_lib.KernelError):
         A.linear(x, w, rope=RopeEpilogue(48, 64, Fn.rope_inv_freq(64, 1e4, "cuda"), None, 1, 0))       # not a whole head
+
+
+@pytest.mark.parametrize("ws,heads,dh,shift,grads", [(12, 6, 32, 6, torch.float32), (7, 3, 32, 3, torch.bfloat16), (7, 48, 32, 0, None), (1, 2, 8, 0, None),
+                                                     (8, 2, 64, 4, torch.float32)])
+def test_windowed_attention(ws, heads, dh, shift, grads):
+    """The windows' rows, the bias of the offsets and the table's gradient against PyTorch expressions in 64 bits on the same values.
+    bf16 operands and outputs, probabilities and their gradients rounded once: 2^-8 and some; the bias gradient sums fp32 terms."""
+    from hetu_galvatron_b200.models import swin
+    from hetu_galvatron_b200.ops.attention import additive_ld, pad_rows
+    torch.manual_seed(7)
+    b, nw = 2, 2
+    res, S = ws * nw, ws * ws
+    rows = b * res * res
+    ids = swin._shift_regions(res, ws, shift) if shift else None
+    perm = torch.randperm(rows, device="cuda")
+    inv = torch.empty_like(perm)
+    inv[perm] = torch.arange(rows, device="cuda")
+    table = _t((2 * ws - 1) ** 2, heads).requires_grad_()
+    qkv, dout = _t(rows, 3 * heads * dh), _t(rows, heads * dh)
+    start = _buffers([table], grads)
+    x = qkv.clone().requires_grad_()
+    o = A.window_attention(x, table, perm, inv, None if ids is None else pad_rows(ids.cuda(), additive_ld(S, S), torch.int32, -1), ws, dh)
+    o.backward(dout)
+    (dtable,) = _grads([table], {table: torch.zeros(1, device="cuda")})
+    if grads is not None:
+        dtable = dtable.double() - start[table].double()
+    xd, td = qkv.double().requires_grad_(), table.detach().double().requires_grad_()
+    w = xd[perm].view(-1, S, 3, heads, dh)
+    bias = td[swin._relative_index(ws).cuda().view(-1)].view(S, S, heads).permute(2, 0, 1)
+    s = torch.einsum("wihd,wjhd->whij", w[:, :, 0], w[:, :, 1]) * dh ** -0.5 + bias
+    if ids is not None:
+        hidden = (ids[:, :, None] != ids[:, None, :]).cuda().repeat(b, 1, 1)
+        s = s.masked_fill(hidden[:, None], float("-inf"))
+    ref = torch.einsum("whij,wjhd->wihd", s.softmax(-1), w[:, :, 2]).reshape(rows, heads * dh)[inv]
+    gx, gt = torch.autograd.grad(ref, (xd, td), dout.double())
+    rel = lambda a, r: ((a.double() - r).norm() / r.norm().clamp(min=1e-6)).item()
+    assert rel(o, ref) < 6e-3
+    if ws > 1:
+        assert rel(x.grad, gx) < 1e-2
+        # a bf16 buffer holds start + gradient to 2^-9 of their size
+        assert rel(dtable, gt) < (1e-2 if grads is not torch.bfloat16 else 1e-2 + 2.0 ** -8 * (start[table].double().norm() / gt.norm()).item())
+    else:
+        assert x.grad[:, :2 * heads * dh].abs().max().item() < 2e-2          # one key: no gradient but of the values
+    assert _lib.read_error() is None
+    assert A.window_attention(qkv, table, perm[:-1], inv, None, ws, dh) is None
