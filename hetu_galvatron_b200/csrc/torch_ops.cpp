@@ -265,6 +265,19 @@ Tensor weight_grad(const Tensor& W, const Tensor& dy2, const Tensor& x2) {
   return dw;
 }
 
+// The same for rows [lo, lo + n) of W, whose other rows belong to another product. Without a main_grad that the kernels take: a gradient of
+// all of W, zero elsewhere. The hook of a whole gradient is not called for a part of it.
+Tensor weight_rows_grad(const Tensor& W, int64_t lo, int64_t n, const Tensor& dy2, const Tensor& x2) {
+  Tensor mg;
+  {
+    py::gil_scoped_acquire gil;
+    mg = buffer_of(W).main_grad;
+  }
+  const Tensor whole = mg.defined() ? mg.view({W.size(0), W.size(1)}) : at::zeros({W.size(0), W.size(1)}, W.options());
+  gemm_into(dy2, true, x2, true, whole.narrow(0, lo, n), mg.defined());
+  return mg.defined() ? Tensor() : whole;
+}
+
 // The gradient of a vector parameter: `fill(buf)` adds it to an fp32 buffer.
 template <class Fill>
 Tensor vector_grad(const Tensor& p, Fill fill) {
@@ -330,6 +343,26 @@ struct LinearFn : Function<LinearFn> {
   }
 };
 
+// x W[lo : lo + n]^T of a weight that holds several projections. As a product with a slice of W, its gradient came back through a
+// cleared buffer of all of W, a copy and an addition, rounded to bf16.
+struct LinearRowsFn : Function<LinearRowsFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& W, int64_t lo, int64_t n) {
+    ctx->saved_data["lo"] = lo;
+    ctx->saved_data["n"] = n;
+    ctx->save_for_backward({x, W});
+    return project(x, W.narrow(0, lo, n));
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &W = saved[1], dy = ready(grads[0]);
+    const int64_t lo = ctx->saved_data["lo"].toInt(), n = ctx->saved_data["n"].toInt();
+    Tensor dx;
+    if (ctx->needs_input_grad(0)) dx = input_grad(dy, W.narrow(0, lo, n));
+    Tensor dW = weight_rows_grad(W, lo, n, dy, x);
+    return {dx, dW, Tensor(), Tensor()};
+  }
+};
+
 bool add_on_ok(const OptTensor& t, int64_t numel) { return !t.has_value() || (plain16(*t) && t->numel() == numel); }
 bool linear_ok(const Tensor& x, const Tensor& W, const OptTensor& bias, const OptTensor& residual) {
   return plain_mode() && input_ok(x) && weight_ok(W) && x.size(-1) == W.size(1) && add_on_ok(bias, W.size(0)) &&
@@ -346,6 +379,11 @@ py::object linear(const Tensor& x, const Tensor& W, const OptTensor& bias, const
       return py::none();
   }
   return py::cast(no_gil([&] { return LinearFn::apply(x, W, bias, residual, r); }));
+}
+
+py::object linear_rows(const Tensor& x, const Tensor& W, int64_t lo, int64_t n) {
+  if (!linear_ok(x, W, std::nullopt, std::nullopt) || x.dim() != 2 || lo < 0 || n <= 0 || lo % 8 != 0 || n % 8 != 0 || lo + n > W.size(0)) return py::none();
+  return py::cast(no_gil([&] { return LinearRowsFn::apply(x, W, lo, n); }));
 }
 
 // ------------------------------------------------------------------ MLP
@@ -719,6 +757,56 @@ py::object attention(const Tensor& q, const Tensor& k, const Tensor& v, bool cau
   return py::make_tuple(out[0], out[1]);
 }
 
+// Attention of queries q [sq * b, hq dh] to keys and values kv [sk * b, 2 hk dh] (keys first), all in sequence-major order, read and
+// written as the projections around it have them: by way of [b, s, h, dh] tensors, output and gradients were copied, and those of the
+// two halves of kv cleared, copied and added.
+struct Cross {
+  int batch, hq, hk, dh;
+  Heads one(const Tensor& t) const { return heads_at(t, 0, static_cast<long long>(hq) * dh, static_cast<long long>(batch) * hq * dh, dh); }
+  Heads half(const Tensor& t, int which) const {
+    const long long w = 2ll * hk * dh;
+    return heads_at(t, static_cast<int64_t>(which) * hk * dh, w, batch * w, dh);
+  }
+};
+
+struct CrossAttentionFn : Function<CrossAttentionFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q_, const Tensor& kv_, const OptTensor& lens_, const Cross& c, const Dropout& drop) {
+    const Tensor q = ready(q_), kv = ready(kv_), lens = lengths(lens_, q_);
+    const int sq = static_cast<int>(q.size(0) / c.batch), sk = static_cast<int>(kv.size(0) / c.batch);
+    const Tensor o = at::empty_like(q), lse = empty32({c.batch, c.hq, sq}, q);
+    const gv_attn_args a = attention_args(c.one(q), c.half(kv, 0), c.half(kv, 1), c.one(o), lse, c.batch, sq, sk, c.hq, c.hk, c.dh, false,
+                                          1.0 / std::sqrt(static_cast<double>(c.dh)), lens, drop);
+    launched(K.gv_attn_fwd(&a, stream()), "gv_attn_fwd");
+    ctx->saved_data["cfg"] = std::vector<int64_t>{c.batch, c.hq, c.hk, c.dh};
+    keep_dropout(ctx, drop);
+    ctx->save_for_backward({q, kv, o, lse, lens});
+    return o;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor q = ready(saved[0]), kv = ready(saved[1]), o = ready(saved[2]), lse = saved[3].contiguous(), &lens = saved[4], dout = ready(grads[0]);
+    const auto n = ctx->saved_data["cfg"].toIntVector();
+    const Cross c = {static_cast<int>(n[0]), static_cast<int>(n[1]), static_cast<int>(n[2]), static_cast<int>(n[3])};
+    const int sq = static_cast<int>(q.size(0) / c.batch), sk = static_cast<int>(kv.size(0) / c.batch);
+    const Tensor dq = at::empty_like(q), dkv = at::empty_like(kv), dq_accum = empty32({c.batch, sq, c.hq, c.dh}, q), delta = empty32({c.batch, c.hq, sq}, q);
+    gv_attn_args a = attention_args(c.one(q), c.half(kv, 0), c.half(kv, 1), c.one(o), lse, c.batch, sq, sk, c.hq, c.hk, c.dh, false,
+                                    1.0 / std::sqrt(static_cast<double>(c.dh)), lens, kept_dropout(ctx));
+    set_grads(a, c.one(dout), c.one(dq), c.half(dkv, 0), c.half(dkv, 1), dq_accum, delta);
+    launched(K.gv_attn_bwd(&a, stream()), "gv_attn_bwd", 3);
+    return {dq, dkv, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+py::object cross_attention(const Tensor& q, const Tensor& kv, int batch, int hq, int hk, int dh, const OptTensor& kv_lens, double p, unsigned long long seed,
+                           int head_offset) {
+  if (!plain_mode() || !input_ok(q) || !input_ok(kv) || q.dim() != 2 || kv.dim() != 2 || batch <= 0 || hk <= 0 || hq % hk != 0 || dh <= 0 || dh % 8 != 0 ||
+      dh > 128 || q.size(0) % batch != 0 || kv.size(0) % batch != 0 || q.size(1) != static_cast<int64_t>(hq) * dh ||
+      kv.size(1) != 2ll * hk * dh || kv.device() != q.device() || (kv_lens.has_value() && (!plain(*kv_lens) || kv_lens->numel() != batch)))
+    return py::none();
+  const Cross c = {batch, hq, hk, dh};
+  return py::cast(no_gil([&] { return CrossAttentionFn::apply(q, kv, kv_lens, c, Dropout{p, seed, head_offset}); }));
+}
+
 // Attention within windows of one projection [tokens, 3 heads dh] whose rows `perm` sorts by window (`inv` undoes it), with the
 // relative-position bias of `table` and, in shifted windows, group ids [n, ld] of the tokens. q, k and v are read out of the sorted
 // rows and their gradients written into one sorted buffer: as three separate ones they came back through three cleared buffers of
@@ -870,6 +958,8 @@ void init(const py::dict& addresses, py::object wgrad, py::object vecgrad, py::o
   name_node<LayerNormBranchFn>("LayerNormBranchFnBackward");
   name_node<PackedAttentionFn>("PackedAttentionFnBackward");
   name_node<AttentionFn>("AttentionFnBackward");
+  name_node<LinearRowsFn>("LinearRowsFnBackward");
+  name_node<CrossAttentionFn>("CrossAttentionFnBackward");
   name_node<WindowAttentionFn>("WindowAttentionFnBackward");
   name_node<LMHeadLossFn>("LMHeadLossFnBackward");
 }
@@ -891,6 +981,8 @@ PYBIND11_MODULE(torch_ops, m) {
   m.def("layernorm", torch::wrap_pybind_function(layernorm));
   m.def("packed_attention", torch::wrap_pybind_function(packed_attention));
   m.def("attention", torch::wrap_pybind_function(attention));
+  m.def("linear_rows", torch::wrap_pybind_function(linear_rows));
+  m.def("cross_attention", torch::wrap_pybind_function(cross_attention));
   m.def("window_attention", torch::wrap_pybind_function(window_attention));
   m.def("lm_head_loss", torch::wrap_pybind_function(lm_head_loss));
 }

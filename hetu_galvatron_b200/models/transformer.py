@@ -384,6 +384,11 @@ class SelfAttention(nn.Module):
         cfg, st = self.cfg, self.st
         dh = cfg.head_dim
         nq = self.hq_w * dh
+        drop = attention_dropout_spec(cfg, ctx, self.layer_idx, (st.tp_rank if st.weight_tp > 1 else 0) * self.hq_w, cross=True)
+        if self.bqkv is None and st.tp == 1 and st.cp == 1:
+            o = A.cross_attention_block(x, kv_source, self.wqkv, ctx.batch, self.hq_w, self.hk_w, dh, key_lengths(ctx, "attention_mask"), drop)
+            if o is not None:
+                return A.linear(o, self.wo, self.bo, residual, st.linear_cfg("row"))
         q = A.linear(x, self.wqkv[:nq], None if self.bqkv is None else self.bqkv[:nq], None, st.linear_cfg("col"))
         kv = A.linear(kv_source, self.wqkv[nq:], None if self.bqkv is None else self.bqkv[nq:], None, st.linear_cfg("col"))
         b = ctx.batch
@@ -391,7 +396,6 @@ class SelfAttention(nn.Module):
         qv = q.view(sq, b, self.hq_w, dh).transpose(0, 1)
         kk = kv[:, : self.hk_w * dh].reshape(sk, b, self.hk_w, dh).transpose(0, 1)
         vv = kv[:, self.hk_w * dh:].reshape(sk, b, self.hk_w, dh).transpose(0, 1)
-        drop = attention_dropout_spec(cfg, ctx, self.layer_idx, (st.tp_rank if st.weight_tp > 1 else 0) * self.hq_w, cross=True)
         o, _ = A.attention(qv, kk, vv, False, None, key_lengths(ctx, "attention_mask"), drop)    # keys = encoder tokens
         o = o.transpose(0, 1).reshape(sq * b, nq)
         return A.linear(o, self.wo, self.bo, residual, st.linear_cfg("row"))

@@ -576,6 +576,20 @@ def attention(q, k, v, causal: bool = True, scale: float | None = None, kv_lens=
     return AttentionFn.apply(q, k, v, causal, scale, kv_lens, dropout)
 
 
+def cross_attention_block(x, kv_source, W, batch: int, hq: int, hk: int, dh: int, kv_lens=None, dropout=None):
+    """Attention of the queries of ``x`` to the keys and values of ``kv_source`` (tokens in sequence-major order), projected by the rows
+    [q | k | v] of ``W``; [sq * batch, hq * dh]. C++ Functions for un-sharded bf16 CUDA operands, else None."""
+    if not x.is_cuda:
+        return None
+    ops, nq = _native(), hq * dh
+    q = ops.linear_rows(x, W, 0, nq)
+    kv = None if q is None else ops.linear_rows(kv_source, W, nq, 2 * hk * dh)
+    if kv is None:
+        return None
+    p, seed, head_offset = dropout or (0.0, 0, 0)
+    return ops.cross_attention(q, kv, batch, hq, hk, dh, kv_lens, p, seed & 0xFFFFFFFFFFFFFFFF, head_offset)
+
+
 class BiasedAttentionFn(torch.autograd.Function):
     """Full (non-causal) attention with extra score terms on the tcgen05 kernels: q, k, v [b, s, h, dh] (any strides the
     kernels accept); ``bias`` [h, sq, sk] additive and shared by the batch (differentiable: its gradient is summed over

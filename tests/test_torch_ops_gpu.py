@@ -324,3 +324,40 @@ def test_windowed_attention(ws, heads, dh, shift, grads):
         assert x.grad[:, :2 * heads * dh].abs().max().item() < 2e-2          # one key: no gradient but of the values
     assert _lib.read_error() is None
     assert A.window_attention(qkv, table, perm[:-1], inv, None, ws, dh) is None
+
+
+@pytest.mark.parametrize("dropout", [None, (0.1, 99, 0)])
+@pytest.mark.parametrize("grads", [None, torch.float32, torch.bfloat16])
+def test_cross_attention_block(grads, dropout):
+    """Against the same products on slices of the weight and attention over [b, s, h, dh] views. Only the weight's gradient differs, by a
+    rounding to bf16 of each slice's (2^-9), and dQ by the order of its fp32 sums."""
+    torch.manual_seed(8)
+    b, sq, sk, hq, hk, dh, hidden = 3, 19, 70, 4, 2, 40, 136
+    nq, nk = hq * dh, hk * dh
+    x, src, dout = _t(sq * b, hidden), _t(sk * b, hidden), _t(sq * b, nq)
+    w = _t(nq + 2 * nk, hidden, scale=0.2).requires_grad_()
+    lens = torch.tensor([70, 1, 33], device="cuda")
+
+    def by_views(x, src):
+        q = A.linear(x, w[:nq]).view(sq, b, hq, dh).transpose(0, 1)
+        kv = A.linear(src, w[nq:])
+        k, v = (t.reshape(sk, b, hk, dh).transpose(0, 1) for t in (kv[:, :nk], kv[:, nk:]))
+        return A.attention(q, k, v, False, None, lens, dropout)[0].transpose(0, 1).reshape(sq * b, nq)
+
+    start = _buffers([w], grads)
+    got = []
+    for fn in (lambda x, s: A.cross_attention_block(x, s, w, b, hq, hk, dh, lens, dropout), by_views):
+        xi, si = x.clone().requires_grad_(), src.clone().requires_grad_()
+        o = fn(xi, si)
+        o.backward(dout)
+        dw = w.grad
+        if grads is not None:
+            dw = (w.main_grad - start[w]).float() + (0 if dw is None else dw.float())
+            w.main_grad.copy_(start[w])
+        w.grad = None
+        got.append((o.detach(), si.grad, xi.grad, dw))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    size = lambda t: t.float().norm().item()
+    assert size(got[0][2] - got[1][2]) < 2e-3 * size(got[1][2])
+    assert size(got[0][3] - got[1][3]) < 2.0 ** -8 * (size(got[1][3]) + (size(start[w]) if grads is torch.bfloat16 else 0.0))
+    assert _lib.read_error() is None
