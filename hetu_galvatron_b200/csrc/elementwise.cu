@@ -380,6 +380,43 @@ xent_loss_grad_kernel(bf16* __restrict__ logits, const long long* __restrict__ l
   }
 }
 
+// Stored logits -> gradient, in place (see gv_kernels.h). One block walks a row: 2048 logits are read by all before any of their
+// gradients are written, and those go to where logits at half the distance stood, which have been read by then. A stream of 4 bytes in and 2
+// out a logit: 8192 x 32000 in 241 us (6.5 TB/s), where multiplying the logits again took 1430 with K = 4096.
+__global__ void __launch_bounds__(256)
+xent_logits_grad_kernel(float* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ lse,
+                        const float* __restrict__ gscale, int cols, long long vocab_start, long long ignore_index) {
+  const long long row = blockIdx.x;
+  float* in = logits + row * cols;
+  const long long lab = labels[row];
+  const bool counted = lab != ignore_index;
+  const float l = lse[row], g = counted ? gscale[row] : 0.f;
+  const long long target = counted ? lab - vocab_start : -1;
+  float4 a, b;
+  int j = threadIdx.x * 8;
+  if (j < cols) {
+    a = __ldcs(reinterpret_cast<const float4*>(in + j));
+    b = __ldcs(reinterpret_cast<const float4*>(in + j) + 1);
+  }
+  for (int c0 = 0; c0 < cols; c0 += 2048, j += 2048) {
+    float4 na, nb;
+    if (j + 2048 < cols) {                       // the next 2048 are on their way while these are worked on
+      na = __ldcs(reinterpret_cast<const float4*>(in + j + 2048));
+      nb = __ldcs(reinterpret_cast<const float4*>(in + j + 2048) + 1);
+    }
+    __syncthreads();
+    if (j < cols) {
+      const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      const int t = target >= j && target < j + 8 ? static_cast<int>(target - j) : -1;
+      float o[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) o[e] = (__expf(x[e] - l) - (t == e ? 1.f : 0.f)) * g;
+      reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(in) + j)[0] = pack8e(o);
+    }
+    a = na; b = nb;
+  }
+}
+
 // ------------------------------------------------------------------ log-sum-exp merge of attention partials
 // Ring / blockwise attention: `acc` (fp32 [b, s, h, dh], contiguous) and `lse_acc` (fp32 [b, h, s]) hold the
 // attention of the key blocks seen so far; a new partial (o_blk bf16 [b, sb, h, dh] with strides, lse_blk fp32
@@ -777,6 +814,14 @@ extern "C" int gv_cast_bf16_to_f32(const void* in, float* out, long long n, floa
   if (n <= 0) return 0;
   cast_bf16_f32_kernel<<<grid_for(n / 4 + 4, 256), 256, 0, (cudaStream_t)s>>>((const bf16*)in, out, n, scale,
                                                                               accumulate);
+  return (int)cudaGetLastError();
+}
+
+extern "C" int gv_xent_logits_grad(float* logits, const long long* labels, const float* lse, const float* gscale, long long rows, int cols,
+                                   long long vocab_start, long long ignore_index, gv_stream_t s) {
+  if (rows <= 0 || cols <= 0) return 0;
+  if (cols % 8 || (reinterpret_cast<uintptr_t>(logits) & 15) || rows > 0x7fffffff) return 2016;
+  xent_logits_grad_kernel<<<static_cast<unsigned>(rows), 256, 0, (cudaStream_t)s>>>(logits, labels, lse, gscale, cols, vocab_start, ignore_index);
   return (int)cudaGetLastError();
 }
 

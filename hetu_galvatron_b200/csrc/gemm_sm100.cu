@@ -43,7 +43,7 @@ struct GemmDev {
   int c_f32, accumulate, act;
   float alpha;
   // cross-entropy epilogues of the language-model head (xent_mode 0 = off)
-  int xent_mode;               // 1: per-tile (max, sum exp) + target logit, nothing stored to C; 2: C = (softmax - onehot) * gscale
+  int xent_mode;               // 1: per-tile (max, sum exp) + target logit, the logits to C in fp32 where C is given; 2: C = (softmax - onehot) * gscale
   const long long* labels;     // [M] global label ids
   long long vocab_start, ignore_index;
   float* stats;                // mode 1: [M, stat_tiles, 2]
@@ -397,6 +397,21 @@ __device__ __forceinline__ void xent_stats_chunk(const GemmDev& p, const uint32_
   }
 }
 
+// One chunk of logits, one row per lane, to C in fp32.
+__device__ __forceinline__ void epi_store_logits(const GemmDev& p, const uint32_t (&r)[32], float4* stage, int row0, int col0, int lane) {
+  epi_stage(r, stage, lane);
+  float4 v[8];
+  epi_fetch(stage, lane, v);
+  const int col = col0 + (lane & 7) * 4, r0 = row0 + (lane >> 3);
+  if (col >= p.N) return;                        // N is a multiple of four here
+  float* cp = reinterpret_cast<float*>(p.C) + static_cast<size_t>(r0) * p.ldc + col;
+#pragma unroll
+  for (int i = 0; i < 8; ++i, cp += 4 * static_cast<size_t>(p.ldc)) {
+    if (r0 + 4 * i >= p.M) continue;
+    *reinterpret_cast<float4*>(cp) = make_float4(v[i].x * p.alpha, v[i].y * p.alpha, v[i].z * p.alpha, v[i].w * p.alpha);
+  }
+}
+
 // One thread polls for the epilogue, the other warps sleep in a barrier. A wait that gave up is everybody's result, so all
 // warps leave together.
 __device__ __forceinline__ bool epilogue_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned int site) {
@@ -486,6 +501,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr,
         tmem_ld_wait();
         if (p.xent_mode == 1) {
           if (row_ok && col0 < p.N) xent_stats_chunk(p, r, row, col0, lcol, xm, xl);
+          if (p.C != nullptr) epi_store_logits(p, r, stage, row0, col0, lane);
         } else {
           // gradient of the cross entropy w.r.t. the logits, straight from the recomputed fp32 logits
           const int t = (lcol >= col0 && lcol < col0 + 32) ? static_cast<int>(lcol - col0) : -1;
@@ -499,13 +515,15 @@ __device__ __forceinline__ bool epilogue_tile(const GemmDev& p, uint32_t t_addr,
         epi_put64(w, stage, lane, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.M, p.N, row0, n0 + c * 32);
     }
     if (p.xent_mode == 1) {
-      // the quarter's second warp hands its half of the statistics to the first; two slots, one barrier per tile: a slot
-      // is written again only after the next tile's barrier, which the reader reaches after reading
-      float2* slot = reinterpret_cast<float2*>(stage - (half ? 4 * (EPI_STAGE_BYTES / 16) : 0)) + parity * 32 + lane;
-      if (half == 1) *slot = make_float2(xm, xl);
+      // the quarter's second warp hands its half of the statistics to the first by way of its own staging buffer, which it may
+      // use again when the first has read them
+      __syncwarp();
+      if (half == 1) reinterpret_cast<float2*>(stage)[lane] = make_float2(xm, xl);
+      named_bar_sync_id(2 + quarter, 64);
+      float2 o = make_float2(-INFINITY, 0.f);
+      if (half == 0) o = reinterpret_cast<const float2*>(stage + 4 * (EPI_STAGE_BYTES / 16))[lane];
       named_bar_sync_id(2 + quarter, 64);
       if (half == 0 && row_ok) {
-        const float2 o = *slot;
         const float m = fmaxf(xm, o.x);
         float* st = p.stats + (static_cast<size_t>(row) * p.stat_tiles + tn) * 2;
         st[0] = m;
@@ -1666,6 +1684,7 @@ extern "C" int gv_gemm_xent(const gv_gemm_args* a, const gv_xent_args* x, gv_str
   if (a->M <= 0 || a->N <= 0 || a->K <= 0) return 0;
   if (x == nullptr || (x->mode != 1 && x->mode != 2) || x->labels == nullptr) return 2011;
   if (x->mode == 1 && (x->stats == nullptr || x->target == nullptr)) return 2012;
+  if (x->mode == 1 && a->C != nullptr && (!a->c_f32 || a->N % 4 || a->ldc % 4 || a->accumulate)) return 2015;
   if (x->mode == 2 && (x->lse == nullptr || x->gscale == nullptr || a->C == nullptr || a->c_f32 || a->accumulate)) return 2013;
   if (a->a_mn_major || a->b_mn_major || a->bias || a->residual || a->act) return 2014;
   if ((a->K % 8) || (a->lda % 8) || (a->ldb % 8) || (x->mode == 2 && (a->ldc % 8))) return 2001;

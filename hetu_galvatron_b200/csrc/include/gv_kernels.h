@@ -67,11 +67,11 @@ int gv_gemm_bf16(const gv_gemm_args* args, gv_stream_t stream);
 // would not. Depends on sizes and options only, not on addresses.
 long long gv_gemm_workspace_bytes(const gv_gemm_args* args);
 
-// Language-model head GEMM (logits = A * B^T, both K-major) with the cross entropy in its epilogue; the logits
-// themselves are never stored.
+// Language-model head GEMM (logits = A * B^T, both K-major) with the cross entropy in its epilogue.
 //   mode 1: per row and per 256-column tile t of this vocabulary shard, stats[row, t, 0] = max and
 //           stats[row, t, 1] = sum exp(logit - max) (the caller merges tiles and ranks); target[row] = logit of the
-//           label when its column lies in this shard (written by exactly one tile; the caller zero-fills target).
+//           label when its column lies in this shard (written by exactly one tile; the caller zero-fills target). With C (fp32, c_f32 set,
+//           N and ldc multiples of 4) the logits are stored too, for gv_xent_logits_grad.
 //   mode 2: C[row, col] (bf16) = (exp(logit - lse[row]) - [col == label]) * gscale[row]: the gradient w.r.t. the
 //           logits from recomputed logits (lse = log-sum-exp over the whole vocabulary, gscale = upstream gradient).
 // labels are global ids; column c of this shard is id vocab_start + c; rows with label == ignore_index match nothing.
@@ -146,6 +146,12 @@ int gv_xent_loss_grad(void* logits, const long long* labels, const float* row_ma
                       const float* tgt_logit, float* loss, float grad_scale, const float* grad_scale_ptr,
                       long long rows, int vocab_local, long long ld, long long vocab_start, long long ignore_index,
                       gv_stream_t stream);
+
+// In place: a row of `cols` fp32 logits becomes, at its start, a row of bf16 (exp(logit - lse[row]) - [col == label]) * gscale[row], the same
+// bits as mode 2 of gv_gemm_xent gives for these logits; rows with label == ignore_index as there. cols a multiple of 8, logits
+// 16-byte aligned; the gradient's row stride is 2 * cols.
+int gv_xent_logits_grad(float* logits, const long long* labels, const float* lse, const float* gscale, long long rows, int cols,
+                        long long vocab_start, long long ignore_index, gv_stream_t stream);
 
 // Joins gv_gemm_xent's mode-1 statistics [rows, tiles, 2] into row_max / row_sum [rows]; target[row] becomes 0 where the label is
 // ignored or not in [vocab_start, vocab_start + vocab_rows). lse = log(sum) + max and loss = lse - target (0 for ignored rows)

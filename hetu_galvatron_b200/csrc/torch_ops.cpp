@@ -10,6 +10,8 @@
 // handed to the Python code.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAGraphsUtils.cuh>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_cpp_function.h>
@@ -41,7 +43,7 @@ namespace {
 #define GV_ENTRIES(X)                                                                                                              \
   X(gv_gemm_bf16) X(gv_gemm_xent) X(gv_gemm_workspace_bytes) X(gv_xent_merge) X(gv_rmsnorm_fwd) X(gv_rmsnorm_bwd) X(gv_layernorm_fwd) \
   X(gv_layernorm_bwd) X(gv_norm_bwd_scratch_elems) X(gv_rope) X(gv_swiglu_bwd) X(gv_gelu_bwd) X(gv_colsum_accum) X(gv_attn_fwd) X(gv_attn_bwd) \
-  X(gv_window_bias) X(gv_window_bias_bwd)
+  X(gv_window_bias) X(gv_window_bias_bwd) X(gv_xent_logits_grad)
 struct Entries {
 #define X(name) decltype(&::name) name = nullptr;
   GV_ENTRIES(X)
@@ -885,16 +887,70 @@ gv_gemm_args head_args(const Tensor& x, const Tensor& W, const Tensor& C) {
   return g;
 }
 
+// Logits kept in fp32 from the forward to the backward pass, where they become their own gradient in place. Otherwise the backward pass
+// multiplies them again, which gives the same bits: whether they are kept is a matter of room only. No more than KEPT_MAX bytes are alive at a
+// time on a device (many micro-batches may be), and only while there is plenty beside.
+constexpr long long KEPT_MAX = 2ll << 30, KEPT_BESIDE = 8ll << 30;
+constexpr int MAX_DEVICES = 64;
+std::atomic<long long> g_kept[MAX_DEVICES];
+
+// Where storing them costs more than it saves they are not kept: with a short K the epilogue, not the product, is what the first pass waits
+// for. us of both products -> of the product that stores and the pass in place: 8192 x 32000 x 4096 2865 -> 1658, 2048 x 151936 x 1536 1239 ->
+// 1069, 8192 x 50304 x 1600 1667 -> 1370, 8192 x 30592 x 1280 784 -> 769, 8192 x 32000 x 1024 680 -> 764. Up to one tile per SM that does
+// not matter.
+bool worth_keeping(int64_t rows, int64_t cols, int64_t k) { return k >= 1280 || rows * cols <= 148ll * 128 * 256; }
+
+Tensor logits_to_keep(int64_t rows, int64_t cols, const Tensor& like) {
+  if (!worth_keeping(rows, cols, like.size(1))) return Tensor();
+  const int device = static_cast<int>(like.device().index());
+  const long long bytes = rows * cols * 4;
+  if (device < 0 || device >= MAX_DEVICES || bytes > KEPT_MAX || at::cuda::currentStreamCaptureStatusMayInitCtx() != at::cuda::CaptureStatus::None) return Tensor();
+  std::atomic<long long>& kept = g_kept[device];
+  if (kept.fetch_add(bytes) + bytes > KEPT_MAX) {
+    kept.fetch_sub(bytes);
+    return Tensor();
+  }
+  auto give_back = [&kept, bytes] { kept.fetch_sub(bytes); };
+  if (bytes >= (64ll << 20)) {
+    size_t free_bytes = 0, total = 0;
+    const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats(static_cast<c10::DeviceIndex>(device));
+    const long long cached = stats.reserved_bytes[0].current - stats.allocated_bytes[0].current;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+      cudaGetLastError();
+      give_back();
+      return Tensor();
+    }
+    if (static_cast<long long>(free_bytes) + cached < bytes + KEPT_BESIDE) {
+      give_back();
+      return Tensor();
+    }
+  }
+  Tensor room;
+  try {
+    room = empty32({rows, cols}, like);
+  } catch (const c10::OutOfMemoryError&) {
+    give_back();
+    return Tensor();
+  }
+  void* at = room.mutable_data_ptr();
+  return at::from_blob(at, {rows, cols}, [room, give_back](void*) mutable {
+    room.reset();
+    give_back();
+  }, room.options());
+}
+
 struct LMHeadLossFn : Function<LMHeadLossFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& W, const Tensor& labels_, int64_t vocab_start, int64_t ignore_index) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& W, const Tensor& labels_, int64_t vocab_start, int64_t ignore_index, bool keep) {
     const Tensor x2 = flat2d(x), labels = labels_.reshape({-1}).to(at::kLong).contiguous();
     const int64_t M = x2.size(0), N = W.size(0), tiles = (N + 255) / 256;
     const Tensor stats = empty32({M, tiles, 2}, x2), rows = empty32({3, M}, x2), lse = empty32({M}, x2), loss = empty32({M}, x2);
+    const Tensor logits = keep ? logits_to_keep(M, N, x2) : Tensor();
     float* r = static_cast<float*>(ptr(rows));                  // max, sum, target
     gv_xent_args xa = {};
     xa.mode = 1; xa.labels = static_cast<const long long*>(cptr(labels)); xa.vocab_start = vocab_start; xa.ignore_index = ignore_index;
     xa.stats = static_cast<float*>(ptr(stats)); xa.target = r + 2 * M;
-    const gv_gemm_args g = head_args(x2, W, Tensor());
+    gv_gemm_args g = head_args(x2, W, logits);
+    g.c_f32 = logits.defined();
     launched(K.gv_gemm_xent(&g, &xa, stream()), "gv_gemm_xent(stats)");
     launched(K.gv_xent_merge(static_cast<const float*>(cptr(stats)), static_cast<int>(tiles), xa.labels, vocab_start, N, ignore_index, r, r + M, r + 2 * M,
                              static_cast<float*>(ptr(lse)), static_cast<float*>(ptr(loss)), M, stream()),
@@ -902,6 +958,7 @@ struct LMHeadLossFn : Function<LMHeadLossFn> {
     ctx->saved_data["sizes"] = x.sizes().vec();
     ctx->saved_data["start"] = vocab_start;
     ctx->saved_data["ignore"] = ignore_index;
+    if (logits.defined()) ctx->saved_data["logits"] = logits;
     ctx->save_for_backward({x2, W, labels, lse});
     return loss;
   }
@@ -909,16 +966,27 @@ struct LMHeadLossFn : Function<LMHeadLossFn> {
     const auto saved = ctx->get_saved_variables();
     const Tensor x2 = row_major(saved[0]), W = row_major(saved[1]), labels = saved[2].contiguous(), lse = saved[3].contiguous();
     const Tensor dloss = grads[0].reshape({-1}).to(at::kFloat).contiguous();
-    const Tensor dlog = empty16({x2.size(0), W.size(0)}, x2);
-    gv_xent_args xa = {};
-    xa.mode = 2; xa.labels = static_cast<const long long*>(cptr(labels));
-    xa.vocab_start = ctx->saved_data["start"].toInt(); xa.ignore_index = ctx->saved_data["ignore"].toInt();
-    xa.lse = static_cast<const float*>(cptr(lse)); xa.gscale = static_cast<const float*>(cptr(dloss));
-    const gv_gemm_args g = head_args(x2, W, dlog);
-    launched(K.gv_gemm_xent(&g, &xa, stream()), "gv_gemm_xent(grad)");
+    const int64_t start = ctx->saved_data["start"].toInt(), ignore = ctx->saved_data["ignore"].toInt(), M = x2.size(0), N = W.size(0);
+    const long long* lab = static_cast<const long long*>(cptr(labels));
+    const float *l = static_cast<const float*>(cptr(lse)), *gs = static_cast<const float*>(cptr(dloss));
+    Tensor dlog;
+    const auto kept = ctx->saved_data.find("logits");
+    if (kept != ctx->saved_data.end()) {
+      // used up: another backward pass over a retained graph multiplies them again
+      const Tensor logits = kept->second.toTensor();
+      ctx->saved_data.erase(kept);
+      launched(K.gv_xent_logits_grad(static_cast<float*>(ptr(logits)), lab, l, gs, M, static_cast<int>(N), start, ignore, stream()), "gv_xent_logits_grad");
+      dlog = logits.view(at::kBFloat16).narrow(1, 0, N);
+    } else {
+      dlog = empty16({M, N}, x2);
+      gv_xent_args xa = {};
+      xa.mode = 2; xa.labels = lab; xa.vocab_start = start; xa.ignore_index = ignore; xa.lse = l; xa.gscale = gs;
+      const gv_gemm_args g = head_args(x2, W, dlog);
+      launched(K.gv_gemm_xent(&g, &xa, stream()), "gv_gemm_xent(grad)");
+    }
     Tensor dx = input_grad(dlog, W).view(ctx->saved_data["sizes"].toIntVector());
     Tensor dW = weight_grad(saved[1], dlog, x2);
-    return {dx, dW, Tensor(), Tensor(), Tensor()};
+    return {dx, dW, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -926,7 +994,8 @@ py::object lm_head_loss(const Tensor& x, const Tensor& W, const Tensor& labels, 
   if (!plain_mode() || !input_ok(x) || !weight_ok(W) || x.size(-1) != W.size(1) || !plain(labels) || labels.numel() * x.size(-1) != x.numel()) return py::none();
   const Tensor x2 = flat2d(x.detach());
   if (!rows_ok(x2)) return py::none();
-  return py::cast(no_gil([&] { return LMHeadLossFn::apply(x, W, labels, vocab_start, ignore_index); }));
+  const bool keep = at::GradMode::is_enabled() && (x.requires_grad() || W.requires_grad());
+  return py::cast(no_gil([&] { return LMHeadLossFn::apply(x, W, labels, vocab_start, ignore_index, keep); }));
 }
 
 // Python sees the nodes under the names that the Python Functions' nodes have.
@@ -970,6 +1039,7 @@ PYBIND11_MODULE(torch_ops, m) {
   m.doc() = "C++ autograd Functions of the un-sharded hot path";
   m.def("init", &init);
   m.def("launch_count", [] { return g_launches.load(std::memory_order_relaxed); });
+  m.def("kept_logits", [](int device) { return g_kept[device].load(); });       // bytes of logits alive on a device
   m.def("no_scratch_for", [](int device, int M, int N, int K_) {
     std::lock_guard<std::mutex> lock(g_no_scratch_lock);
     g_no_scratch_products.insert(std::make_tuple(device, M, N, K_));

@@ -131,7 +131,8 @@ PROTOTYPES["gv_pad_heads"] = [POINTER(PadHeadsArgs), _I, _P]
 # what csrc/torch_ops.cpp calls
 TORCH_OPS_ENTRIES = ("gv_gemm_bf16", "gv_gemm_xent", "gv_gemm_workspace_bytes", "gv_xent_merge", "gv_rmsnorm_fwd", "gv_rmsnorm_bwd",
                      "gv_layernorm_fwd", "gv_layernorm_bwd", "gv_norm_bwd_scratch_elems", "gv_rope", "gv_swiglu_bwd", "gv_gelu_bwd",
-                     "gv_colsum_accum", "gv_attn_fwd", "gv_attn_bwd", "gv_window_bias", "gv_window_bias_bwd")
+                     "gv_colsum_accum", "gv_attn_fwd", "gv_attn_bwd", "gv_window_bias", "gv_window_bias_bwd",
+                     "gv_xent_logits_grad")
 
 
 def available() -> bool:

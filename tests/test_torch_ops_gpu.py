@@ -206,6 +206,45 @@ def test_language_model_head(grads):
     assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
+@pytest.mark.parametrize("tokens,hidden,vocab", [(1, 64, 8), (300, 72, 2048), (130, 64, 2056), (77, 128, 10000), (2500, 1280, 50304)])
+def test_kept_logits_give_the_bits_of_a_second_product(tokens, hidden, vocab):
+    """Gradients from logits that the forward pass left, in place, against those of the product done again: rows that end within and at
+    the end of a block's step, ignored rows, single and pair tiles. A second pass over a retained graph does the product again."""
+    torch.manual_seed(9)
+    x, w = _t(tokens, hidden).requires_grad_(), _t(vocab, hidden, scale=0.1).requires_grad_()
+    labels = torch.randint(0, vocab, (tokens,), device="cuda")
+    labels[2::5] = -100
+    g = torch.rand(tokens, device="cuda")
+    loss = A.lm_head_loss(x, w, labels)
+    assert _lib.torch_ops().kept_logits(0) == 4 * tokens * vocab
+    first = torch.autograd.grad(loss, (x, w), g, retain_graph=True)
+    assert _lib.torch_ops().kept_logits(0) == 0
+    again = torch.autograd.grad(loss, (x, w), g)
+    ref = A.LMHeadLossFn.apply(x, w, labels, A.LossCfg())
+    other = torch.autograd.grad(ref, (x, w), g)
+    assert torch.equal(loss, ref)
+    for a, b, c in zip(first, again, other):
+        assert torch.equal(a, c) and torch.equal(b, c)
+    with torch.no_grad():
+        A.lm_head_loss(x, w, labels)
+    assert _lib.torch_ops().kept_logits(0) == 0 and _lib.read_error() is None
+
+
+def test_kept_logits_are_bounded_and_given_back():
+    tokens, vocab = 4096, 40000
+    x, w = _t(tokens, 1280).requires_grad_(), _t(vocab, 1280, scale=0.1).requires_grad_()
+    labels = torch.randint(0, vocab, (tokens,), device="cuda")
+    losses = [A.lm_head_loss(x, w, labels) for _ in range(5)]
+    kept = _lib.torch_ops().kept_logits(0)
+    assert kept in (3 * 4 * tokens * vocab, 0)                    # of five, as many as fit into 2 GB, or none where the device is full
+    grads = [torch.autograd.grad(l.sum(), w)[0] for l in losses]
+    assert all(torch.equal(g, grads[0]) for g in grads)
+    assert _lib.torch_ops().kept_logits(0) == 0
+    loss = A.lm_head_loss(x, w, labels)
+    del loss, losses
+    assert _lib.torch_ops().kept_logits(0) == 0
+
+
 def test_saved_tensors_go_through_hooks():
     """Hooks that hand back other tensors (here: the same values in transposed storage) see every saved tensor and are believed."""
     torch.manual_seed(6)
