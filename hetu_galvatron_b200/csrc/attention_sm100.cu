@@ -206,6 +206,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int kv_head = head / (p.hq / p.hk);
   const int q0 = q_tile * FWD_BM;
   const int shift = p.sk - p.sq;  // causal: query i sees keys <= i + shift
+  if (p.kv_lens) wait_for_previous_kernel();      // else not before everything is set up
   const int sk_eff = p.kv_lens ? max(0, min(p.sk, p.kv_lens[batch])) : p.sk;   // keys that are not padding
   int kv_end = sk_eff;
   if (p.causal) kv_end = min(sk_eff, min(p.sq, q0 + FWD_BM) + shift);
@@ -238,6 +239,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   auto wait_pv = [&](int block, unsigned int site) {    // until P V of this block has been added to O
     const PvPhase ph = pv_phase(block);
     return mbar_wait(&pv_done[ph.barrier], ph.parity, abort_flag, site);
@@ -607,6 +610,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int kv0 = kv_tile * BWD_BKV;
   const int rep = p.hq / p.hk;
   const int shift = p.sk - p.sq;
+  if (p.kv_lens) wait_for_previous_kernel();      // else not before everything is set up
   const int sk_eff = p.kv_lens ? max(0, min(p.sk, p.kv_lens[batch])) : p.sk;   // keys that are not padding
   // first query block that can see this KV tile (causal): q + shift >= kv0
   int q_start = 0;
@@ -666,6 +670,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous_kernel();
+  let_next_kernel_start();
 
   // (each warpgroup sets its registers in its own branch: where branches join again the compiler counts on the fewest)
   if (warp < 4) {
@@ -1083,6 +1089,8 @@ template <int LPR>
 __global__ void attn_delta_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, float* __restrict__ delta,
                                   int b, int sq, int hq, int dh, long long o_sb, long long o_ss, long long o_sh,
                                   long long do_sb, long long do_ss, long long do_sh) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const long long total = static_cast<long long>(b) * hq * sq;
   const int sub = threadIdx.x % LPR;
   // whole warps stay in the loop together (the shuffles below are warp-wide): rows are padded up to a multiple of 32 / LPR
@@ -1117,6 +1125,8 @@ template <bool ROPE>
 __global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, int b, int sq, int hq, int dh,
                                        long long sb, long long ss, long long sh, const float* __restrict__ inv_freq,
                                        const int* __restrict__ pos, int pos_offset) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   constexpr int PARTS = ROPE ? 2 : 1;
   const int span = dh / PARTS, vec = span >> 3, groups = (sq + 3) >> 2;
   const long long total = static_cast<long long>(b) * hq * groups * vec;
@@ -1248,7 +1258,7 @@ static int launch_fwd(const gv_attn_args* a, cudaStream_t stream) {
   const long long blocks = static_cast<long long>(q_tiles) * a->hq * a->b;
   if (blocks > 0x7fffffff) return 2317;
   const dim3 grid = tile_grid(a->causal, q_tiles, a->hq, a->b, p.tile_group);
-  kern<<<grid, FWD_THREADS, smem, stream>>>(tmQ, tmK, tmV, p);
+  gv::launch_early(kern, grid, FWD_THREADS, smem, stream, 1, tmQ, tmK, tmV, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1297,7 +1307,7 @@ extern "C" int gv_attn_bwd(const gv_attn_args* a, gv_stream_t s) {
     const long long cap = static_cast<long long>(num_sms()) * 8;
     if (blocks > cap) blocks = cap;
     auto delta_kern = lpr == 4 ? attn_delta_kernel<4> : (lpr == 8 ? attn_delta_kernel<8> : attn_delta_kernel<16>);
-    delta_kern<<<static_cast<int>(blocks), 256, 0, stream>>>(
+    gv::launch_early(delta_kern, static_cast<int>(blocks), 256, 0, stream, 1,
         reinterpret_cast<const bf16*>(a->o), reinterpret_cast<const bf16*>(a->dout), a->delta, a->b, a->sq, a->hq,
         a->dh, a->o_stride_b, a->o_stride_s, a->o_stride_h, a->do_stride_b, a->do_stride_s, a->do_stride_h);
     cudaError_t e = cudaMemsetAsync(a->dq_accum, 0, sizeof(float) * static_cast<size_t>(a->b) * a->sq * a->hq * a->dh,
@@ -1342,7 +1352,7 @@ extern "C" int gv_attn_bwd(const gv_attn_args* a, gv_stream_t s) {
   auto launch = [&](auto kern, PerDeviceOnce& once) -> cudaError_t {
     cudaError_t e = ensure_max_dynamic_smem(once, kern, BwdSmem::TOTAL);
     if (e != cudaSuccess) return e;
-    kern<<<grid, BWD_THREADS, BwdSmem::TOTAL, stream>>>(tmQ, tmK, tmV, tmDO, p);
+    gv::launch_early(kern, grid, BWD_THREADS, BwdSmem::TOTAL, stream, 1, tmQ, tmK, tmV, tmDO, p);
     return cudaSuccess;
   };
   static PerDeviceOnce once_plain, once_bias, once_drop;
@@ -1360,7 +1370,7 @@ extern "C" int gv_attn_bwd(const gv_attn_args* a, gv_stream_t s) {
     const long long cap = static_cast<long long>(num_sms()) * 8;
     if (blocks > cap) blocks = cap;
     auto convert = rope ? attn_dq_convert_kernel<true> : attn_dq_convert_kernel<false>;
-    convert<<<static_cast<int>(blocks), 256, 0, stream>>>(a->dq_accum, reinterpret_cast<bf16*>(a->dq), a->b, a->sq, a->hq, a->dh,
+    gv::launch_early(convert, static_cast<int>(blocks), 256, 0, stream, 1, a->dq_accum, reinterpret_cast<bf16*>(a->dq), a->b, a->sq, a->hq, a->dh,
                                                           a->dq_stride_b, a->dq_stride_s, a->dq_stride_h, a->dq_rope_inv_freq,
                                                           a->dq_rope_pos, a->dq_rope_pos_offset);
   }

@@ -9,6 +9,7 @@
 //   cross entropy megatron/core/tensor_parallel/cross_entropy.py:16-152
 //   Adam          galvatron/core/runtime/utils.py:137-149 (apex FusedAdam)
 //   grad norm     megatron/core/optimizer/clip_grads.py:80-107 (amp_C multi_tensor_l2norm / scale)
+#include "include/gv_host.h"
 #include "include/gv_kernels.h"
 #include "include/gv_ptx.cuh"
 
@@ -59,6 +60,8 @@ template <int ROPE_RUN>
 __global__ void rope_kernel(bf16* __restrict__ x, const int* __restrict__ pos, const float* __restrict__ inv_freq,
                             long long tokens, int heads, int dh, long long ld, int pos_div, int pos_mod,
                             int pos_offset, int inverse) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const int half = dh >> 1;
   const int vec_per_head = half >> 3;
   const int runs = (heads + ROPE_RUN - 1) / ROPE_RUN, per_token = runs * vec_per_head;
@@ -103,6 +106,8 @@ __global__ void rope_kernel(bf16* __restrict__ x, const int* __restrict__ pos, c
 
 // ------------------------------------------------------------------ SwiGLU / GELU
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long long rows, int f) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const int vec = f >> 3;
   const long long total = rows * vec;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -121,6 +126,8 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
 
 __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu,
                                   long long rows, int f) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const int vec = f >> 3;
   const long long total = rows * vec;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -145,6 +152,8 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __r
 }
 
 __global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long long nvec) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < nvec;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float a[8], o[8];
@@ -156,6 +165,8 @@ __global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y
 }
 __global__ void gelu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, bf16* __restrict__ dx,
                                 long long nvec) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < nvec;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float a[8], d[8], o[8];
@@ -170,6 +181,8 @@ __global__ void gelu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restr
 // db[c] += sum_r dy[r, c]. CTA = 32 x 8 threads; each thread owns 8 columns of a 256-column
 // strip and walks rows with stride 8 * gridDim.y; partial sums meet in shared memory.
 __global__ void colsum_kernel(const bf16* __restrict__ dy, float* __restrict__ out, long long rows, int cols) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   __shared__ float sm[8][256];
   const int c0 = blockIdx.x * 256 + threadIdx.x * 8;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -197,6 +210,8 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const bf
                                      const int* __restrict__ pos_ids, const bf16* __restrict__ pos_table,
                                      bf16* __restrict__ out, long long tokens, int hidden, long long vocab_start,
                                      long long vocab_rows) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const int vec = hidden >> 3;
   for (long long t = blockIdx.x; t < tokens; t += gridDim.x) {
     const long long id = ids[t] - vocab_start;
@@ -386,6 +401,8 @@ xent_loss_grad_kernel(bf16* __restrict__ logits, const long long* __restrict__ l
 __global__ void __launch_bounds__(256)
 xent_logits_grad_kernel(float* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ lse,
                         const float* __restrict__ gscale, int cols, long long vocab_start, long long ignore_index) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const long long row = blockIdx.x;
   float* in = logits + row * cols;
   const long long lab = labels[row];
@@ -463,6 +480,8 @@ __device__ __forceinline__ float scaled_sum(float sum, float max, float new_max)
 __global__ void xent_merge_kernel(const float2* __restrict__ stats, int tiles, const long long* __restrict__ labels, long long vocab_start,
                                   long long vocab_rows, long long ignore_index, float* __restrict__ row_max, float* __restrict__ row_sum,
                                   float* __restrict__ target, float* __restrict__ lse, float* __restrict__ loss, long long rows) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const int lane = threadIdx.x & 31;
   const long long row = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   if (row >= rows) return;
@@ -495,6 +514,8 @@ __global__ void xent_merge_kernel(const float2* __restrict__ stats, int tiles, c
 // strided copy per tensor took 39 us, three tensors now share a launch.
 template <bool PAD>
 __global__ void pad_heads_kernel(const gv_pad_heads_args a) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const int t = blockIdx.y;
   const int units = a.wide >> 3, total = a.h[t] * units, narrow = a.narrow;
   const long long rows = static_cast<long long>(a.b) * a.s[t];
@@ -528,6 +549,8 @@ __global__ void adamw_kernel(float* __restrict__ master, float* __restrict__ m, 
                              const void* __restrict__ grad, bf16* __restrict__ param, long long n, float lr, float b1,
                              float b2, float eps, float wd, float bc1, float bc2, float grad_scale,
                              const float* __restrict__ clip_coef) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const float gs = grad_scale * (clip_coef ? *clip_coef : 1.f);
   const long long nvec = n >> 2;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < nvec;
@@ -583,6 +606,8 @@ __global__ void adamw_kernel(float* __restrict__ master, float* __restrict__ m, 
 
 template <bool IS_BF16>
 __global__ void sumsq_kernel(const void* __restrict__ x, long long n, float* __restrict__ out) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   __shared__ float sm[32];
   float acc = 0.f;
   if (IS_BF16) {
@@ -668,7 +693,7 @@ extern "C" int gv_rope(void* x, const int* pos, const float* inv_freq, long long
   if (dh % 16 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15)) return 2201;
   auto go = [&](auto kern, int run) {
     const long long total = tokens * ((heads + run - 1) / run) * (dh / 16);
-    kern<<<grid_for(total, 256), 256, 0, (cudaStream_t)s>>>((bf16*)x, pos, inv_freq, tokens, heads, dh, ld, pos_div > 0 ? pos_div : 1,
+    gv::launch_early(kern, grid_for(total, 256), 256, 0, (cudaStream_t)s, 1, (bf16*)x, pos, inv_freq, tokens, heads, dh, ld, pos_div > 0 ? pos_div : 1,
                                                             pos_mod > 0 ? pos_mod : 0x7fffffff, pos_offset, inverse);
   };
   if (heads == 1 || tokens * heads * (dh / 16) <= 256ll * num_sms()) go(rope_kernel<1>, 1);
@@ -679,26 +704,26 @@ extern "C" int gv_rope(void* x, const int* pos, const float* inv_freq, long long
 extern "C" int gv_swiglu_fwd(const void* gu, void* out, long long rows, int f, gv_stream_t s) {
   if (rows <= 0) return 0;
   if (f % 8) return 2202;
-  swiglu_fwd_kernel<<<grid_for(rows * (f / 8), 256, ONCE_THROUGH), 256, 0, (cudaStream_t)s>>>((const bf16*)gu, (bf16*)out, rows, f);
+  gv::launch_early(swiglu_fwd_kernel, grid_for(rows * (f / 8), 256, ONCE_THROUGH), 256, 0, (cudaStream_t)s, 1, (const bf16*)gu, (bf16*)out, rows, f);
   return (int)cudaGetLastError();
 }
 extern "C" int gv_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long rows, int f, gv_stream_t s) {
   if (rows <= 0) return 0;
   if (f % 8) return 2202;
-  swiglu_bwd_kernel<<<grid_for(rows * (f / 8), 256, ONCE_THROUGH), 256, 0, (cudaStream_t)s>>>((const bf16*)dout, (const bf16*)gu,
+  gv::launch_early(swiglu_bwd_kernel, grid_for(rows * (f / 8), 256, ONCE_THROUGH), 256, 0, (cudaStream_t)s, 1, (const bf16*)dout, (const bf16*)gu,
                                                                                 (bf16*)dgu, rows, f);
   return (int)cudaGetLastError();
 }
 extern "C" int gv_gelu_fwd(const void* x, void* y, long long n, gv_stream_t s) {
   if (n <= 0) return 0;
   if (n % 8) return 2203;
-  gelu_fwd_kernel<<<grid_for(n / 8, 256, 32), 256, 0, (cudaStream_t)s>>>((const bf16*)x, (bf16*)y, n / 8);
+  gv::launch_early(gelu_fwd_kernel, grid_for(n / 8, 256, 32), 256, 0, (cudaStream_t)s, 1, (const bf16*)x, (bf16*)y, n / 8);
   return (int)cudaGetLastError();
 }
 extern "C" int gv_gelu_bwd(const void* dy, const void* x, void* dx, long long n, gv_stream_t s) {
   if (n <= 0) return 0;
   if (n % 8) return 2203;
-  gelu_bwd_kernel<<<grid_for(n / 8, 256, 32), 256, 0, (cudaStream_t)s>>>((const bf16*)dy, (const bf16*)x, (bf16*)dx, n / 8);
+  gv::launch_early(gelu_bwd_kernel, grid_for(n / 8, 256, 32), 256, 0, (cudaStream_t)s, 1, (const bf16*)dy, (const bf16*)x, (bf16*)dx, n / 8);
   return (int)cudaGetLastError();
 }
 extern "C" int gv_colsum_accum(const void* dy, float* out, long long rows, int cols, gv_stream_t s) {
@@ -710,7 +735,7 @@ extern "C" int gv_colsum_accum(const void* dy, float* out, long long rows, int c
   const long long cap = (static_cast<long long>(num_sms()) * 4 + gx - 1) / gx;
   if (gy > cap) gy = cap;
   if (gy < 1) gy = 1;
-  colsum_kernel<<<dim3(gx, (unsigned)gy), block, 0, (cudaStream_t)s>>>((const bf16*)dy, out, rows, cols);
+  gv::launch_early(colsum_kernel, dim3(gx, (unsigned)gy), block, 0, (cudaStream_t)s, 1, (const bf16*)dy, out, rows, cols);
   return (int)cudaGetLastError();
 }
 
@@ -720,7 +745,7 @@ extern "C" int gv_embedding_fwd(const long long* ids, const void* table, const i
   if (tokens <= 0) return 0;
   if (hidden % 8) return 2205;
   int grid = (int)(tokens < (long long)num_sms() * 16 ? tokens : (long long)num_sms() * 16);
-  embedding_fwd_kernel<<<grid, 128, 0, (cudaStream_t)s>>>(ids, (const bf16*)table, pos_ids, (const bf16*)pos_table,
+  gv::launch_early(embedding_fwd_kernel, grid, 128, 0, (cudaStream_t)s, 1, ids, (const bf16*)table, pos_ids, (const bf16*)pos_table,
                                                           (bf16*)out, tokens, hidden, vocab_start, vocab_rows);
   return (int)cudaGetLastError();
 }
@@ -779,11 +804,11 @@ extern "C" int gv_adamw(float* master, float* m, float* v, const void* grad, int
   if (n <= 0) return 0;
   const int grid = grid_for((n + 3) / 4 + 4, 256, ONCE_THROUGH);
   if (grad_is_bf16)
-    adamw_kernel<true><<<grid, 256, 0, (cudaStream_t)s>>>(master, m, v, grad, (bf16*)param_bf16, n, lr, beta1, beta2,
+    gv::launch_early(adamw_kernel<true>, grid, 256, 0, (cudaStream_t)s, 1, master, m, v, grad, (bf16*)param_bf16, n, lr, beta1, beta2,
                                                           eps, weight_decay, bias_corr1, bias_corr2, grad_scale,
                                                           clip_coef);
   else
-    adamw_kernel<false><<<grid, 256, 0, (cudaStream_t)s>>>(master, m, v, grad, (bf16*)param_bf16, n, lr, beta1, beta2,
+    gv::launch_early(adamw_kernel<false>, grid, 256, 0, (cudaStream_t)s, 1, master, m, v, grad, (bf16*)param_bf16, n, lr, beta1, beta2,
                                                            eps, weight_decay, bias_corr1, bias_corr2, grad_scale,
                                                            clip_coef);
   return (int)cudaGetLastError();
@@ -793,9 +818,9 @@ extern "C" int gv_sumsq_accum(const void* x, int is_bf16, long long n, float* ou
   if (n <= 0) return 0;
   const int grid = grid_for(n / 8 + 1, 256, 4);
   if (is_bf16)
-    sumsq_kernel<true><<<grid, 256, 0, (cudaStream_t)s>>>(x, n, out);
+    gv::launch_early(sumsq_kernel<true>, grid, 256, 0, (cudaStream_t)s, 1, x, n, out);
   else
-    sumsq_kernel<false><<<grid, 256, 0, (cudaStream_t)s>>>(x, n, out);
+    gv::launch_early(sumsq_kernel<false>, grid, 256, 0, (cudaStream_t)s, 1, x, n, out);
   return (int)cudaGetLastError();
 }
 
@@ -821,7 +846,7 @@ extern "C" int gv_xent_logits_grad(float* logits, const long long* labels, const
                                    long long vocab_start, long long ignore_index, gv_stream_t s) {
   if (rows <= 0 || cols <= 0) return 0;
   if (cols % 8 || (reinterpret_cast<uintptr_t>(logits) & 15) || rows > 0x7fffffff) return 2016;
-  xent_logits_grad_kernel<<<static_cast<unsigned>(rows), 256, 0, (cudaStream_t)s>>>(logits, labels, lse, gscale, cols, vocab_start, ignore_index);
+  gv::launch_early(xent_logits_grad_kernel, static_cast<unsigned>(rows), 256, 0, (cudaStream_t)s, 1, logits, labels, lse, gscale, cols, vocab_start, ignore_index);
   return (int)cudaGetLastError();
 }
 
@@ -830,7 +855,7 @@ extern "C" int gv_xent_merge(const float* stats, int tiles, const long long* lab
                              long long rows, gv_stream_t st) {
   if (rows <= 0) return 0;
   if (tiles <= 0 || (reinterpret_cast<uintptr_t>(stats) & 7)) return 2207;
-  xent_merge_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, (cudaStream_t)st>>>(reinterpret_cast<const float2*>(stats), tiles, labels, vocab_start,
+  gv::launch_early(xent_merge_kernel, (unsigned)((rows + 7) / 8), 256, 0, (cudaStream_t)st, 1, reinterpret_cast<const float2*>(stats), tiles, labels, vocab_start,
                                                                              vocab_rows, ignore_index, row_max, row_sum, target, lse, loss, rows);
   return (int)cudaGetLastError();
 }
@@ -853,8 +878,8 @@ extern "C" int gv_pad_heads(const gv_pad_heads_args* a, int pad, gv_stream_t st)
   const int threads = units >= 256 ? 256 : (units + 31) / 32 * 32;
   const long long cap = static_cast<long long>(num_sms()) * 16;
   const dim3 grid(static_cast<unsigned>(rows < cap ? rows : cap), static_cast<unsigned>(a->count));
-  if (pad) pad_heads_kernel<true><<<grid, threads, 0, (cudaStream_t)st>>>(*a);
-  else pad_heads_kernel<false><<<grid, threads, 0, (cudaStream_t)st>>>(*a);
+  if (pad) gv::launch_early(pad_heads_kernel<true>, grid, threads, 0, (cudaStream_t)st, 1, *a);
+  else gv::launch_early(pad_heads_kernel<false>, grid, threads, 0, (cudaStream_t)st, 1, *a);
   return (int)cudaGetLastError();
 }
 

@@ -691,6 +691,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous_kernel();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -728,6 +729,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
+      let_next_kernel_start();
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
@@ -1072,6 +1074,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
   cluster_sync_all();                   // the peer's barriers exist before anything arrives on them remotely
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous_kernel();
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
@@ -1109,6 +1112,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
           if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
         }
       }
+      let_next_kernel_start();
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (CTA 0 only) --------------------------------
@@ -1340,7 +1344,7 @@ static int launch_gemm(const gv_gemm_args* a, cudaStream_t stream, const gv_xent
   }
   const int tiles = ((a->M + BM - 1) / BM) * (a->swiglu_out ? a->N / 256 : (a->N + BN - 1) / BN);
   const int grid = tiles < num_sms() ? tiles : num_sms();
-  kern<<<grid, GEMM_THREADS, smem, stream>>>(tmA, tmB, p);
+  launch_early(kern, grid, GEMM_THREADS, smem, stream, 1, tmA, tmB, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1422,7 +1426,7 @@ static int launch_gemm_pair(const gv_gemm_args* a, cudaStream_t stream, const gv
   static int max_pairs = 0;
   if (max_pairs == 0) max_pairs = resident_clusters(kern, 2);
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  kern<<<2 * pairs, GEMM_THREADS, P_SMEM_TOTAL, stream>>>(tmA, tmB, p);
+  launch_early(kern, 2 * pairs, GEMM_THREADS, P_SMEM_TOTAL, stream, 1, tmA, tmB, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1439,7 +1443,7 @@ static int launch_gemm_share(const gv_gemm_args* a, cudaStream_t stream, const T
     cudaError_t e = ensure_max_dynamic_smem(smem_once, kern, P_SMEM_TOTAL);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  kern<<<2 * gemm_pairs(), GEMM_THREADS, P_SMEM_TOTAL, stream>>>(tmA, tmB, p);
+  launch_early(kern, 2 * gemm_pairs(), GEMM_THREADS, P_SMEM_TOTAL, stream, 1, tmA, tmB, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1475,17 +1479,7 @@ static int launch_gemm_split(const gv_gemm_args* a, cudaStream_t stream, int S) 
   }
   const int tiles = ((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + 255) / 256);
   const int clusters = tiles < split_clusters(S) ? tiles : split_clusters(S);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(2 * S * clusters));
-  cfg.blockDim = dim3(GEMM_THREADS);
-  cfg.dynamicSmemBytes = P_SMEM_TOTAL;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = static_cast<unsigned>(2 * S); attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, S, reinterpret_cast<float4*>(a->workspace)));
+  return static_cast<int>(launch_early(kern, 2 * S * clusters, GEMM_THREADS, P_SMEM_TOTAL, stream, 2 * S, tmA, tmB, p, S, reinterpret_cast<float4*>(a->workspace)));
 }
 
 // GV_GEMM_PAIR: 0 never, 1 (default) when there is a 256 x 256 tile for every SM pair, 2 always (used by the

@@ -48,6 +48,8 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                 __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out, float* __restrict__ mean_out,
                 float* __restrict__ rstd_out, int rows, int cols, float eps) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   constexpr int TEAMS = FWD_THREADS / 32 / WARPS;
   __shared__ float scratch[2][FWD_THREADS / 32];
   const int nvec = cols >> 3;
@@ -182,6 +184,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                 const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean_in,
                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                 __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows, int cols) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   extern __shared__ __align__(128) uint8_t ring[];      // [BWD_STAGES][x row | dy row | dres row]
   __shared__ float2 scratch[2][NORM_THREADS / 32];
   __shared__ uint64_t full[BWD_STAGES];
@@ -306,6 +310,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
 __global__ void __launch_bounds__(1024)
 norm_partial_reduce_kernel(const float* __restrict__ partial, int parts, int cols, float* __restrict__ dw_accum,
                            float* __restrict__ db_accum) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   __shared__ float sm[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   const float* src = blockIdx.y == 0 ? partial : partial + static_cast<size_t>(parts) * cols;
@@ -352,7 +358,7 @@ template <bool LAYER, bool KEEP32>
 static int launch_norm_fwd_rows(const void* x, const void* res, const void* w, const void* b, void* y, void* h_out, float* mean,
                            float* rstd, int rows, int cols, float eps, cudaStream_t s) {
   auto go = [&](auto kern, int teams) {
-    kern<<<(rows + teams - 1) / teams, FWD_THREADS, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)w, (const bf16*)b,
+    gv::launch_early(kern, (rows + teams - 1) / teams, FWD_THREADS, 0, s, 1, (const bf16*)x, (const bf16*)res, (const bf16*)w, (const bf16*)b,
                                                             (bf16*)y, (bf16*)h_out, mean, rstd, rows, cols, eps);
     return (int)cudaGetLastError();
   };
@@ -403,7 +409,7 @@ static int launch_norm_bwd_v(const BwdShape& b, const void* dy, const void* x, c
   constexpr int most = BWD_STAGES * 3 * 2 * 8 * NORM_THREADS * V;      // widest row of this V
   cudaError_t e = ensure_max_dynamic_smem(once, kern, most);
   if (e != cudaSuccess) return static_cast<int>(e);
-  kern<<<b.grid, b.threads, BWD_STAGES * (dres ? 3 : 2) * cols * 2, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd,
+  gv::launch_early(kern, b.grid, b.threads, BWD_STAGES * (dres ? 3 : 2) * cols * 2, s, 1, (const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd,
                                                                          (const bf16*)dres, (bf16*)dx, partial, rows, cols);
   return static_cast<int>(cudaGetLastError());
 }
@@ -420,7 +426,7 @@ static int launch_norm_bwd(const void* dy, const void* x, const void* w, const f
     default: rc = launch_norm_bwd_v<LAYER, 4>(b, dy, x, w, mean, rstd, dres, dx, scratch, rows, cols, s); break;
   }
   if (rc) return rc;
-  norm_partial_reduce_kernel<<<dim3((cols + 31) / 32, db_accum ? 2 : 1), dim3(32, 32), 0, s>>>(scratch, b.grid, cols, dw_accum, db_accum);
+  gv::launch_early(norm_partial_reduce_kernel, dim3((cols + 31) / 32, db_accum ? 2 : 1), dim3(32, 32), 0, s, 1, scratch, b.grid, cols, dw_accum, db_accum);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -5,6 +5,7 @@
 // Bound by launches and latency, not by bytes (a few MB): as index, permutation, two padded copies and their gradients, among them a
 // sort of all ws^4 indices for the table's gradient, these were 17 launches and 120 us of kernels a layer at ws = 12; now two launches,
 // 5 us together at 6 heads and 12 at 48.
+#include "include/gv_host.h"
 #include "include/gv_kernels.h"
 #include "include/gv_ptx.cuh"
 
@@ -14,6 +15,8 @@ typedef __nv_bfloat16 bf16;
 
 // Eight columns of a row of both matrices per thread. The table (a few 10 KB) stays in L1, so the scattered reads cost little.
 __global__ void window_bias_kernel(const bf16* __restrict__ table, int heads, int ws, int ld, bf16* __restrict__ bias, bf16* __restrict__ bias_t) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const int S = ws * ws, vecs = ld >> 3, span = 2 * ws - 1;
   const long long total = static_cast<long long>(heads) * S * vecs;
   for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total; t += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -36,6 +39,8 @@ __global__ void window_bias_kernel(const bf16* __restrict__ table, int heads, in
 
 // One warp per table entry and head sums the pairs of tokens with that offset, always in the same order.
 __global__ void window_bias_bwd_kernel(const float* __restrict__ dbias, int heads, int ws, int ld, float* __restrict__ dtable) {
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   const int S = ws * ws, span = 2 * ws - 1, lane = threadIdx.x & 31;
   const long long total = static_cast<long long>(span) * span * heads;
   for (long long t = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5; t < total; t += static_cast<long long>(gridDim.x) * (blockDim.x >> 5)) {
@@ -63,7 +68,7 @@ static bool window_args_ok(int heads, int ws, int ld) { return heads > 0 && ws >
 
 extern "C" int gv_window_bias(const void* table, int heads, int ws, int ld, void* bias, void* bias_t, gv_stream_t s) {
   if (!window_args_ok(heads, ws, ld) || ((reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(bias_t)) & 15)) return 2501;
-  gv::window_bias_kernel<<<gv::blocks_for(static_cast<long long>(heads) * ws * ws * (ld / 8)), 256, 0, reinterpret_cast<cudaStream_t>(s)>>>(
+  gv::launch_early(gv::window_bias_kernel, gv::blocks_for(static_cast<long long>(heads) * ws * ws * (ld / 8)), 256, 0, reinterpret_cast<cudaStream_t>(s), 1,
       reinterpret_cast<const gv::bf16*>(table), heads, ws, ld, reinterpret_cast<gv::bf16*>(bias), reinterpret_cast<gv::bf16*>(bias_t));
   return static_cast<int>(cudaGetLastError());
 }
@@ -71,6 +76,6 @@ extern "C" int gv_window_bias(const void* table, int heads, int ws, int ld, void
 extern "C" int gv_window_bias_bwd(const float* dbias, int heads, int ws, int ld, float* dtable, gv_stream_t s) {
   if (!window_args_ok(heads, ws, ld)) return 2501;
   const long long span = 2 * ws - 1;
-  gv::window_bias_bwd_kernel<<<gv::blocks_for(span * span * heads * 32), 256, 0, reinterpret_cast<cudaStream_t>(s)>>>(dbias, heads, ws, ld, dtable);
+  gv::launch_early(gv::window_bias_bwd_kernel, gv::blocks_for(span * span * heads * 32), 256, 0, reinterpret_cast<cudaStream_t>(s), 1, dbias, heads, ws, ld, dtable);
   return static_cast<int>(cudaGetLastError());
 }

@@ -400,3 +400,61 @@ def test_cross_attention_block(grads, dropout):
     assert size(got[0][2] - got[1][2]) < 2e-3 * size(got[1][2])
     assert size(got[0][3] - got[1][3]) < 2.0 ** -8 * (size(got[1][3]) + (size(start[w]) if grads is torch.bfloat16 else 0.0))
     assert _lib.read_error() is None
+
+
+def _chain(x, p, sync):
+    """Kernels of all kinds one after the other, each reading what the one before wrote; ``sync``: with the device waited for in between."""
+    out = []
+
+    def step(t):
+        if sync:
+            torch.cuda.synchronize()
+        out.append(t)
+        return t
+
+    y, h = A.rmsnorm_branch(x, p["n"], 1e-5)
+    qkv = step(A.linear(step(y), p["qkv"]))
+    o = step(A.packed_attention(qkv, A.AttnCfg(batch=2, hq=4, hk=2, dh=64)))
+    h = step(A.linear(o, p["o"], None, h))
+    y = step(A.layernorm(h, p["n"], p["b"], 1e-5))
+    h = step(A.swiglu_mlp(y, p["up"], p["down"], h))
+    h = step(A.linear(step(A.linear_gelu(h, p["g"], p["gb"])), p["g2"], p["b"]))
+    loss = step(A.lm_head_loss(h, p["head"], p["labels"]))
+    grads = torch.autograd.grad(loss, (x, p["n"], p["b"], p["up"], p["gb"], p["head"]), torch.full_like(loss, 1e-3))
+    return out, grads
+
+
+@pytest.mark.parametrize("rows,hidden", [(96, 256), (2048, 512)])
+def test_kernels_started_early_wait_for_what_they_read(rows, hidden):
+    """A chain issued at once gives the bits of the same chain with the device waited for after every kernel, over and over, on new inputs
+    in reused memory; the gradients, of which dQ is summed in the order that blocks finish in, within a rounding to bf16. Replayed from a
+    graph too."""
+    torch.manual_seed(11)
+    shapes = {"qkv": (512, hidden), "o": (hidden, 256), "up": (1024, hidden), "down": (hidden, 512), "g": (1024, hidden), "g2": (hidden, 1024), "head": (4096, hidden)}
+    p = {k: _t(*v, scale=0.05).requires_grad_() for k, v in shapes.items()}
+    p.update(n=(1 + _t(hidden, scale=0.1)).requires_grad_(), b=_t(hidden, scale=0.1).requires_grad_(), gb=_t(1024, scale=0.1).requires_grad_(),
+             labels=torch.randint(0, 4096, (rows,), device="cuda"))
+    for i in range(8):
+        x = _t(rows, hidden).requires_grad_()
+        want, wg = _chain(x, p, True)
+        for _ in range(4):
+            got, gg = _chain(x, p, False)
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+            for a, b in zip(gg, wg):
+                assert (a - b).float().norm() <= 4e-3 * b.float().norm()
+    static = _t(rows, hidden)
+    with torch.no_grad():
+        run = lambda: A.linear(A.swiglu_mlp(A.rmsnorm(static, p["n"]), p["up"], p["down"], static), p["qkv"])
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            run()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            y = run()
+        for _ in range(4):
+            static.copy_(_t(rows, hidden))
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, run())
+    assert _lib.read_error() is None
