@@ -889,10 +889,12 @@ gv_gemm_args head_args(const Tensor& x, const Tensor& W, const Tensor& C) {
 
 // Logits kept in fp32 from the forward to the backward pass, where they become their own gradient in place. Otherwise the backward pass
 // multiplies them again, which gives the same bits: whether they are kept is a matter of room only. No more than KEPT_MAX bytes are alive at a
-// time on a device (many micro-batches may be), and only while there is plenty beside.
-constexpr long long KEPT_MAX = 2ll << 30, KEPT_BESIDE = 8ll << 30;
+// time on a device (many micro-batches may be), and only while an eighth of its memory stays free of this process's tensors: by the
+// allocator's own count, since asking the driver took 0.2 ms, and 12 to 80 where other processes held its lock. Sizes that once did not
+// fit are not tried again: each failed allocation first empties the allocator's cache.
+constexpr long long KEPT_MAX = 2ll << 30;
 constexpr int MAX_DEVICES = 64;
-std::atomic<long long> g_kept[MAX_DEVICES];
+std::atomic<long long> g_kept[MAX_DEVICES], g_did_not_fit[MAX_DEVICES];      // bytes alive; the smallest that failed, 0: none
 
 // Where storing them costs more than it saves they are not kept: with a short K the epilogue, not the product, is what the first pass waits
 // for. us of both products -> of the product that stores and the pass in place: 8192 x 32000 x 4096 2865 -> 1658, 2048 x 151936 x 1536 1239 ->
@@ -911,24 +913,18 @@ Tensor logits_to_keep(int64_t rows, int64_t cols, const Tensor& like) {
     return Tensor();
   }
   auto give_back = [&kept, bytes] { kept.fetch_sub(bytes); };
-  if (bytes >= (64ll << 20)) {
-    size_t free_bytes = 0, total = 0;
-    const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats(static_cast<c10::DeviceIndex>(device));
-    const long long cached = stats.reserved_bytes[0].current - stats.allocated_bytes[0].current;
-    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
-      cudaGetLastError();
-      give_back();
-      return Tensor();
-    }
-    if (static_cast<long long>(free_bytes) + cached < bytes + KEPT_BESIDE) {
-      give_back();
-      return Tensor();
-    }
+  const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats(static_cast<c10::DeviceIndex>(device));
+  const long long total = static_cast<long long>(at::cuda::getDeviceProperties(static_cast<c10::DeviceIndex>(device))->totalGlobalMem);
+  const long long failed = g_did_not_fit[device].load();
+  if (stats.allocated_bytes[0].current + bytes > total / 8 * 7 || (failed != 0 && bytes >= failed)) {
+    give_back();
+    return Tensor();
   }
   Tensor room;
   try {
     room = empty32({rows, cols}, like);
   } catch (const c10::OutOfMemoryError&) {
+    g_did_not_fit[device].store(bytes);
     give_back();
     return Tensor();
   }
